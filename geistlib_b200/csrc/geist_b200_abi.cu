@@ -222,8 +222,8 @@ struct geist_b200_ctx {
         unsigned long long rng_in;
         unsigned long long rng_out;
     };
-    Small *d_small = nullptr;
-    Small *h_small = nullptr; /* pinned */
+    Small *d_small = nullptr; /* what a greedy row's launch reads: temperature 0, never written again but for its generator word */
+    Small *h_small = nullptr; /* pinned: settings in, token and status out, read and written by the kernels where it lies */
     std::mutex small_mu;      /* one synchronous host-pointer call at a time stages through the two words above */
 
     /* kernel scratch: part records, candidate groups, segment sums, row counters, multi-pass row copies. kLanes
@@ -267,6 +267,12 @@ extern "C" enum geist_status geist_b200_ctx_create(int device, struct geist_b200
     }
     if (e == cudaSuccess) {
         e = cudaHostAlloc(&c->h_small, sizeof(geist_b200_ctx::Small), cudaHostAllocDefault);
+    }
+    if (e == cudaSuccess) {
+        memset(c->h_small, 0, sizeof *c->h_small);
+        c->h_small->top_p  = 1.0f;
+        c->h_small->rng_in = 1;
+        e                  = cudaMemcpy(c->d_small, c->h_small, sizeof *c->h_small, cudaMemcpyHostToDevice);
     }
     if (e != cudaSuccess) {
         geist_b200_ctx_destroy(c);
@@ -655,53 +661,57 @@ geist_token_t sample_host_row(size_t n, const float *logits, float *staging, flo
         }
     }
     if (e == cudaSuccess) {
-        const float *src = logits;
-        if (staging != nullptr) {
-            memcpy(staging, logits, n * sizeof(float));
-            src = staging;
+        if (staging == nullptr) {
+            e = cudaMemcpyAsync(c->d_row, logits, n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+        } else {
+            /* through the pinned buffer in pieces: one is on the link while the next is copied */
+            const size_t piece = 32768;
+            for (size_t at = 0; at < n && e == cudaSuccess; at += piece) {
+                const size_t m = std::min(piece, n - at);
+                memcpy(staging + at, logits + at, m * sizeof(float));
+                e = cudaMemcpyAsync(c->d_row + at, staging + at, m * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+            }
         }
-        e = cudaMemcpyAsync(c->d_row, src, n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
     }
     if (e != cudaSuccess) {
         fail(GEIST_E_BACKEND, "sampler: staging the row: %s", cudaGetErrorString(e));
         return -1;
     }
-    geist_b200_ctx::Small *h = c->h_small;
+    geist_b200_ctx::Small *h = c->h_small; /* the kernels read it and write to it over the host link: a few words, no copies */
     h->T                     = T;
     h->top_k                 = top_k;
     h->top_p                 = top_p;
-    h->token                 = -1;
-    h->status                = 0;
     h->rng_in                = rng ? rng->state : 1ull;
     h->rng_out               = h->rng_in;
-    e                        = cudaMemcpyAsync(c->d_small, h, sizeof *h, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) {
-        fail(GEIST_E_BACKEND, "sampler: %s", cudaGetErrorString(e));
-        return -1;
-    }
     geist_b200_batch b{};
     b.logits       = c->d_row;
     b.row_stride   = n;
     b.n_seq        = 1;
     b.rows_per_seq = 1;
     b.n_vocab      = n;
-    b.temperature  = &c->d_small->T;
-    b.top_k        = &c->d_small->top_k;
-    b.top_p        = &c->d_small->top_p;
-    b.rng_in       = reinterpret_cast<const uint64_t *>(&c->d_small->rng_in);
-    b.rng_out      = reinterpret_cast<uint64_t *>(&c->d_small->rng_out);
-    b.tokens       = &c->d_small->token;
-    b.row_status   = &c->d_small->status;
-    if (geist_b200_sample_batch(c, &b, c->stream) != GEIST_OK) {
-        return -1;
-    }
-    e = cudaMemcpyAsync(h, c->d_small, sizeof *h, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) {
+    b.temperature  = &h->T;
+    b.top_k        = &h->top_k;
+    b.top_p        = &h->top_p;
+    b.rng_in       = reinterpret_cast<const uint64_t *>(&h->rng_in);
+    b.rng_out      = reinterpret_cast<uint64_t *>(&h->rng_out);
+    b.tokens       = &h->token;
+    b.row_status   = &h->status;
+    b.finish_hint  = !(T > 0.0f) ? GEIST_B200_FINISH_GREEDY : (top_k > 1 && (size_t) top_k < n && top_k <= gb::kFastKMax) ? GEIST_B200_FINISH_GREEDY_TOPK : GEIST_B200_FINISH_AUTO;
+    for (int attempt = 0; attempt < 2; attempt++) {
+        h->token  = -1;
+        h->status = 0;
+        if (geist_b200_sample_batch(c, &b, c->stream) != GEIST_OK) {
+            return -1;
+        }
         e = cudaStreamSynchronize(c->stream);
-    }
-    if (e != cudaSuccess) {
-        fail(GEIST_E_BACKEND, "sampler: %s", cudaGetErrorString(e));
-        return -1;
+        if (e != cudaSuccess) {
+            fail(GEIST_E_BACKEND, "sampler: %s", cudaGetErrorString(e));
+            return -1;
+        }
+        if (!(h->status & GEIST_B200_ROW_RETRY)) {
+            break;
+        }
+        b.finish_hint = GEIST_B200_FINISH_AUTO; /* thousands of equal values at the top: the general kernel takes the row */
     }
     if (h->status & (GEIST_B200_ROW_LOAD_TIMEOUT | GEIST_B200_ROW_HIST_OVERFLOW | GEIST_B200_ROW_INTERNAL)) {
         fail(GEIST_E_BACKEND, "sampler: kernel reported row status 0x%x", h->status);
@@ -787,11 +797,8 @@ extern "C" enum geist_status geist_b200_argmax_f32(struct geist_b200_ctx *ctx, c
     std::lock_guard<std::mutex> lk(ctx->small_mu); /* callers on several threads share the context's staging words */
     CUDA_TRY(cudaSetDevice(ctx->device));
     geist_b200_ctx::Small *h = ctx->h_small;
-    memset(h, 0, sizeof *h);
-    h->top_p  = 1.0f;
-    h->token  = -1;
-    h->rng_in = 1;
-    CUDA_TRY(cudaMemcpyAsync(ctx->d_small, h, sizeof *h, cudaMemcpyHostToDevice, ctx->stream));
+    h->token                 = -1;
+    h->status                = 0;
     geist_b200_batch b{};
     b.logits       = logits_dev;
     b.row_stride   = n;
@@ -803,13 +810,13 @@ extern "C" enum geist_status geist_b200_argmax_f32(struct geist_b200_ctx *ctx, c
     b.top_p        = &ctx->d_small->top_p;
     b.rng_in       = reinterpret_cast<const uint64_t *>(&ctx->d_small->rng_in);
     b.rng_out      = reinterpret_cast<uint64_t *>(&ctx->d_small->rng_out);
-    b.tokens       = &ctx->d_small->token;
-    b.row_status   = &ctx->d_small->status;
+    b.tokens       = &h->token; /* written over the host link by the one kernel that the hint leaves */
+    b.row_status   = &h->status;
+    b.finish_hint  = GEIST_B200_FINISH_GREEDY;
     enum geist_status s = geist_b200_sample_batch(ctx, &b, ctx->stream);
     if (s != GEIST_OK) {
         return s;
     }
-    CUDA_TRY(cudaMemcpyAsync(h, ctx->d_small, sizeof *h, cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     if ((h->status & ~(GEIST_B200_ROW_SLOW_PATH | GEIST_B200_ROW_KEPT_PARTIAL)) != 0 || h->token < 0 || (size_t) h->token >= n) {
         return fail(GEIST_E_BACKEND, "argmax_f32: row status 0x%x, index %d", h->status, h->token);
@@ -837,11 +844,11 @@ struct geist_b200_batcher {
     long long          *d_hist_tot = nullptr;
 
     /* per-call device scratch, sized for max_sessions * GEIST_B200_SPEC_KMAX rows */
-    int   *d_slot = nullptr, *d_tokens = nullptr, *d_status = nullptr, *d_fed = nullptr;
-    int   *d_accepted = nullptr, *d_nemit = nullptr, *d_emitted = nullptr, *d_ones = nullptr;
+    int   *d_slot = nullptr, *d_tokens = nullptr, *d_fed = nullptr, *d_ones = nullptr;
     float *d_logits     = nullptr; /* staging for host logits, grown on demand */
     size_t d_logits_cap = 0;
-    int   *h_pin        = nullptr; /* pinned: slots | fed | tokens | status | accepted | nemit | emitted */
+    int   *h_pin        = nullptr; /* pinned, written and read by the kernels where it lies: slots | fed | tokens | status | accepted | nemit | emitted */
+    std::vector<int32_t> slots_sent; /* the session list that d_slot holds */
     size_t h_pin_ints   = 0;
 
     cudaStream_t copy_stream[2] = {nullptr, nullptr};
@@ -884,7 +891,7 @@ extern "C" void geist_b200_batcher_destroy(struct geist_b200_batcher *b) {
     cudaSetDevice(b->ctx->device);
     cudaDeviceSynchronize();
     void *dev[] = {b->d_T, b->d_P, b->d_rep, b->d_freq, b->d_pres, b->d_K, b->d_rng, b->d_rng_tmp, b->d_hist, b->d_hist_len, b->d_hist_tot, b->d_slot, b->d_tokens,
-                   b->d_status, b->d_fed, b->d_accepted, b->d_nemit, b->d_emitted, b->d_ones, b->d_logits, b->d_pending, b->d_cap, b->d_mask, b->d_peek,
+                   b->d_fed, b->d_ones, b->d_logits, b->d_pending, b->d_cap, b->d_mask, b->d_peek,
                    b->d_drafts, b->d_ndrafts, b->d_matchL, b->d_skip};
     for (void *p : dev) {
         cudaFree(p);
@@ -957,11 +964,7 @@ extern "C" enum geist_status geist_b200_batcher_create(struct geist_b200_ctx *ct
     A((void **) &b->d_hist_tot, S * 8);
     A((void **) &b->d_slot, S * 4);
     A((void **) &b->d_tokens, R * 4);
-    A((void **) &b->d_status, R * 4);
     A((void **) &b->d_fed, R * 4);
-    A((void **) &b->d_accepted, S * 4);
-    A((void **) &b->d_nemit, S * 4);
-    A((void **) &b->d_emitted, S * (GEIST_B200_SPEC_KMAX + 1) * 4);
     A((void **) &b->d_ones, S * 4);
     A((void **) &b->d_pending, S * 4);
     A((void **) &b->d_cap, S * 4);
@@ -1237,8 +1240,13 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
     int *h_acc  = h_stat + b->max_sessions * GEIST_B200_SPEC_KMAX;
     int *h_nem  = h_acc + b->max_sessions;
     int *h_emit = h_nem + b->max_sessions; /* [n, k+1] */
-    memcpy(h_slot, sessions, n * 4);
-    CUDA_TRY(cudaMemcpyAsync(b->d_slot, h_slot, n * 4, cudaMemcpyHostToDevice, st));
+    if (b->slots_sent.size() != n || memcmp(b->slots_sent.data(), sessions, n * 4) != 0) { /* a decode loop names the same sessions step after step */
+        memcpy(h_slot, sessions, n * 4);
+        b->slots_sent.clear();
+        CUDA_TRY(cudaMemcpyAsync(b->d_slot, h_slot, n * 4, cudaMemcpyHostToDevice, st));
+        b->slots_sent.assign(sessions, sessions + n);
+    }
+    const bool pen = b->n_pen_active > 0 && b->max_history > 0;
     if (verify) {
         memcpy(h_fed, fed, rows * 4);
         for (size_t i = 0; i < n; i++) {
@@ -1246,9 +1254,10 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
                 h_fed[i * k] = b->pending[(size_t) sessions[i]];
             }
         }
-        CUDA_TRY(cudaMemcpyAsync(b->d_fed, h_fed, rows * 4, cudaMemcpyHostToDevice, st));
+        if (pen) { /* the sampling kernels read the fed tokens many times, the accept kernel once: that one reads them here */
+            CUDA_TRY(cudaMemcpyAsync(b->d_fed, h_fed, rows * 4, cudaMemcpyHostToDevice, st));
+        }
     }
-    const bool pen = b->n_pen_active > 0 && b->max_history > 0;
     if (logits_on_host) { /* the staging block is about to be overwritten: rows remembered in it are gone */
         for (auto &lr : b->last_row) {
             if (lr.valid && b->d_logits != nullptr && lr.ptr >= b->d_logits && lr.ptr < b->d_logits + b->d_logits_cap) {
@@ -1257,6 +1266,9 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
         }
     }
 
+    /* Results go to the pinned block straight from the kernels (a few words each); only what a kernel behind reads more
+     * than once stays on the device. Every small copy cost the stream 2 us and the host as much. */
+    int *const       tok_dst = verify ? b->d_tokens : h_tok;
     geist_b200_batch d{};
     d.n_vocab            = b->V;
     d.rows_per_seq       = k;
@@ -1285,8 +1297,8 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
             d.n_seq      = n;
             d.slot       = b->d_slot;
             d.fed_tokens = (pen && verify) ? b->d_fed : nullptr;
-            d.tokens     = b->d_tokens;
-            d.row_status = b->d_status;
+            d.tokens     = tok_dst;
+            d.row_status = h_stat;
             enum geist_status s = geist_b200_sample_batch(b->ctx, &d, st);
             if (s != GEIST_OK) {
                 return s;
@@ -1322,8 +1334,8 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
                 d.n_seq      = ns;
                 d.slot       = b->d_slot + s0;
                 d.fed_tokens = (pen && verify) ? b->d_fed + s0 * k : nullptr;
-                d.tokens     = b->d_tokens + s0 * k;
-                d.row_status = b->d_status + s0 * k;
+                d.tokens     = tok_dst + s0 * k;
+                d.row_status = h_stat + s0 * k;
                 enum geist_status s = geist_b200_sample_batch(b->ctx, &d, cs);
                 if (s != GEIST_OK) {
                     return s;
@@ -1336,13 +1348,13 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
         }
         return GEIST_OK;
     };
-    const int *append_tok = b->d_tokens;
+    const int *append_tok = h_tok; /* read behind this call: the block's part is written again by kernels alone, in stream order */
     const int *append_cnt = b->d_ones;
     int        per_seq    = 1;
     int        first      = 0;
     if (verify) {
-        append_tok = b->d_emitted;
-        append_cnt = b->d_nemit;
+        append_tok = h_emit;
+        append_cnt = h_nem;
         per_seq    = (int) k + 1;
         first      = 1; /* emitted[0] is the pending token, which joined the history when it was sampled */
     }
@@ -1352,16 +1364,8 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
             return ls;
         }
         if (verify) {
-            gb::AcceptParams ap{b->d_fed, b->d_tokens, (int) n, (int) k, b->d_accepted, b->d_nemit, b->d_emitted};
+            gb::AcceptParams ap{h_fed, b->d_tokens, (int) n, (int) k, h_acc, h_nem, h_emit};
             CUDA_TRY(gb::launch_accept(ap, st));
-        }
-        CUDA_TRY(cudaMemcpyAsync(h_stat, b->d_status, rows * 4, cudaMemcpyDeviceToHost, st));
-        if (verify) {
-            CUDA_TRY(cudaMemcpyAsync(h_acc, b->d_accepted, n * 4, cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaMemcpyAsync(h_nem, b->d_nemit, n * 4, cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaMemcpyAsync(h_emit, b->d_emitted, n * (k + 1) * 4, cudaMemcpyDeviceToHost, st));
-        } else {
-            CUDA_TRY(cudaMemcpyAsync(h_tok, b->d_tokens, rows * 4, cudaMemcpyDeviceToHost, st));
         }
         CUDA_TRY(cudaStreamSynchronize(st));
         bool retry = false;
@@ -1622,7 +1626,9 @@ extern "C" enum geist_status geist_b200_batcher_propose_drafts(struct geist_b200
     CUDA_TRY(cudaSetDevice(b->ctx->device));
     cudaStream_t st = b->ctx->stream;
     const int    oc = GEIST_B200_SPEC_KMAX + 1; /* row length of the device-side draft table */
+    b->slots_sent.clear();
     CUDA_TRY(cudaMemcpyAsync(b->d_slot, h_slot, n * 4, cudaMemcpyHostToDevice, st));
+    b->slots_sent.assign(sessions, sessions + n);
     CUDA_TRY(cudaMemcpyAsync(b->d_pending, h_seed, n * 4, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(b->d_skip, h_skip, n * 4, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemsetAsync(b->d_drafts, 0xff, n * oc * 4, st));

@@ -177,6 +177,22 @@ def test_post_filter_probability_vector(ctx):
     assert rel_err(dense[exp > 0], exp[exp > 0]) <= 1e-5 and abs(dense.sum() - 1.0) < 1e-5
 
 
+@pytest.mark.parametrize("V", [1, 3, 4095, 4096, 4097, 12289])
+def test_dense_vector_at_the_edges_of_its_pieces(ctx, V):
+    """Sizes around the piece that one thread block writes; odd sizes put rows off the 16-byte grid. Every column comes
+    back, kept or zero, whatever the memory held."""
+    rows, k = 3, min(40, V)
+    x = normal_logits(rows, V, 2.5, V)
+    dT, dK, dP = per_seq(rows, 0.8, 40, 0.9)
+    out = ctx.sample_batch(to_dev(x), dT, dK, dP, u64_to_dev(independent_states(port, V, rows)), kept_cap=k)
+    dense = ctx.scatter_kept(out, V).cpu().numpy()
+    n, idx, prob = (out[name].cpu().numpy() for name in ("kept_n", "kept_idx", "kept_prob"))
+    exp = np.zeros((rows, V), np.float32)
+    for r in range(rows):
+        exp[r, idx[r, :min(n[r], k)]] = prob[r, :min(n[r], k)]
+    assert np.array_equal(dense, exp)
+
+
 def test_invalid_arguments_are_refused(ctx):
     import torch
     x = torch.zeros(4, 100, device="cuda")

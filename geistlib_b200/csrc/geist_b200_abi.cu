@@ -112,7 +112,7 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
         }
         pl.id_slots   = (int) slots;
         pl.row_cap    = (int) round_up(hist_max, 4);
-        pl.bucket_cap = (int) round_up(n_slices + 1, 4);
+        pl.bucket_cap = (int) round_up(n_slices * (size_t) gb::kWarps + 1, 4);
     }
     pl.hist_cap = hist_max ? (int) round_up(std::min<size_t>(hist_max, 1024), 4) : 0; /* the finisher walks segments of at most 1024 ids */
     pl.smem     = gb::sample_stream_smem(pl.n_slices, pl.id_slots > 0 ? 1 : 0);
@@ -411,9 +411,7 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     const size_t gen_str  = round_up(b->n_vocab, 4);
     const size_t gen_bmw  = (b->n_vocab + 31) / 32;
     const size_t gen_hcap = hist_max ? std::min(hist_max, b->n_vocab) : 0;
-    const size_t off_gv   = 0;
-    const size_t off_gb   = round_up(off_gv + n_rows * parts * (size_t) gb::kPartSlots * 16, 256);
-    const size_t off_seg  = round_up(off_gb + n_rows * parts * (size_t) gb::kPartSlots * 4, 256);
+    const size_t off_seg  = round_up(n_rows * parts * (size_t) gb::kPartBytes, 256);
     const int    fin_grid = (int) std::min<size_t>((size_t) pl.fin_ctas, n_rows);
     const size_t slots    = (size_t) fin_grid; /* row copies of the multi-pass path: one per finishing thread block that can run at a time */
     const size_t off_rows = round_up(off_seg + n_items * (size_t) gb::kWarps * sizeof(gb::SegRec), 256);
@@ -423,7 +421,7 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     const size_t off_ls   = round_up(off_dl + slots * gen_hcap * sizeof(gb::Pair), 256);
     const size_t off_pl   = round_up(off_ls + slots * gen_lcap * sizeof(gb::Pair), 256);
     const size_t off_po   = round_up(off_pl + (pl.id_slots ? n_rows * (size_t) pl.row_cap * 4 : 0), 256);
-    const size_t need     = round_up(off_po + (pl.id_slots ? n_rows * (size_t) (pl.n_slices + 1) * 4 : 0), 256) + 256;
+    const size_t need     = round_up(off_po + (pl.id_slots ? n_rows * ((size_t) pl.n_slices * (size_t) gb::kWarps + 1) * 4 : 0), 256) + 256;
     geist_b200_ctx::Lane *ln;
     {
         std::lock_guard<std::mutex> lk(ctx->lane_mu);
@@ -460,8 +458,7 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     p.pool             = ln->counters;
     p.arrive           = ln->arrive;
     p.pool_slots       = (int) slots;
-    p.grp_v            = reinterpret_cast<float4 *>(ln->buf + off_gv);
-    p.grp_b            = reinterpret_cast<int *>(ln->buf + off_gb);
+    p.parts            = ln->buf;
     p.segs             = reinterpret_cast<gb::SegRec *>(ln->buf + off_seg);
     p.gen_rows         = reinterpret_cast<float *>(ln->buf + off_rows);
     p.gen_stride       = (long long) gen_str;

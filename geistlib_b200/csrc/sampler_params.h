@@ -10,7 +10,8 @@ namespace gb {
 
 constexpr int kWarps        = 8;              /* warps of one thread block; each streams its own share of every slice */
 constexpr int kThreads      = kWarps * 32;
-constexpr int kNV4          = 8;              /* float4 one thread holds of a slice */
+constexpr int kNV4Log       = 3;
+constexpr int kNV4          = 1 << kNV4Log;   /* float4 one thread holds of a slice */
 constexpr int kSliceMax     = kThreads * kNV4 * 4; /* floats of one row slice: 8192 */
 constexpr int kStages       = 2;              /* depth of each warp's bulk-copy ring */
 constexpr int kWarpStageBytes = kSliceMax * 4 / kWarps; /* one warp's share of a slice: 4 KB */
@@ -25,9 +26,10 @@ constexpr int kMaxSlices    = 1024;           /* slices per row */
 constexpr int kMaxParts     = 64;             /* thread blocks a row may be spread over before the finisher gives the row to the multi-pass path */
 constexpr int kFinBitmapWords = 32;           /* finisher: one bit per entry of a crossing segment (at most 1024) */
 constexpr int kHistBins     = 256;            /* value histograms (threshold, select) */
-constexpr int kGroupCapWarp = 160;            /* candidate groups (one float4 each) a warp can hold of one row part */
-constexpr int kPartGroups   = kWarps * kGroupCapWarp; /* ... and a whole thread block: 1280 */
-constexpr int kPartSlots    = kPartGroups + 2;        /* a part in global scratch: its record in the first two 16-byte slots, then its groups */
+constexpr int kGroupSlots   = 16;             /* group maxima a thread keeps of one row part */
+constexpr int kPartCand     = 1024;           /* candidates that one row part can hand on */
+constexpr int kPartBytes    = 32 + kPartCand * 8; /* a part in global scratch: its record, then its candidates */
+constexpr int kSliceCs      = 32;             /* slices of a part whose units are remembered */
 constexpr int kRowIds       = 256;            /* ids of a row (history + fed tokens) counted inside the stream kernel, one per thread */
 
 /* status word, one per row (bit set) */
@@ -57,18 +59,18 @@ struct Pair {
 struct __align__(16) PartRec {
     float  max;      /* maximum of the part after penalties */
     int    arg;      /* first global id of that maximum */
-    int    n_groups; /* candidate groups this part found (more than kPartGroups: some were dropped) */
+    int    n_cand;   /* candidates this part found (more than kPartCand: some were dropped) */
     int    st;       /* status bits raised while the part streamed */
     float  tau;      /* the part's final select threshold: a lower bound of the row's kq-th largest value */
-    float  bulk_ref; /* top-p: the sum below is relative to this value ... */
-    double bulk_sum; /* ... sum of expf((x - bulk_ref) * inv_t) over everything outside the candidate groups */
+    float  bulk_c;   /* top-p: the sum below is in units of 2^bulk_c ... */
+    double bulk_sum; /* ... sum of 2^(x * log2(e) / T) over everything that is no candidate */
 };
 
 /* Temperature rows: one warp's share of one slice, ids in order. */
 struct __align__(16) SegRec {
-    float  ref;  /* maximum of the segment */
+    float  ref;  /* the sum is in units of 2^ref (a whole number, at least that of the segment's maximum); kNoUnit: nothing there */
     float  pad;
-    double sum;  /* sum of expf((x - ref) * inv_t) over the segment */
+    double sum;  /* sum of 2^(x * log2(e) / T) over the segment */
 };
 
 /* Which (row, slice) items a thread block of the stream kernel takes: always one contiguous run of the row-major
@@ -132,9 +134,9 @@ struct SampleParams {
     /* rows with more than kRowIds ids: their distinct ids are prepared by a kernel of their own */
     int       id_slots;    /* slots of that kernel's id table (a power of two, at least twice the ids a row can bring); 0: no such rows */
     int       row_cap;     /* entries of one row's prepared list */
-    int       bucket_cap;  /* n_slices + 1 rounded up to a multiple of 4 */
-    unsigned *pre_list;    /* [n_rows][row_cap] (position in the slice) | (count << 14), grouped by slice */
-    int      *pre_off;     /* [n_rows][n_slices + 1] where each slice's run starts */
+    int       bucket_cap;  /* n_slices * kWarps + 1 rounded up to a multiple of 4 */
+    unsigned *pre_list;    /* [n_rows][row_cap] (offset in the share) | (count << 10), grouped by (slice, warp) share */
+    int      *pre_off;     /* [n_rows][n_slices * kWarps + 1] where each share's run starts */
     int      hist_cap;     /* distinct-id entries the finisher reserves for one walked segment */
     int      aligned;      /* rows start on 16-byte boundaries: bulk copies allowed */
     unsigned flags;
@@ -143,8 +145,7 @@ struct SampleParams {
     int       *arrive;      /* [n_rows] greedy launches: how many parts of the row have published their record; zero between launches */
     int       *pool;        /* [pool_slots] 1: the row copy of this number is taken; zero between launches */
     int        pool_slots;
-    float4    *grp_v;       /* [n_rows, parts_max, kPartSlots] per part: its PartRec (two slots), then its candidate groups: four consecutive values ... */
-    int       *grp_b;       /* ... and the global id of the first */
+    unsigned char *parts;   /* [n_rows, parts_max, kPartBytes] per part: its PartRec, then its candidates (value, id) */
     SegRec    *segs;        /* [n_rows, n_slices, kWarps] temperature rows */
     float     *gen_rows;    /* [pool_slots, gen_stride]: private copies of one row for the multi-pass path */
     long long  gen_stride;  /* floats */

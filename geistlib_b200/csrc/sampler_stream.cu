@@ -10,19 +10,17 @@
  *   mbarriers): it waits for its share, applies the penalties that fall into it, lifts it into registers, asks
  *   for the share two items ahead and works on the registers. Inside a part no warp waits for another one.
  *
- *   Greedy rows keep (maximum, first id) per warp. Top-k / top-p rows pick candidates against a select
- *   threshold tau, a lower bound of the row's kq-th largest value: the part's first slice sets it (the thread
- *   maxima of all warps are binned by key; the only barriers inside a part), a histogram of the candidates
- *   raises it as the part streams. What is kept is the float4 GROUP that holds a candidate (four values and the
- *   id of the first): the lanes that hold any place them into the warp's own list themselves, one pass per
- *   slice, the places counted in shared memory. Temperature and top-p rows also sum
- *   expf((x - warp maximum) * inv_t) per warp and slice.
+ *   Greedy rows keep (maximum, first id) per warp. Top-k / top-p rows keep, per thread, the maximum of its 32
+ *   floats of every slice (a group) and its maximum over the part: nothing else of the select happens while the
+ *   part streams. When it is through, the kq-th largest of the 256 thread maxima is a threshold that k and a few
+ *   more values of the part reach; the few dozen groups that hold them are read again. Temperature rows sum
+ *   2^(x * log2(e) / T) per warp and slice, top-p rows per thread over the part.
  *
  *   Before any of this a row's share may pass the soft cap tanhf(x / c) * c and the mask of allowed columns,
  *   in place in the stage (head.c:145-159; only launches that carry one pay for it).
  *
  *   Part boundaries. The thread block meets and writes the part's record (maximum, first id, threshold, sums;
- *   two 16-byte slots) followed by its candidate groups to the part's place in global scratch. Nothing else is
+ *   two 16-byte slots) followed by its candidates to the part's place in global scratch. Nothing else is
  *   shared between thread blocks: no counters, no thread block waits for another one.
  *
  *   Finishing is left to a kernel of its own behind the stream kernel, launched as a programmatic dependent so
@@ -156,9 +154,8 @@ struct __align__(16) GroupShared {
 /* float4 of a slice that one warp owns: an equal share, rounded up to whole warp steps */
 __host__ __device__ __forceinline__ int share_len(int nv4) { return ((nv4 + kWarps - 1) / kWarps + 31) & ~31; }
 
-constexpr int kLiBits = 14; /* an id list entry is (position in the slice) | (count << kLiBits) */
-static_assert(kSliceMax <= (1 << kLiBits), "slice positions must fit the id list entry");
-static_assert((long long) kMaxSlices * kSliceMax <= (1ll << 28), "a candidate group keeps four flag bits above the id of its first value");
+static_assert(kSliceMax / kWarps <= 1024, "an offset in a share takes ten bits of an id list entry");
+static_assert(kNV4 == 1 << kNV4Log, "the float4 of a group are named by bits");
 
 enum Mode { M_ARGMAX, M_TOPK, M_TOPP, M_TEMP };
 
@@ -381,6 +378,36 @@ __device__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const Ro
     }
     g.sync();
     return st;
+}
+
+/* ------------------------------------------------------- sums over a row -- */
+
+/* The sums of temperature and top-p rows are formed of 2^(x * scale - c), scale = log2(e) / T in two floats (their sum is
+ * good to 2^-48) and c a whole number near the largest x * scale: one rounding of the argument at the size of the
+ * difference, whatever the size of x, and changing c moves a sum by a power of two, exactly. The high float is
+ * rounded down so that both products of an x of -inf are -inf. */
+constexpr float kNoUnit = -1e30f; /* c before anything finite has been met */
+__device__ __forceinline__ double sum_scale(float inv_t) { return (double) inv_t * 1.4426950408889634; }
+struct SumScale {
+    float hi, lo;
+};
+__device__ __forceinline__ SumScale sum_scale2(float inv_t) {
+    SumScale k;
+    k.hi = __double2float_rz(sum_scale(inv_t));
+    k.lo = fmaxf(__double2float_rn(sum_scale(inv_t) - (double) k.hi), 1e-37f);
+    return k;
+}
+__device__ __forceinline__ float sum_term(float x, const SumScale &k, float c) { return exp2_fast(__fmaf_rn(x, k.lo, __fmaf_rn(x, k.hi, -c))); }
+__device__ __forceinline__ float sum_unit(float m, float inv_t) { return m == -CUDART_INF_F ? kNoUnit : ceilf(__fmul_rn(m, sum_scale2(inv_t).hi)); }
+/* 2^(a - b) for whole numbers, 0 below the range of double */
+__device__ __forceinline__ double pow2_diff(float a, float b) {
+    const double d = (double) a - (double) b;
+    return d < -1022.0 ? 0.0 : __longlong_as_double((long long) (1023 + (int) fmin(d, 1023.0)) << 52);
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
 /* ------------------------------------------------------- group reductions -- */
@@ -1211,31 +1238,26 @@ __device__ __forceinline__ void row_epilogue(const SampleParams &p, const RowCfg
 /* ------------------------------------------------------------ shared state -- */
 
 /* What the warps of one thread block share. The ring (every warp's two stages) lies in front of it in dynamic
- * shared memory, the candidate groups of the part in work behind it. */
-constexpr int kInlineCap = 1024; /* candidates of a row that the stream kernel can order by itself */
+ * shared memory, the group maxima of the part in work behind it. */
 struct __align__(16) StreamShared {
     unsigned long long full[kWarps][kStages]; /* warp w's share of item j has landed in its stage j % kStages */
     /* the part in work */
-    unsigned           tau_key;   /* ordered key of the raised select threshold (0: not raised yet) */
-    int                tau_lock;  /* one warp at a time reads the candidate histogram */
     int                st;        /* status bits of the part */
-    unsigned           wkey[kWarps], wlow[kWarps]; /* first slice: largest / smallest group maximum per warp */
-    int                wown[kWarps];               /* ... and how many groups the warp holds */
-    int                wn[kWarps], wn_all[kWarps]; /* candidate groups per warp: held / found */
     unsigned long long best[kWarps];               /* (key of the maximum, ~first id) per warp */
-    float              wb_ref[kWarps];             /* top-p: per warp, sum of expf((x - ref) * inv_t) over what is no candidate */
-    double             wb_sum[kWarps];
-    int                bhist[kHistBins];           /* first slice: group maxima binned by key */
-    int                thist[kHistBins];           /* candidates binned by value between threshold and maximum */
+    float              wb_c[kWarps];               /* temperature / top-p: the warp's sums are in units of 2^wb_c ... */
+    double             wb_sum[kWarps];             /* ... and top-p's sum over the part */
+    float              c_at[kSliceCs][kWarps];     /* top-p: the unit that a slice's terms were formed in */
+    double             fix[kWarps];                /* top-p: what the candidates' leaving changes in that sum */
     int                rl_id[kRowIds], rl_cnt[kRowIds + 4]; /* the row's distinct history ids as (offset in the share | count << 10 | tag << 20),
                                                              * grouped by the (slice, warp) share they fall into, and where each group's run starts */
-    /* finishing inside the stream kernel (F_INLINE_TOPK): the row's candidates, its k best in order, their weights */
-    int                fin_n, cur_rr;
-    alignas(8) Pair    fin_c[kInlineCap]; /* also holds the draw's running sums (doubles) once the ranking is done */
+    /* the part's select */
+    int                n_grp, n_cand;         /* groups that reach the threshold; candidates in them */
+    unsigned short     grp[kPartCand];        /* (slot << 8) | thread */
+    alignas(8) Pair    cand[kPartCand];
+    /* finishing inside the stream kernel (F_INLINE_TOPK): the k best in order, their weights */
+    int                cur_rr;
     Pair               fin_s[kFastKMax];
     float              fin_q[kFastKMax];
-    int                wcur[kWarps];    /* groups in each warp's list (the lanes count themselves in) */
-    float              wsq[kWarps];     /* top-k: the threshold at which each warp last cleared its candidate list of what had fallen below */
     unsigned long long cur_rng;         /* the generator word the part's sequence came with, its sequence, and whether the row is the sequence's last */
     int                cur_seq, cur_last;
     float              cap;             /* the part's soft cap and mask row (0 / null: none) */
@@ -1246,6 +1268,7 @@ struct __align__(16) StreamShared {
 };
 
 constexpr int kStagedParts = 4;
+constexpr int kStagedCand  = 120; /* candidates of each that come in with the record */
 
 /* What the threads of one finishing thread block share; the merged candidate list lies behind it. */
 struct __align__(16) FinishShared {
@@ -1259,19 +1282,24 @@ struct __align__(16) FinishShared {
     Pair        fsort[kFastKMax];
     float       fq[kFastKMax];
     PenEntry    fdlist[512];
-    float4      st_v[kStagedParts][kThreads]; /* the first 256 slots of the row's first parts, as they came in ... */
-    int         st_b[kStagedParts][kThreads]; /* ... in one round trip */
+    alignas(16) unsigned long long stage[kStagedParts][kStagedCand + 4]; /* the records and first candidates of the row's first parts, in one round trip */
+    unsigned long long save[256 + 128];                      /* the multi-pass path keeps a histogram here */
 };
 
-constexpr int kGroupBytes = kPartGroups * 20; /* float4 + first id per group */
-constexpr int kSqueezeAt  = 64;               /* a warp holding more candidate groups than this looks whether the threshold has left some behind */
+constexpr int kGroupBytes = kGroupSlots * kThreads * 4; /* one maximum per slot and thread */
 constexpr int kListSmem   = 1024;             /* prepared id-list entries of a part that are kept in shared memory */
 constexpr int kFinCap     = 2048;             /* candidates the finisher can order per row (8 per thread) */
 constexpr int kFinPer     = kFinCap / kThreads;
 constexpr int kRankAll    = 384;              /* up to this many candidates are ranked one against all */
 constexpr int kFinBytes   = kWarps * 256 * 12;    /* finisher: the merged candidate list; the multi-pass path keeps one byte histogram per warp there */
 static_assert(kFinCap * (int) sizeof(Pair) <= kFinBytes, "the merged list fits");
-static_assert(kGroupBytes >= 4 * kRowIds * 4, "the id table of a part's set-up lies in the groups' memory");
+static_assert(kGroupBytes >= 4 * kRowIds * 4, "the id table of a part's set-up lies in the group maxima's memory");
+static_assert(kGroupSlots <= 256 && kThreads == 256, "a group's name fits 16 bits");
+
+/* Part `k` of a row in global scratch: its record (two int4), then its candidates. */
+__device__ __forceinline__ int4 *part_rec(const SampleParams &p, int row, int k) {
+    return reinterpret_cast<int4 *>(p.parts + ((size_t) row * (size_t) p.parts_max + (size_t) k) * (size_t) kPartBytes);
+}
 
 /* n things dealt out in runs of q + 1 (the first r runs) and q: which run holds thing i */
 __device__ __forceinline__ int run_of(int i, int q, int r) { return i < r * (q + 1) ? i / (q + 1) : r + (i - r * (q + 1)) / q; }
@@ -1334,20 +1362,6 @@ __device__ __forceinline__ int top_bin(const int *hist, int lane, int kq) {
         }
     }
     return __shfl_sync(0xffffffffu, b, ball != 0u ? 31 - __clz(ball) : 0);
-}
-
-/* Group f of this thread block's own candidates: the warps' lists one after the other. */
-__device__ __forceinline__ int own_slot(const StreamShared *sh, int f) {
-    int w = 0;
-#pragma unroll
-    for (int i = 0; i < kWarps - 1; i++) {
-        const int n = sh->wn[i];
-        if (w == i && f >= n) {
-            f -= n;
-            w = i + 1;
-        }
-    }
-    return w * kGroupCapWarp + f;
 }
 
 /* ------------------------------------------- finisher: ordered select of kq -- */
@@ -1463,23 +1477,19 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
 
     g.sync(); /* the staging of the row before is no longer read */
     {
-        /* one round trip: the first 256 slots (record + 254 groups) of up to four parts, whatever their counts are */
-        float4 tv[kStagedParts];
-        int    tb[kStagedParts];
+        /* one round trip: the record and the first candidates of up to four parts, whatever their counts are */
+        unsigned long long tv[2];
 #pragma unroll
-        for (int k = 0; k < kStagedParts; k++) {
-            tv[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            tb[k] = 0;
-            if (k < n_parts) {
-                const size_t at = ((size_t) row * (size_t) p.parts_max + (size_t) k) * (size_t) kPartSlots + (size_t) g.tid;
-                tv[k]           = __ldcg(p.grp_v + at);
-                tb[k]           = __ldcg(p.grp_b + at);
-            }
+        for (int q = 0; q < 2; q++) {
+            const int t = g.tid + q * kThreads, k = t / (kStagedCand + 4), i = t - k * (kStagedCand + 4);
+            tv[q]       = k < min(n_parts, kStagedParts) ? __ldcg(reinterpret_cast<const unsigned long long *>(part_rec(p, row, k)) + i) : 0ull;
         }
 #pragma unroll
-        for (int k = 0; k < kStagedParts; k++) {
-            sh->st_v[k][g.tid] = tv[k];
-            sh->st_b[k][g.tid] = tb[k];
+        for (int q = 0; q < 2; q++) {
+            const int t = g.tid + q * kThreads;
+            if (t < kStagedParts * (kStagedCand + 4)) {
+                (&sh->stage[0][0])[t] = tv[q];
+            }
         }
     }
     g.sync();
@@ -1489,7 +1499,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         float m = -CUDART_INF_F;
         int   a = 0x7fffffff;
         for (int i = g.tid; i < n_parts; i += g.n) {
-            const int4  h  = __ldcg(reinterpret_cast<const int4 *>(p.grp_v + ((size_t) row * (size_t) p.parts_max + (size_t) i) * (size_t) kPartSlots));
+            const int4  h  = __ldcg(part_rec(p, row, i));
             const float pm = __int_as_float(h.x);
             st |= h.w;
             if (pair_before(pm, h.y, m, a)) {
@@ -1524,10 +1534,10 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     if (g.tid < n_parts) {
         int4 h, h2;
         if (g.tid < kStagedParts) { /* the record came in with the part's first slots */
-            h  = *reinterpret_cast<const int4 *>(&sh->st_v[g.tid][0]);
-            h2 = *reinterpret_cast<const int4 *>(&sh->st_v[g.tid][1]);
+            h  = *reinterpret_cast<const int4 *>(&sh->stage[g.tid][0]);
+            h2 = *reinterpret_cast<const int4 *>(&sh->stage[g.tid][2]);
         } else {
-            const int4 *rec = reinterpret_cast<const int4 *>(p.grp_v + ((size_t) row * (size_t) p.parts_max + (size_t) g.tid) * (size_t) kPartSlots);
+            const int4 *rec = part_rec(p, row, g.tid);
             h               = __ldcg(rec);
             h2              = __ldcg(rec + 1);
         }
@@ -1560,11 +1570,11 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             row_arg = a;
         }
         tau_row = fmaxf(tau_row, sh->ptau[i]);
-        overflow |= sh->pn[i] > kPartGroups;
+        overflow |= sh->pn[i] > kPartCand;
         if (g.tid == 0) {
             sh->poff[i] = others;
         }
-        others += sh->pn[i];
+        others += min(sh->pn[i], kPartCand + 1);
     }
 
     if (r.mode == M_ARGMAX) {
@@ -1585,11 +1595,16 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         /* segment sums (one per warp and slice, ids in order), moved from their own maximum to the row maximum */
         const int     nseg   = p.n_slices * kWarps;
         const SegRec *segs   = p.segs + (size_t) row * (size_t) nseg;
+        /* every segment's sum is in units of a power of two of its own; all are moved to the row's, that of its
+         * maximum, which is the largest of them: exact but for what leaves the range of double */
+        const float   row_c  = sum_unit(row_max, r.inv_t);
         auto          seg_at = [&](int t) {
-            const float  ref = __ldcg(&segs[t].ref);
-            const double sm  = __ldcg(&segs[t].sum);
-            return ref == -CUDART_INF_F ? 0.0 : sm * exp(((double) ref - (double) row_max) * (double) r.inv_t);
+            const float  c  = __ldcg(&segs[t].ref);
+            const double sm = __ldcg(&segs[t].sum);
+            return c == kNoUnit ? 0.0 : sm * pow2_diff(c, row_c);
         };
+        /* ... and the crossing segment's terms, evaluated against the maximum itself */
+        const double  unit   = exp2((double) row_max * sum_scale(r.inv_t) - (double) row_c);
         double part = 0.0;
         for (int t = g.tid; t < nseg; t += g.n) {
             part += seg_at(t);
@@ -1682,7 +1697,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             for (int q = 0; q < 4; q++) {
                 const int i = i0 + q;
                 ev[q]       = (q < per && i < seg_n) ? expf(scaled_arg(wbuf[i], row_max, r.inv_t)) : 0.0f;
-                mine += (double) ev[q];
+                mine += (double) ev[q] * unit;
             }
             double incl = mine;
 #pragma unroll
@@ -1718,7 +1733,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 int    hit = min(i0 + per - 1, seg_n - 1);
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    a += (double) ev[q];
+                    a += (double) ev[q] * unit;
                     if (q < per && u < a) {
                         hit = i0 + q;
                         break;
@@ -1735,9 +1750,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     }
 
     }
-    /* ---- top-k and top-p: merge the parts' candidate groups ---- */
-    const int n_groups       = others;
-    bool      need_multipass = !(r.kq > 0 && r.kq <= kFastKMax) || overflow || n_groups > 8 * kFinCap; /* what counts is how many stay above the row's threshold: checked below */
+    /* ---- top-k and top-p: merge the parts' candidates ---- */
+    bool need_multipass = !(r.kq > 0 && r.kq <= kFastKMax) || overflow; /* what counts is how many stay above the row's threshold: checked below */
     if (!need_multipass) {
         const bool keep_all = r.mode == M_TOPP; /* every marked entry was left out of the bulk sums */
         /* The candidates of all parts are merged in up to three passes of one rolled loop. The first keeps what
@@ -1749,51 +1763,31 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         int   bin_min   = 0;
         auto  bin_of    = [&](float v) { return min(kHistBins - 1, max(0, __float2int_rz((v - tau_row) * bin_scale))); };
         int   pass      = 0; /* 0 keep by threshold, 1 bin, 2 keep by bin */
-        /* A group is four consecutive values, the id of the first and, in the id's top four bits, which of them
-         * passed. The whole warp calls: the entries that stay are counted over the warp and get their places
-         * with one atomic per warp. */
-        auto place_group = [&](bool valid, const float4 &v, int raw) {
-            const int      b  = raw & 0x0fffffff;
-            const unsigned cm = valid ? (unsigned) raw >> 28 : 0u;
-            bool           k0 = (cm & 1u) && b < p.V && (keep_all || v.x >= tau_row);
-            bool           k1 = (cm & 2u) && b + 1 < p.V && (keep_all || v.y >= tau_row);
-            bool           k2 = (cm & 4u) && b + 2 < p.V && (keep_all || v.z >= tau_row);
-            bool           k3 = (cm & 8u) && b + 3 < p.V && (keep_all || v.w >= tau_row);
+        /* The whole warp calls: the entries that stay are counted over the warp and get their places with one atomic
+         * per warp. */
+        auto place = [&](bool valid, const Pair &e) {
+            bool keep = valid && (keep_all || e.v >= tau_row);
             if (pass == 1) {
-                if (k0) atomicAdd(&sh->bhist[bin_of(v.x)], 1);
-                if (k1) atomicAdd(&sh->bhist[bin_of(v.y)], 1);
-                if (k2) atomicAdd(&sh->bhist[bin_of(v.z)], 1);
-                if (k3) atomicAdd(&sh->bhist[bin_of(v.w)], 1);
+                if (keep) {
+                    atomicAdd(&sh->bhist[bin_of(e.v)], 1);
+                }
                 return;
             }
             if (pass == 2) {
-                k0 = k0 && bin_of(v.x) >= bin_min;
-                k1 = k1 && bin_of(v.y) >= bin_min;
-                k2 = k2 && bin_of(v.z) >= bin_min;
-                k3 = k3 && bin_of(v.w) >= bin_min;
+                keep = keep && bin_of(e.v) >= bin_min;
             }
-            const int      cnt = (int) k0 + (int) k1 + (int) k2 + (int) k3;
-            if (__ballot_sync(0xffffffffu, cnt > 0) == 0u) {
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            if (m == 0u) {
                 return;
             }
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, incl, o);
-                if (g.lane >= o) {
-                    incl += up;
-                }
-            }
             int base = 0;
-            if (g.lane == 31) {
-                base = atomicAdd(&sh->n_ent, incl);
+            if (g.lane == 0) {
+                base = atomicAdd(&sh->n_ent, __popc(m));
             }
-            base    = __shfl_sync(0xffffffffu, base, 31);
-            int pos = base + incl - cnt;
-            if (k0) { if (pos < kFinCap) { cbuf[pos].v = v.x; cbuf[pos].idx = b; } pos++; }
-            if (k1) { if (pos < kFinCap) { cbuf[pos].v = v.y; cbuf[pos].idx = b + 1; } pos++; }
-            if (k2) { if (pos < kFinCap) { cbuf[pos].v = v.z; cbuf[pos].idx = b + 2; } pos++; }
-            if (k3) { if (pos < kFinCap) { cbuf[pos].v = v.w; cbuf[pos].idx = b + 3; } pos++; }
+            const int pos = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << g.lane) - 1u));
+            if (keep && pos < kFinCap) {
+                cbuf[pos] = e;
+            }
         };
         int total = 0;
 #pragma unroll 1
@@ -1805,7 +1799,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 sh->bhist[g.tid] = 0;
             }
             g.sync();
-            /* one loop over the groups of all parts (rolled: code that runs once per row costs what it weighs) */
+            /* one loop over the candidates of all parts (rolled: code that runs once per row costs what it weighs) */
 #pragma unroll 1
             for (int f0 = 0; f0 < others; f0 += g.n) {
                 const int  f  = f0 + g.tid;
@@ -1816,20 +1810,16 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                         pi = q; /* offsets ascend */
                     }
                 }
-                const int slot = f - sh->poff[pi] + 2; /* behind the part's record */
-                float4    v    = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                int       b    = 0;
+                const int i = f - sh->poff[pi];
+                Pair      e{0.0f, 0};
                 if (ok) {
-                    if (pi < kStagedParts && slot < kThreads) {
-                        v = sh->st_v[pi][slot];
-                        b = sh->st_b[pi][slot];
-                    } else {
-                        const size_t at = ((size_t) row * (size_t) p.parts_max + (size_t) pi) * (size_t) kPartSlots + (size_t) slot;
-                        v               = __ldcg(p.grp_v + at);
-                        b               = __ldcg(p.grp_b + at);
-                    }
+                    const unsigned long long w = pi < kStagedParts && i < kStagedCand
+                                                         ? sh->stage[pi][4 + i]
+                                                         : __ldcg(reinterpret_cast<const unsigned long long *>(part_rec(p, row, pi)) + 4 + i);
+                    e.v                        = __uint_as_float((unsigned) w);
+                    e.idx                      = (int) (w >> 32);
                 }
-                place_group(ok, v, b);
+                place(ok, e);
             }
             g.sync();
             if (pass == 1) { /* the bin in which the kq-th candidate from the top falls */
@@ -1972,8 +1962,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         if constexpr (!kFast) {
         if (!need_multipass) {
             /* top-p over a small nucleus (sampler.c:245-300). Candidates get their exact e_i relative to the row
-             * maximum; the rest of the row was summed per part with expf relative to a maximum of its own and is
-             * rescaled here. */
+             * maximum; the rest of the row was summed per part in units of a power of two and is rescaled
+             * here. */
             double part = 0.0;
             for (int i = g.tid; i < total; i += g.n) {
                 const float e = exp_exact(scaled_arg(cbuf[i].v, row_max, r.inv_t));
@@ -1981,8 +1971,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 part += (double) e;
             }
             if (g.tid < n_parts) {
-                const float  ref = sh->pbref[g.tid];
-                const double sc  = ref == -CUDART_INF_F ? 0.0 : exp(((double) ref - (double) row_max) * (double) r.inv_t);
+                const float  c  = sh->pbref[g.tid];
+                const double sc = c == kNoUnit ? 0.0 : exp2((double) c - (double) row_max * sum_scale(r.inv_t));
                 part += sc * sh->pbsum[g.tid];
             }
             const double S = group_sum_d(g, gs, part);
@@ -2063,47 +2053,21 @@ __device__ __forceinline__ int row_id_count(const SampleParams &p, int hist_len,
 }
 
 /*
- * A top-k row that went through one thread block as a whole, finished by that thread block from its own candidate
- * lists (all threads call): the candidates above the part's final threshold are gathered, ranked one against all,
- * the k best get their exact weights and the draw is made as in finish_row. What does not fit here (a warp's list
- * ran over, more than kInlineCap candidates, fewer than k) is handed back with ST_RETRY.
+ * A top-k row that went through one thread block as a whole, finished by that thread block from its own candidates
+ * (all threads call): ranked one against all, the k best get their exact weights and the draw is made as in
+ * finish_row. What does not fit here (more candidates than the list holds, fewer than k) is handed back with ST_RETRY.
  */
-__device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, const float4 *grp_v, const int *grp_b, int row, int held, bool complete, float tau_fin,
-                                                int k, float inv_t, int st_bits) {
+__device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, int row, int total, int k, float inv_t, int st_bits) {
     const int tid = (int) threadIdx.x;
-    if (tid == 0) {
-        sh->fin_n = 0;
-    }
-    __syncthreads();
-    for (int f = tid; f < held; f += kThreads) {
-        const int      slot = own_slot(sh, f);
-        const float4   v    = grp_v[slot];
-        const int      raw  = grp_b[slot];
-        const int      b    = raw & 0x0fffffff;
-        const unsigned cm   = (unsigned) raw >> 28;
-        const float    c4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            if (((cm >> c) & 1u) != 0u && b + c < p.V && c4[c] >= tau_fin) {
-                const int pos = atomicAdd(&sh->fin_n, 1);
-                if (pos < kInlineCap) {
-                    sh->fin_c[pos].v   = c4[c];
-                    sh->fin_c[pos].idx = b + c;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    const int  total = sh->fin_n;
-    const bool ok    = complete && total <= kInlineCap && total >= k && k <= kFastKMax;
+    const bool ok = total <= kPartCand && total >= k && k <= kFastKMax;
     if (ok) {
 #pragma unroll 1
         for (int i = tid; i < total; i += kThreads) {
-            const Pair me   = sh->fin_c[i];
+            const Pair me   = sh->cand[i];
             int        rank = 0;
 #pragma unroll 4
             for (int j = 0; j < total; j++) {
-                rank += pair_before(sh->fin_c[j].v, sh->fin_c[j].idx, me.v, me.idx) ? 1 : 0;
+                rank += pair_before(sh->cand[j].v, sh->cand[j].idx, me.v, me.idx) ? 1 : 0;
             }
             if (rank < k) {
                 sh->fin_s[rank] = me;
@@ -2233,6 +2197,21 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
     stage = kPrefetchDone;
 }
 
+/* The largest of the warps' units of a part. */
+__device__ __forceinline__ float unit_max(const StreamShared *sh) {
+    float c = kNoUnit;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        c = fmaxf(c, sh->wb_c[w]);
+    }
+    return c;
+}
+
+/* The terms of a float4, added up as every place that forms them adds them up. */
+__device__ __forceinline__ float sum_terms(const float4 &x, const SumScale &k, float c) {
+    return __fadd_rn(__fadd_rn(sum_term(x.x, k, c), sum_term(x.y, k, c)), __fadd_rn(sum_term(x.z, k, c), sum_term(x.w, k, c)));
+}
+
 /* Which kinds of rows an instantiation of the stream kernel carries the code for: every one carries greedy rows;
  * K_SEL adds the candidate select of top-k rows, K_SUMS the sums of temperature and top-p rows (and top-p's select).
  * A launch whose caller vouched for its rows' kinds (finish_hint) runs the instantiation without the rest: less
@@ -2250,10 +2229,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     unsigned char *ring    = smem_raw;
     StreamShared  *sh      = reinterpret_cast<StreamShared *>(smem_raw + (size_t) kWarps * kStages * kWarpStageBytes);
     unsigned char *gmem    = reinterpret_cast<unsigned char *>(sh + 1); /* candidate groups of the part in work */
-    float4        *grp_v   = reinterpret_cast<float4 *>(gmem);
-    int           *grp_b   = reinterpret_cast<int *>(gmem + (size_t) kPartGroups * 16);
-    int           *sl_off  = reinterpret_cast<int *>(gmem + kGroupBytes); /* long histories: where each slice's run of the prepared list starts */
-    unsigned      *sl_list = reinterpret_cast<unsigned *>(gmem + kGroupBytes + ((((size_t) p.n_slices + 1) * 4 + 15) & ~(size_t) 15)); /* ... and the part's entries, when they fit */
+    float         *gmax    = reinterpret_cast<float *>(gmem); /* [kGroupSlots][kThreads] */
+    unsigned      *sl_list = reinterpret_cast<unsigned *>(gmem + kGroupBytes); /* long histories: the part's entries of the row's prepared list, when they fit */
 
     Grp g;
     g.tid  = (int) threadIdx.x;
@@ -2263,7 +2240,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     g.nw   = kWarps;
     g.bar  = 0;
     const int      tid = g.tid, lane = g.lane, warp = g.warp;
-    const unsigned lt  = (1u << lane) - 1u;
 
     /* every thread block takes a contiguous run of the (row, slice) items */
     int my_first, my_count;
@@ -2403,23 +2379,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         const int   part_idx = (int) blockIdx.x - b_first;
         const int   n_parts = cta_of_item(p, row * p.n_slices + p.n_slices - 1) - b_first + 1;
 
+        const int  *long_off  = (kKinds & K_SHORT) == 0 && long_ids ? p.pre_off + (size_t) row * (size_t) (p.n_slices * kWarps + 1) + c0 * kWarps : nullptr;
+        bool        long_smem = true; /* a long list's part lies in shared memory like a short one's */
+
         /* ---- part set-up ---- */
         if (tid == 0) {
-            sh->st       = 0;
-            sh->tau_key  = 0u;
-            sh->tau_lock = 0;
-            sh->fin_n    = 0;
-        }
-        if (tid < kHistBins) {
-            sh->thist[tid] = 0;
-            sh->bhist[tid] = 0;
-        }
-        if (tid < kWarps) {
-            sh->wcur[tid] = 0;
-            sh->wsq[tid] = -CUDART_INF_F;
+            sh->st     = 0;
+            sh->n_grp  = 0;
+            sh->n_cand = 0;
         }
         if (pen_on && !long_ids) {
-            /* The row's distinct ids with their counts: an open-addressing table in the groups' memory (free
+            /* The row's distinct ids with their counts: an open-addressing table in the group maxima's memory (free
              * between two parts), one id per thread; the thread whose id opened a slot speaks for that id. The ids
              * are then grouped by the (slice, warp) share of the part that they fall into, so that a warp looks at
              * its own share's run alone (most shares hold none): kRowIds groups, slice c of the part and slice
@@ -2504,21 +2474,23 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 sh->rl_id[sh->rl_cnt[grp] + place] = rest | (id_cnt[slot] << 10);
             }
         } else if (pen_on) {
-            /* long histories: a kernel that ran before this one left the row's distinct ids with their counts
-             * in global memory, grouped by slice; the part copies where its slices' runs start */
-            const int *off = p.pre_off + (size_t) row * (size_t) (p.n_slices + 1) + c0;
-            for (int i = tid; i <= part_len; i += kThreads) {
-                sl_off[i] = off[i];
+            /* long histories: a kernel that ran before this one left the row's distinct ids with their counts in
+             * global memory, grouped by share. The part copies where its shares' runs start, and the entries
+             * themselves when there are at most kListSmem of them: the slices then read them from shared memory
+             * instead of paying a round trip to L2 each. */
+            if (part_len * kWarps <= kRowIds) {
+                for (int i = tid; i <= part_len * kWarps; i += kThreads) {
+                    sh->rl_cnt[i] = long_off[i] - long_off[0];
+                }
             }
-            /* the part's entries themselves come along when there are at most kListSmem of them: the slices then
-             * read them from shared memory instead of paying a round trip to L2 each */
-            const int e_lo = off[0], e_n = off[part_len] - e_lo;
+            const int e_lo = long_off[0], e_n = long_off[part_len * kWarps] - e_lo;
             if (e_n <= kListSmem) {
                 const unsigned *src = p.pre_list + (size_t) row * (size_t) p.row_cap + e_lo;
                 for (int i = tid; i < e_n; i += kThreads) {
                     sl_list[i] = src[i];
                 }
             }
+            long_smem = part_len * kWarps <= kRowIds && e_n <= kListSmem;
         }
         __syncthreads();
         static_assert(2 * kRowIds == 512, "the id table's hash keeps 9 bits");
@@ -2526,15 +2498,35 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         PROF_ONCE(3);
         CYC(5);
         const double rep_rcp = pen_on ? 1.0 / (double) rep : 1.0;
-        unsigned run_key = 0u; /* this warp's maximum of the part so far (key) and its first id */
-        int      run_arg = 0x7fffffff;
-        float    tau_reg = -CUDART_INF_F, t_lo = 0.0f, t_scale = 0.0f;
-        int      wcnt = 0, since = 0; /* this warp's candidate groups of the part; those since it last looked at the threshold */
-        float    b_ref = -CUDART_INF_F; /* top-p: running sum of what is no candidate, relative to b_ref */
-        double   b_sum = 0.0;
-        int      wst   = 0;
-        float4  *seg_v = grp_v + warp * kGroupCapWarp;
-        int     *seg_b = grp_b + warp * kGroupCapWarp;
+        /* the entries of the ids that fall into warp w's share of the part's slice s_: an entry that belongs to
+         * another slice of the same group has another tag */
+        auto ids_of = [&](int s_, int w, const unsigned *&ent, int &lo, int &hi, unsigned &tag) {
+            if (!long_ids) {
+                const int grp = (s_ & 31) * kWarps + w;
+                ent           = reinterpret_cast<const unsigned *>(sh->rl_id);
+                lo            = sh->rl_cnt[grp];
+                hi            = sh->rl_cnt[grp + 1];
+                tag           = (unsigned) s_ >> 5;
+            } else {
+                const int grp = s_ * kWarps + w;
+                ent           = long_smem ? sl_list : p.pre_list + (size_t) row * (size_t) p.row_cap;
+                lo            = long_smem ? sh->rl_cnt[grp] : long_off[grp];
+                hi            = long_smem ? sh->rl_cnt[grp + 1] : long_off[grp + 1];
+                tag           = 0u;
+            }
+        };
+        const unsigned cnt_mask = long_ids ? 0x3fffffu : 0x3ffu; /* above the offset's ten bits; a short list's entries carry a tag on top */
+        unsigned       run_key = 0u; /* greedy: this warp's maximum of the part so far (key) and its first id */
+        int            run_arg = 0x7fffffff;
+        float          top0 = -CUDART_INF_F, top1 = -CUDART_INF_F; /* others: the thread's maxima over the first and the second half of its float4 */
+        float          unit = kNoUnit; /* the warp's sums are in units of 2^unit */
+        double         acc  = 0.0;     /* top-p: the thread's sum over the part */
+        int            wst  = 0;
+        const SumScale ks   = sum_scale2(inv_t);
+        int            gm_shift = 0; /* slices that share one slot of the group maxima: 2^gm_shift */
+        while (((part_len - 1) >> gm_shift) >= kGroupSlots) {
+            gm_shift++;
+        }
 
         /* ---- the part's slices, every warp on its own ---- */
         for (int s = 0; s < part_len; s++, j++) {
@@ -2586,28 +2578,16 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             /* ---- 2. penalties on the share ---- */
             if (pen_on) {
                 bool touched = false; /* most shares hold none of the row's ids: those need no fence before the refill */
-                if (!long_ids) {
-                    const int grp = (s & 31) * kWarps + warp;
-                    const int lo = sh->rl_cnt[grp], hi = sh->rl_cnt[grp + 1];
-                    for (int e = lo + lane; e < hi; e += 32) {
-                        const unsigned en = (unsigned) sh->rl_id[e];
-                        if ((int) (en >> 20) == (s >> 5)) {
-                            float *q = sl + (en & 0x3ffu);
-                            *q       = penalise_rcp(*q, (int) ((en >> 10) & 0x3ffu), rep_rcp, rep, freq, pres);
-                            touched  = true;
-                        }
-                    }
-                } else {
-                    const unsigned *src = p.pre_list + (size_t) row * (size_t) p.row_cap;
-                    const int       lo = sl_off[s], hi = sl_off[s + 1], e_lo = sl_off[0];
-                    const bool      in_smem = sl_off[part_len] - e_lo <= kListSmem;
-                    for (int i = lo + lane; i < hi; i += 32) {
-                        const unsigned e  = in_smem ? sl_list[i - e_lo] : src[i];
-                        const int      li = (int) (e & ((1u << kLiBits) - 1u));
-                        if (li >= 4 * w4lo && li < 4 * (w4lo + mine4) && li < n) {
-                            sl[li - 4 * w4lo] = penalise_rcp(sl[li - 4 * w4lo], (int) (e >> kLiBits), rep_rcp, rep, freq, pres);
-                            touched           = true;
-                        }
+                const unsigned *ent;
+                int             lo, hi;
+                unsigned        tag;
+                ids_of(s, warp, ent, lo, hi, tag);
+                for (int e = lo + lane; e < hi; e += 32) {
+                    const unsigned en = ent[e];
+                    if (long_ids || (en >> 20) == tag) {
+                        float *q = sl + (en & 0x3ffu);
+                        *q       = penalise_rcp(*q, (int) ((en >> 10) & cnt_mask), rep_rcp, rep, freq, pres);
+                        touched  = true;
                     }
                 }
                 wrote |= __any_sync(0xffffffffu, touched); /* also orders the stores before the loads below */
@@ -2621,24 +2601,37 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
 
             /* ---- 3. the share in registers; what a thread does not own reads as -inf ---- */
             const float4 *s4 = reinterpret_cast<const float4 *>(sl) + lane;
-            float4        x[kNV4];
-            float         gm[kNV4]; /* maximum of each float4 group */
-            float         bv = -CUDART_INF_F;
-#pragma unroll
-            for (int i = 0; i < kNV4; i++) {
-                x[i]  = lane + 32 * i < mine4 ? s4[32 * i] : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
-                gm[i] = fmaxf(fmaxf(x[i].x, x[i].y), fmaxf(x[i].z, x[i].w));
-                bv    = fmaxf(bv, gm[i]);
-            }
-            CYC(1);
-            const unsigned bkey = order_key(bv + 0.0f); /* -0 and +0 are one value, as the comparison of floats has it */
-            const bool     own  = lane < mine4;
-            const unsigned wkey = __reduce_max_sync(0xffffffffu, own ? bkey : 0u);
-            const float    wmax = wkey == 0u ? -CUDART_INF_F : key_to_float(wkey);
-
+            /* the share has been read: the stage is free again and the warp refills it itself */
+            auto refill = [&]() {
+                __syncwarp();
+                if (lane == 0 && aligned && j + kStages < my_count && ring_dead < 0) {
+                    if (wrote) { /* ordinary stores of this warp come before the copy engine's */
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    }
+                    issue_next();
+                }
+            };
+            auto note_maxima = [&](int s_, float m0, float m1) {
+                top0          = fmaxf(top0, m0);
+                top1          = fmaxf(top1, m1);
+                float      *q = &gmax[(s_ >> gm_shift) * kThreads + tid];
+                const float m = fmaxf(m0, m1);
+                *q            = (s_ & ((1 << gm_shift) - 1)) == 0 ? m : fmaxf(*q, m);
+            };
             if (smode == M_ARGMAX) {
+                float4 x[kNV4];
+                float  bv = -CUDART_INF_F;
+#pragma unroll
+                for (int i = 0; i < kNV4; i++) {
+                    x[i] = lane + 32 * i < mine4 ? s4[32 * i] : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+                    bv   = max3(max3(bv, x[i].x, x[i].y), x[i].z, x[i].w);
+                }
+                const unsigned bkey = order_key(bv);
+                const bool     own  = lane < mine4;
+                const unsigned wkey = __reduce_max_sync(0xffffffffu, own ? bkey : 0u);
                 if (wkey > run_key) { /* rare: the warp's running maximum moves; its first id in this slice */
-                    int best = 0x7fffffff;
+                    const float wmax = key_to_float(wkey);
+                    int         best = 0x7fffffff;
                     if (own && bkey == wkey) {
 #pragma unroll
                         for (int i = kNV4 - 1; i >= 0; i--) {
@@ -2653,257 +2646,223 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                     run_key = wkey;
                     run_arg = s0 + best;
                 }
-            } else if (wkey > run_key) {
-                run_key = wkey; /* the maximum alone: no other mode asks where it is */
-            }
-
-            float tau = CUDART_INF_F;
-            if (sel) {
-                if (s == 0) {
-                    /* The part's first slice sets the threshold; all warps meet here (the only barriers inside a
-                     * part). The thread maxima (wide k: the float4 maxima) are binned by their ordered keys into 256
-                     * bins below the largest, and tau = the lower edge of the highest bin above which at least kq of
-                     * them lie: at least kq entries of this slice alone are >= tau, so tau cannot exceed the row's
-                     * kq-th largest value. Fewer than kq groups: everything passes. */
-                    const bool fine = kq > 64;
-                    float      gmin = bv;
-                    int        ng   = own ? 1 : 0;
-                    if (fine) {
-                        gmin = CUDART_INF_F;
-                        ng   = 0;
+                refill();
+            } else if (!sums) {
+                /* top-k: the largest value of the thread's floats is all that the select asks of a slice */
+                float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F;
+                if (mine4 == 32 * kNV4) {
 #pragma unroll
-                        for (int i = 0; i < kNV4; i++) {
-                            if (lane + 32 * i < mine4) {
-                                gmin = fminf(gmin, gm[i]);
-                                ng++;
-                            }
+                    for (int i = 0; i < kNV4; i++) {
+                        const float4 x = s4[32 * i];
+                        float       &m = i < kNV4 / 2 ? m0 : m1;
+                        m              = max3(max3(m, x.x, x.y), x.z, x.w);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kNV4; i++) {
+                        if (lane + 32 * i < mine4) {
+                            const float4 x = s4[32 * i];
+                            float       &m = i < kNV4 / 2 ? m0 : m1;
+                            m              = max3(max3(m, x.x, x.y), x.z, x.w);
                         }
                     }
-                    const unsigned wlow = __reduce_min_sync(0xffffffffu, own ? order_key(gmin + 0.0f) : 0xffffffffu);
-                    ng                  = __reduce_add_sync(0xffffffffu, ng);
-                    if (lane == 0) {
-                        sh->wkey[warp] = wkey;
-                        sh->wlow[warp] = wlow;
-                        sh->wown[warp] = ng;
-                    }
-                    __syncthreads();
-                    unsigned khi = 0u, klo = 0xffffffffu;
-                    int      n_own = 0;
-#pragma unroll
-                    for (int w = 0; w < kWarps; w++) {
-                        khi = max(khi, sh->wkey[w]);
-                        klo = min(klo, sh->wlow[w]);
-                        n_own += sh->wown[w];
-                    }
-                    /* values far below the largest all go to bin 0: the walk comes from the top */
-                    const unsigned klo2  = max(klo, khi > (1u << 27) ? khi - (1u << 27) : 0u);
-                    const unsigned span  = khi - klo2;
-                    const int      shift = max(0, (32 - __clz(span)) - 8); /* (span >> shift) < 256 */
-                    if (n_own >= kq) {
-                        if (fine) {
-#pragma unroll
-                            for (int i = 0; i < kNV4; i++) {
-                                if (lane + 32 * i < mine4) {
-                                    atomicAdd(&sh->bhist[(max(order_key(gm[i] + 0.0f), klo2) - klo2) >> shift], 1);
-                                }
-                            }
-                        } else {
-                            /* most thread maxima fall into a few low bins: the lanes of a warp that share a bin
-                             * add once for all of them */
-                            const int      bin   = own ? (int) ((max(bkey, klo2) - klo2) >> shift) : -1;
-                            const unsigned peers = __match_any_sync(0xffffffffu, bin);
-                            if (own && lane == __ffs(peers) - 1) {
-                                atomicAdd(&sh->bhist[bin], __popc(peers));
-                            }
-                        }
-                    }
-                    __syncthreads();
-                    unsigned tkey = 0u; /* below everything: all entries pass */
-                    if (n_own >= kq) { /* every warp reads the bins for itself */
-                        const int b = top_bin(sh->bhist, lane, kq);
-                        tkey        = b == 0 ? klo : klo2 + ((unsigned) b << shift); /* bin 0 also holds what was clamped */
-                    }
-                    tau_reg = tkey == 0u ? -CUDART_INF_F : key_to_float(tkey);
-                    /* the part's candidates are binned between tau and this slice's maximum; the bins are read from
-                     * the top to raise the threshold for the slices to come */
-                    const float top = key_to_float(khi);
-                    t_lo            = tau_reg;
-                    t_scale         = (n_own >= kq && top > tau_reg && top - tau_reg < CUDART_INF_F) ? (float) kHistBins / (top - tau_reg) : 0.0f;
                 }
-                CYC(7);
-                PROF_ONCE(7);
-                const unsigned pkey = *reinterpret_cast<volatile unsigned *>(&sh->tau_key);
-                tau                 = pkey == 0u ? tau_reg : fmaxf(tau_reg, key_to_float(pkey));
-                /* Candidates: the float4 groups whose maximum passes. Which of a thread's eight groups do is one bit
-                 * each; a lane that holds any takes them one after the other in ONE rolled loop (rarely run code
-                 * inside the hot loop is kept in one copy: it has to come from the instruction cache each time), the
-                 * values re-read from the stage. */
-                unsigned mybits = 0u;
+                refill();
+                note_maxima(s, m0, m1);
+            } else if constexpr ((kKinds & K_SUMS) != 0) {
+                float4 x[kNV4];
+                float  m0 = -CUDART_INF_F, m1 = -CUDART_INF_F;
 #pragma unroll
                 for (int i = 0; i < kNV4; i++) {
-                    mybits |= (gm[i] >= tau && lane + 32 * i < mine4) ? (1u << i) : 0u;
+                    x[i]     = lane + 32 * i < mine4 ? s4[32 * i] : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+                    float &m = i < kNV4 / 2 ? m0 : m1;
+                    m        = max3(max3(m, x[i].x, x[i].y), x[i].z, x[i].w);
                 }
-                if (__any_sync(0xffffffffu, mybits != 0u)) {
-                    /* every lane that holds candidates places its groups itself, the places counted in shared memory:
-                     * one pass whatever the number of lanes and groups (the order inside the list means nothing) */
-                    unsigned mb = mybits;
-                    while (mb != 0u) {
-                        const int i = __ffs(mb) - 1;
-                        mb &= mb - 1u;
-                        const float4 v   = s4[32 * i];
-                        const int    pos = atomicAdd(&sh->wcur[warp], 1);
-                        if (pos < kGroupCapWarp) {
-                            /* which of the four pass: the finisher takes those, the sums below leave those out */
-                            const unsigned cm = (v.x >= tau ? 1u : 0u) | (v.y >= tau ? 2u : 0u) | (v.z >= tau ? 4u : 0u) | (v.w >= tau ? 8u : 0u);
-                            seg_v[pos]        = v;
-                            seg_b[pos]        = (s0 + 4 * (w4lo + lane + 32 * i)) | (int) (cm << 28);
-                        }
-                        if (t_scale > 0.0f) {
-                            const float gmax = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
-                            atomicAdd(&sh->thist[min(kHistBins - 1, max(0, __float2int_rz((gmax - t_lo) * t_scale)))], 1);
-                        }
-                    }
-                    __syncwarp();
-                    const int now = *reinterpret_cast<volatile int *>(&sh->wcur[warp]);
-                    since += now - wcnt;
-                    wcnt = now;
+                refill();
+                /* the unit follows the maximum: a temperature row's terms stay below 1 (their sum is added up in fixed
+                 * point), a top-p row's may grow to 2^60 before the sums so far are moved */
+                if (__any_sync(0xffffffffu, __fmul_rn(fmaxf(m0, m1), ks.hi) > unit + (smode == M_TEMP ? 0.0f : 60.0f))) {
+                    const unsigned wk = __reduce_max_sync(0xffffffffu, order_key(fmaxf(m0, m1)));
+                    const float    u  = ceilf(__fmul_rn(key_to_float(wk), ks.hi));
+                    acc               = unit == kNoUnit ? 0.0 : acc * pow2_diff(unit, u);
+                    unit              = u;
                 }
-            }
-            CYC(2);
-            /* the stage is free again: the warp refills it itself */
-            __syncwarp();
-            if (lane == 0 && aligned && j + kStages < my_count && ring_dead < 0) {
-                if (wrote) { /* ordinary stores of this warp come before the copy engine's */
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                }
-                issue_next();
-            }
-            CYC(1);
-            if (sums) {
-                /* sum of e_i relative to the WARP's maximum of this slice (top-p: of what is in no candidate
-                 * group); -inf padding gives exp(-inf) = 0 */
-                const float ref = wmax == -CUDART_INF_F ? 0.0f : wmax;
-                const float k2  = inv_t * 1.4426950408889634f; /* e^(a / T) = 2^(a * log2(e) / T) */
-                double      sum = 0.0;
+                double sum = 0.0;
 #pragma unroll
                 for (int i = 0; i < kNV4; i++) {
-                    /* a candidate's argument becomes -inf (exp gives 0), so that the evaluations stay one straight
-                     * line and overlap */
-                    const float e0 = exp2_fast(x[i].x >= tau ? -CUDART_INF_F : (x[i].x - ref) * k2);
-                    const float e1 = exp2_fast(x[i].y >= tau ? -CUDART_INF_F : (x[i].y - ref) * k2);
-                    const float e2 = exp2_fast(x[i].z >= tau ? -CUDART_INF_F : (x[i].z - ref) * k2);
-                    const float e3 = exp2_fast(x[i].w >= tau ? -CUDART_INF_F : (x[i].w - ref) * k2);
-                    sum += (double) ((e0 + e1) + (e2 + e3));
+                    sum += (double) sum_terms(x[i], ks, unit);
                 }
-                sum = warp_sum_d(sum);
-                if (smode == M_TEMP) {
+                if (smode == M_TOPP) {
+                    acc += sum;
+                    if (lane == 0 && s < kSliceCs) {
+                        sh->c_at[s][warp] = unit;
+                    }
+                    note_maxima(s, m0, m1);
+                } else {
+                    /* the warp's sum in fixed point, 2^-42 of the largest possible term: two integer reductions
+                     * instead of five rounds of double additions between lanes */
+                    const long long q  = __double_as_longlong(sum + 0x1.8p10) & 0xfffffffffffffll;
+                    const unsigned  lo = __reduce_add_sync(0xffffffffu, (unsigned) q & 0x3ffffffu);
+                    const unsigned  hi = __reduce_add_sync(0xffffffffu, (unsigned) (q >> 26));
+                    top0               = fmaxf(top0, fmaxf(m0, m1));
                     if (lane == 0) {
                         SegRec sr;
-                        sr.ref = wmax;
+                        sr.ref = unit;
                         sr.pad = 0.0f;
-                        sr.sum = sum;
+                        sr.sum = ((double) hi - 32.0 * 0x1p25) * 0x1p-16 + (double) lo * 0x1p-42;
                         p.segs[((size_t) row * (size_t) p.n_slices + (size_t) c) * kWarps + warp] = sr;
                     }
-                } else if (wmax != -CUDART_INF_F) {
-                    if (wmax > b_ref) {
-                        b_sum = b_ref == -CUDART_INF_F ? 0.0 : b_sum * exp(((double) b_ref - (double) wmax) * (double) inv_t);
-                        b_ref = wmax;
-                    }
-                    b_sum += sum * exp(((double) wmax - (double) b_ref) * (double) inv_t);
-                }
-            }
-            if (sel && since >= 8 && t_scale > 0.0f) {
-                /* after a few new candidates of its own the warp looks whether the threshold can go up: the lowest
-                 * bin edge above which at least kq candidates lie, one bin lower to be safe against rounding */
-                since  = 0;
-                int go = 0;
-                if (lane == 0) {
-                    go = atomicCAS(&sh->tau_lock, 0, 1) == 0 ? 1 : 0;
-                }
-                go = __shfl_sync(0xffffffffu, go, 0);
-                if (go) {
-                    const int b = top_bin(sh->thist, lane, kq);
-                    if (lane == 0) {
-                        if (b >= 2) {
-                            const float t_new = t_lo + (float) (b - 1) / t_scale;
-                            if (t_new > t_lo) {
-                                atomicMax(&sh->tau_key, order_key(t_new));
-                            }
-                        }
-                        __threadfence_block();
-                        sh->tau_lock = 0;
-                    }
-                }
-            }
-            if ((kKinds & K_SEL) != 0 && smode == M_TOPK && wcnt > kSqueezeAt && wcnt <= kGroupCapWarp) {
-                /* The threshold has gone up since most of the warp's groups were taken: those whose maximum has
-                 * fallen below it cannot hold one of the row's kq largest any more and leave the list (top-k rows
-                 * only: a top-p row's candidates were left out of its sums and must all arrive). Without this a
-                 * wide k fills a warp's list before the row is through. */
-                const unsigned pk    = *reinterpret_cast<volatile unsigned *>(&sh->tau_key);
-                const float    tau_c = pk == 0u ? tau_reg : fmaxf(tau_reg, key_to_float(pk));
-                if (tau_c > sh->wsq[warp]) {
-                    int kept = 0;
-                    for (int base = 0; base < wcnt; base += 32) {
-                        const int j    = base + lane;
-                        float4    v    = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        int       bb   = 0;
-                        bool      keep = false;
-                        if (j < wcnt) {
-                            v    = seg_v[j];
-                            bb   = seg_b[j];
-                            keep = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) >= tau_c;
-                        }
-                        const unsigned m = __ballot_sync(0xffffffffu, keep); /* every lane has read its entry before any is overwritten */
-                        if (keep) {
-                            const int pos = kept + __popc(m & lt);
-                            seg_v[pos]    = v;
-                            seg_b[pos]    = bb;
-                        }
-                        kept += __popc(m);
-                        __syncwarp();
-                    }
-                    wcnt = kept;
-                    if (lane == 0) {
-                        sh->wcur[warp] = kept;
-                        sh->wsq[warp] = tau_c;
-                    }
-                    __syncwarp();
                 }
             }
             CYC(2);
         }
 
         PROF(2);
-        /* ---- the part is through: one record and the candidate groups go to global scratch ---- */
+        /* ---- the part is through ---- */
         wst = __reduce_or_sync(0xffffffffu, (unsigned) wst);
+        if (smode != M_ARGMAX) {
+            run_key = __reduce_max_sync(0xffffffffu, order_key(fmaxf(top0, top1)));
+        }
+        if ((kKinds & K_SUMS) != 0 && smode == M_TOPP && sums) {
+            acc = warp_sum_d(acc);
+        }
         if (lane == 0) {
             sh->best[warp]   = ((unsigned long long) run_key << 32) | (unsigned long long) (0xffffffffu - (unsigned) run_arg);
-            sh->wn[warp]     = min(wcnt, kGroupCapWarp);
-            sh->wn_all[warp] = wcnt;
-            sh->wb_ref[warp] = b_ref;
-            sh->wb_sum[warp] = b_sum;
+            sh->wb_c[warp]   = unit;
+            sh->wb_sum[warp] = acc;
             if (wst != 0) {
                 atomicOr(&sh->st, wst);
             }
         }
-        __syncthreads();
-        int held = 0;
+        float tau = CUDART_INF_F;
+        if (sel) {
+            /*
+             * The threshold: the kq-th largest (or one a little below) of the 256 thread maxima, a lower bound of the
+             * part's kq-th largest value that lies close to it (k of 256 threads hold about k + k^2 / 512 of the
+             * values above it; beyond k = 128 the 512 half maxima are asked). Found by building its key from the top
+             * bit down, each step counting the threads that reach it: a dozen short barriers, no memory.
+             * Against capturing candidates above a rising threshold while the part streams (465 instead of about 100
+             * instructions per warp and slice, two barriers and shared-memory atomics inside the part): 256 x 128256
+             * top-k 40 with penalties 33.2 -> 32.2 us, 4096 x 128256 top-k 50 549 -> 541 us, 256 x 262144 top-p
+             * 97.0 -> 85.2 us with the sums' new form, 48 x 262144 soft-capped top-k 64 116 -> 104 us a step.
+             */
+            const unsigned key0 = order_key(kq <= kThreads / 2 ? fmaxf(top0, top1) : top0), key1 = kq <= kThreads / 2 ? 0u : order_key(top1);
+            unsigned       tkey = 0u;
+            for (int bit = 31; bit >= 0; bit--) {
+                const unsigned t = tkey | (1u << bit);
+                int            n = __syncthreads_count(key0 >= t);
+                if (kq > kThreads / 2) {
+                    n += __syncthreads_count(key1 >= t);
+                }
+                if (n >= kq) {
+                    tkey = t;
+                    if (n <= kq + kq / 8) {
+                        break;
+                    }
+                }
+            }
+            tau = tkey <= order_key(-CUDART_INF_F) ? -CUDART_INF_F : key_to_float(tkey); /* fewer than kq of them: everything passes */
+            /* the thread's groups that reach it */
+            const int slots = ((part_len - 1) >> gm_shift) + 1;
+#pragma unroll 4
+            for (int i = 0; i < slots; i++) {
+                if (gmax[i * kThreads + tid] >= tau) {
+                    const int pos = atomicAdd(&sh->n_grp, 1);
+                    if (pos < kPartCand) {
+                        sh->grp[pos] = (unsigned short) ((i << 8) | tid);
+                    }
+                }
+            }
+            __syncthreads();
+            /* their float4, read again (L2 holds them), changed as they were while the part streamed */
+            const int n_grp = min(sh->n_grp, kPartCand), per_log = kNV4Log + gm_shift;
+            double    fix   = 0.0;
+            for (int t = tid; t < n_grp << per_log; t += kThreads) {
+                const int  name = sh->grp[t >> per_log], f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
+                const int  s = ((name >> 8) << gm_shift) + f / kNV4, c = c0 + s, i4 = l + 32 * (f % kNV4);
+                const bool last_c = c == p.n_slices - 1;
+                const int  n = last_c ? n_last : n_full, nv4 = (n + 3) >> 2, L = share_len(nv4), w4 = min(w * L, nv4);
+                if (s >= part_len || i4 >= min(L, nv4 - w4)) {
+                    continue;
+                }
+                const int    e0  = 4 * (w4 + i4), id0 = c * p.slice + e0;
+                const float *src = p.logits + (size_t) row * (size_t) p.row_stride + id0;
+                float        v[4];
+                if (aligned && e0 + 4 <= n) {
+                    const float4 q = *reinterpret_cast<const float4 *>(src);
+                    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+                } else {
 #pragma unroll
-        for (int w = 0; w < kWarps; w++) {
-            held += sh->wn[w];
+                    for (int q = 0; q < 4; q++) {
+                        v[q] = e0 + q < n ? src[q] : -CUDART_INF_F;
+                    }
+                }
+                if (pro_on) {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (e0 + q < n) {
+                            v[q] = prologue_one(v[q], id0 + q, sh->cap, sh->mrow);
+                        }
+                    }
+                }
+                if (pen_on) {
+                    const unsigned *ent;
+                    int             lo, hi;
+                    unsigned        tag;
+                    ids_of(s, w, ent, lo, hi, tag);
+                    for (int e = lo; e < hi; e++) {
+                        const unsigned en = ent[e];
+                        if ((int) ((en & 0x3ffu) >> 2) == i4 && (long_ids || (en >> 20) == tag)) {
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                if ((int) (en & 3u) == q) {
+                                    v[q] = penalise_rcp(v[q], (int) ((en >> 10) & cnt_mask), rep_rcp, rep, freq, pres);
+                                }
+                            }
+                        }
+                    }
+                }
+                bool any = false;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (v[q] >= tau && e0 + q < n) {
+                        const int pos = atomicAdd(&sh->n_cand, 1);
+                        if (pos < kPartCand) {
+                            sh->cand[pos].v   = v[q];
+                            sh->cand[pos].idx = id0 + q;
+                        }
+                        any = true;
+                    }
+                }
+                if ((kKinds & K_SUMS) != 0 && sums && any) {
+                    /* a candidate's weight is evaluated exactly where the row is finished: it leaves the sum, as the
+                     * term of its float4 entered it, and what shares its float4 comes back one by one */
+                    const float u   = s < kSliceCs ? sh->c_at[s][w] : sh->wb_c[w];
+                    double      now = -(double) sum_terms(make_float4(v[0], v[1], v[2], v[3]), ks, u);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (!(v[q] >= tau)) {
+                            now += (double) sum_term(v[q], ks, u);
+                        }
+                    }
+                    fix += now * pow2_diff(u, sh->wb_c[w]) * pow2_diff(sh->wb_c[w], unit_max(sh));
+                }
+            }
+            if ((kKinds & K_SUMS) != 0 && sums) {
+                fix = warp_sum_d(fix);
+                if (lane == 0) {
+                    sh->fix[warp] = fix;
+                }
+            }
         }
+        __syncthreads();
+        const int n_cand = sh->n_grp > kPartCand ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
+        const int held   = sel ? min(n_cand, kPartCand) : 0;
         if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
             /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
              * part); a row of another kind is reported as the small finishing kernel would */
             if (mode == M_TOPK) {
-                int n_all = 0;
-#pragma unroll
-                for (int w = 0; w < kWarps; w++) {
-                    n_all += sh->wn_all[w];
-                }
-                const unsigned pkey = sh->tau_key;
-                inline_finish_topk(p, sh, grp_v, grp_b, row, held, held == n_all, pkey == 0u ? tau_reg : fmaxf(tau_reg, key_to_float(pkey)), kq, inv_t, sh->st);
+                inline_finish_topk(p, sh, row, n_cand, kq, inv_t, sh->st);
             } else {
                 if (tid == 0) {
                     p.tokens[row] = -1;
@@ -2915,37 +2874,32 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             continue;
         }
         if (tid == 0) {
-            unsigned long long bw    = 0ull;
-            int                n_all = 0;
-            float              bref  = -CUDART_INF_F;
+            unsigned long long bw = 0ull;
 #pragma unroll
             for (int w = 0; w < kWarps; w++) {
                 bw = max(bw, sh->best[w]);
-                n_all += sh->wn_all[w];
-                bref = fmaxf(bref, sh->wb_ref[w]);
             }
+            float  bc   = kNoUnit;
             double bsum = 0.0;
-            if (mode == M_TOPP && sel) {
+            if ((kKinds & K_SUMS) != 0 && smode == M_TOPP && sums) {
+                bc = unit_max(sh);
 #pragma unroll
                 for (int w = 0; w < kWarps; w++) {
-                    const float wr = sh->wb_ref[w];
-                    if (wr != -CUDART_INF_F) {
-                        bsum += sh->wb_sum[w] * exp(((double) wr - (double) bref) * (double) inv_t);
-                    }
+                    bsum += (sh->wb_c[w] == kNoUnit ? 0.0 : sh->wb_sum[w] * pow2_diff(sh->wb_c[w], bc)) + sh->fix[w];
                 }
+                bsum = fmax(bsum, 0.0);
             }
-            const unsigned pkey = sh->tau_key;
             int4           h, h2;
             h.x  = __float_as_int((unsigned) (bw >> 32) == 0u ? -CUDART_INF_F : key_to_float((unsigned) (bw >> 32)));
             h.y  = (int) (0xffffffffu - (unsigned) (bw & 0xffffffffull));
-            h.z  = held == n_all ? n_all : kPartGroups + 1; /* a warp ran out of room for its groups */
+            h.z  = sel ? n_cand : 0;
             h.w  = sh->st;
-            h2.x = __float_as_int(pkey == 0u ? tau_reg : fmaxf(tau_reg, key_to_float(pkey)));
-            h2.y = __float_as_int(bref);
+            h2.x = __float_as_int(sel ? tau : -CUDART_INF_F);
+            h2.y = __float_as_int(bc);
             h2.z = __double2loint(bsum);
             h2.w = __double2hiint(bsum);
-            int4 *rec = reinterpret_cast<int4 *>(p.grp_v + ((size_t) row * (size_t) p.parts_max + (size_t) part_idx) * (size_t) kPartSlots);
-            rec[0]    = h; /* the part's record takes the first two slots of its group list */
+            int4 *rec = part_rec(p, row, part_idx);
+            rec[0]    = h; /* the record lies in front of the part's candidates */
             rec[1]    = h2;
             if ((p.flags & (F_GREEDY_ONLY | F_INLINE_TOPK)) != 0u) { /* in a launch that finishes its top-k rows here, the greedy ones are finished here as well */
                 /* The caller said that every row is greedy: no finishing kernel follows. A row that went through
@@ -2963,7 +2917,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                         float m       = -CUDART_INF_F;
                         best_arg      = 0x7fffffff;
                         for (int q = 0; q < n_parts; q++) {
-                            const int4 o = __ldcg(reinterpret_cast<const int4 *>(p.grp_v + ((size_t) row * (size_t) p.parts_max + (size_t) q) * (size_t) kPartSlots));
+                            const int4 o = __ldcg(part_rec(p, row, q));
                             stq |= o.w;
                             if (pair_before(__int_as_float(o.x), o.y, m, best_arg)) {
                                 m        = __int_as_float(o.x);
@@ -2990,11 +2944,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 }
             }
         }
-        const size_t at = ((size_t) row * (size_t) p.parts_max + (size_t) part_idx) * (size_t) kPartSlots + 2;
-        for (int f = tid; f < held; f += kThreads) {
-            const int slot  = own_slot(sh, f);
-            p.grp_v[at + f] = grp_v[slot];
-            p.grp_b[at + f] = grp_b[slot];
+        {
+            unsigned long long *dst = reinterpret_cast<unsigned long long *>(part_rec(p, row, part_idx)) + 4;
+            for (int f = tid; f < held; f += kThreads) {
+                dst[f] = *reinterpret_cast<const unsigned long long *>(&sh->cand[f]);
+            }
         }
         __syncthreads(); /* the lists are free for the next part */
         CYC(6);
@@ -3081,7 +3035,7 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
                 if (slot < 0) {
                     st = (st & ~ST_DEFERRED) | ST_INTERNAL;
                 } else {
-                    st = (st & ~ST_DEFERRED) | multipass_row(g, p, &sh->gs, r, bm, ba, cmem, kFinBytes, slot, &sh->st_v[0][0]); /* the staging of the parts' first slots is free by now: 3 KB of it keep a histogram */
+                    st = (st & ~ST_DEFERRED) | multipass_row(g, p, &sh->gs, r, bm, ba, cmem, kFinBytes, slot, sh->save);
                     __syncthreads();
                     if (g.tid == 0) {
                         __threadfence();
@@ -3102,20 +3056,30 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
 
 constexpr int kRowIdThreads = 256;
 
+/* Which (slice, warp) share a column lies in, and where in it. */
+__device__ __forceinline__ int share_of(const SampleParams &p, int id, int &off) {
+    const int c = id / p.slice, local = id - c * p.slice;
+    const int L = share_len((min(p.slice, p.V - c * p.slice) + 3) >> 2);
+    const int w = (local >> 2) / L;
+    off         = local - 4 * w * L;
+    return c * kWarps + w;
+}
+
 /* One CTA per row whose history (plus fed tokens) is longer than the stream kernel counts
- * by itself: the row's distinct ids with their counts, grouped by the slice they fall into.
- * pre_off[row][c] .. pre_off[row][c + 1] is slice c's run in pre_list[row]; an entry is
- * (position in the slice) | (count << kLiBits). Shorter rows are left to the stream kernel. */
+ * by itself: the row's distinct ids with their counts, grouped by the (slice, warp) share they fall into.
+ * pre_off[row][g] .. pre_off[row][g + 1] is share g's run in pre_list[row]; an entry is
+ * (offset in the share) | (count << 10). Shorter rows are left to the stream kernel. */
 __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_constant__ SampleParams p) {
     extern __shared__ __align__(16) int row_ids_smem[];
     int *tkey = row_ids_smem;          /* open-addressing table: the id ... */
     int *tcnt = tkey + p.id_slots;     /* ... and how often it occurs */
-    int *bcnt = tcnt + p.id_slots;     /* entry c + 1: distinct ids in slice c; after the scan, entry c: ids in slices < c */
-    int *bpos = bcnt + p.bucket_cap;   /* next free place of each slice's run */
+    int *bcnt = tcnt + p.id_slots;     /* entry g + 1: distinct ids in share g; after the scan, entry g: ids in the shares before */
+    int *bpos = bcnt + p.bucket_cap;   /* next free place of each share's run */
 
     /* the stream kernel behind this one may start now: it copies logits and sets itself up while the
      * lists are made, and waits for them where it first needs one */
     asm volatile("griddepcontrol.launch_dependents;");
+    const int n_shares = p.n_slices * kWarps;
     const int row  = (int) blockIdx.x, tid = (int) threadIdx.x;
     const int seq0 = p.rows_per_seq == 1 ? row : row / p.rows_per_seq;
     const int seq  = p.slot ? p.slot[seq0] : seq0;
@@ -3130,7 +3094,7 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
         tkey[i] = -1;
         tcnt[i] = 0;
     }
-    for (int i = tid; i <= p.n_slices; i += kRowIdThreads) {
+    for (int i = tid; i <= n_shares; i += kRowIdThreads) {
         bcnt[i] = 0;
     }
     __syncthreads();
@@ -3144,7 +3108,8 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
                 if (old == -1 || old == id) {
                     atomicAdd(&tcnt[hsh], 1);
                     if (old == -1) {
-                        atomicAdd(&bcnt[id / p.slice + 1], 1);
+                        int off;
+                        atomicAdd(&bcnt[share_of(p, id, off) + 1], 1);
                     }
                     break;
                 }
@@ -3154,11 +3119,11 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
     }
     __syncthreads();
     if (tid < 32) {
-        int *off   = p.pre_off + (size_t) row * (size_t) (p.n_slices + 1);
+        int *off   = p.pre_off + (size_t) row * (size_t) (n_shares + 1);
         int  carry = 0;
-        for (int base = 0; base <= p.n_slices; base += 32) {
+        for (int base = 0; base <= n_shares; base += 32) {
             const int i    = base + tid;
-            int       incl = i <= p.n_slices ? bcnt[i] : 0;
+            int       incl = i <= n_shares ? bcnt[i] : 0;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const int up = __shfl_up_sync(0xffffffffu, incl, d);
@@ -3166,7 +3131,7 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
                     incl += up;
                 }
             }
-            if (i <= p.n_slices) {
+            if (i <= n_shares) {
                 bcnt[i] = carry + incl;
                 bpos[i] = carry + incl;
                 off[i]  = carry + incl;
@@ -3179,9 +3144,9 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
     for (int i = tid; i < p.id_slots; i += kRowIdThreads) {
         const int id = tkey[i];
         if (id >= 0) {
-            const int c   = id / p.slice;
-            const int pos = atomicAdd(&bpos[c], 1);
-            list[pos]     = (unsigned) (id - c * p.slice) | ((unsigned) tcnt[i] << kLiBits);
+            int       off;
+            const int pos = atomicAdd(&bpos[share_of(p, id, off)], 1);
+            list[pos]     = (unsigned) off | ((unsigned) tcnt[i] << 10);
         }
     }
 }
@@ -3199,7 +3164,6 @@ extern "C" int geist_b200_debug_cyc(long long *out) { return (int) cudaMemcpyFro
 size_t sample_stream_smem(int n_slices, int long_ids) {
     size_t b = (size_t) kWarps * kStages * kWarpStageBytes + sizeof(StreamShared) + (size_t) kGroupBytes;
     if (long_ids) {
-        b += (((size_t) n_slices + 1) * 4 + 15) & ~(size_t) 15;
         b += (size_t) kListSmem * 4;
     }
     return b;

@@ -460,3 +460,18 @@ def test_history_sizes_up_to_the_limit(ctx):
         check_tokens(g, o)
     with pytest.raises(api.GeistError):
         run_gpu(ctx, x, 0.0, 0, 1.0, st, rep=1.3, history=histories(rows, 9000, V, 8504))
+
+
+@pytest.mark.parametrize("k", [2, 127, 128, 129, 255, 256])
+@pytest.mark.parametrize("V", [513, 1027, 8200, 33001])
+def test_select_widths_around_the_half_maxima(ctx, k, V):
+    """Up to k = 128 the threshold comes from one maximum per thread, beyond from two; rows with fewer groups than k let
+    everything pass; values that repeat put many entries on the threshold."""
+    rows = 8
+    x = normal_logits(rows, V, 2.5, 7 * V + k)
+    x[::2] = np.round(x[::2] * 4) / 4
+    st = independent_states(oracle.port, V + k, rows)
+    g = run_gpu(ctx, x, 0.9, k, 1.0, st, kept_cap=256)
+    o = oracle.port.sample_batch(x, 0.9, k, 1.0, st)
+    check_tokens(g, o)
+    assert (g["kept_n"] == min(k, V)).all() or k >= V

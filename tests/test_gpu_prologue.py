@@ -305,3 +305,30 @@ def test_stream_kernel_finishes_whole_rows_itself(ctx):
     sv = independent_states(oracle.port, 779, S)
     g = run_gpu(ctx, xv, 0.9, 50, 1.0, sv, rows_per_seq=R, finish_hint=api.FINISH_GREEDY_TOPK)
     check_tokens(g, oracle.port.sample_batch(xv, 0.9, 50, 1.0, sv, rows_per_seq=R))
+
+
+@pytest.mark.parametrize("c,sigma,shiftx", [(30.0, 3.0, 0.0), (30.0, 12.0, 0.0), (5.0, 2.0, 20.0), (1.0, 4.0, 0.0), (30.0, 2.0, -40.0), (1e6, 3.0, 0.0)])
+@pytest.mark.parametrize("hint", [0, 1])
+def test_softcap_after_the_select_equals_softcap_before(ctx, c, sigma, shiftx, hint):
+    """Top-k rows without ids are selected from uncapped logits and capped afterwards. Asking for the capped logits makes
+    the launch cap every logit while it streams, with the same device functions: tokens and kept sets are the same ones,
+    from the linear range of the cap to where it saturates and thousands of values are equal."""
+    rows, V = 24, 33001
+    x = normal_logits(rows, V, sigma, 61) + np.float32(shiftx)
+    x[::4, ::3] = -np.inf
+    x[3] = np.inf
+    x[3, 500:] = 0.0
+    st = independent_states(oracle.port, 61, rows)
+    K = np.resize(np.array([2, 40, 64, 200], np.int32), rows)
+    mask = np.random.default_rng(62).random((rows, V)) < 0.5
+    for extra in ({}, {"logit_mask": to_dev(mask_words(mask))}):
+        for cap in (0, 256):
+            late = run_gpu(ctx, x, 0.8, K, 1.0, st, softcap=cap_dev(rows, c), kept_cap=cap, finish_hint=hint if cap == 0 else 0, **extra)
+            full = run_gpu(ctx, x, 0.8, K, 1.0, st, softcap=cap_dev(rows, c), kept_cap=cap, want_logits=True, **extra)
+            done = (late["status"] & api.ROW_RETRY) == 0
+            assert done.any() or hint
+            assert np.array_equal(late["tokens"][done], full["tokens"][done])
+            if cap:
+                both = ((late["status"] | full["status"]) & api.ROW_KEPT_PARTIAL) == 0
+                for name in ("kept_n", "kept_idx", "kept_prob"):
+                    assert np.array_equal(late[name][both], full[name][both]), name

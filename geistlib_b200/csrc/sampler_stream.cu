@@ -1842,6 +1842,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 break;
             }
             bin_scale = (float) kHistBins / (row_max - tau_row);
+            g.sync(); /* every thread has read n_ent: the next pass puts it back to zero */
         }
         PROF(10);
         if (total > kFinCap || total < r.kq) {

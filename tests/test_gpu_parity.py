@@ -475,3 +475,20 @@ def test_select_widths_around_the_half_maxima(ctx, k, V):
     o = oracle.port.sample_batch(x, 0.9, k, 1.0, st)
     check_tokens(g, o)
     assert (g["kept_n"] == min(k, V)).all() or k >= V
+
+
+@pytest.mark.parametrize("rows,V", [(1, 151936), (2, 131072), (18, 128256)])
+@pytest.mark.parametrize("k", [100, 200, 256])
+def test_wide_sets_merged_from_many_parts(ctx, rows, V, k):
+    """A row cut into many parts, each with at least k candidates of its own: more than the finisher can order at once
+    (2048), so it bins them and takes them in again. The second half of the batch has its values on a grid of 1/8: the
+    bin that holds the k-th is full of ties."""
+    x = normal_logits(rows, V, 2.5, V + k)
+    x[rows // 2:] = np.round(x[rows // 2:] * 8) / 8
+    st = independent_states(oracle.port, V + k, rows)
+    g = run_gpu(ctx, x, 0.9, k, 1.0, st, kept_cap=256)
+    o = oracle.port.sample_batch(x, 0.9, k, 1.0, st, detail_cap=256)
+    check_tokens(g, o)
+    listed = (g["status"] & 8) == 0
+    for r in np.nonzero(listed)[0]:
+        assert np.array_equal(g["kept_idx"][r, :k], o["detail_idx"][r, :k])

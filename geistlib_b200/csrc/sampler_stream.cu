@@ -2311,6 +2311,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         if (b4 > 0) {
             mbar_expect_tx(&sh->full[warp][stage], (unsigned) b4 * 16u);
             bulk_g2s(wring + (size_t) stage * kWarpStageBytes, isrc + 4 * (last ? w4lo_l : w4lo_f), (unsigned) b4 * 16u, &sh->full[warp][stage]);
+        } else {
+            /* Every item moves its stage's barrier on by one phase, also one of which the warp owns nothing: the waits
+             * below go by the item's number. A share can be empty in one of the two slice shapes alone (V = 18436:
+             * the last warp owns no float4 of a full slice and 191 of the row's last one). */
+            mbar_arrive(&sh->full[warp][stage]);
         }
         ijj++;
         ic++;
@@ -2551,10 +2556,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             CYC(4);
             /* ---- 1. the warp's share of the slice is in its stage; the slice's tail is padded with -inf ---- */
             if (aligned) {
-                const int full4 = last_c ? bulk4_l : bulk4_f;
                 if (ring_dead >= 0) {
                     wst |= ST_LOAD_TIMEOUT; /* every row the warp still touches is reported as not loaded */
-                } else if (full4 > 0 && !mbar_wait_bounded(&sh->full[warp][stage], parity)) {
+                } else if (!mbar_wait_bounded(&sh->full[warp][stage], parity)) {
                     wst |= ST_LOAD_TIMEOUT;
                     ring_dead = j; /* the warp asks for no further copy and waits for none; see the kernel's end */
                 }

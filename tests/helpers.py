@@ -63,3 +63,15 @@ def rel_err(a, b):
     a = np.asarray(a, np.float64)
     b = np.asarray(b, np.float64)
     return np.max(np.abs(a - b) / np.maximum(np.abs(b), 1e-30)) if a.size else 0.0
+
+
+def slice_shares(V):
+    """How a row is cut: per slice shape (full, last), how many whole float4 each of the eight warps owns of it."""
+    n_slices = -(-V // 8192)
+    full = -(-(-(-V // n_slices)) // 4) * 4 if n_slices > 1 else V
+    out = []
+    for n in (full, V - (n_slices - 1) * full):
+        nv4 = -(-n // 4)
+        per = (-(-nv4 // 8) + 31) // 32 * 32
+        out.append([max(0, min(per, nv4 - w * per, n // 4 - w * per)) for w in range(8)])
+    return n_slices, out

@@ -1,6 +1,8 @@
 """Host-side checks of arithmetic identities that the kernels rely on (no GPU)."""
 import numpy as np
 
+from helpers import slice_shares
+
 
 def test_float_division_as_double_product_with_the_reciprocal():
     """The stream kernel's penalty loop computes x / rep as float(double(x) * (1.0 / double(rep))), which keeps the
@@ -30,3 +32,14 @@ def test_float_division_as_double_product_with_the_reciprocal():
             qf = a / ys
             qp = (np.float64(a) * (1.0 / ys.astype(np.float64))).astype(np.float32)
         assert np.array_equal(qf.view(np.uint32), qp.view(np.uint32)), (a, qf, qp)
+
+
+def test_vocabularies_whose_shares_differ_in_emptiness():
+    """The vocabularies below 28672 (on the 16-byte grid, three slices and more) where a warp owns something of one slice
+    shape and nothing of the other: the GPU tests of the copy ring are run on sizes out of this list."""
+    got = []
+    for V in range(16388, 28672, 4):
+        _, (full, last) = slice_shares(V)
+        if any((a == 0) != (b == 0) for a, b in zip(full, last)):
+            got.append(V)
+    assert got == [18436, 18440, 18448, 18820, 18824, 18832, 24580, 24584, 24588, 24596, 24600, 24612, 25092, 25096, 25100, 25108, 25112, 25124]

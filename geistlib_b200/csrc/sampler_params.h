@@ -29,7 +29,7 @@ constexpr int kHistBins     = 256;            /* value histograms (threshold, se
 constexpr int kGroupSlots   = 16;             /* group maxima a thread keeps of one row part */
 constexpr int kPartCand     = 1024;           /* candidates that one row part can hand on */
 constexpr int kPartBytes    = 32 + kPartCand * 8; /* a part in global scratch: its record, then its candidates */
-constexpr int kSliceCs      = 32;             /* slices of a part whose units are remembered */
+constexpr int kSliceRefs    = 32;             /* slices of a part whose references are remembered in shared memory */
 constexpr int kRowIds       = 256;            /* ids of a row (history + fed tokens) counted inside the stream kernel, one per thread */
 
 /* status word, one per row (bit set) */
@@ -62,15 +62,15 @@ struct __align__(16) PartRec {
     int    n_cand;   /* candidates this part found (more than kPartCand: some were dropped) */
     int    st;       /* status bits raised while the part streamed */
     float  tau;      /* the part's final select threshold: a lower bound of the row's kq-th largest value */
-    float  bulk_c;   /* top-p: the sum below is in units of 2^bulk_c ... */
-    double bulk_sum; /* ... sum of 2^(x * log2(e) / T) over everything that is no candidate */
+    float  bulk_ref; /* top-p: the sum below is relative to this value ... */
+    double bulk_sum; /* ... sum of e^((x - bulk_ref) / T) over everything that is no candidate */
 };
 
 /* Temperature rows: one warp's share of one slice, ids in order. */
 struct __align__(16) SegRec {
-    float  ref;  /* the sum is in units of 2^ref (a whole number, at least that of the segment's maximum); kNoUnit: nothing there */
+    float  ref;  /* maximum of the segment */
     float  pad;
-    double sum;  /* sum of 2^(x * log2(e) / T) over the segment */
+    double sum;  /* sum of e^((x - ref) / T) over the segment */
 };
 
 /* Which (row, slice) items a thread block of the stream kernel takes: always one contiguous run of the row-major

@@ -14,7 +14,7 @@
  *   floats of every slice (a group) and its maximum over the part: nothing else of the select happens while the
  *   part streams. When it is through, the kq-th largest of the 256 thread maxima is a threshold that k and a few
  *   more values of the part reach; the few dozen groups that hold them are read again. Temperature rows sum
- *   2^(x * log2(e) / T) per warp and slice, top-p rows per thread over the part.
+ *   e^((x - maximum) / T) per warp and slice, top-p rows per thread over the part.
  *
  *   Before any of this a row's share may pass the soft cap tanhf(x / c) * c and the mask of allowed columns,
  *   in place in the stage (head.c:145-159; only launches that carry one pay for it).
@@ -382,27 +382,29 @@ __device__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const Ro
 
 /* ------------------------------------------------------- sums over a row -- */
 
-/* The sums of temperature and top-p rows are formed of 2^(x * scale - c), scale = log2(e) / T in two floats (their sum is
- * good to 2^-48) and c a whole number near the largest x * scale: one rounding of the argument at the size of the
- * difference, whatever the size of x, and changing c moves a sum by a power of two, exactly. The high float is
- * rounded down so that both products of an x of -inf are -inf. */
-constexpr float kNoUnit = -1e30f; /* c before anything finite has been met */
+/* The sums of temperature and top-p rows are formed of 2^((x - ref) * scale), ref a value of the row and scale =
+ * log2(e) / T in two floats (their sum is good to 2^-48): the difference comes first, so a term's argument is rounded at
+ * its own size, whatever the sizes of x and T. The high float is rounded down, both are at least the
+ * smallest float and the low one is finite, so that an x of -inf (which pads a row) gives 0 and the x that is ref gives
+ * 1 at every T whose inverse is finite. */
 __device__ __forceinline__ double sum_scale(float inv_t) { return (double) inv_t * 1.4426950408889634; }
 struct SumScale {
     float hi, lo;
 };
 __device__ __forceinline__ SumScale sum_scale2(float inv_t) {
     SumScale k;
-    k.hi = __double2float_rz(sum_scale(inv_t));
-    k.lo = fmaxf(__double2float_rn(sum_scale(inv_t) - (double) k.hi), 1e-37f);
+    const float hi = __double2float_rz(sum_scale(inv_t));
+    k.hi           = fmaxf(hi, 0x1p-149f);
+    k.lo           = fminf(fmaxf(__double2float_rn(sum_scale(inv_t) - (double) hi), 0x1p-149f), 3.4028235e38f);
     return k;
 }
-__device__ __forceinline__ float sum_term(float x, const SumScale &k, float c) { return exp2_fast(__fmaf_rn(x, k.lo, __fmaf_rn(x, k.hi, -c))); }
-__device__ __forceinline__ float sum_unit(float m, float inv_t) { return m == -CUDART_INF_F ? kNoUnit : ceilf(__fmul_rn(m, sum_scale2(inv_t).hi)); }
-/* 2^(a - b) for whole numbers, 0 below the range of double */
-__device__ __forceinline__ double pow2_diff(float a, float b) {
-    const double d = (double) a - (double) b;
-    return d < -1022.0 ? 0.0 : __longlong_as_double((long long) (1023 + (int) fmin(d, 1023.0)) << 52);
+__device__ __forceinline__ float sum_term(float x, const SumScale &k, float ref) {
+    const float d = __fsub_rn(x, ref);
+    return exp2_fast(__fmaf_rn(d, k.lo, __fmul_rn(d, k.hi)));
+}
+/* what a sum relative to `from` is multiplied with to be relative to `to`; nothing has been summed relative to -inf */
+__device__ __forceinline__ double ref_move(float from, float to, float inv_t) {
+    return from == -CUDART_INF_F ? 0.0 : exp(((double) from - (double) to) * (double) inv_t);
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
@@ -1244,10 +1246,9 @@ struct __align__(16) StreamShared {
     /* the part in work */
     int                st;        /* status bits of the part */
     unsigned long long best[kWarps];               /* (key of the maximum, ~first id) per warp */
-    float              wb_c[kWarps];               /* temperature / top-p: the warp's sums are in units of 2^wb_c ... */
-    double             wb_sum[kWarps];             /* ... and top-p's sum over the part */
-    float              c_at[kSliceCs][kWarps];     /* top-p: the unit that a slice's terms were formed in */
-    double             fix[kWarps];                /* top-p: what the candidates' leaving changes in that sum */
+    float              wb_ref[kWarps];             /* top-p: what the warp's sum is relative to ... */
+    double             wb_sum[kWarps];             /* ... and that sum without the candidates, relative to the part's reference */
+    float              ref_at[kSliceRefs][kWarps]; /* top-p: what a slice's terms were formed relative to */
     int                rl_id[kRowIds], rl_cnt[kRowIds + 4]; /* the row's distinct history ids as (offset in the share | count << 10 | tag << 20),
                                                              * grouped by the (slice, warp) share they fall into, and where each group's run starts */
     /* the part's select */
@@ -1595,16 +1596,11 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         /* segment sums (one per warp and slice, ids in order), moved from their own maximum to the row maximum */
         const int     nseg   = p.n_slices * kWarps;
         const SegRec *segs   = p.segs + (size_t) row * (size_t) nseg;
-        /* every segment's sum is in units of a power of two of its own; all are moved to the row's, that of its
-         * maximum, which is the largest of them: exact but for what leaves the range of double */
-        const float   row_c  = sum_unit(row_max, r.inv_t);
         auto          seg_at = [&](int t) {
-            const float  c  = __ldcg(&segs[t].ref);
-            const double sm = __ldcg(&segs[t].sum);
-            return c == kNoUnit ? 0.0 : sm * pow2_diff(c, row_c);
+            const float  ref = __ldcg(&segs[t].ref);
+            const double sm  = __ldcg(&segs[t].sum);
+            return sm * ref_move(ref, row_max, r.inv_t);
         };
-        /* ... and the crossing segment's terms, evaluated against the maximum itself */
-        const double  unit   = exp2((double) row_max * sum_scale(r.inv_t) - (double) row_c);
         double part = 0.0;
         for (int t = g.tid; t < nseg; t += g.n) {
             part += seg_at(t);
@@ -1697,7 +1693,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             for (int q = 0; q < 4; q++) {
                 const int i = i0 + q;
                 ev[q]       = (q < per && i < seg_n) ? expf(scaled_arg(wbuf[i], row_max, r.inv_t)) : 0.0f;
-                mine += (double) ev[q] * unit;
+                mine += (double) ev[q];
             }
             double incl = mine;
 #pragma unroll
@@ -1733,7 +1729,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 int    hit = min(i0 + per - 1, seg_n - 1);
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    a += (double) ev[q] * unit;
+                    a += (double) ev[q];
                     if (q < per && u < a) {
                         hit = i0 + q;
                         break;
@@ -1963,8 +1959,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         if constexpr (!kFast) {
         if (!need_multipass) {
             /* top-p over a small nucleus (sampler.c:245-300). Candidates get their exact e_i relative to the row
-             * maximum; the rest of the row was summed per part in units of a power of two and is rescaled
-             * here. */
+             * maximum; the rest of the row was summed per part relative to the part's own maximum and is
+             * rescaled here. */
             double part = 0.0;
             for (int i = g.tid; i < total; i += g.n) {
                 const float e = exp_exact(scaled_arg(cbuf[i].v, row_max, r.inv_t));
@@ -1972,9 +1968,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 part += (double) e;
             }
             if (g.tid < n_parts) {
-                const float  c  = sh->pbref[g.tid];
-                const double sc = c == kNoUnit ? 0.0 : exp2((double) c - (double) row_max * sum_scale(r.inv_t));
-                part += sc * sh->pbsum[g.tid];
+                part += ref_move(sh->pbref[g.tid], row_max, r.inv_t) * sh->pbsum[g.tid];
             }
             const double S = group_sum_d(g, gs, part);
             for (int i = g.tid; i < total; i += g.n) {
@@ -2198,19 +2192,19 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
     stage = kPrefetchDone;
 }
 
-/* The largest of the warps' units of a part. */
-__device__ __forceinline__ float unit_max(const StreamShared *sh) {
-    float c = kNoUnit;
+/* The largest of the warps' references of a part. */
+__device__ __forceinline__ float part_ref(const StreamShared *sh) {
+    float m = -CUDART_INF_F;
 #pragma unroll
     for (int w = 0; w < kWarps; w++) {
-        c = fmaxf(c, sh->wb_c[w]);
+        m = fmaxf(m, sh->wb_ref[w]);
     }
-    return c;
+    return m;
 }
 
 /* The terms of a float4, added up as every place that forms them adds them up. */
-__device__ __forceinline__ float sum_terms(const float4 &x, const SumScale &k, float c) {
-    return __fadd_rn(__fadd_rn(sum_term(x.x, k, c), sum_term(x.y, k, c)), __fadd_rn(sum_term(x.z, k, c), sum_term(x.w, k, c)));
+__device__ __forceinline__ float sum_terms(const float4 &x, const SumScale &k, float ref) {
+    return __fadd_rn(__fadd_rn(sum_term(x.x, k, ref), sum_term(x.y, k, ref)), __fadd_rn(sum_term(x.z, k, ref), sum_term(x.w, k, ref)));
 }
 
 /* Which kinds of rows an instantiation of the stream kernel carries the code for: every one carries greedy rows;
@@ -2530,7 +2524,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         unsigned       run_key = 0u; /* greedy: this warp's maximum of the part so far (key) and its first id */
         int            run_arg = 0x7fffffff;
         float          top0 = -CUDART_INF_F, top1 = -CUDART_INF_F; /* others: the thread's maxima over the first and the second half of its float4 */
-        float          unit = kNoUnit; /* the warp's sums are in units of 2^unit */
+        float          ref  = -CUDART_INF_F; /* top-p: what the warp's sum is relative to */
         double         acc  = 0.0;     /* top-p: the thread's sum over the part */
         int            wst  = 0;
         const SumScale ks   = sum_scale2(inv_t);
@@ -2689,37 +2683,52 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                     m        = max3(max3(m, x[i].x, x[i].y), x[i].z, x[i].w);
                 }
                 refill();
-                /* the unit follows the maximum: a temperature row's terms stay below 1 (their sum is added up in fixed
-                 * point), a top-p row's may grow to 2^60 before the sums so far are moved */
-                if (__any_sync(0xffffffffu, __fmul_rn(fmaxf(m0, m1), ks.hi) > unit + (smode == M_TEMP ? 0.0f : 60.0f))) {
-                    const unsigned wk = __reduce_max_sync(0xffffffffu, order_key(fmaxf(m0, m1)));
-                    const float    u  = ceilf(__fmul_rn(key_to_float(wk), ks.hi));
-                    acc               = unit == kNoUnit ? 0.0 : acc * pow2_diff(unit, u);
-                    unit              = u;
+                /* A temperature row's share is summed relative to its own maximum, a top-p row's relative to a value that the
+                 * warp's maximum may leave behind by 2^60: the row's largest values are candidates, which leave the
+                 * sum again. Where it has gone further, what was summed so far is too little for its factor's last bits
+                 * to count. */
+                const float m = fmaxf(m0, m1);
+                float       from;
+                if (smode == M_TEMP) {
+                    from = key_to_float(__reduce_max_sync(0xffffffffu, order_key(m)));
+                } else {
+                    if (__any_sync(0xffffffffu, m > ref && !(__fmul_rn(__fsub_rn(m, ref), ks.hi) <= 60.0f))) {
+                        const float now = key_to_float(__reduce_max_sync(0xffffffffu, order_key(m)));
+                        acc *= (double) sum_term(ref, ks, now);
+                        ref = now;
+                    }
+                    from = ref;
                 }
-                double sum = 0.0;
+                const float from0 = from == -CUDART_INF_F ? 0.0f : from; /* nothing but -inf so far: its terms are 0 */
+                double      sum   = 0.0;
 #pragma unroll
                 for (int i = 0; i < kNV4; i++) {
-                    sum += (double) sum_terms(x[i], ks, unit);
+                    sum += (double) sum_terms(x[i], ks, from0);
                 }
                 if (smode == M_TOPP) {
                     acc += sum;
-                    if (lane == 0 && s < kSliceCs) {
-                        sh->c_at[s][warp] = unit;
+                    if (lane == 0) {
+                        if (s < kSliceRefs) {
+                            sh->ref_at[s][warp] = from;
+                        } else { /* parts of more slices keep the rest where a temperature row's sums would lie */
+                            p.segs[((size_t) row * (size_t) p.n_slices + (size_t) c) * kWarps + warp].ref = from;
+                        }
                     }
                     note_maxima(s, m0, m1);
                 } else {
-                    /* the warp's sum in fixed point, 2^-42 of the largest possible term: two integer reductions
-                     * instead of five rounds of double additions between lanes */
-                    const long long q  = __double_as_longlong(sum + 0x1.8p10) & 0xfffffffffffffll;
-                    const unsigned  lo = __reduce_add_sync(0xffffffffu, (unsigned) q & 0x3ffffffu);
-                    const unsigned  hi = __reduce_add_sync(0xffffffffu, (unsigned) (q >> 26));
-                    top0               = fmaxf(top0, fmaxf(m0, m1));
+                    /* The warp's sum in fixed point: a lane's is at most 32, in steps of 2^-57 its double loses nothing that
+                     * a double of the total would hold. Three integer reductions instead of five rounds of double
+                     * additions between lanes. */
+                    const long long q   = __double2ll_rn(sum * 0x1p57);
+                    const unsigned  lo  = __reduce_add_sync(0xffffffffu, (unsigned) q & 0x1fffffu);
+                    const unsigned  mid = __reduce_add_sync(0xffffffffu, (unsigned) (q >> 21) & 0x1fffffu);
+                    const unsigned  hi  = __reduce_add_sync(0xffffffffu, (unsigned) (q >> 42));
+                    top0                = fmaxf(top0, m);
                     if (lane == 0) {
                         SegRec sr;
-                        sr.ref = unit;
+                        sr.ref = from;
                         sr.pad = 0.0f;
-                        sr.sum = ((double) hi - 32.0 * 0x1p25) * 0x1p-16 + (double) lo * 0x1p-42;
+                        sr.sum = (double) hi * 0x1p-15 + ((double) mid * 0x1p-36 + (double) lo * 0x1p-57);
                         p.segs[((size_t) row * (size_t) p.n_slices + (size_t) c) * kWarps + warp] = sr;
                     }
                 }
@@ -2738,8 +2747,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         }
         if (lane == 0) {
             sh->best[warp]   = ((unsigned long long) run_key << 32) | (unsigned long long) (0xffffffffu - (unsigned) run_arg);
-            sh->wb_c[warp]   = unit;
-            sh->wb_sum[warp] = acc;
+            sh->wb_ref[warp] = ref;
             if (wst != 0) {
                 atomicOr(&sh->st, wst);
             }
@@ -2860,21 +2868,22 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 if ((kKinds & K_SUMS) != 0 && sums && any) {
                     /* a candidate's weight is evaluated exactly where the row is finished: it leaves the sum, as the
                      * term of its float4 entered it, and what shares its float4 comes back one by one */
-                    const float u   = s < kSliceCs ? sh->c_at[s][w] : sh->wb_c[w];
-                    double      now = -(double) sum_terms(make_float4(v[0], v[1], v[2], v[3]), ks, u);
+                    const float u  = s < kSliceRefs ? sh->ref_at[s][w] : p.segs[((size_t) row * (size_t) p.n_slices + (size_t) c) * kWarps + w].ref;
+                    const float u0 = u == -CUDART_INF_F ? 0.0f : u;
+                    double      now = -(double) sum_terms(make_float4(v[0], v[1], v[2], v[3]), ks, u0);
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         if (!(v[q] >= tau)) {
-                            now += (double) sum_term(v[q], ks, u);
+                            now += (double) sum_term(v[q], ks, u0);
                         }
                     }
-                    fix += now * pow2_diff(u, sh->wb_c[w]) * pow2_diff(sh->wb_c[w], unit_max(sh));
+                    fix += now * ref_move(u, part_ref(sh), inv_t);
                 }
             }
             if ((kKinds & K_SUMS) != 0 && sums) {
                 fix = warp_sum_d(fix);
-                if (lane == 0) {
-                    sh->fix[warp] = fix;
+                if (lane == 0) { /* with the warp's own sum: each warp moves its own */
+                    sh->wb_sum[warp] = acc * ref_move(ref, part_ref(sh), inv_t) + fix;
                 }
             }
         }
@@ -2902,13 +2911,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             for (int w = 0; w < kWarps; w++) {
                 bw = max(bw, sh->best[w]);
             }
-            float  bc   = kNoUnit;
+            float  bref = -CUDART_INF_F;
             double bsum = 0.0;
             if ((kKinds & K_SUMS) != 0 && smode == M_TOPP && sums) {
-                bc = unit_max(sh);
+                bref = part_ref(sh);
 #pragma unroll
                 for (int w = 0; w < kWarps; w++) {
-                    bsum += (sh->wb_c[w] == kNoUnit ? 0.0 : sh->wb_sum[w] * pow2_diff(sh->wb_c[w], bc)) + sh->fix[w];
+                    bsum += sh->wb_sum[w];
                 }
                 bsum = fmax(bsum, 0.0);
             }
@@ -2918,7 +2927,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             h.z  = sel ? n_cand : 0;
             h.w  = sh->st;
             h2.x = __float_as_int(sel ? tau : -CUDART_INF_F);
-            h2.y = __float_as_int(bc);
+            h2.y = __float_as_int(bref);
             h2.z = __double2loint(bsum);
             h2.w = __double2hiint(bsum);
             int4 *rec = part_rec(p, row, part_idx);

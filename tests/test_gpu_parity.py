@@ -514,3 +514,54 @@ def test_shares_that_are_empty_in_one_slice_shape(ctx, V):
         # a draw over a whole row may fall within the sums' last bits of a step (two of 1536 rows of 128256 were seen to)
         assert differ <= (0 if hint != 2 else 0.008 * rows), (T, K, hint, differ)
         assert np.array_equal(u64_from_dev(out["rng_state"]), o["rng_state"])
+
+
+@pytest.mark.parametrize("T", [1e-3, 1e-5, 1e-6, 3e-7, 1e-7, 5e-8, 1e-9, 1e-12, 1e-30, 1e-37, 1e30, np.inf])
+@pytest.mark.parametrize("P", [1.0, 0.9])
+def test_row_sums_at_extreme_temperatures(ctx, T, P):
+    """"Nearly greedy" temperatures (and, last, nearly uniform ones): the row's sum is its few largest terms, whatever the size and the sign of the logits
+    (confident rows, log-probabilities, far offsets, values that rise along the ids, the type's lowest values as a mask,
+    two equal maxima)."""
+    V, rows = 33001, 56
+    x = normal_logits(rows, V, 2.5, 91)
+    rg = np.random.default_rng(92)
+    for r in range(rows):
+        kind = r % 7
+        if kind == 0:
+            x[r, rg.integers(0, V, 8)] += 12
+        elif kind == 1:
+            x[r] -= 30
+        elif kind == 2:
+            x[r] += 3000
+        elif kind == 3:
+            x[r] += np.linspace(-80, 80, V, dtype=np.float32)
+        elif kind == 4:
+            x[r, rg.random(V) < 0.999] = np.finfo(np.float32).min
+        elif kind == 5:
+            x[r] = np.finfo(np.float32).min
+        else:
+            x[r, rg.integers(0, V, 2)] = 25.0
+    st = independent_states(oracle.port, 93, rows)
+    g = run_gpu(ctx, x, T, 0, P, st)
+    o = oracle.port.sample_batch(x, T, 0, P, st)
+    check_tokens(g, o)
+
+
+@pytest.mark.parametrize("T,P", [(1.0, 1.0), (0.8, 0.9), (0.3, 0.95)])
+def test_row_sums_where_the_maximum_rises_along_the_row(ctx, T, P):
+    """Sums whose reference moves slice after slice, in parts of more slices than are remembered in shared memory (33 a
+    row, whole rows per thread block); rows 3 of 4 end in a small nucleus whose ids leave the sum again."""
+    import torch
+    V, rows = 270336, 600
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(rows, V, generator=gen, device="cuda").mul_(2.0) + torch.linspace(0.0, 30.0, V, device="cuda")
+    x[::4] -= torch.linspace(0.0, 30.0, V, device="cuda")
+    x[1::2, -5000::625] += 9.0
+    st = independent_states(oracle.port, 95, rows)
+    dT, dK, dP = per_seq(rows, T, 0, P)
+    out = ctx.sample_batch(x, dT, dK, dP, u64_to_dev(st), finish_hint=2)
+    assert (out["status"].cpu().numpy() & INVALID == 0).all()
+    tok = out["tokens"].cpu().numpy()
+    some = np.arange(0, rows, 60) + np.arange(10) % 4
+    o = oracle.port.sample_batch(np.ascontiguousarray(x[torch.from_numpy(some).cuda()].cpu().numpy()), T, 0, P, st[some])
+    assert np.array_equal(tok[some], o["tokens"]), (tok[some], o["tokens"])

@@ -1721,8 +1721,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             g.sync();
             const int pk = gs->pick;
             if (pk == 0x7fffffff) {
-                if (g.tid == 0) { /* regrouped sums can end a hair below the segment's share */
-                    p.tokens[row] = s0c + e0 + max(seg_n - 1, 0) + p.vocab_offset;
+                if (g.tid == 0) { /* regrouped sums can end a hair below the segment's share; the row's last segment may be empty */
+                    p.tokens[row] = max(s0c + e0 + seg_n - 1, 0) + p.vocab_offset;
                 }
             } else if (g.tid == pk) {
                 double a   = base + (incl - mine);
@@ -2718,17 +2718,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 } else {
                     /* The warp's sum in fixed point: a lane's is at most 32, in steps of 2^-57 its double loses nothing that
                      * a double of the total would hold. Three integer reductions instead of five rounds of double
-                     * additions between lanes. */
+                     * additions between lanes. A lane whose sum is NaN adds what no sum of lanes comes to. */
                     const long long q   = __double2ll_rn(sum * 0x1p57);
                     const unsigned  lo  = __reduce_add_sync(0xffffffffu, (unsigned) q & 0x1fffffu);
                     const unsigned  mid = __reduce_add_sync(0xffffffffu, (unsigned) (q >> 21) & 0x1fffffu);
-                    const unsigned  hi  = __reduce_add_sync(0xffffffffu, (unsigned) (q >> 42));
+                    const unsigned  hi  = __reduce_add_sync(0xffffffffu, sum <= 32.0 ? (unsigned) (q >> 42) : 1u << 26);
                     top0                = fmaxf(top0, m);
                     if (lane == 0) {
                         SegRec sr;
                         sr.ref = from;
                         sr.pad = 0.0f;
-                        sr.sum = (double) hi * 0x1p-15 + ((double) mid * 0x1p-36 + (double) lo * 0x1p-57);
+                        sr.sum = hi < (1u << 26) ? (double) hi * 0x1p-15 + ((double) mid * 0x1p-36 + (double) lo * 0x1p-57) : CUDART_NAN;
                         p.segs[((size_t) row * (size_t) p.n_slices + (size_t) c) * kWarps + warp] = sr;
                     }
                 }
@@ -2919,7 +2919,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 for (int w = 0; w < kWarps; w++) {
                     bsum += sh->wb_sum[w];
                 }
-                bsum = fmax(bsum, 0.0);
+                bsum = bsum < 0.0 ? 0.0 : bsum; /* a NaN stays one: the walk ends on the row's last id, as the reference's does */
             }
             int4           h, h2;
             h.x  = __float_as_int((unsigned) (bw >> 32) == 0u ? -CUDART_INF_F : key_to_float((unsigned) (bw >> 32)));

@@ -565,3 +565,23 @@ def test_row_sums_where_the_maximum_rises_along_the_row(ctx, T, P):
     some = np.arange(0, rows, 60) + np.arange(10) % 4
     o = oracle.port.sample_batch(np.ascontiguousarray(x[torch.from_numpy(some).cuda()].cpu().numpy()), T, 0, P, st[some])
     assert np.array_equal(tok[some], o["tokens"]), (tok[some], o["tokens"])
+
+
+@pytest.mark.parametrize("V", [33, 100, 4096, 18820, 33001])
+@pytest.mark.parametrize("P", [1.0, 0.9])
+def test_nan_in_a_summed_row(ctx, V, P):
+    """A NaN reaches the row's total and the walk ends on the last id, as the reference's does (every comparison with the
+    running sum fails); so does a row that holds nothing but -inf. The rows around them are drawn as ever. (100 and
+    18820 columns leave the last warp's share of the last slice empty.)"""
+    rows = 40
+    x = normal_logits(rows, V, 2.5, V)
+    for r in range(0, rows, 4):
+        x[r, 1 + (r * 7919) % (V - 1)] = np.nan
+    x[1] = -np.inf
+    x[5, V // 2:] = -np.inf
+    x[5, V - 1] = np.nan
+    st = independent_states(oracle.port, V, rows)
+    o = oracle.port.sample_batch(x, 0.9, 0, P, st)
+    assert (o["tokens"][[0, 1, 4, 5, 36]] == V - 1).all()
+    for hint in (0, 2):
+        check_tokens(run_gpu(ctx, x, 0.9, 0, P, st, finish_hint=hint), o)

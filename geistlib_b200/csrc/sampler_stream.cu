@@ -780,6 +780,16 @@ __device__ unsigned long long resolve_ties(const Grp &g, GroupShared *sh, Sweep 
     return bisect_mass(g, sh, sweep, idx_bits, target, inclusive, key, mass, (unsigned long long) ro.key << idx_bits, idx_bits - 1);
 }
 
+/* Where a row is read again once it has been streamed, and whether it starts on a 16-byte boundary there. A launch that
+ * asks for the rows as they are sampled from reads those back and changes nothing a second time: they may lie over the
+ * logits themselves. */
+__device__ __forceinline__ const float *row_again(const SampleParams &p, int row) {
+    return p.out_logits != nullptr ? p.out_logits + (size_t) row * (size_t) p.V : p.logits + (size_t) row * (size_t) p.row_stride;
+}
+__device__ __forceinline__ bool again_aligned(const SampleParams &p) {
+    return p.out_logits != nullptr ? (reinterpret_cast<unsigned long long>(p.out_logits) & 15ull) == 0ull && (p.V & 3) == 0 : p.aligned != 0;
+}
+
 /* All threads of the thread block serve a row whose kept set does not fit the one-pass path. */
 __device__ __noinline__ int multipass_row(const Grp &g, const SampleParams &p, GroupShared *sh, RowCfg &r, float row_max, int row_arg, void *hist_mem, int hist_bytes, int slot, void *save_mem) {
     /* room for the byte histograms of the radix walks: per warp where it fits, else one for all */
@@ -790,12 +800,13 @@ __device__ __noinline__ int multipass_row(const Grp &g, const SampleParams &p, G
     const int    idx_bits = 32 - __clz(max(V - 1, 1));
     int          st       = ST_SLOW_PATH;
     float       *gr       = p.gen_rows + (size_t) slot * (size_t) p.gen_stride;
-    const float *src      = p.logits + (size_t) r.row * (size_t) p.row_stride;
+    const float *src      = row_again(p, r.row);
+    const bool   src_al   = again_aligned(p);
     int         *kept_i   = p.kept_cap > 0 ? p.kept_idx + (size_t) r.row * (size_t) p.kept_cap : nullptr;
     float       *kept_v   = p.kept_cap > 0 ? p.kept_val + (size_t) r.row * (size_t) p.kept_cap : nullptr;
     /* Nothing changes the row's values (no penalties, cap or mask) and it lies on a 16-byte boundary: it is read
      * where it is, and the private copy only takes what a top-p row is rewritten into. */
-    const bool   in_place = !r.pen_on && !(r.cap > 0.0f) && r.mrow == nullptr && p.aligned != 0;
+    const bool   in_place = !r.pen_on && !(r.cap > 0.0f) && r.mrow == nullptr && src_al;
     const float *cur      = in_place ? src : gr; /* what the sweeps read */
     auto         row_sw   = [&](auto &&f) { row_sweep(g, cur, V, f); };
     /* the entries that pred(value, id) names, picked out of the row into this thread block's list (any order);
@@ -824,7 +835,7 @@ __device__ __noinline__ int multipass_row(const Grp &g, const SampleParams &p, G
     MP(0);
     /* private copy of the row, penalties applied once */
     if (in_place) {
-    } else if (p.aligned) { /* rows start on 16-byte boundaries: four values per load */
+    } else if (src_al) { /* rows start on 16-byte boundaries: four values per load */
         const float4 *s4 = reinterpret_cast<const float4 *>(src);
         float4       *d4 = reinterpret_cast<float4 *>(gr);
         for (int i = g.tid; i < (V >> 2); i += g.n) {
@@ -1665,7 +1676,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         const int    e1    = min(4 * min((w + 1) * Lc, nv4c), nc);
         const int    seg_n = max(e1 - e0, 0);
         float       *wbuf  = reinterpret_cast<float *>(cmem); /* >= 1024 floats */
-        const float *src   = p.logits + (size_t) row * (size_t) p.row_stride + s0c + e0;
+        const float *src   = row_again(p, row) + s0c + e0;
         g.sync();
         for (int i = g.tid; i < seg_n; i += g.n) {
             wbuf[i] = prologue_one(src[i], s0c + e0 + i, r.cap, r.mrow);
@@ -2806,6 +2817,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             }
             __syncthreads();
             /* their float4, read again (L2 holds them), changed as they were while the part streamed */
+            const bool rewritten = !kPlain && p.out_logits != nullptr, src_al = kPlain || again_aligned(p);
             const int n_grp = min(sh->n_grp, kPartCand), per_log = kNV4Log + gm_shift;
             double    fix   = 0.0;
             for (int t = tid; t < n_grp << per_log; t += kThreads) {
@@ -2817,9 +2829,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                     continue;
                 }
                 const int    e0  = 4 * (w4 + i4), id0 = c * p.slice + e0;
-                const float *src = p.logits + (size_t) row * (size_t) p.row_stride + id0;
+                const float *src = (kPlain ? p.logits + (size_t) row * (size_t) p.row_stride : row_again(p, row)) + id0;
                 float        v[4];
-                if (aligned && e0 + 4 <= n) {
+                if (src_al && e0 + 4 <= n) {
                     const float4 q = *reinterpret_cast<const float4 *>(src);
                     v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
                 } else {
@@ -2828,7 +2840,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                         v[q] = e0 + q < n ? src[q] : -CUDART_INF_F;
                     }
                 }
-                if (pro_on) {
+                if (pro_on && !rewritten) {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         if (e0 + q < n) {
@@ -2836,7 +2848,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                         }
                     }
                 }
-                if (pen_on) {
+                if (pen_on && !rewritten) {
                     const unsigned *ent;
                     int             lo, hi;
                     unsigned        tag;
@@ -3033,6 +3045,11 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     for (int row = (int) blockIdx.x; row < p.n_rows; row += (int) gridDim.x) {
         const RawCfg rc = row == (int) blockIdx.x ? rc0 : raw_config(p, row, true);
         RowCfg       r  = row_config(p, row, rc, true);
+        if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
+            r.cap    = 0.0f;
+            r.mrow   = nullptr;
+            r.pen_on = false;
+        }
         PROF(8);
         int          st = finish_row<kFast>(g, p, sh, r, cmem);
         PROF(13);

@@ -167,7 +167,10 @@ struct geist_b200_batch {
     int32_t *tokens;     /* [n_seq * rows_per_seq] */
     int32_t *row_status; /* [n_seq * rows_per_seq] */
 
-    float *out_logits; /* optional [rows, n_vocab]: rows after penalties */
+    /* Optional [rows, n_vocab]: the rows as they are sampled from, after soft cap, mask and penalties. May be `logits`
+     * itself (row_stride == n_vocab): the rows are then rewritten where they lie, and a row that answers
+     * GEIST_B200_ROW_RETRY is launched again without cap, mask and penalties. Any other overlap is undefined. */
+    float *out_logits;
 
     int32_t  kept_cap; /* 0 = off; else entries per row below */
     int32_t *kept_n;   /* [rows] size of the kept set (k, nucleus size, 0 for argmax/temperature) */

@@ -6,7 +6,7 @@ import pytest
 
 import oracle
 from geistlib_b200 import api
-from helpers import gumbel_logits, histories, independent_states, normal_logits, rel_err, seq_states, to_dev
+from helpers import gumbel_logits, histories, independent_states, normal_logits, per_seq, rel_err, seq_states, to_dev, u64_to_dev
 from test_gpu_parity import check_tokens, run_gpu
 
 pytestmark = pytest.mark.gpu
@@ -332,3 +332,29 @@ def test_softcap_after_the_select_equals_softcap_before(ctx, c, sigma, shiftx, h
                 both = ((late["status"] | full["status"]) & api.ROW_KEPT_PARTIAL) == 0
                 for name in ("kept_n", "kept_idx", "kept_prob"):
                     assert np.array_equal(late[name][both], full[name][both]), name
+
+
+@pytest.mark.parametrize("V", [4096, 33001, 33004, 151936])
+@pytest.mark.parametrize("T,K,P", [(0.0, 0, 1.0), (0.9, 40, 1.0), (0.9, 300, 1.0), (0.8, 0, 0.9), (1.0, 0, 1.0)])
+def test_logits_rewritten_where_they_lie(ctx, V, T, K, P):
+    """out_logits over logits: the rows end up as they are sampled from and the tokens are those of a launch that writes
+    elsewhere, on every route that reads a row again (select, segment walk, the multi-pass path)."""
+    rows, H = 12, 90
+    x = normal_logits(rows, V, 2.5, V)
+    x[::3, :6] += 9.0
+    h = histories(rows, H, V, V)
+    h[:, :8] = np.argsort(-x, axis=1)[:, :8]
+    st = independent_states(oracle.port, V, rows)
+    mask = np.random.default_rng(V).random((rows, V)) < 0.7
+    kw = dict(rep=1.3, freq=0.2, history=h, softcap=cap_dev(rows, np.resize([30.0, 0.0], rows)), logit_mask=to_dev(mask_words(mask)))
+    apart = run_gpu(ctx, x, T, K, P, st, want_logits=True, **kw)
+    dT, dK, dP = per_seq(rows, T, K, P)
+    dx, drng = to_dev(x), u64_to_dev(st)
+    like = ctx.sample_batch(dx, dT, dK, dP, drng, want_logits=True, launch=False)
+    like["logits"] = dx
+    dev = {"rep": to_dev(np.full(rows, 1.3, np.float32)), "freq": to_dev(np.full(rows, 0.2, np.float32)), "history": to_dev(h),
+           "history_len": to_dev(np.full(rows, H, np.int32)), "softcap": kw["softcap"], "logit_mask": kw["logit_mask"]}
+    over = ctx.sample_batch(dx, dT, dK, dP, drng, out=like, **dev)
+    assert (over["status"].cpu().numpy() & api.ROW_INVALID == 0).all()
+    assert np.array_equal(over["logits"].cpu().numpy().view(np.uint32), apart["logits"].view(np.uint32))
+    assert np.array_equal(over["tokens"].cpu().numpy(), apart["tokens"])

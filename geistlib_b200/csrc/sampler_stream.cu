@@ -1250,6 +1250,10 @@ __device__ __forceinline__ void row_epilogue(const SampleParams &p, const RowCfg
 
 /* ------------------------------------------------------------ shared state -- */
 
+constexpr int kIdBits = 4 * kSliceMax;
+/* Where the bit of a value lies: slice of the part, warp, offset in the share. */
+__device__ __forceinline__ int id_bit(int s, int w, int off) { return ((s & 3) * kWarps + w) * (kSliceMax / kWarps) + off; }
+
 /* What the warps of one thread block share. The ring (every warp's two stages) lies in front of it in dynamic
  * shared memory, the group maxima of the part in work behind it. */
 struct __align__(16) StreamShared {
@@ -1262,8 +1266,10 @@ struct __align__(16) StreamShared {
     float              ref_at[kSliceRefs][kWarps]; /* top-p: what a slice's terms were formed relative to */
     int                rl_id[kRowIds], rl_cnt[kRowIds + 4]; /* the row's distinct history ids as (offset in the share | count << 10 | tag << 20),
                                                              * grouped by the (slice, warp) share they fall into, and where each group's run starts */
+    alignas(16) unsigned id_bits[kIdBits / 32];             /* which values of the part an id has changed (slices s and s + 4 share their bits) */
     /* the part's select */
     int                n_grp, n_cand;         /* groups that reach the threshold; candidates in them */
+    int                max_cnt;               /* how often the part's most frequent id occurs (asked where that raises a value) */
     unsigned short     grp[kPartCand];        /* (slot << 8) | thread */
     alignas(8) Pair    cand[kPartCand];
     /* finishing inside the stream kernel (F_INLINE_TOPK): the k best in order, their weights */
@@ -2403,6 +2409,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             sh->st     = 0;
             sh->n_grp  = 0;
             sh->n_cand = 0;
+            sh->max_cnt = 1;
+        }
+        if (pen_on && sel) {
+            for (int i = tid; i < kIdBits / 128; i += kThreads) {
+                reinterpret_cast<uint4 *>(sh->id_bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+            }
         }
         if (pen_on && !long_ids) {
             /* The row's distinct ids with their counts: an open-addressing table in the group maxima's memory (free
@@ -2537,7 +2549,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         float          top0 = -CUDART_INF_F, top1 = -CUDART_INF_F; /* others: the thread's maxima over the first and the second half of its float4 */
         float          ref  = -CUDART_INF_F; /* top-p: what the warp's sum is relative to */
         double         acc  = 0.0;     /* top-p: the thread's sum over the part */
-        int            wst  = 0;
+        int            wst  = 0, most = 0; /* most: how often the most frequent id occurs */
         const SumScale ks   = sum_scale2(inv_t);
         int            gm_shift = 0; /* slices that share one slot of the group maxima: 2^gm_shift */
         while (((part_len - 1) >> gm_shift) >= kGroupSlots) {
@@ -2600,9 +2612,14 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 for (int e = lo + lane; e < hi; e += 32) {
                     const unsigned en = ent[e];
                     if (long_ids || (en >> 20) == tag) {
+                        most    = max(most, (int) ((en >> 10) & cnt_mask));
                         float *q = sl + (en & 0x3ffu);
                         *q       = penalise_rcp(*q, (int) ((en >> 10) & cnt_mask), rep_rcp, rep, freq, pres);
                         touched  = true;
+                        if (sel) {
+                            const int bit = id_bit(s, warp, (int) (en & 0x3ffu));
+                            atomicOr(&sh->id_bits[bit >> 5], 1u << (bit & 31));
+                        }
                     }
                 }
                 wrote |= __any_sync(0xffffffffu, touched); /* also orders the stores before the loads below */
@@ -2750,6 +2767,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         PROF(2);
         /* ---- the part is through ---- */
         wst = __reduce_or_sync(0xffffffffu, (unsigned) wst);
+        if (pen_on && sel && freq < 0.0f) {
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (lane == 0) {
+                atomicMax(&sh->max_cnt, most);
+            }
+        }
         if (smode != M_ARGMAX) {
             run_key = __reduce_max_sync(0xffffffffu, order_key(fmaxf(top0, top1)));
         }
@@ -2818,49 +2841,93 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             __syncthreads();
             /* their float4, read again (L2 holds them), changed as they were while the part streamed */
             const bool rewritten = !kPlain && p.out_logits != nullptr, src_al = kPlain || again_aligned(p);
+            const bool bits_say  = part_len <= 4 && freq == 0.0f; /* every value has a bit of its own and its penalty does not ask how often */
+            /* no value below tau_raw reaches tau with the penalties that raise it most (a repetition penalty below 1, negative
+             * ones); the margins are eight times what the roundings of a penalised value add up to */
+            float tau_raw = tau;
+            if (pen_on && !(rep >= 1.0f && freq >= 0.0f && pres >= 0.0f)) {
+                const float f = (float) (freq < 0.0f ? sh->max_cnt : 1) * freq, y = tau + f + pres - (fabsf(tau) + fabsf(f) + fabsf(pres)) * 0x1p-20f;
+                const float x = y > 0.0f ? y * rep : __fdiv_rn(y, rep);
+                tau_raw       = fminf(tau, x - fabsf(x) * 0x1p-20f);
+            }
             const int n_grp = min(sh->n_grp, kPartCand), per_log = kNV4Log + gm_shift;
             double    fix   = 0.0;
-            for (int t = tid; t < n_grp << per_log; t += kThreads) {
-                const int  name = sh->grp[t >> per_log], f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
+            for (int t0 = 0; t0 < n_grp << per_log; t0 += kThreads) { /* whole warps: ids are looked up by all lanes together */
+                const int  t = t0 + tid, name = t < n_grp << per_log ? sh->grp[t >> per_log] : 0, f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
                 const int  s = ((name >> 8) << gm_shift) + f / kNV4, c = c0 + s, i4 = l + 32 * (f % kNV4);
                 const bool last_c = c == p.n_slices - 1;
                 const int  n = last_c ? n_last : n_full, nv4 = (n + 3) >> 2, L = share_len(nv4), w4 = min(w * L, nv4);
-                if (s >= part_len || i4 >= min(L, nv4 - w4)) {
+                const bool own = t < n_grp << per_log && s < part_len && i4 < min(L, nv4 - w4);
+                const int  e0  = 4 * (w4 + i4), id0 = c * p.slice + e0;
+                float      v[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+                if ((kKinds & K_PEN) == 0 && !own) {
                     continue;
                 }
-                const int    e0  = 4 * (w4 + i4), id0 = c * p.slice + e0;
-                const float *src = (kPlain ? p.logits + (size_t) row * (size_t) p.row_stride : row_again(p, row)) + id0;
-                float        v[4];
-                if (src_al && e0 + 4 <= n) {
-                    const float4 q = *reinterpret_cast<const float4 *>(src);
-                    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-                } else {
+                if (own) {
+                    const float *src = (kPlain ? p.logits + (size_t) row * (size_t) p.row_stride : row_again(p, row)) + id0;
+                    if (src_al && e0 + 4 <= n) {
+                        const float4 q = *reinterpret_cast<const float4 *>(src);
+                        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+                    } else {
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        v[q] = e0 + q < n ? src[q] : -CUDART_INF_F;
+                        for (int q = 0; q < 4; q++) {
+                            v[q] = e0 + q < n ? src[q] : -CUDART_INF_F;
+                        }
                     }
-                }
-                if (pro_on && !rewritten) {
+                    if (pro_on && !rewritten) {
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        if (e0 + q < n) {
-                            v[q] = prologue_one(v[q], id0 + q, sh->cap, sh->mrow);
+                        for (int q = 0; q < 4; q++) {
+                            if (e0 + q < n) {
+                                v[q] = prologue_one(v[q], id0 + q, sh->cap, sh->mrow);
+                            }
                         }
                     }
                 }
                 if (pen_on && !rewritten) {
-                    const unsigned *ent;
-                    int             lo, hi;
-                    unsigned        tag;
-                    ids_of(s, w, ent, lo, hi, tag);
-                    for (int e = lo; e < hi; e++) {
-                        const unsigned en = ent[e];
-                        if ((int) ((en & 0x3ffu) >> 2) == i4 && (long_ids || (en >> 20) == tag)) {
+                    /* Which of the four an id has changed (a bit each, which may be another slice's where the part is long).
+                     * Where the bits are the value's own and the penalty does not ask how often the id occurs, that is
+                     * all there is to know. Else the ids are looked up, the warp's lanes going through the share's
+                     * list together, for values that can reach the threshold (a sum wants all four of a candidate's
+                     * float4). Against every float4 going through its share's list by itself, us: 1000 rows of 4096
+                     * columns, top-k 40, rep 1.1: 64 ids 45.1 -> 39.8, 256 ids 63.2 -> 44.9, 1000 ids 132 -> 64.7;
+                     * 256 x 128256 with 64 ids 32.2 -> 31.2; 4096 x 128256 with 1024 ids, top-k 50: 539 -> 509. */
+                    const int bit   = id_bit(s, w, 4 * i4);
+                    unsigned  mark  = own ? (sh->id_bits[bit >> 5] >> (bit & 31)) & 15u : 0u;
+                    int       cnt[4] = {1, 1, 1, 1};
+                    if (!bits_say) {
+                        unsigned reach = 0u, found = 0u;
 #pragma unroll
-                            for (int q = 0; q < 4; q++) {
-                                if ((int) (en & 3u) == q) {
-                                    v[q] = penalise_rcp(v[q], (int) ((en >> 10) & cnt_mask), rep_rcp, rep, freq, pres);
+                        for (int q = 0; q < 4; q++) {
+                            reach |= v[q] < tau_raw ? 0u : 1u << q;
+                        }
+                        mark = (kKinds & K_SUMS) != 0 && sums ? (reach != 0u ? mark : 0u) : mark & reach;
+                        for (unsigned ask = __ballot_sync(0xffffffffu, mark != 0u); ask != 0u; ask &= ask - 1u) {
+                            const int       from = __ffs(ask) - 1, i4_ = __shfl_sync(0xffffffffu, i4, from);
+                            const unsigned *ent;
+                            int             lo, hi;
+                            unsigned        tag;
+                            ids_of(__shfl_sync(0xffffffffu, s, from), __shfl_sync(0xffffffffu, w, from), ent, lo, hi, tag);
+                            for (int base = lo; base < hi; base += 32) {
+                                const unsigned en = base + lane < hi ? ent[base + lane] : 0u;
+                                for (unsigned hit = __ballot_sync(0xffffffffu, base + lane < hi && (int) ((en & 0x3ffu) >> 2) == i4_ && (long_ids || (en >> 20) == tag)); hit != 0u; hit &= hit - 1u) {
+                                    const unsigned eh = __shfl_sync(0xffffffffu, en, __ffs(hit) - 1);
+                                    if (lane == from) {
+                                        found |= 1u << (eh & 3u);
+#pragma unroll
+                                        for (int q = 0; q < 4; q++) {
+                                            cnt[q] = (int) (eh & 3u) == q ? (int) ((eh >> 10) & cnt_mask) : cnt[q];
+                                        }
+                                    }
                                 }
+                            }
+                        }
+                        mark = found;
+                    }
+                    if (mark != 0u) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if ((mark >> q) & 1u) {
+                                v[q] = penalise_rcp(v[q], cnt[q], rep_rcp, rep, freq, pres);
                             }
                         }
                     }
@@ -2868,7 +2935,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 bool any = false;
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    if (v[q] >= tau && e0 + q < n) {
+                    if (own && v[q] >= tau && e0 + q < n) {
                         const int pos = atomicAdd(&sh->n_cand, 1);
                         if (pos < kPartCand) {
                             sh->cand[pos].v   = v[q];

@@ -585,3 +585,28 @@ def test_nan_in_a_summed_row(ctx, V, P):
     assert (o["tokens"][[0, 1, 4, 5, 36]] == V - 1).all()
     for hint in (0, 2):
         check_tokens(run_gpu(ctx, x, 0.9, 0, P, st, finish_hint=hint), o)
+
+
+@pytest.mark.parametrize("H", [200, 1000, 1500])
+@pytest.mark.parametrize("V", [4096, 32768, 40000, 70001])
+def test_candidates_among_many_ids(ctx, V, H):
+    """Rows most of whose likely ids are in their history: what is read again at a part's end is penalised as it was while
+    it streamed, by its bit alone (short parts) or by looking the id up, for penalties that lower values, that raise
+    them and that count. Ids four slices apart share a bit."""
+    rows = 36
+    x = normal_logits(rows, V, 2.5, V + H)
+    order = np.argsort(-x, axis=1)
+    rg = np.random.default_rng(V + H)
+    n_slices = -(-V // 8192)
+    slice_ = -(-(-(-V // n_slices)) // 4) * 4
+    h = np.empty((rows, H), np.int32)
+    for r in range(rows):
+        top = order[r, :300]
+        pool = np.concatenate([top[rg.random(300) < 0.5], (top + 4 * slice_) % V, rg.integers(0, V, H)])
+        h[r] = rg.choice(pool[:H], H)
+    st = independent_states(oracle.port, V + H, rows)
+    for rep, freq, pres in [(1.1, 0.0, 0.0), (1.0, 0.2, 0.3), (0.8, 0.0, 0.0), (1.1, -0.1, 0.0), (1.0, 0.0, -0.5)]:
+        for T, K, P, hint in [(0.9, 40, 1.0, 1), (0.9, 40, 1.0, 0), (0.7, 0, 0.8, 0)]:
+            g = run_gpu(ctx, x, T, K, P, st, rep=rep, freq=freq, pres=pres, history=h, finish_hint=hint)
+            assert (g["status"] & 32 == 0).all()
+            check_tokens(g, oracle.port.sample_batch(x, T, K, P, st, rep=rep, freq=freq, pres=pres, hist=h))

@@ -610,3 +610,25 @@ def test_candidates_among_many_ids(ctx, V, H):
             g = run_gpu(ctx, x, T, K, P, st, rep=rep, freq=freq, pres=pres, history=h, finish_hint=hint)
             assert (g["status"] & 32 == 0).all()
             check_tokens(g, oracle.port.sample_batch(x, T, K, P, st, rep=rep, freq=freq, pres=pres, hist=h))
+
+
+@pytest.mark.parametrize("k", [2, 64, 127, 128, 129, 200, 256])
+@pytest.mark.parametrize("V", [700, 1500, 4096, 8200, 16384])
+def test_wide_sets_finished_by_the_stream_kernel(ctx, k, V):
+    """Whole rows per thread block, wide sets drawn nearly evenly so that every place of the order counts: plain rows, values
+    on a grid (bins full of ties), one far outlier (all others in the lowest bins), an infinite one, rows of equal values.
+    Rows of 4096 and fewer give a thread four float4 or less, every other one a maximum of its own."""
+    rows = 320
+    x = normal_logits(rows, V, 2.5, V + k)
+    x[1::5] = np.round(x[1::5] * 8) / 8
+    x[2::5, V // 3] = 3e4
+    x[3::15, V // 2] = np.inf
+    x[4::15] = 0.25
+    st = independent_states(oracle.port, V + k, rows)
+    g = run_gpu(ctx, x, 3.0, k, 1.0, st, finish_hint=1)
+    done = (g["status"] & 32) == 0
+    few_ties = np.ones(rows, bool)
+    few_ties[4::15] = V <= 1024  # more equal values than a part hands on
+    assert done[few_ties].all()
+    o = oracle.port.sample_batch(x, 3.0, k, 1.0, st)
+    assert np.array_equal(g["tokens"][done], o["tokens"][done])

@@ -1270,7 +1270,7 @@ struct __align__(16) StreamShared {
     /* the part's select */
     int                n_grp, n_cand;         /* groups that reach the threshold; candidates in them */
     int                max_cnt;               /* how often the part's most frequent id occurs (asked where that raises a value) */
-    unsigned short     grp[kPartCand];        /* (slot << 8) | thread */
+    unsigned short     grp[kGroupSlots * kThreads]; /* (slot << 8) | thread */
     alignas(8) Pair    cand[kPartCand];
     /* finishing inside the stream kernel (F_INLINE_TOPK): the k best in order, their weights */
     int                cur_rr;
@@ -2280,6 +2280,17 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
     stage = kPrefetchDone;
 }
 
+/* The part's maximum, as its candidates are. */
+__device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late) {
+    unsigned long long b = 0ull;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        b = max(b, sh->best[w]);
+    }
+    const float top = key_to_float((unsigned) (b >> 32));
+    return cap_late && top > -CUDART_INF_F ? soft_cap(top, sh->cap) : top;
+}
+
 /* The largest of the warps' references of a part. */
 __device__ __forceinline__ float part_ref(const StreamShared *sh) {
     float m = -CUDART_INF_F;
@@ -2447,9 +2458,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             pres   = r.pres;
             pro_on = !kPlain && (r.cap > 0.0f || r.mrow != nullptr); /* something happens to a logit before the penalties ... */
             /* ... and it has to while the part streams. The soft cap is monotone: a top-k row that brings no ids is
-             * selected from its uncapped logits, and only what is read again is capped. A tanhf, a division and a
-             * call per logit less: 48 rows of 262144 columns, half of them masked, top-k 64: 104.6 -> 93.8 us a step. */
-            cap_late = !kPlain && (kKinds & K_SEL) != 0 && r.cap > 0.0f && mode == M_TOPK && kq <= kFastKMax && !pen_on && p.out_logits == nullptr;
+             * selected from its uncapped logits, and only what is read again is capped: a tanhf, a division and a
+             * call per logit less. 48 rows of 262144 columns, half of them masked, top-k 64: 104.6 us a step with every
+             * logit capped and 93.8 with these (then; 78 by now). */
+            cap_late = !kPlain && (kKinds & K_SEL) != 0 && r.cap > 0.0f && r.cap < 1e38f && mode == M_TOPK && kq <= kFastKMax && !pen_on && p.out_logits == nullptr;
             pro_part = !kPlain && ((r.cap > 0.0f && !cap_late) || r.mrow != nullptr);
             if (tid == 0) { /* read again by the warps only if pro_on; the barriers of the part set-up lie between */
                 sh->cap      = r.cap;
@@ -2857,7 +2869,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 atomicOr(&sh->st, wst);
             }
         }
-        float tau = CUDART_INF_F;
+        float tau  = CUDART_INF_F;
+        bool  over = false;
         if (sel) {
             /*
              * The threshold: the kq-th largest (or one a little below) of the 256 thread maxima, a lower bound of the
@@ -2869,7 +2882,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
              * top-k 40 with penalties 33.2 -> 32.2 us, 4096 x 128256 top-k 50 549 -> 541 us, 256 x 262144 top-p
              * 97.0 -> 85.2 us with the sums' new form, 48 x 262144 soft-capped top-k 64 116 -> 104 us a step.
              */
-            const unsigned key0 = order_key(kq <= kThreads / 2 ? fmaxf(top0, top1) : top0), key1 = kq <= kThreads / 2 ? 0u : order_key(top1);
+            float sel0 = kq <= kThreads / 2 ? fmaxf(top0, top1) : top0, sel1 = kq <= kThreads / 2 ? -CUDART_INF_F : top1;
+            if (cap_late) { /* as the values they belong to will be once they are read again */
+                sel0 = sel0 == -CUDART_INF_F ? sel0 : soft_cap(sel0, sh->cap);
+                sel1 = sel1 == -CUDART_INF_F ? sel1 : soft_cap(sel1, sh->cap);
+            }
+            const unsigned key0 = order_key(sel0), key1 = order_key(sel1);
             unsigned       tkey = 0u;
             for (int bit = 31; bit >= 0; bit--) {
                 const unsigned t = tkey | (1u << bit);
@@ -2887,26 +2905,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             tau = tkey <= order_key(-CUDART_INF_F) ? -CUDART_INF_F : key_to_float(tkey); /* fewer than kq of them: everything passes */
             float tau_grp = tau;
             if (cap_late && tau > -CUDART_INF_F) {
-                /* From an uncapped threshold to a capped one: what reaches tau uncapped has a capped value of at least
-                 * y * cap (tanhf is good to a few 2^-24 and so may fall that much where its argument grows), and what
-                 * has a capped value of at least y * cap lies above the place where the cap takes a value a margin
-                 * below y. The margins, 2^-19 of y and 2^-21, are eight times what the functions' errors add up to;
-                 * where the cap saturates the place moves down to 6.8 cap, behind which all values are one. */
-                const float c = sh->cap, y0 = tanhf(__fdiv_rn(tau, c));
-                const float y1 = y0 - (fabsf(y0) * 0x1p-19f + 0x1p-21f), y2 = y1 - (fabsf(y1) * 0x1p-19f + 0x1p-21f);
-                const float t  = y2 > -1.0f ? c * atanhf(y2) : -CUDART_INF_F;
-                tau_grp        = fminf(tau, t - (fabsf(t) + c) * 0x1p-16f);
-                tau            = y1 * c;
+                /* The place of the uncapped row below which no capped value reaches tau. tanhf, the division and the product
+                 * are good to 2^-21 together, so such a value's true tanh(x / c) is at least y; the margins are four times
+                 * that and cover atanhf, the last two what falls below the smallest normal float. */
+                const float c = sh->cap, y0 = __fdiv_rn(tau, c), y = y0 - fabsf(y0) * 0x1p-19f;
+                const float t = y > -1.0f ? c * atanhf(y) : -CUDART_INF_F;
+                tau_grp       = t - fabsf(t) * 0x1p-20f - c * 0x1p-140f - 0x1p-120f;
             }
             /* the thread's groups that reach it */
             const int slots = ((part_len - 1) >> gm_shift) + 1;
 #pragma unroll 4
             for (int i = 0; i < slots; i++) {
                 if (gmax[i * kThreads + tid] >= tau_grp) {
-                    const int pos = atomicAdd(&sh->n_grp, 1);
-                    if (pos < kPartCand) {
-                        sh->grp[pos] = (unsigned short) ((i << 8) | tid);
-                    }
+                    sh->grp[atomicAdd(&sh->n_grp, 1)] = (unsigned short) ((i << 8) | tid);
                 }
             }
             __syncthreads();
@@ -2921,7 +2932,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 const float x = y > 0.0f ? y * rep : __fdiv_rn(y, rep);
                 tau_raw       = fminf(tau, x - fabsf(x) * 0x1p-20f);
             }
-            const int n_grp = min(sh->n_grp, kPartCand), per_log = kNV4Log + gm_shift;
+            /* a candidate at least in each: more groups than candidates fit need no look (uncapped values may fall short) */
+            over            = sh->n_grp > kPartCand && !(cap_late && tau > -CUDART_INF_F);
+            const int  n_grp = over ? 0 : sh->n_grp, per_log = kNV4Log + gm_shift;
             double    fix   = 0.0;
             for (int t0 = 0; t0 < n_grp << per_log; t0 += kThreads) { /* whole warps: ids are looked up by all lanes together */
                 const int  t = t0 + tid, name = t < n_grp << per_log ? sh->grp[t >> per_log] : 0, f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
@@ -3038,19 +3051,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             }
         }
         __syncthreads();
-        const int n_cand = sh->n_grp > kPartCand ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
+        const int n_cand = over ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
         const int held   = sel ? min(n_cand, kPartCand) : 0;
         if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
             /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
              * part); a row of another kind is reported as the small finishing kernel would */
             if (mode == M_TOPK) {
-                unsigned long long bw = 0ull;
-#pragma unroll
-                for (int w = 0; w < kWarps; w++) {
-                    bw = max(bw, sh->best[w]);
-                }
-                const float top = key_to_float((unsigned) (bw >> 32));
-                inline_finish_topk(p, sh, gmem, row, n_cand, kq, tau, cap_late ? soft_cap(top, sh->cap) : top, inv_t, sh->st);
+                inline_finish_topk(p, sh, gmem, row, n_cand, kq, tau, part_top(sh, cap_late), inv_t, sh->st);
             } else {
                 if (tid == 0) {
                     p.tokens[row] = -1;
@@ -3078,7 +3085,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 bsum = bsum < 0.0 ? 0.0 : bsum; /* a NaN stays one: the walk ends on the row's last id, as the reference's does */
             }
             int4           h, h2;
-            h.x  = __float_as_int((unsigned) (bw >> 32) == 0u ? -CUDART_INF_F : key_to_float((unsigned) (bw >> 32)));
+            h.x  = __float_as_int((unsigned) (bw >> 32) == 0u ? -CUDART_INF_F : part_top(sh, cap_late));
             h.y  = (int) (0xffffffffu - (unsigned) (bw & 0xffffffffull));
             h.z  = sel ? n_cand : 0;
             h.w  = sh->st;

@@ -132,10 +132,13 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
 
 /* How a launch's (row, slice) items are dealt out to the stream kernel's thread blocks (gb::RunMap), the grid that
  * goes with it, and over how many thread blocks a row can be spread. A thread block's cost is taken as its items
- * plus kPartCost items' worth for every part of a row it touches (set-up, the first slice's threshold, the
- * record): five where rows may be top-k rows (measured: 256 whole rows beat 296 equal runs by 5 us of 51), one
- * where the caller said they are temperature / top-p rows (their parts set no threshold; equal runs measured
- * 6 - 10 % faster there), eight where the caller said they are greedy (whole rows need no finishing kernel). */
+ * plus kPartCost items' worth for every part of a row it touches (set-up, threshold, groups read again, record): five
+ * where rows may be top-k rows (with three, us: 200 x 128256 top-k 40 26.0 -> 31.7, 1000 x 65536 64.0 -> 76.2; with eight
+ * 150 x 128256 29.3 -> 22.3, 350 x 65536 34.9 -> 31.0, single rows of 8192 5 % slower), one where the caller said they
+ * are temperature / top-p rows (a temperature part has no threshold: 150 x 65536 23.9 us against 26.3 with three; a
+ * top-p part has one: 256 x 128256 on Gumbel rows 55.5 against 49.9, the hint does not tell them apart), eight where
+ * the caller said they are greedy (whole rows need no finishing kernel; with three 200 x 128256 19.6 -> 21.5, with five
+ * 350 x 65536 21.4 -> 19.7). */
 struct Deal {
     gb::RunMap map;
     int        grid;
@@ -226,7 +229,7 @@ struct geist_b200_ctx {
     Small *h_small = nullptr; /* pinned: settings in, token and status out, read and written by the kernels where it lies */
     std::mutex small_mu;      /* one synchronous host-pointer call at a time stages through the two words above */
 
-    /* kernel scratch: part records, candidate groups, segment sums, row counters, multi-pass row copies. kLanes
+    /* kernel scratch: part records with their candidates, segment sums, row counters, multi-pass row copies. kLanes
      * independent sets, used round-robin, so that up to kLanes launches may overlap on the GPU. */
     struct Lane {
         unsigned char *buf         = nullptr;

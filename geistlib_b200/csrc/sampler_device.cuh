@@ -72,12 +72,6 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
 /* mbarrier + bulk copy (global -> this CTA's shared memory only) */
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 /* Several barriers, then one pair of fences for all of them. */
 __device__ __forceinline__ void mbar_init_only(unsigned long long *bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -121,19 +115,6 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned 
     asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-    return ok != 0;
-}
-
-/* Non-blocking test of a phase (try_wait may suspend the thread for a while). */
-__device__ __forceinline__ bool mbar_test(unsigned long long *bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok)
             : "r"(smem_u32(bar)), "r"(parity)

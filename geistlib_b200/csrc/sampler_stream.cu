@@ -57,8 +57,8 @@ namespace gb {
 /* Optional instrumentation, compiled in with -DGB_PROFILE (and -DGB_PROFILE_CYC): PROF(i) stamps %globaltimer
  * at fixed points of a thread block's life (stream kernel 0-4, finishing kernels 5-13), MP(i) at the stages of
  * the multi-pass path, CYC(i) adds up a warp's cycles per section of the stream kernel's slice loop (0 wait for
- * data, 1 load + maxima + refill, 2 argmax / capture / raise, 4 loop top, 5 part set-up, 6 part end, 7 first
- * slice's threshold). The arrays are read back through geist_b200_debug_*. All of it is empty otherwise. */
+ * data, 2 maxima or sums with the refill, 4 loop top, 5 part set-up, 6 part end with the select). The arrays are
+ * read back through geist_b200_debug_*. All of it is empty otherwise. */
 #ifdef GB_PROFILE
 __device__ long long g_prof[1024][16];
 __device__ __forceinline__ long long gtime() {
@@ -132,23 +132,15 @@ struct __align__(16) GroupShared {
     int       wred_a[32];
     double    wred_d[32];
     long long wred_l[32];
-    int       bins[kHistBins];
     double    S;
-    float     tau;
     float     blk_max;
     int       blk_arg;
-    int       n_cand;
     int       n_dlist;
     int       n_sel;
-    int       n_border;
     int       b_star;
     int       n_hi;
     int       flag;
     int       pick;
-    unsigned  tau_key;       /* ordered key of the select threshold */
-    int       cur_row;
-    float     hmax[kHistBins]; /* finisher: slice maxima of the row */
-    int       harg[kHistBins]; /* finisher: their first ids */
 };
 
 /* float4 of a slice that one warp owns: an equal share, rounded up to whole warp steps */
@@ -451,24 +443,6 @@ __device__ __forceinline__ void group_argmax(const Grp &g, GroupShared *sh, floa
     g.sync();
     v = sh->blk_max;
     a = sh->blk_arg;
-}
-
-/* Maximum over the group (values only); one barrier less than group_argmax. */
-__device__ __forceinline__ float group_max(const Grp &g, GroupShared *sh, float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    }
-    g.sync();
-    if (g.lane == 0) {
-        sh->wred_f[g.warp] = v;
-    }
-    g.sync();
-    float m = sh->wred_f[0];
-    for (int w = 1; w < g.nw; w++) {
-        m = fmaxf(m, sh->wred_f[w]);
-    }
-    return m;
 }
 
 /* Every thread gets the same total (fixed order of additions). */
@@ -2322,7 +2296,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *ring    = smem_raw;
     StreamShared  *sh      = reinterpret_cast<StreamShared *>(smem_raw + (size_t) kWarps * kStages * kWarpStageBytes);
-    unsigned char *gmem    = reinterpret_cast<unsigned char *>(sh + 1); /* candidate groups of the part in work */
+    unsigned char *gmem    = reinterpret_cast<unsigned char *>(sh + 1); /* what belongs to the part in work alone */
     float         *gmax    = reinterpret_cast<float *>(gmem); /* [kGroupSlots][kThreads] */
     unsigned      *sl_list = reinterpret_cast<unsigned *>(gmem + kGroupBytes); /* long histories: the part's entries of the row's prepared list, when they fit */
 

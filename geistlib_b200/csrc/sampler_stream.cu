@@ -2039,12 +2039,23 @@ __device__ __forceinline__ int row_id_count(const SampleParams &p, int hist_len,
     return H + E;
 }
 
-/* The `total` candidates in sh->cand by (value desc, id asc): the k best to sh->fin_s. All of them lie between lo and hi.
+/* The part's maximum, as its candidates are. */
+__device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late) {
+    unsigned long long b = 0ull;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        b = max(b, sh->best[w]);
+    }
+    const float top = key_to_float((unsigned) (b >> 32));
+    return cap_late && top > -CUDART_INF_F ? soft_cap(top, sh->cap) : top;
+}
+
+/* The `total` candidates in sh->cand by (value desc, id asc): the k best to sh->fin_s. None lies below lo.
  * Up to 128 are ranked one against all. More are dealt out to 256 bins of values first, the highest in front, and
  * ranked against their own bin: one against all costs a thread block total^2 / 32 rounds of six instructions. 1000 rows
  * of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9; 256 x 128256 top-k 200 48.9 -> 41.0. */
 constexpr int kRankFew = 128;
-__device__ __forceinline__ void rank_candidates(StreamShared *sh, unsigned char *gmem, int total, int k, float lo, float hi) {
+__device__ __forceinline__ void rank_candidates(StreamShared *sh, unsigned char *gmem, int total, int k, float lo, bool cap_late) {
     const int tid = (int) threadIdx.x, lane = tid & 31;
     if (total <= kRankFew) {
 #pragma unroll 1
@@ -2063,6 +2074,7 @@ __device__ __forceinline__ void rank_candidates(StreamShared *sh, unsigned char 
     }
     Pair       *srt   = reinterpret_cast<Pair *>(gmem); /* the group maxima are done with */
     int        *start = reinterpret_cast<int *>(srt + kPartCand), *next = start + kHistBins + 1;
+    const float hi    = part_top(sh, cap_late);
     const float scale = hi > lo && hi - lo < CUDART_INF_F ? (float) kHistBins / (hi - lo) : 0.0f; /* 0: one bin for all */
     auto        bin_of = [&](float v) { return kHistBins - 1 - min(kHistBins - 1, max(0, __float2int_rz((v - lo) * scale))); };
     for (int i = tid; i <= kHistBins; i += kThreads) {
@@ -2121,15 +2133,15 @@ __device__ __forceinline__ void rank_candidates(StreamShared *sh, unsigned char 
 
 /*
  * A top-k row that went through one thread block as a whole, finished by that thread block from its own candidates
- * (all threads call): put in order, the k best get their exact weights and the draw is made as in finish_row. lo and hi:
- * no candidate lies below or above. What does not fit here (more candidates than the list holds, fewer than k) is handed
- * back with ST_RETRY.
+ * (all threads call): put in order, the k best get their exact weights and the draw is made as in finish_row. No
+ * candidate lies below lo. What does not fit here (more candidates than the list holds, fewer than k) is handed back
+ * with ST_RETRY.
  */
-__device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, unsigned char *gmem, int row, int total, int k, float lo, float hi, float inv_t, int st_bits) {
+__device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, unsigned char *gmem, int row, int total, int k, float lo, bool cap_late, float inv_t, int st_bits) {
     const int tid = (int) threadIdx.x;
     const bool ok = total <= kPartCand && total >= k && k <= kFastKMax;
     if (ok) {
-        rank_candidates(sh, gmem, total, k, lo, hi);
+        rank_candidates(sh, gmem, total, k, lo, cap_late);
         __syncthreads();
         const float m = sh->fin_s[0].v;
         for (int i = tid; i < k; i += kThreads) {
@@ -2252,17 +2264,6 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
         }
     }
     stage = kPrefetchDone;
-}
-
-/* The part's maximum, as its candidates are. */
-__device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late) {
-    unsigned long long b = 0ull;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        b = max(b, sh->best[w]);
-    }
-    const float top = key_to_float((unsigned) (b >> 32));
-    return cap_late && top > -CUDART_INF_F ? soft_cap(top, sh->cap) : top;
 }
 
 /* The largest of the warps' references of a part. */
@@ -2910,8 +2911,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             over            = sh->n_grp > kPartCand && !(cap_late && tau > -CUDART_INF_F);
             const int  n_grp = over ? 0 : sh->n_grp, per_log = kNV4Log + gm_shift;
             double    fix   = 0.0;
-            for (int t0 = 0; t0 < n_grp << per_log; t0 += kThreads) { /* whole warps: ids are looked up by all lanes together */
-                const int  t = t0 + tid, name = t < n_grp << per_log ? sh->grp[t >> per_log] : 0, f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
+            for (int t0 = 32 * warp; t0 < n_grp << per_log; t0 += kThreads) { /* whole warps: ids are looked up by all lanes together */
+                const int  t = t0 + lane, name = t < n_grp << per_log ? sh->grp[t >> per_log] : 0, f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
                 const int  s = ((name >> 8) << gm_shift) + f / kNV4, c = c0 + s, i4 = l + 32 * (f % kNV4);
                 const bool last_c = c == p.n_slices - 1;
                 const int  n = last_c ? n_last : n_full, nv4 = (n + 3) >> 2, L = share_len(nv4), w4 = min(w * L, nv4);
@@ -3031,7 +3032,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
              * part); a row of another kind is reported as the small finishing kernel would */
             if (mode == M_TOPK) {
-                inline_finish_topk(p, sh, gmem, row, n_cand, kq, tau, part_top(sh, cap_late), inv_t, sh->st);
+                inline_finish_topk(p, sh, gmem, row, n_cand, kq, tau, cap_late, inv_t, sh->st);
             } else {
                 if (tid == 0) {
                     p.tokens[row] = -1;

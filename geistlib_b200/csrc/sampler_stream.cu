@@ -2050,28 +2050,13 @@ __device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late)
     return cap_late && top > -CUDART_INF_F ? soft_cap(top, sh->cap) : top;
 }
 
-/* The `total` candidates in sh->cand by (value desc, id asc): the k best to sh->fin_s. None lies below lo.
- * Up to 128 are ranked one against all. More are dealt out to 256 bins of values first, the highest in front, and
- * ranked against their own bin: one against all costs a thread block total^2 / 32 rounds of six instructions. 1000 rows
- * of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9; 256 x 128256 top-k 200 48.9 -> 41.0. */
+/* More than kRankFew candidates in order, the k best to sh->fin_s; none lies below lo. They are dealt out to 256 bins of
+ * values, the highest in front, and ranked against their own bin: one against all costs a thread block total^2 / 32
+ * rounds of six instructions. 1000 rows of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9;
+ * 256 x 128256 top-k 200 48.9 -> 41.0. */
 constexpr int kRankFew = 128;
-__device__ __forceinline__ void rank_candidates(StreamShared *sh, unsigned char *gmem, int total, int k, float lo, bool cap_late) {
+__device__ __noinline__ void rank_in_bins(StreamShared *sh, unsigned char *gmem, int total, int k, float lo, bool cap_late) {
     const int tid = (int) threadIdx.x, lane = tid & 31;
-    if (total <= kRankFew) {
-#pragma unroll 1
-        for (int i = tid; i < total; i += kThreads) {
-            const Pair me   = sh->cand[i];
-            int        rank = 0;
-#pragma unroll 4
-            for (int j = 0; j < total; j++) {
-                rank += pair_before(sh->cand[j].v, sh->cand[j].idx, me.v, me.idx) ? 1 : 0;
-            }
-            if (rank < k) {
-                sh->fin_s[rank] = me;
-            }
-        }
-        return;
-    }
     Pair       *srt   = reinterpret_cast<Pair *>(gmem); /* the group maxima are done with */
     int        *start = reinterpret_cast<int *>(srt + kPartCand), *next = start + kHistBins + 1;
     const float hi    = part_top(sh, cap_late);
@@ -2131,17 +2116,177 @@ __device__ __forceinline__ void rank_candidates(StreamShared *sh, unsigned char 
     }
 }
 
+/* The largest of the warps' references of a part. */
+__device__ __forceinline__ float part_ref(const StreamShared *sh) {
+    float m = -CUDART_INF_F;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        m = fmaxf(m, sh->wb_ref[w]);
+    }
+    return m;
+}
+
+/* The terms of a float4, added up as every place that forms them adds them up. */
+__device__ __forceinline__ float sum_terms(const float4 &x, const SumScale &k, float ref) {
+    return __fadd_rn(__fadd_rn(sum_term(x.x, k, ref), sum_term(x.y, k, ref)), __fadd_rn(sum_term(x.z, k, ref), sum_term(x.w, k, ref)));
+}
+
+/* A part whose candidates outran their list, for raise_threshold. */
+struct PartAgain {
+    int             row, c0, part_len, gm_shift, kq;
+    bool            pro, sums; /* cap or mask to apply; top-p: the candidates leave the sum */
+    float           inv_t, ref;
+    double          acc;       /* the warp's sum, relative to ref */
+    bool            pen, long_ids;
+    float           rep, freq, pres;
+    double          rep_rcp;
+    const int      *long_off;  /* long histories: where the part's shares' runs start ... */
+    const unsigned *long_list; /* ... in this list */
+    bool            long_smem; /* the runs are in shared memory, as a short history's are */
+};
+
+/*
+ * A part whose candidates outran their list: its large values lie with a few threads (a row sorted along its ids, say),
+ * so the thread maxima let too many through. The threshold becomes the part's kq-th largest value, or less where the
+ * list has room for what reaches that: its key is built byte by byte from counts of the values that reach tau, read
+ * again in the groups that do; then the candidates are taken once more. Only equal values outrun the list now. All
+ * threads call; the caller's barrier follows. Out of line: rare, and in line its code cost every part of a row of a
+ * slice 2 - 4 %.
+ */
+__device__ __noinline__ float raise_threshold(const SampleParams &p, StreamShared *sh, const PartAgain &a, float tau) {
+    const int      tid = (int) threadIdx.x, lane = tid & 31, per_log = kNV4Log + a.gm_shift, n_grp = sh->n_grp;
+    const int      n_full = min(p.slice, p.V), n_last = p.V - (p.n_slices - 1) * p.slice;
+    const float   *src    = row_again(p, a.row);
+    const SumScale ks     = sum_scale2(a.inv_t);
+    int           *bins   = reinterpret_cast<int *>(sh->fin_q);
+    unsigned       prefix = 0u;
+    int            need   = a.kq;
+    for (int level = 3;; level--) { /* the byte that is counted; -1: the candidates are taken */
+        __syncthreads(); /* the counts, and before them the candidates, have been read */
+        bins[tid] = 0;
+        if (tid == 0) {
+            sh->n_cand = 0;
+        }
+        __syncthreads();
+        double fix = 0.0;
+        for (int t = tid; t < n_grp << per_log; t += kThreads) {
+            const int name = sh->grp[t >> per_log], f = t & ((1 << per_log) - 1), w = (name & 255) >> 5;
+            const int s = ((name >> 8) << a.gm_shift) + f / kNV4, c = a.c0 + s, i4 = (name & 31) + 32 * (f % kNV4);
+            const int n = c == p.n_slices - 1 ? n_last : n_full, nv4 = (n + 3) >> 2, L = share_len(nv4), w4 = min(w * L, nv4);
+            if (s >= a.part_len || i4 >= min(L, nv4 - w4)) {
+                continue;
+            }
+            float v[4];
+            bool  any = false;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int e = 4 * (w4 + i4) + q, id = c * p.slice + e, off = 4 * i4 + q, bit = id_bit(s, w, off);
+                v[q] = -CUDART_INF_F;
+                if (e >= n) {
+                    continue;
+                }
+                v[q] = src[id];
+                if (a.pro) {
+                    v[q] = prologue_one(v[q], id, sh->cap, sh->mrow);
+                }
+                if (a.pen && ((sh->id_bits[bit >> 5] >> (bit & 31)) & 1u) != 0u) {
+                    const int       g   = a.long_ids ? s * kWarps + w : (s & 31) * kWarps + w;
+                    const unsigned *ent = a.long_ids ? a.long_list : reinterpret_cast<const unsigned *>(sh->rl_id);
+                    const int       lo  = a.long_smem ? sh->rl_cnt[g] : a.long_off[g], hi = a.long_smem ? sh->rl_cnt[g + 1] : a.long_off[g + 1];
+                    for (int i = lo; i < hi; i++) {
+                        if ((int) (ent[i] & 0x3ffu) == off && (a.long_ids || (int) (ent[i] >> 20) == s >> 5)) {
+                            v[q] = penalise_rcp(v[q], (int) ((ent[i] >> 10) & (a.long_ids ? 0x3fffffu : 0x3ffu)), a.rep_rcp, a.rep, a.freq, a.pres);
+                        }
+                    }
+                }
+                if (v[q] >= tau) {
+                    const unsigned key = order_key(v[q]);
+                    if (level < 0) {
+                        const int pos = atomicAdd(&sh->n_cand, 1);
+                        if (pos < kPartCand) {
+                            sh->cand[pos].v   = v[q];
+                            sh->cand[pos].idx = id;
+                        }
+                        any = true;
+                    } else if (level == 3 || (key >> (8 * level + 8)) == (prefix >> (8 * level + 8))) {
+                        atomicAdd(&bins[(key >> (8 * level)) & 255u], 1);
+                    }
+                }
+            }
+            if (a.sums && any) { /* as where the candidates are taken first */
+                const float u  = s < kSliceRefs ? sh->ref_at[s][w] : p.segs[((size_t) a.row * (size_t) p.n_slices + (size_t) c) * kWarps + w].ref;
+                const float u0 = u == -CUDART_INF_F ? 0.0f : u;
+                double      now = -(double) sum_terms(make_float4(v[0], v[1], v[2], v[3]), ks, u0);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (!(v[q] >= tau)) {
+                        now += (double) sum_term(v[q], ks, u0);
+                    }
+                }
+                fix += now * ref_move(u, part_ref(sh), a.inv_t);
+            }
+        }
+        if (level < 0) {
+            if (a.sums) {
+                fix = warp_sum_d(fix);
+                if (lane == 0) {
+                    sh->wb_sum[tid >> 5] = a.acc * ref_move(a.ref, part_ref(sh), a.inv_t) + fix;
+                }
+            }
+            return tau;
+        }
+        __syncthreads();
+        const int b     = top_bin(bins, lane, need);
+        int       above = 0;
+        for (int i = b + 1 + lane; i < 256; i += 32) {
+            above += bins[i];
+        }
+        need -= __reduce_add_sync(0xffffffffu, above);
+        prefix |= (unsigned) b << (8 * level);
+        if (level == 0 || a.kq - need + bins[b] <= kPartCand) { /* what has a larger key, and this byte's */
+            tau   = fmaxf(tau, prefix <= order_key(-CUDART_INF_F) ? -CUDART_INF_F : key_to_float(prefix));
+            level = 0;
+        }
+    }
+}
+
 /*
  * A top-k row that went through one thread block as a whole, finished by that thread block from its own candidates
  * (all threads call): put in order, the k best get their exact weights and the draw is made as in finish_row. No
- * candidate lies below lo. What does not fit here (more candidates than the list holds, fewer than k) is handed back
- * with ST_RETRY.
+ * candidate lies below lo. Where they outran their list, finish_raised raises the threshold first. What does not fit
+ * then (more equal values than the list holds, fewer than k) is handed back with ST_RETRY. What is rare is called out of
+ * line and from branches that are there anyway: code that every row jumps over costs rows of a slice 2 - 4 %, code that
+ * is called for the first time in a while a microsecond (k = 100 on 256 x 128256: 36.6 us with all of this behind one call).
  */
-__device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, unsigned char *gmem, int row, int total, int k, float lo, bool cap_late, float inv_t, int st_bits) {
+__device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, const PartAgain &again, float lo, bool cap_late, float inv_t, int st_bits);
+template <bool kRaise, class Again>
+__device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, unsigned char *gmem, int row, int total, int k, float lo, bool cap_late, float inv_t, int st_bits,
+                                                   Again &&again) {
     const int tid = (int) threadIdx.x;
     const bool ok = total <= kPartCand && total >= k && k <= kFastKMax;
+    if constexpr (kRaise) {
+        if (!ok && total > kPartCand && lo > -CUDART_INF_F) { /* below -inf there is nothing to raise: fewer than kq threads met a finite value */
+            finish_raised(p, sh, gmem, again(), lo, cap_late, inv_t, st_bits);
+            return;
+        }
+    }
     if (ok) {
-        rank_candidates(sh, gmem, total, k, lo, cap_late);
+        if (total <= kRankFew) {
+#pragma unroll 1
+            for (int i = tid; i < total; i += kThreads) {
+                const Pair me   = sh->cand[i];
+                int        rank = 0;
+#pragma unroll 4
+                for (int j = 0; j < total; j++) {
+                    rank += pair_before(sh->cand[j].v, sh->cand[j].idx, me.v, me.idx) ? 1 : 0;
+                }
+                if (rank < k) {
+                    sh->fin_s[rank] = me;
+                }
+            }
+        } else {
+            rank_in_bins(sh, gmem, total, k, lo, cap_late);
+        }
         __syncthreads();
         const float m = sh->fin_s[0].v;
         for (int i = tid; i < k; i += kThreads) {
@@ -2212,6 +2357,12 @@ __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, Stream
     __syncthreads();
 }
 
+__device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, const PartAgain &again, float lo, bool cap_late, float inv_t, int st_bits) {
+    const float tau = raise_threshold(p, sh, again, lo);
+    __syncthreads();
+    inline_finish_topk<false>(p, sh, gmem, again.row, min(sh->n_cand, kPartCand + 1), again.kq, tau, cap_late, inv_t, st_bits, 0);
+}
+
 /*
  * A row's parameters cost up to two dependent memory round trips (slot -> parameters and history ids). Warp 0
  * fetches them for the NEXT row of the run with 4-byte asynchronous copies into shared memory, one step per
@@ -2264,21 +2415,6 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
         }
     }
     stage = kPrefetchDone;
-}
-
-/* The largest of the warps' references of a part. */
-__device__ __forceinline__ float part_ref(const StreamShared *sh) {
-    float m = -CUDART_INF_F;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        m = fmaxf(m, sh->wb_ref[w]);
-    }
-    return m;
-}
-
-/* The terms of a float4, added up as every place that forms them adds them up. */
-__device__ __forceinline__ float sum_terms(const float4 &x, const SumScale &k, float ref) {
-    return __fadd_rn(__fadd_rn(sum_term(x.x, k, ref), sum_term(x.y, k, ref)), __fadd_rn(sum_term(x.z, k, ref), sum_term(x.w, k, ref)));
 }
 
 /* Which kinds of rows an instantiation of the stream kernel carries the code for: every one carries greedy rows;
@@ -3026,13 +3162,37 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             }
         }
         __syncthreads();
-        const int n_cand = over ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
-        const int held   = sel ? min(n_cand, kPartCand) : 0;
+        auto part_again = [&]() {
+            constexpr bool kPen = (kKinds & K_PEN) != 0, kLong = kPen && (kKinds & K_SHORT) == 0, kSums = (kKinds & K_SUMS) != 0;
+            const bool     done = !kPlain && p.out_logits != nullptr;
+            PartAgain      again;
+            again.row       = row;
+            again.c0        = c0;
+            again.part_len  = part_len;
+            again.gm_shift  = gm_shift;
+            again.kq        = kq;
+            again.pro       = !kPlain && pro_on && !done;
+            again.sums      = kSums && sums;
+            again.inv_t     = kSums ? inv_t : 1.0f;
+            again.ref       = kSums ? ref : 0.0f;
+            again.acc       = kSums ? acc : 0.0;
+            again.pen       = kPen && pen_on && !done;
+            again.rep       = kPen ? rep : 1.0f;
+            again.freq      = kPen ? freq : 0.0f;
+            again.pres      = kPen ? pres : 0.0f;
+            again.rep_rcp   = kPen ? rep_rcp : 1.0;
+            again.long_ids  = kLong && long_ids;
+            again.long_off  = kLong ? long_off : nullptr;
+            again.long_smem = !kLong || long_smem;
+            again.long_list = !kLong ? nullptr : long_smem ? sl_list : p.pre_list + (size_t) row * (size_t) p.row_cap;
+            return again;
+        };
+        int       n_cand = over ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
         if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
             /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
              * part); a row of another kind is reported as the small finishing kernel would */
             if (mode == M_TOPK) {
-                inline_finish_topk(p, sh, gmem, row, n_cand, kq, tau, cap_late, inv_t, sh->st);
+                inline_finish_topk<true>(p, sh, gmem, row, n_cand, kq, tau, cap_late, inv_t, sh->st, part_again);
             } else {
                 if (tid == 0) {
                     p.tokens[row] = -1;
@@ -3043,6 +3203,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             CYC(6);
             continue;
         }
+        if (sel && n_cand > kPartCand && tau > -CUDART_INF_F) {
+            tau = raise_threshold(p, sh, part_again(), tau);
+            __syncthreads();
+            n_cand = min(sh->n_cand, kPartCand + 1);
+        }
+        const int held = sel ? min(n_cand, kPartCand) : 0;
         if (tid == 0) {
             unsigned long long bw = 0ull;
 #pragma unroll

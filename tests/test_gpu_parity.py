@@ -632,3 +632,29 @@ def test_wide_sets_finished_by_the_stream_kernel(ctx, k, V):
     assert done[few_ties].all()
     o = oracle.port.sample_batch(x, 3.0, k, 1.0, st)
     assert np.array_equal(g["tokens"][done], o["tokens"][done])
+
+
+@pytest.mark.parametrize("V", [1450, 3748, 24268, 70000])
+@pytest.mark.parametrize("slope", [-80.0, 80.0, -25.0])
+def test_rows_sorted_along_their_ids(ctx, V, slope):
+    """Rows whose large values lie with a few threads (logits that fall or rise along the ids): the thread maxima alone let
+    thousands of values through, the threshold is raised until the k best fit. No row asks to be launched again or goes
+    the long way; kept sets come in order."""
+    rows = 310
+    x = normal_logits(rows, V, 0.5, V) + np.linspace(0.0, slope, V, dtype=np.float32)
+    x[1::4] -= 100.0
+    K = np.resize(np.array([2, 40, 100, 128, 129, 200, 256], np.int32), rows)
+    st = independent_states(oracle.port, V, rows)
+    o = oracle.port.sample_batch(x, 2.0, K, 1.0, st, detail_cap=256)
+    for hint, cap in [(1, 0), (0, 0), (0, 256)]:
+        g = run_gpu(ctx, x, 2.0, K, 1.0, st, finish_hint=hint, kept_cap=cap)
+        assert (g["status"] & (32 | 2) == 0).all()
+        check_tokens(g, o)
+    for r in range(rows):
+        assert np.array_equal(g["kept_idx"][r, :K[r]], o["detail_idx"][r, :K[r]]), r
+    h = histories(rows, 300, V, V)
+    h[:, :100] = np.argsort(-x, axis=1)[:, :100]
+    g = run_gpu(ctx, x, 2.0, K, 1.0, st, finish_hint=1, history=h, rep=1.2, freq=0.1)
+    assert (g["status"] & 32 == 0).all()
+    check_tokens(g, oracle.port.sample_batch(x, 2.0, K, 1.0, st, hist=h, rep=1.2, freq=0.1))
+    check_tokens(run_gpu(ctx, x, 0.4, 0, 0.9, st), oracle.port.sample_batch(x, 0.4, 0, 0.9, st))

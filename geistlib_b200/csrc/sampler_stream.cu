@@ -1228,6 +1228,19 @@ constexpr int kIdBits = 4 * kSliceMax;
 /* Where the bit of a value lies: slice of the part, warp, offset in the share. */
 __device__ __forceinline__ int id_bit(int s, int w, int off) { return ((s & 3) * kWarps + w) * (kSliceMax / kWarps) + off; }
 
+/* A part whose candidates outran their list, for raise_threshold. */
+struct PartAgain {
+    int             row, c0, part_len, gm_shift, kq;
+    bool            pro, sums; /* cap or mask to apply; top-p: the candidates leave the sum */
+    float           inv_t;
+    bool            pen, long_ids;
+    float           rep, freq, pres;
+    double          rep_rcp;
+    const int      *long_off;  /* long histories: where the part's shares' runs start ... */
+    const unsigned *long_list; /* ... in this list */
+    bool            long_smem; /* the runs are in shared memory, as a short history's are */
+};
+
 /* What the warps of one thread block share. The ring (every warp's two stages) lies in front of it in dynamic
  * shared memory, the group maxima of the part in work behind it. */
 struct __align__(16) StreamShared {
@@ -1236,7 +1249,8 @@ struct __align__(16) StreamShared {
     int                st;        /* status bits of the part */
     unsigned long long best[kWarps];               /* (key of the maximum, ~first id) per warp */
     float              wb_ref[kWarps];             /* top-p: what the warp's sum is relative to ... */
-    double             wb_sum[kWarps];             /* ... and that sum without the candidates, relative to the part's reference */
+    double             wb_acc[kWarps];             /* ... that sum ... */
+    double             wb_sum[kWarps];             /* ... and the sum without the candidates, relative to the part's reference */
     float              ref_at[kSliceRefs][kWarps]; /* top-p: what a slice's terms were formed relative to */
     int                rl_id[kRowIds], rl_cnt[kRowIds + 4]; /* the row's distinct history ids as (offset in the share | count << 10 | tag << 20),
                                                              * grouped by the (slice, warp) share they fall into, and where each group's run starts */
@@ -1246,6 +1260,7 @@ struct __align__(16) StreamShared {
     int                max_cnt;               /* how often the part's most frequent id occurs (asked where that raises a value) */
     unsigned short     grp[kGroupSlots * kThreads]; /* (slot << 8) | thread */
     alignas(8) Pair    cand[kPartCand];
+    PartAgain          again;                 /* what raise_threshold needs to know of the part */
     /* finishing inside the stream kernel (F_INLINE_TOPK): the k best in order, their weights */
     int                cur_rr;
     Pair               fin_s[kFastKMax];
@@ -2131,20 +2146,6 @@ __device__ __forceinline__ float sum_terms(const float4 &x, const SumScale &k, f
     return __fadd_rn(__fadd_rn(sum_term(x.x, k, ref), sum_term(x.y, k, ref)), __fadd_rn(sum_term(x.z, k, ref), sum_term(x.w, k, ref)));
 }
 
-/* A part whose candidates outran their list, for raise_threshold. */
-struct PartAgain {
-    int             row, c0, part_len, gm_shift, kq;
-    bool            pro, sums; /* cap or mask to apply; top-p: the candidates leave the sum */
-    float           inv_t, ref;
-    double          acc;       /* the warp's sum, relative to ref */
-    bool            pen, long_ids;
-    float           rep, freq, pres;
-    double          rep_rcp;
-    const int      *long_off;  /* long histories: where the part's shares' runs start ... */
-    const unsigned *long_list; /* ... in this list */
-    bool            long_smem; /* the runs are in shared memory, as a short history's are */
-};
-
 /*
  * A part whose candidates outran their list: its large values lie with a few threads (a row sorted along its ids, say),
  * so the thread maxima let too many through. The threshold becomes the part's kq-th largest value, or less where the
@@ -2153,7 +2154,9 @@ struct PartAgain {
  * threads call; the caller's barrier follows. Out of line: rare, and in line its code cost every part of a row of a
  * slice 2 - 4 %.
  */
-__device__ __noinline__ float raise_threshold(const SampleParams &p, StreamShared *sh, const PartAgain &a, float tau) {
+__device__ __noinline__ float raise_threshold(const SampleParams &p, StreamShared *sh, float tau) {
+    __syncthreads(); /* the part's description is there */
+    const PartAgain &a = sh->again;
     const int      tid = (int) threadIdx.x, lane = tid & 31, per_log = kNV4Log + a.gm_shift, n_grp = sh->n_grp;
     const int      n_full = min(p.slice, p.V), n_last = p.V - (p.n_slices - 1) * p.slice;
     const float   *src    = row_again(p, a.row);
@@ -2230,7 +2233,7 @@ __device__ __noinline__ float raise_threshold(const SampleParams &p, StreamShare
             if (a.sums) {
                 fix = warp_sum_d(fix);
                 if (lane == 0) {
-                    sh->wb_sum[tid >> 5] = a.acc * ref_move(a.ref, part_ref(sh), a.inv_t) + fix;
+                    sh->wb_sum[tid >> 5] = sh->wb_acc[tid >> 5] * ref_move(sh->wb_ref[tid >> 5], part_ref(sh), a.inv_t) + fix;
                 }
             }
             return tau;
@@ -2258,7 +2261,7 @@ __device__ __noinline__ float raise_threshold(const SampleParams &p, StreamShare
  * line and from branches that are there anyway: code that every row jumps over costs rows of a slice 2 - 4 %, code that
  * is called for the first time in a while a microsecond (k = 100 on 256 x 128256: 36.6 us with all of this behind one call).
  */
-__device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, const PartAgain &again, float lo, bool cap_late, float inv_t, int st_bits);
+__device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, float lo, bool cap_late, int st_bits);
 template <bool kRaise, class Again>
 __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, StreamShared *sh, unsigned char *gmem, int row, int total, int k, float lo, bool cap_late, float inv_t, int st_bits,
                                                    Again &&again) {
@@ -2266,7 +2269,8 @@ __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, Stream
     const bool ok = total <= kPartCand && total >= k && k <= kFastKMax;
     if constexpr (kRaise) {
         if (!ok && total > kPartCand && lo > -CUDART_INF_F) { /* below -inf there is nothing to raise: fewer than kq threads met a finite value */
-            finish_raised(p, sh, gmem, again(), lo, cap_late, inv_t, st_bits);
+            again();
+            finish_raised(p, sh, gmem, lo, cap_late, st_bits);
             return;
         }
     }
@@ -2357,10 +2361,10 @@ __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, Stream
     __syncthreads();
 }
 
-__device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, const PartAgain &again, float lo, bool cap_late, float inv_t, int st_bits) {
-    const float tau = raise_threshold(p, sh, again, lo);
+__device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, float lo, bool cap_late, int st_bits) {
+    const float tau = raise_threshold(p, sh, lo);
     __syncthreads();
-    inline_finish_topk<false>(p, sh, gmem, again.row, min(sh->n_cand, kPartCand + 1), again.kq, tau, cap_late, inv_t, st_bits, 0);
+    inline_finish_topk<false>(p, sh, gmem, sh->again.row, min(sh->n_cand, kPartCand + 1), sh->again.kq, tau, cap_late, sh->again.inv_t, st_bits, 0);
 }
 
 /*
@@ -3157,15 +3161,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             if ((kKinds & K_SUMS) != 0 && sums) {
                 fix = warp_sum_d(fix);
                 if (lane == 0) { /* with the warp's own sum: each warp moves its own */
+                    sh->wb_acc[warp] = acc;
                     sh->wb_sum[warp] = acc * ref_move(ref, part_ref(sh), inv_t) + fix;
                 }
             }
         }
         __syncthreads();
-        auto part_again = [&]() {
+        auto part_again = [&]() { /* raise_threshold is called next; its arguments lie here and not in a stack frame */
+            if (tid != 0) {
+                return;
+            }
             constexpr bool kPen = (kKinds & K_PEN) != 0, kLong = kPen && (kKinds & K_SHORT) == 0, kSums = (kKinds & K_SUMS) != 0;
             const bool     done = !kPlain && p.out_logits != nullptr;
-            PartAgain      again;
+            PartAgain     &again = sh->again;
             again.row       = row;
             again.c0        = c0;
             again.part_len  = part_len;
@@ -3173,9 +3181,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             again.kq        = kq;
             again.pro       = !kPlain && pro_on && !done;
             again.sums      = kSums && sums;
-            again.inv_t     = kSums ? inv_t : 1.0f;
-            again.ref       = kSums ? ref : 0.0f;
-            again.acc       = kSums ? acc : 0.0;
+            again.inv_t     = inv_t;
             again.pen       = kPen && pen_on && !done;
             again.rep       = kPen ? rep : 1.0f;
             again.freq      = kPen ? freq : 0.0f;
@@ -3185,7 +3191,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             again.long_off  = kLong ? long_off : nullptr;
             again.long_smem = !kLong || long_smem;
             again.long_list = !kLong ? nullptr : long_smem ? sl_list : p.pre_list + (size_t) row * (size_t) p.row_cap;
-            return again;
         };
         int       n_cand = over ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
         if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
@@ -3204,7 +3209,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             continue;
         }
         if (sel && n_cand > kPartCand && tau > -CUDART_INF_F) {
-            tau = raise_threshold(p, sh, part_again(), tau);
+            part_again();
+            tau = raise_threshold(p, sh, tau);
             __syncthreads();
             n_cand = min(sh->n_cand, kPartCand + 1);
         }

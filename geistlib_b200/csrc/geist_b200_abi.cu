@@ -66,6 +66,7 @@ extern "C" const char *geist_b200_errmsg(void) { return g_err.c_str(); }
 namespace {
 
 constexpr size_t kSmemMax = 227 * 1024; /* opt-in shared memory per CTA on sm_100 */
+constexpr size_t kHeadInts = 16;       /* words in front of a lane's per-slot words */
 constexpr int    kLanes   = 4;          /* launches of one context that may overlap on the GPU */
 
 struct Plan {
@@ -234,7 +235,7 @@ struct geist_b200_ctx {
     struct Lane {
         unsigned char *buf         = nullptr;
         size_t         bytes       = 0;
-        int           *counters    = nullptr; /* one flag per row copy of the multi-pass path */
+        int           *counters    = nullptr; /* kHeadInts words of the launch, then per row copy a wide row's words, its histogram, a flag */
         int           *arrive      = nullptr; /* one counter per row: parts that have published (greedy launches); zero between launches */
         size_t         arrive_cap  = 0;
         size_t         counter_cap = 0;
@@ -415,14 +416,19 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     const size_t gen_bmw  = (b->n_vocab + 31) / 32;
     const size_t gen_hcap = hist_max ? std::min(hist_max, b->n_vocab) : 0;
     const size_t off_seg  = round_up(n_rows * parts * (size_t) gb::kPartBytes, 256);
-    const int    fin_grid = (int) std::min<size_t>((size_t) pl.fin_ctas, n_rows);
-    const size_t slots    = (size_t) fin_grid; /* row copies of the multi-pass path: one per finishing thread block that can run at a time */
+    const size_t slots    = std::min<size_t>((size_t) pl.fin_ctas, n_rows); /* row copies of the multi-pass path: one per finishing thread block that can run at a time */
+    /* The general finishing kernel gets thread blocks that own no row as well: they help with wide top-p rows, two pieces
+     * per warp. */
+    const bool   general  = (p.flags & (gb::F_FAST_ONLY | gb::F_SELECT_ONLY)) == 0u;
+    const size_t pieces   = (b->n_vocab + gb::kWidePiece - 1) / gb::kWidePiece;
+    const int    fin_grid = (int) std::min<size_t>((size_t) pl.fin_ctas, general ? n_rows * std::max<size_t>(1, pieces / (2 * gb::kWarps)) : n_rows);
     const size_t off_rows = round_up(off_seg + n_items * (size_t) gb::kWarps * sizeof(gb::SegRec), 256);
     const size_t off_bm   = round_up(off_rows + slots * gen_str * 4, 256);
     const size_t off_dl   = round_up(off_bm + slots * gen_bmw * 4, 256);
     const size_t gen_lcap = std::min<size_t>(b->n_vocab, 16384); /* entries of one histogram bin that the multi-pass path picks out of a row */
     const size_t off_ls   = round_up(off_dl + slots * gen_hcap * sizeof(gb::Pair), 256);
-    const size_t off_pl   = round_up(off_ls + slots * gen_lcap * sizeof(gb::Pair), 256);
+    const size_t off_wp   = round_up(off_ls + slots * gen_lcap * sizeof(gb::Pair), 256);
+    const size_t off_pl   = round_up(off_wp + slots * pieces * (size_t) gb::kWidePartBytes, 256);
     const size_t off_po   = round_up(off_pl + (pl.id_slots ? n_rows * (size_t) pl.row_cap * 4 : 0), 256);
     const size_t need     = round_up(off_po + (pl.id_slots ? n_rows * ((size_t) pl.n_slices * (size_t) gb::kWarps + 1) * 4 : 0), 256) + 256;
     geist_b200_ctx::Lane *ln;
@@ -436,15 +442,17 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
             CUDA_TRY(cudaMalloc((void **) &ln->buf, need));
             ln->bytes = need;
         }
-        if (ln->counter_cap < slots) {
+        if (ln->counter_cap < slots && (p.flags & gb::F_FAST_ONLY) == 0u) {
             cudaFree(ln->counters);
             ln->counters    = nullptr;
             ln->counter_cap = 0;
-            const size_t cap = round_up(slots, 1024);
-            /* one flag per row copy of the multi-pass path, zero between launches (whoever takes a copy gives it
-             * back). Zeroed on the launch's own stream, so the first kernel that uses them comes behind it. */
-            CUDA_TRY(cudaMalloc((void **) &ln->counters, cap * sizeof(int)));
-            CUDA_TRY(cudaMemsetAsync(ln->counters, 0, cap * sizeof(int), st));
+            const size_t cap = round_up(slots, 32);
+            /* per row copy of the multi-pass path a flag, and a wide row's words and histogram, all zero between launches
+             * (whoever takes a copy gives it back as it was). Zeroed on the launch's own stream, so the first kernel that
+             * uses them comes behind it. */
+            const size_t bytes = (kHeadInts + cap * (size_t) (1 + gb::kWideCtlInts + gb::kWideBins)) * sizeof(int);
+            CUDA_TRY(cudaMalloc((void **) &ln->counters, bytes));
+            CUDA_TRY(cudaMemsetAsync(ln->counters, 0, bytes, st));
             ln->counter_cap = cap;
         }
         if ((p.flags & gb::F_GREEDY_ONLY) != 0u && ln->arrive_cap < n_rows) {
@@ -458,7 +466,13 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
             ln->arrive_cap = cap;
         }
     }
-    p.pool             = ln->counters;
+    if (ln->counters != nullptr) {
+        p.wide_head = reinterpret_cast<gb::WideHead *>(ln->counters);
+        p.wide_ctl  = reinterpret_cast<gb::WideCtl *>(ln->counters + kHeadInts);
+        p.wide_hist = reinterpret_cast<unsigned *>(ln->counters + kHeadInts + ln->counter_cap * (size_t) gb::kWideCtlInts);
+        p.pool      = ln->counters + kHeadInts + ln->counter_cap * (size_t) (gb::kWideCtlInts + gb::kWideBins);
+    }
+    p.wide_part        = reinterpret_cast<gb::WidePart *>(ln->buf + off_wp);
     p.arrive           = ln->arrive;
     p.pool_slots       = (int) slots;
     p.parts            = ln->buf;

@@ -88,6 +88,21 @@ struct RunMap {
     int P; /* RUN_PARTS: thread blocks per row */
 };
 
+/* Wide top-p rows (sampler_wide.cuh) */
+struct WideCtl;
+struct WidePart;
+struct WideHead {
+    unsigned long long rows; /* rows of the launch that are done or open for everybody; in the upper half those that were opened */
+    int                any;  /* there are top-p rows */
+    int                pad;
+};
+constexpr int kWidePiece     = 512;  /* columns that are dealt out at a time, to a warp */
+constexpr int kWidePiecesMax = 4096; /* rows of more pieces go the multi-pass way */
+constexpr int kWideBinsLog   = 12;
+constexpr int kWideBins      = 1 << kWideBinsLog; /* bins of a row's histogram */
+constexpr int kWideCtlInts   = 16;
+constexpr int kWidePartBytes = 32;
+
 struct SampleParams {
     const float *logits;      /* [n_rows, V], row_stride floats apart */
     long long    row_stride;
@@ -154,6 +169,11 @@ struct SampleParams {
     Pair      *gen_dlist;   /* [pool_slots, gen_hist_cap] (id, original value) */
     Pair      *gen_list;    /* [pool_slots, gen_list_cap] (probability, id): the entries of one histogram bin, picked out of the row */
     int        gen_list_cap;
+    /* per slot (row copy) a wide row's words and its histogram, both zero between launches, and what its pieces add up to */
+    WideHead  *wide_head;
+    WideCtl   *wide_ctl;    /* [pool_slots] */
+    unsigned  *wide_hist;   /* [pool_slots, kWideBins] */
+    WidePart  *wide_part;   /* [pool_slots, pieces of a row] */
     int        gen_hist_cap;
 };
 

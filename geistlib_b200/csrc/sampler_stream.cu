@@ -126,6 +126,17 @@ struct Grp {
     __device__ __forceinline__ void sync() const { __syncthreads(); }
 };
 
+__device__ __forceinline__ Grp whole_block() {
+    Grp g;
+    g.tid  = (int) threadIdx.x;
+    g.lane = g.tid & 31;
+    g.warp = g.tid >> 5;
+    g.n    = kThreads;
+    g.nw   = kWarps;
+    g.bar  = 0;
+    return g;
+}
+
 /* Reduction scratch, one instance per group. */
 struct __align__(16) GroupShared {
     float     wred_f[32];
@@ -307,7 +318,7 @@ __device__ __forceinline__ float penalise(float x, int cnt, float rep, float fre
  * did not prefetch: have_first = false). All threads of the group call this.
  * Returns status bits.
  */
-__device__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const RowCfg &r, int V, int vocab_offset, unsigned *bitmap, PenEntry *dlist, int cap, int *n_dlist,
+__device__ __forceinline__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const RowCfg &r, int V, int vocab_offset, unsigned *bitmap, PenEntry *dlist, int cap, int *n_dlist,
                                bool have_first, int first_id) {
     int       st    = 0;
     const int total = r.H + r.E;
@@ -1222,6 +1233,12 @@ __device__ __forceinline__ void row_epilogue(const SampleParams &p, const RowCfg
     }
 }
 
+} /* namespace gb */
+
+#include "sampler_wide.cuh"
+
+namespace gb {
+
 /* ------------------------------------------------------------ shared state -- */
 
 constexpr int kIdBits = 4 * kSliceMax;
@@ -1291,6 +1308,7 @@ struct __align__(16) FinishShared {
     PenEntry    fdlist[512];
     alignas(16) unsigned long long stage[kStagedParts][kStagedCand + 4]; /* the records and first candidates of the row's first parts, in one round trip */
     unsigned long long save[256 + 128];                      /* the multi-pass path keeps a histogram here */
+    double      wide_S; /* a top-p row that the candidates could not serve: its sum, 0 where it is not known */
 };
 
 constexpr int kGroupBytes = kGroupSlots * kThreads * 4; /* one maximum per slot and thread */
@@ -1300,6 +1318,7 @@ constexpr int kFinPer     = kFinCap / kThreads;
 constexpr int kRankAll    = 220;              /* up to this many candidates the finisher ranks one against all (220 against 384, us: 1000 x 16384 top-k 128 79.5 -> 71.7,
                                                * top-k 200 97.9 -> 88.0; 64 x 128256 top-k 64 30.4 -> 23.4; against 128: 8 x 128256 top-k 128 46.1 -> 43.9) */
 constexpr int kFinBytes   = kWarps * 256 * 12;    /* finisher: the merged candidate list; the multi-pass path keeps one byte histogram per warp there */
+constexpr int kFinGeneralBytes = sizeof(WideShared) > (size_t) kFinBytes ? (int) sizeof(WideShared) : kFinBytes; /* the general kernel works on wide rows there as well */
 static_assert(kFinCap * (int) sizeof(Pair) <= kFinBytes, "the merged list fits");
 static_assert(kGroupBytes >= 4 * kRowIds * 4, "the id table of a part's set-up lies in the group maxima's memory");
 static_assert(kGroupSlots <= 256 && kThreads == 256, "a group's name fits 16 bits");
@@ -1380,7 +1399,8 @@ __device__ __forceinline__ int top_bin(const int *hist, int lane, int kq) {
  * the bin that holds the kq-th entry; entries in higher bins are in, only that one bin is ranked exactly. cand is
  * overwritten. Called by the whole thread block.
  */
-__device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int total, int kq, Pair *sorted) {
+__device__ __noinline__ void select_sorted(FinishShared *sh, Pair *cand, int total, int kq, Pair *sorted) {
+    const Grp g = whole_block();
     Pair     e[kFinPer];
     unsigned lo = 0xffffffffu, hi = 0u;
 #pragma unroll
@@ -1472,7 +1492,7 @@ __device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int to
  * room for the merged list. Returns the row's status bits (ST_DEFERRED: the multi-pass path has to serve it).
  */
 template <bool kFast>
-__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, unsigned char *cmem) {
+__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, unsigned char *cmem, int &any) {
     const int  row     = r.row;
     int       *kept_i  = p.kept_cap > 0 ? p.kept_idx + (size_t) row * (size_t) p.kept_cap : nullptr;
     float     *kept_v  = p.kept_cap > 0 ? p.kept_val + (size_t) row * (size_t) p.kept_cap : nullptr;
@@ -1484,6 +1504,9 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     int        st      = 0;
 
     g.sync(); /* the staging of the row before is no longer read */
+    if (!kFast && g.tid == 0) {
+        sh->wide_S = 0.0;
+    }
     {
         /* one round trip: the record and the first candidates of up to four parts, whatever their counts are */
         unsigned long long tv[2];
@@ -1563,6 +1586,9 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     }
     g.sync();
     PROF(9);
+    if constexpr (!kFast) {
+        any = ld_volatile(&p.wide_head->any); /* wanted when the row is done */
+    }
     for (int w = 0; w < g.nw; w++) {
         st |= gs->wred_a[w];
     }
@@ -1870,7 +1896,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 }
                 g.sync();
             } else {
-                select_sorted(g, sh, cbuf, total, k, sh->fsort);
+                select_sorted(sh, cbuf, total, k, sh->fsort);
             }
             PROF(11);
             if (r.select_only) {
@@ -1978,55 +2004,74 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 part += ref_move(sh->pbref[g.tid], row_max, r.inv_t) * sh->pbsum[g.tid];
             }
             const double S = group_sum_d(g, gs, part);
+            if (g.tid == 0) {
+                sh->wide_S = S;
+            }
             for (int i = g.tid; i < total; i += g.n) {
                 cbuf[i].v = __double2float_rn((double) cbuf[i].v / S); /* p_i as the reference normalises it */
             }
             g.sync();
             /* the walk order is (p desc, id asc); the row's kq most probable ids are all candidates */
             const int kq = min(r.kq, total);
-            select_sorted(g, sh, cbuf, total, kq, sh->fsort);
-            if (g.tid == 0) {
-                const float p_floor = sh->fsort[kq - 1].v; /* nothing outside fsort has a larger p */
-                double      cum     = 0.0;
-                int         cut     = -1;
-                for (int i = 0; i < kq; i++) {
-                    cum += (double) sh->fsort[i].v;
-                    if (cum >= (double) r.top_p) {
-                        cut = i + 1;
-                        break;
+            if (total <= kRankAll) {
+#pragma unroll 1
+                for (int i = g.tid; i < total; i += g.n) {
+                    const Pair me   = cbuf[i];
+                    int        rank = 0;
+#pragma unroll 4
+                    for (int j = 0; j < total; j++) {
+                        rank += pair_before(cbuf[j].v, cbuf[j].idx, me.v, me.idx) ? 1 : 0;
+                    }
+                    if (rank < kq) {
+                        sh->fsort[rank] = me;
                     }
                 }
-                const bool all_in = kq >= p.V;
-                bool       ok     = cut > 0 && (sh->fsort[cut - 1].v > p_floor || all_in);
-                if (cut < 0 && all_in) { /* never reached top_p: the nucleus is the whole row */
-                    cut = kq;
-                    ok  = true;
+                g.sync();
+            } else {
+                select_sorted(sh, cbuf, total, kq, sh->fsort);
+            }
+            /* The walks over the kq entries, one per lane of a warp. Their running sums are exact wherever no entry is smaller
+             * than 2^-29, so the order of additions is not seen; one thread that adds them one by one, three times over,
+             * took 4 us of a row's 15. */
+            static_assert(kNucleusProbe <= 32, "an entry per lane");
+            if (g.warp == 0) {
+                const Pair e    = g.lane < kq ? sh->fsort[g.lane] : Pair{0.0f, 0};
+                double     cum  = (double) e.v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double up = __shfl_up_sync(0xffffffffu, cum, o);
+                    if (g.lane >= o) {
+                        cum += up;
+                    }
                 }
+                const float    p_floor = __shfl_sync(0xffffffffu, e.v, kq - 1); /* nothing outside fsort has a larger p */
+                const unsigned reached = __ballot_sync(0xffffffffu, g.lane < kq && cum >= (double) r.top_p);
+                const bool     all_in  = kq >= p.V;
+                /* never reached top_p: the nucleus is the whole row, if all of it is here */
+                const int      cut = reached != 0u ? __ffs(reached) : (all_in ? kq : -1);
+                const float    p_cut = __shfl_sync(0xffffffffu, e.v, max(cut - 1, 0));
+                const bool     ok    = cut > 0 && (reached == 0u || p_cut > p_floor || all_in);
                 if (ok) {
-                    double N = 0.0;
-                    for (int i = 0; i < cut; i++) {
-                        N += (double) sh->fsort[i].v;
+                    const double   N    = __shfl_sync(0xffffffffu, cum, cut - 1);
+                    const double   u    = (double) unit_from(xorshift_next(r.rng)) * N;
+                    const unsigned over = __ballot_sync(0xffffffffu, g.lane < cut && u < cum);
+                    const int      pick = over != 0u ? __ffs(over) - 1 : cut - 1;
+                    if (g.lane == pick) {
+                        p.tokens[row] = e.idx + p.vocab_offset;
                     }
-                    const double u    = (double) unit_from(xorshift_next(r.rng)) * N;
-                    double       a    = 0.0;
-                    int          pick = cut - 1;
-                    for (int i = 0; i < cut; i++) {
-                        a += (double) sh->fsort[i].v;
-                        if (u < a) {
-                            pick = i;
-                            break;
-                        }
-                    }
-                    p.tokens[row] = sh->fsort[pick].idx + p.vocab_offset;
                     if (p.kept_cap > 0) {
-                        p.kept_n[row] = cut;
-                        for (int i = 0; i < min(cut, p.kept_cap); i++) {
-                            kept_i[i] = sh->fsort[i].idx + p.vocab_offset;
-                            kept_v[i] = __double2float_rn((double) sh->fsort[i].v / N);
+                        if (g.lane == 0) {
+                            p.kept_n[row] = cut;
+                        }
+                        if (g.lane < min(cut, p.kept_cap)) {
+                            kept_i[g.lane] = e.idx + p.vocab_offset;
+                            kept_v[g.lane] = __double2float_rn((double) e.v / N);
                         }
                     }
                 }
-                gs->flag = ok ? 1 : 0;
+                if (g.lane == 0) {
+                    gs->flag = ok ? 1 : 0;
+                }
             }
             g.sync();
             if (gs->flag) {
@@ -2485,6 +2530,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if ((kKinds & K_SUMS) != 0 && tid == 0 && blockIdx.x == 0 && p.wide_head != nullptr) { /* the finishing kernel's count of rows begins at nothing */
+        *reinterpret_cast<int4 *>(p.wide_head) = make_int4(0, 0, 0, 0);
+    }
     asm volatile("griddepcontrol.launch_dependents;");
 #ifdef GB_PROFILE
     if (tid == 0 && blockIdx.x < 1024) {
@@ -3318,6 +3366,60 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
  * less per launch; it is launched instead when the caller vouched for such rows, and reports any other row as
  * ROW_INTERNAL. Both write the row's status and, behind a sequence's last row, its generator.
  */
+/*
+ * A row that the candidates could not serve, all threads of its thread block: a wide nucleus becomes everybody's, any
+ * other row takes the multi-pass path over a private copy. Out of line, and it asks for the row's parameters again: with
+ * them handed on by reference the kernel had a stack frame that every launch paid for.
+ */
+__device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *sh, unsigned char *cmem, int row, int st) {
+    const Grp    g  = whole_block();
+    const RawCfg rc = raw_config(p, row, true);
+    RowCfg       r  = row_config(p, row, rc, true);
+    if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
+        r.cap    = 0.0f;
+        r.mrow   = nullptr;
+        r.pen_on = false;
+    }
+    const float bm = sh->gs.blk_max;
+    const int   ba = sh->gs.blk_arg;
+    if (g.tid == 0) {
+        /* claim a row copy: bounded search, the holders always make progress; with a copy per row there is nothing to claim */
+        int got = p.n_rows <= p.pool_slots ? row : -1;
+        for (long long t = 0; t < (1ll << 24) && got < 0; t++) {
+            const int c = (int) ((blockIdx.x + t) % (unsigned) p.pool_slots);
+            if (atomicCAS(&p.pool[c], 0, 1) == 0) {
+                got = c;
+            }
+        }
+        __threadfence();
+        sh->slot = got;
+    }
+    __syncthreads();
+    const int    slot = sh->slot;
+    const double S0   = sh->wide_S;
+    if (slot >= 0 && r.mode == M_TOPP && S0 > 0.0 && S0 < CUDART_INF && p.V <= kWidePiecesMax * kWidePiece) {
+        wide_open(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), slot, row, st, bm, ba, S0, sh->save); /* done by whoever completes it */
+        return;
+    }
+    if (g.tid == 0) {
+        atomicAdd(&p.wide_head->rows, 1ull);
+    }
+    if (slot < 0) {
+        st |= ST_INTERNAL;
+    } else {
+        st |= multipass_row(g, p, &sh->gs, r, bm, ba, cmem, kFinGeneralBytes, slot, sh->save);
+        __syncthreads();
+        if (g.tid == 0 && p.n_rows > p.pool_slots) {
+            __threadfence();
+            atomicExch(&p.pool[slot], 0);
+        }
+    }
+    if (g.tid == 0) {
+        row_epilogue(p, r, row, st, rc.rng);
+    }
+    __syncthreads();
+}
+
 template <bool kFast>
 __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_constant__ SampleParams p) {
     extern __shared__ __align__(128) unsigned char fsmem[];
@@ -3340,6 +3442,7 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     asm volatile("griddepcontrol.wait;" ::: "memory"); /* the records of the kernel before this one are complete and visible */
     asm volatile("griddepcontrol.launch_dependents;");
     PROF(kFast ? 5 : 7);
+    int any = 0; /* the launch has top-p rows */
     for (int row = (int) blockIdx.x; row < p.n_rows; row += (int) gridDim.x) {
         const RawCfg rc = row == (int) blockIdx.x ? rc0 : raw_config(p, row, true);
         RowCfg       r  = row_config(p, row, rc, true);
@@ -3349,7 +3452,12 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
             r.pen_on = false;
         }
         PROF(8);
-        int          st = finish_row<kFast>(g, p, sh, r, cmem);
+        if constexpr (!kFast) {
+            if (g.tid == 0 && r.mode == M_TOPP) {
+                *reinterpret_cast<volatile int *>(&p.wide_head->any) = 1;
+            }
+        }
+        int          st = finish_row<kFast>(g, p, sh, r, cmem, any);
         PROF(13);
         if (st & ST_DEFERRED) {
             if constexpr (kFast) {
@@ -3361,40 +3469,29 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
                     p.tokens[row] = -1;
                 }
             } else {
-                /* the multi-pass path: all threads of this thread block, over a private copy of the row */
-                __syncthreads();
-                const float bm = sh->gs.blk_max;
-                const int   ba = sh->gs.blk_arg;
-                if (g.tid == 0) {
-                    /* claim a row copy: bounded search, the holders always make progress */
-                    int got = -1;
-                    for (long long t = 0; t < (1ll << 24) && got < 0; t++) {
-                        const int c = (int) ((blockIdx.x + t) % (unsigned) p.pool_slots);
-                        if (atomicCAS(&p.pool[c], 0, 1) == 0) {
-                            got = c;
-                        }
-                    }
-                    __threadfence();
-                    sh->slot = got;
-                }
-                __syncthreads();
-                const int slot = sh->slot;
-                if (slot < 0) {
-                    st = (st & ~ST_DEFERRED) | ST_INTERNAL;
-                } else {
-                    st = (st & ~ST_DEFERRED) | multipass_row(g, p, &sh->gs, r, bm, ba, cmem, kFinBytes, slot, sh->save);
-                    __syncthreads();
-                    if (g.tid == 0) {
-                        __threadfence();
-                        atomicExch(&p.pool[slot], 0);
-                    }
-                }
+                deferred_row(p, sh, cmem, row, st & ~ST_DEFERRED);
+                continue;
+            }
+        } else if constexpr (!kFast) {
+            if (g.tid == 0) {
+                atomicAdd(&p.wide_head->rows, 1ull);
             }
         }
         if (g.tid == 0) {
             row_epilogue(p, r, row, st, rc.rng);
         }
         __syncthreads();
+    }
+    if constexpr (!kFast) {
+        if ((int) blockIdx.x >= p.n_rows && g.tid == 0) { /* here to help alone: top-p rows say so when their blocks begin */
+            const unsigned long long t0 = global_ns();
+            do {
+                any = ld_volatile(&p.wide_head->any);
+            } while (any == 0 && global_ns() - t0 < 3000ull);
+        }
+        if (__syncthreads_or(any) != 0) {
+            wide_help(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), sh->save);
+        }
     }
     PROF(kFast ? 6 : 7);
 }
@@ -3580,7 +3677,7 @@ static cudaError_t ensure_row_ids_attributes(size_t smem_bytes) {
     return cudaSuccess;
 }
 
-size_t finish_rows_smem() { return sizeof(FinishShared) + (size_t) kFinBytes; }
+size_t finish_rows_smem(bool fast) { return sizeof(FinishShared) + (size_t) (fast ? kFinBytes : kFinGeneralBytes); }
 
 static cudaError_t ensure_finish_attributes() {
     static int  configured[64] = {0};
@@ -3593,9 +3690,9 @@ static cudaError_t ensure_finish_attributes() {
         return cudaErrorInvalidDevice;
     }
     if (!configured[dev]) {
-        e = cudaFuncSetAttribute(finish_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) finish_rows_smem());
+        e = cudaFuncSetAttribute(finish_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) finish_rows_smem(true));
         if (e == cudaSuccess) {
-            e = cudaFuncSetAttribute(finish_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) finish_rows_smem());
+            e = cudaFuncSetAttribute(finish_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) finish_rows_smem(false));
         }
         if (e != cudaSuccess) {
             return e;
@@ -3612,7 +3709,7 @@ cudaError_t finish_rows_max_ctas(int sms, int *out) {
         return e;
     }
     int per_sm = 0;
-    e          = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, finish_rows_kernel<false>, kThreads, finish_rows_smem());
+    e          = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, finish_rows_kernel<false>, kThreads, finish_rows_smem(false));
     *out       = per_sm * sms;
     return e;
 }
@@ -3672,7 +3769,7 @@ cudaError_t launch_sample_stream(const SampleParams &p, int grid, size_t smem_by
         return e;
     }
     cfg.gridDim          = dim3((unsigned) finish_grid);
-    cfg.dynamicSmemBytes = finish_rows_smem();
+    cfg.dynamicSmemBytes = finish_rows_smem((p.flags & F_FAST_ONLY) != 0u);
     if ((p.flags & (F_GREEDY_ONLY | F_INLINE_TOPK)) != 0u) {
         return cudaSuccess; /* the stream kernel writes the tokens itself */
     }

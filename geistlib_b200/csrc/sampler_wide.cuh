@@ -1,0 +1,732 @@
+/*
+ * sampler_wide.cuh — top-p rows whose nucleus is wide, part of finish_rows_kernel<false> (included by
+ * sampler_stream.cu behind the helpers it uses).
+ *
+ * Such a row is worked on by every thread block of the finishing kernel that has nothing else to do. It is cut into
+ * pieces of kWidePiece columns, dealt out one by one to warps, which share nothing but counters while they work:
+ *
+ *   pass 1  e_i = expf((x_i - max) / T), correctly rounded, kept in the row's scratch; their sum per piece in double; and
+ *           a histogram of their mass over kWideBins bins of their bits, in whole units of S0 / 2^30 (S0: the row's sum
+ *           as the stream kernel formed it).
+ *   pass 2  starts when every piece is through pass 1: S is known, and from the histogram the bins in which the walk
+ *           reaches top_p and in which the draw will fall, with a margin for the units' rounding. p_i = (float)(e_i / S);
+ *           what lies above a window is summed in double, what lies in it is listed (a few entries, or a few hundred).
+ *   end     the thread block that completes pass 2 walks the two lists exactly, in (p desc, id asc) order, and has the
+ *           token. Whatever the lists do not decide (more entries than they hold, a crossing outside its window, equal
+ *           probabilities at a window's edge) goes to multipass_row.
+ *
+ * Nobody waits for a thread block that has not begun: the block that owns the row takes pieces like any other, and once
+ * they are all dealt out, every piece lies with a block that runs. Sums and lists do not depend on who took which piece.
+ */
+#pragma once
+
+namespace gb {
+
+constexpr int kWideRank = 512;  /* lists up to here are walked by ranking */
+constexpr int kWideIds  = 1024; /* ids of a row that a thread block keeps at hand; more are read from memory for every piece */
+
+/* What the wide row that a slot (row copy) holds is. */
+struct __align__(16) WideCtl {
+    int    rem1, rem2;    /* pieces not yet dealt out of pass 1 and pass 2; rem1 at most 0: no row to help with */
+    int    done1, done2;  /* pieces through pass 1; pieces whose thread block of pass 1 has left pass 2 */
+    int    n_cut, n_pick; /* entries of the two lists */
+    int    row, st;
+    float  row_max;
+    int    row_arg;
+    double S0;
+    double pad[2];
+};
+static_assert(sizeof(WideCtl) == 4 * kWideCtlInts, "a slot's words");
+
+/* What a piece adds up to. */
+struct __align__(16) WidePart {
+    double sum;                   /* of e */
+    double above_cut, above_pick; /* of p, above the two windows */
+    int    n_above;               /* entries above the window of the crossing */
+    int    pad;
+};
+static_assert(sizeof(WidePart) == kWidePartBytes, "the host sizes the parts");
+
+/* A thread block's memory while it works on wide rows (the merged candidates' memory). */
+struct __align__(16) WideShared {
+    unsigned           hist[kWideBins];
+    float              x[kWarps][2][kWidePiece];    /* every warp's pieces: the one in work and the next on its way */
+    unsigned           cnt[kWarps][kWidePiece / 2]; /* how often an id of the warp's piece occurs, 16 bits each; zero between pieces */
+    int                ids[kWideIds];
+    unsigned           wsum[kWarps];
+    int                win[4]; /* the crossing's window, lowest and highest bin; the draw's */
+    int                next, slot, mine;
+    int                best_rank;
+    unsigned long long best, best_mass;
+};
+
+/*
+ * expf as a correctly rounded one gives it, for a <= 0: 2^m * 2^(j/32) * e^r by Tang's table-driven scheme (P. Tang, ACM
+ * TOMS 15, 1989) in double, the table one entry per lane (t32 = 2^(lane / 32)): all lanes of the warp call. r is at most
+ * ln 2 / 64, where the series cut behind r^6 / 720 is good to 4e-18, so the value before its rounding to binary32 is as
+ * good as exp()'s. A NaN does not come back (the caller has excluded it).
+ */
+__device__ __forceinline__ float wide_exp(float a, double t32) {
+    const double ad = (double) fmaxf(a, -120.0f);
+    const double t  = __fma_rn(ad, 46.166241308446829, 0x1.8p52); /* 32 / ln 2; the addend leaves the nearest whole number in the low word */
+    const int    n  = __double2loint(t);
+    const double nd = t - 0x1.8p52;
+    double       r  = __fma_rn(nd, -0x1.62e42fefa39efp-6, ad); /* ln 2 / 32 in two doubles */
+    r               = __fma_rn(nd, -0x1.abc9e3b39803fp-61, r);
+    double q        = __fma_rn(r, 1.0 / 720.0, 1.0 / 120.0);
+    q               = __fma_rn(q, r, 1.0 / 24.0);
+    q               = __fma_rn(q, r, 1.0 / 6.0);
+    q               = __fma_rn(q, r, 0.5);
+    q               = __fma_rn(q, r, 1.0);
+    q               = q * r;
+    const int    lo = __shfl_sync(0xffffffffu, __double2loint(t32), n); /* lane n modulo 32 */
+    const int    hi = __shfl_sync(0xffffffffu, __double2hiint(t32), n) + ((n << 15) & (int) 0xfff00000);
+    const double T  = __hiloint2double(hi, lo);
+    return __double2float_rn(__fma_rn(T, q, T));
+}
+
+/* (float) (e / S): the quotient to 2^-47, then one rounding (inv_hi + inv_lo = 1 / S). */
+__device__ __forceinline__ float wide_prob(float e, float inv_hi, float inv_lo) {
+    const float q = __fmul_rn(e, inv_hi);
+    return __fadd_rn(q, __fmaf_rn(e, inv_lo, __fmaf_rn(e, inv_hi, -q)));
+}
+
+__device__ __forceinline__ void copy_quad_async(void *dst_shared, const void *src_global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned) __cvta_generic_to_shared(dst_shared)), "l"(src_global) : "memory");
+}
+__device__ __forceinline__ int ld_volatile(const int *q) { return *reinterpret_cast<const volatile int *>(q); }
+
+/* Bins of a row's histogram: the bits of e from the floor up to 1, in at most kWideBins equal steps of a power of two.
+ * Entries with p < (1 - top_p) / V add up to less than 1 - top_p, so the walk crosses above half of that. */
+struct WideBins {
+    unsigned k_floor;
+    int      shift;
+    float    unit; /* 2^30 / S0 */
+    __device__ __forceinline__ WideBins(double S0, float top_p, int V) {
+        const float f       = __double2float_rn(0.5 * (1.0 - (double) top_p) / (double) V * S0);
+        k_floor             = f > 0.0f && f < 1.0f ? __float_as_uint(f) : 1u;
+        const unsigned span = __float_as_uint(1.0f) - k_floor;
+        shift               = max(0, 32 - __clz(span) - kWideBinsLog);
+        unit                = __double2float_rn(0x1p30 / S0);
+    }
+    __device__ __forceinline__ unsigned bin(unsigned k) const { return (k - k_floor) >> shift; } /* kWideBins and more: below the floor */
+    __device__ __forceinline__ unsigned edge(int b) const { return k_floor + ((unsigned) b << shift); } /* lowest bits of bin b */
+};
+
+/* Where one of the two walks ends. */
+struct WideHit {
+    bool               found;
+    unsigned long long word; /* (bits of p, id) as composite() packs them */
+    double             mass; /* of everything up to and with it */
+    long long          rank; /* its place, from 1, in its list */
+};
+
+/* The first of the n listed entries, in (p desc, id asc) order, at which base + running mass reaches (inclusive) or
+ * exceeds the target. Masses are added in units of 2^-62, so the order of the list does not matter. All threads call. */
+__device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, const Pair *list, int n, double base, double target, bool inclusive, int idx_bits) {
+    WideHit out;
+    if (n <= kWideRank) {
+        unsigned long long *word = reinterpret_cast<unsigned long long *>(&ws->x[0][0][0]), *mass = word + kWideRank;
+        static_assert(sizeof(ws->x) >= 2 * kWideRank * 8, "the list fits");
+        g.sync();
+        for (int i = g.tid; i < n; i += g.n) {
+            const unsigned long long w  = __ldcg(reinterpret_cast<const unsigned long long *>(list + i)); /* p, then the id */
+            const float              pv = __uint_as_float((unsigned) w);
+            word[i]                     = composite(__float_as_uint(pv), (int) (w >> 32), idx_bits);
+            mass[i]                     = __double2ull_rz((double) pv * 0x1p62);
+        }
+        if (g.tid == 0) {
+            ws->best = 0ull;
+        }
+        g.sync();
+        unsigned long long mine = 0ull, my_sum[kWideRank / kThreads];
+        int                my_rank[kWideRank / kThreads];
+#pragma unroll
+        for (int q = 0; q < kWideRank / kThreads; q++) {
+            const int i = g.tid + q * kThreads;
+            my_sum[q]   = 0ull;
+            my_rank[q]  = 0;
+            if (i < n) {
+                const unsigned long long me = word[i];
+#pragma unroll 4
+                for (int j = 0; j < n; j++) {
+                    const bool up = word[j] >= me;
+                    my_sum[q] += up ? mass[j] : 0ull;
+                    my_rank[q] += up ? 1 : 0;
+                }
+                const double at = base + (double) my_sum[q] * 0x1p-62;
+                if (inclusive ? at >= target : at > target) {
+                    mine = max(mine, me);
+                }
+            }
+        }
+        if (mine != 0ull) {
+            atomicMax(&ws->best, mine);
+        }
+        g.sync();
+        out.word = ws->best;
+#pragma unroll
+        for (int q = 0; q < kWideRank / kThreads; q++) {
+            const int i = g.tid + q * kThreads;
+            if (i < n && word[i] == out.word) {
+                ws->best_mass = my_sum[q];
+                ws->best_rank = my_rank[q];
+            }
+        }
+        g.sync();
+        out.found = out.word != 0ull;
+        out.mass  = base + (double) ws->best_mass * 0x1p-62;
+        out.rank  = (long long) ws->best_rank;
+        g.sync();
+        return out;
+    }
+    /* long lists (many equal values): byte by byte as the multi-pass path walks its own */
+    auto     sweep = [&](auto &&f) { list_sweep(g, list, n, f); };
+    auto     keyf  = [](float pv) { return __float_as_uint(pv); };
+    auto     massf = [](float pv, int) { return (double) pv; };
+    double  *hm    = reinterpret_cast<double *>(&ws->x[0][0][0]);
+    int     *hc    = reinterpret_cast<int *>(hm + kWarps * 256);
+    static_assert(sizeof(ws->x) >= (size_t) kWarps * 256 * 12, "a byte histogram per warp fits");
+    const RadixOut ro = radix_mass(g, gs, hm, hc, kWarps, 0x1p62, sweep, target - base, inclusive, keyf, massf);
+    out.found         = ro.found;
+    out.word          = ro.found ? resolve_ties(g, gs, sweep, idx_bits, ro, target - base, inclusive, keyf, massf) : 0ull;
+    double    m = 0.0;
+    long long c = 0;
+    sweep([&](float pv, int i) {
+        if (composite(__float_as_uint(pv), i, idx_bits) >= out.word) {
+            m += (double) pv;
+            c++;
+        }
+    });
+    out.mass = base + group_sum_d(g, gs, m);
+    out.rank = group_sum_ll(g, gs, c);
+    return out;
+}
+
+/* Takes a piece of a row of which *rem were left: its number, -1 when there was none. Called by a whole warp; the answer
+ * takes a round trip, so a warp asks a piece ahead (lane 0 holds what came back). */
+__device__ __forceinline__ int wide_ask(int *rem, int lane) { return lane == 0 ? atomicSub(rem, 1) : 0; }
+__device__ __forceinline__ int wide_got(int left, int pieces) {
+    const int l = __shfl_sync(0xffffffffu, left, 0);
+    return l > 0 ? pieces - l : -1;
+}
+
+/* The last of a row's thread blocks: the two walks, the token, and the slot made ready for its next row. */
+__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, RowCfg &r, int slot, float inv_hi, float inv_lo, unsigned long long rng0, void *save_mem) {
+    const Grp       g      = whole_block();
+    WideCtl        *ctl    = p.wide_ctl + slot;
+    const int       V      = p.V, pieces = (V + kWidePiece - 1) / kWidePiece, idx_bits = 32 - __clz(max(V - 1, 1));
+    const WidePart *parts  = p.wide_part + (size_t) slot * (size_t) pieces;
+    const Pair     *list   = p.gen_list + (size_t) slot * (size_t) p.gen_list_cap;
+    const int       half   = p.gen_list_cap / 2;
+    const WideBins  bins(__ldcg(&ctl->S0), r.top_p, V);
+    double          a_cut = 0.0, a_pick = 0.0;
+    long long       above = 0;
+    for (int t = g.tid; t < pieces; t += g.n) {
+        a_cut += __ldcg(&parts[t].above_cut);
+        a_pick += __ldcg(&parts[t].above_pick);
+        above += __ldcg(&parts[t].n_above);
+    }
+    const int n_cut = __ldcg(&ctl->n_cut), n_pick = __ldcg(&ctl->n_pick);
+    a_cut           = group_sum_d(g, gs, a_cut);
+    a_pick          = group_sum_d(g, gs, a_pick);
+    above           = group_sum_ll(g, gs, above);
+    /* p of the nearest entries outside a window: an entry of the window that shares it cannot be placed */
+    auto p_at   = [&](unsigned k) { return wide_prob(__uint_as_float(k), inv_hi, inv_lo); };
+    auto inside = [&](unsigned long long word, int lo, int hi) {
+        const float pv = __uint_as_float((unsigned) (word >> idx_bits));
+        return pv > 0.0f && (hi >= kWideBins - 1 || pv < p_at(bins.edge(hi + 1))) && pv > p_at(bins.edge(lo) - 1u);
+    };
+    const int w0 = ws->win[0], w1 = ws->win[1], w2 = ws->win[2], w3 = ws->win[3];
+    bool      ok = n_cut <= half && n_pick <= half && n_cut > 0 && a_cut < (double) r.top_p;
+    WideHit   cut{}, pick{};
+    if (ok) {
+        cut = wide_walk(g, gs, ws, list, n_cut, a_cut, (double) r.top_p, true, idx_bits);
+        ok  = cut.found && inside(cut.word, w0, w1);
+    }
+    if (ok) {
+        unsigned long long rng = r.rng;
+        const double       u   = (double) unit_from(xorshift_next(rng)) * cut.mass;
+        ok                     = a_pick <= u;
+        if (ok) {
+            pick = wide_walk(g, gs, ws, list + half, n_pick, a_pick, u, false, idx_bits);
+            ok   = pick.found && inside(pick.word, w2, w3);
+        }
+    }
+    int st = __ldcg(&ctl->st);
+    if (ok) {
+        if (g.tid == 0) {
+            const unsigned long long id_mask = (1ull << idx_bits) - 1ull;
+            const unsigned long long word    = max(pick.word, cut.word); /* the draw does not leave the nucleus (sampler.c:292) */
+            p.tokens[r.row]                  = min((int) (id_mask - (word & id_mask)), V - 1) + p.vocab_offset;
+            if (p.kept_cap > 0) {
+                p.kept_n[r.row] = (int) (above + cut.rank);
+            }
+        }
+        st |= ST_SLOW_PATH | (p.kept_cap > 0 ? (int) ST_KEPT_PARTIAL : 0);
+    } else {
+        st |= multipass_row(g, p, gs, r, __ldcg(&ctl->row_max), __ldcg(&ctl->row_arg), ws, (int) sizeof(WideShared), slot, save_mem);
+    }
+    if (g.tid == 0) {
+        row_epilogue(p, r, r.row, st, rng0);
+    }
+    uint4 *gh = reinterpret_cast<uint4 *>(p.wide_hist + (size_t) slot * kWideBins);
+    for (int i = g.tid; i < kWideBins / 4; i += g.n) {
+        gh[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __threadfence();
+    g.sync();
+    if (g.tid == 0 && p.n_rows > p.pool_slots) {
+        __threadfence();
+        atomicExch(&p.pool[slot], 0);
+    }
+    g.sync();
+}
+
+/* Works on the row of a slot. `first`: a piece that the thread block has been dealt already, its first warp's (all threads call). */
+__device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, WideShared *ws, int slot, int first, void *save_mem) {
+    const Grp       g       = whole_block();
+    WideCtl        *ctl     = p.wide_ctl + slot;
+    const int       V       = p.V, pieces = (V + kWidePiece - 1) / kWidePiece;
+    int             left    = wide_ask(&ctl->rem1, g.lane);
+    const int       row     = __ldcg(&ctl->row);
+    const float     row_max = __ldcg(&ctl->row_max);
+    const double    S0      = __ldcg(&ctl->S0);
+    for (int i = g.tid; i < kWideBins / 4; i += g.n) {
+        reinterpret_cast<uint4 *>(ws->hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    for (int i = g.tid; i < kWarps * kWidePiece / 8; i += g.n) {
+        reinterpret_cast<uint4 *>(ws->cnt)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (g.tid == 0) {
+        ws->mine = 0;
+    }
+    const RawCfg rc = raw_config(p, row, true);
+    RowCfg       r  = row_config(p, row, rc, true);
+    if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
+        r.cap    = 0.0f;
+        r.mrow   = nullptr;
+        r.pen_on = false;
+    }
+    const WideBins bins(S0, r.top_p, V);
+    const float   *src    = row_again(p, row);
+    const bool     src_al = again_aligned(p);
+    float         *gr     = p.gen_rows + (size_t) slot * (size_t) p.gen_stride;
+    WidePart      *parts  = p.wide_part + (size_t) slot * (size_t) pieces;
+    const double   t32    = exp2((double) g.lane * 0x1p-5);
+    const int      n_ids  = r.pen_on ? r.H + r.E : 0;
+    const bool     pro    = r.cap > 0.0f || r.mrow != nullptr;
+    for (int j = g.tid; j < min(n_ids, kWideIds); j += g.n) {
+        ws->ids[j] = hist_id(r, j, p.vocab_offset);
+    }
+    g.sync();
+    /* ---- pass 1 ---- */
+    constexpr int kPer = 8, kSteps = kWidePiece / (32 * kPer); /* eight values of a lane at a time: as many independent chains */
+    auto column = [&](int step, int q) { return step * (32 * kPer) + (q >> 2) * 128 + 4 * g.lane + (q & 3); }; /* inside the piece */
+    /* A piece on its way into one of the warp's two buffers. What bounds the passes is the bytes on their way: with eight
+     * values per lane in registers and none ahead 16 KB per SM, 3.5 TB/s with nothing else done. */
+    auto fetch = [&](const float *from, bool al, int end, int pc, int to, float pad) {
+        const int    s0  = pc * kWidePiece, n = min(kWidePiece, end - s0);
+        float       *buf = ws->x[g.warp][to];
+        const float *at  = from + s0;
+        if (al) {
+#pragma unroll
+            for (int i = 4 * g.lane; i < kWidePiece; i += 128) {
+                if (i + 4 <= n) {
+                    copy_quad_async(buf + i, at + i);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        buf[i + q] = i + q < n ? at[i + q] : pad;
+                    }
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (int i = g.lane; i < kWidePiece; i += 32) {
+                if (i < n) {
+                    copy_word_async(buf + i, at + i);
+                } else {
+                    buf[i] = pad;
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto take_values = [&](int from, int step, float (&e)[kPer]) {
+#pragma unroll
+        for (int h = 0; h < kPer; h += 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(&ws->x[g.warp][from][column(step, h)]);
+            e[h] = v.x, e[h + 1] = v.y, e[h + 2] = v.z, e[h + 3] = v.w;
+        }
+    };
+    auto one_behind = [&](bool more) { /* the piece in work has arrived; the next may be on its way */
+        if (more) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+    };
+    int       mine  = 0;
+    int       piece = first >= 0 && g.warp == 0 ? first : -1;
+    unsigned *cnt   = ws->cnt[g.warp];
+    if (piece < 0) {
+        piece = wide_got(left, pieces);
+        left  = piece >= 0 ? wide_ask(&ctl->rem1, g.lane) : 0;
+    }
+    if (piece >= 0) {
+        fetch(src, src_al, V, piece, 0, -CUDART_INF_F);
+    }
+    for (int in = 0; piece >= 0; in ^= 1) {
+        const int s0   = piece * kWidePiece;
+        const int next = wide_got(left, pieces);
+        if (next >= 0) {
+            left = wide_ask(&ctl->rem1, g.lane);
+            fetch(src, src_al, V, next, in ^ 1, -CUDART_INF_F);
+        }
+        if (n_ids > 0) { /* how often each id of the piece occurs */
+            for (int j = g.lane; j < n_ids; j += 32) {
+                const int li = (j < kWideIds ? ws->ids[j] : hist_id(r, j, p.vocab_offset)) - s0;
+                if (li >= 0 && li < kWidePiece && li + s0 < V) {
+                    atomicAdd(&cnt[li >> 1], 1u << (16 * (li & 1)));
+                }
+            }
+            __syncwarp();
+        }
+        one_behind(next >= 0);
+        double sum = 0.0;
+#pragma unroll 1
+        for (int step = 0; step < kSteps; step++) {
+            float e[kPer];
+            take_values(in, step, e);
+            if (pro || n_ids > 0) {
+#pragma unroll
+                for (int h = 0; h < kPer; h += 4) {
+                    const int      c     = s0 + column(step, h);
+                    uint2         &cw    = *reinterpret_cast<uint2 *>(cnt + (column(step, h) >> 1));
+                    const unsigned c4[4] = {cw.x & 0xffffu, cw.x >> 16, cw.y & 0xffffu, cw.y >> 16};
+                    if (pro) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (c + q < V) {
+                                e[h + q] = prologue_one(e[h + q], c + q, r.cap, r.mrow);
+                            }
+                        }
+                    }
+                    if ((cw.x | cw.y) != 0u) {
+                        cw = make_uint2(0u, 0u);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (c4[q] != 0u) {
+                                e[h + q] = penalise(e[h + q], (int) c4[q], r.rep, r.freq, r.pres);
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int q = 0; q < kPer; q++) {
+                e[q] = wide_exp(scaled_arg(e[q], row_max, r.inv_t), t32);
+            }
+#pragma unroll
+            for (int h = 0; h < kPer; h += 4) {
+                const int c = s0 + column(step, h);
+                sum += ((double) e[h] + (double) e[h + 1]) + ((double) e[h + 2] + (double) e[h + 3]);
+                if (c + 4 <= p.gen_stride) {
+                    *reinterpret_cast<float4 *>(gr + c) = make_float4(e[h], e[h + 1], e[h + 2], e[h + 3]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kPer; q++) {
+                const unsigned b = bins.bin(__float_as_uint(e[q])), m = __float2uint_rn(e[q] * bins.unit);
+                if (b < (unsigned) kWideBins) {
+                    atomicAdd(&ws->hist[b], m);
+                }
+            }
+        }
+        sum = warp_sum_d(sum);
+        if (g.lane == 0) {
+            parts[piece].sum = sum;
+        }
+        mine++;
+        piece = next;
+        __syncwarp(); /* the buffer is free */
+    }
+    if (g.lane == 0 && mine > 0) {
+        atomicAdd(&ws->mine, mine);
+    }
+    g.sync();
+    unsigned *gh = p.wide_hist + (size_t) slot * kWideBins;
+    for (int i = g.tid; i < kWideBins; i += g.n) {
+        const unsigned v = ws->hist[i];
+        if (v != 0u) {
+            atomicAdd(&gh[i], v);
+        }
+    }
+    __threadfence();
+    g.sync();
+    if (g.tid == 0) {
+        atomicAdd(&ctl->done1, ws->mine);
+        /* every piece lies with a thread block that runs: the wait ends */
+        const unsigned long long t0 = global_ns();
+        bool                     in = true;
+        while (ld_volatile(&ctl->done1) < pieces && in) {
+            __nanosleep(50);
+            in = global_ns() - t0 < kWaitLimitNs;
+        }
+        __threadfence();
+        ws->next = in ? 1 : 0;
+    }
+    g.sync();
+    if (ws->next == 0) {
+        if (g.tid == 0) {
+            p.tokens[row] = -1;
+            p.status[row] = ST_INTERNAL;
+        }
+        g.sync();
+        return;
+    }
+    left = wide_ask(&ctl->rem2, g.lane);
+    /* ---- S, and the two windows ---- */
+    constexpr int kOwn = kWideBins / kThreads;
+    unsigned      h[kOwn], run = 0u; /* thread t holds kOwn bins, the highest with thread 0 */
+    const int     b0 = kWideBins - kOwn * (g.tid + 1);
+#pragma unroll
+    for (int q = 0; q < kOwn / 4; q++) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(gh + b0) + q);
+        h[4 * q] = v.x, h[4 * q + 1] = v.y, h[4 * q + 2] = v.z, h[4 * q + 3] = v.w;
+    }
+    double S = 0.0;
+    for (int t = g.tid; t < pieces; t += g.n) {
+        S += __ldcg(&parts[t].sum);
+    }
+    S = group_sum_d(g, gs, S);
+    const double inv    = 1.0 / S;
+    const float  inv_hi = __double2float_rn(inv), inv_lo = __double2float_rn(inv - (double) inv_hi);
+    {
+#pragma unroll
+        for (int q = 0; q < kOwn; q++) {
+            run += h[q];
+        }
+        unsigned incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (g.lane >= o) {
+                incl += up;
+            }
+        }
+        if (g.lane == 31) {
+            ws->wsum[g.warp] = incl;
+        }
+        if (g.tid < 4) {
+            ws->win[g.tid] = 0;
+        }
+        g.sync();
+        unsigned before = incl - run;
+        for (int w = 0; w < g.warp; w++) {
+            before += ws->wsum[w];
+        }
+        /* Units that reach a target, less and more the margin (the units' rounding moves the sum of n entries by 0.29
+         * sqrt(n), rms): the highest bin up to which the target can be reached, and the one up to which it surely is. */
+        unsigned long long rng    = r.rng;
+        const double       u01    = (double) unit_from(xorshift_next(rng));
+        const double       margin = 1024.0 + (double) (V >> 8);
+        const double       t_cut  = (double) r.top_p * S * (double) bins.unit;
+        auto place = [&](int which, double target) { /* the highest bin b so that the units in bins >= b reach the target */
+            target = fmax(target, 1e-3);
+            if ((double) before < target && (double) (before + run) >= target) {
+                unsigned acc = before;
+                int      b   = b0;
+#pragma unroll
+                for (int q = kOwn - 1; q >= 0; q--) {
+                    const bool below = (double) acc < target;
+                    acc += h[q];
+                    b = below && (double) acc >= target ? b0 + q : b;
+                }
+                ws->win[which] = b;
+            }
+        };
+        place(1, t_cut - margin);
+        place(0, t_cut + margin);
+        g.sync();
+        /* the draw's target lies between u and u times what the crossing entry can add at most */
+        const double p_one = (double) __uint_as_float(bins.edge(ws->win[1] + 1)) * (double) bins.unit;
+        place(3, u01 * t_cut - margin);
+        place(2, u01 * (t_cut + p_one) + margin);
+        g.sync();
+        if (g.tid == 0) {
+            ws->win[2] = max(ws->win[2], ws->win[0]);
+        }
+        g.sync();
+    }
+    /* ---- pass 2 ---- */
+    const unsigned c_lo = bins.edge(ws->win[0]), c_hi = ws->win[1] >= kWideBins - 1 ? 0xffffffffu : bins.edge(ws->win[1] + 1);
+    const unsigned k_lo = bins.edge(ws->win[2]), k_hi = ws->win[3] >= kWideBins - 1 ? 0xffffffffu : bins.edge(ws->win[3] + 1);
+    const int      half = p.gen_list_cap / 2;
+    Pair          *list = p.gen_list + (size_t) slot * (size_t) p.gen_list_cap;
+    auto           note = [&](int *count, Pair *to, float pv, int id) {
+        const int pos = atomicAdd(count, 1);
+        if (pos < half) {
+            to[pos].v   = pv;
+            to[pos].idx = id;
+        }
+    };
+    piece = wide_got(left, pieces);
+    left  = piece >= 0 ? wide_ask(&ctl->rem2, g.lane) : 0;
+    if (piece >= 0) {
+        fetch(gr, true, (int) p.gen_stride, piece, 0, 0.0f);
+    }
+    for (int in = 0; piece >= 0; in ^= 1) {
+        const int s0   = piece * kWidePiece;
+        const int next = wide_got(left, pieces);
+        if (next >= 0) {
+            left = wide_ask(&ctl->rem2, g.lane);
+            fetch(gr, true, (int) p.gen_stride, next, in ^ 1, 0.0f);
+        }
+        one_behind(next >= 0);
+        double a_cut = 0.0, a_pick = 0.0;
+        int    above = 0;
+#pragma unroll 1
+        for (int step = 0; step < kSteps; step++) {
+            float    e[kPer];
+            unsigned listed = 0u; /* which of the lane's values lie in a window */
+            take_values(in, step, e);
+#pragma unroll
+            for (int q = 0; q < kPer; q++) {
+                const unsigned k = __float_as_uint(e[q]);
+                if (__any_sync(0xffffffffu, k >= c_lo)) { /* most of a row lies below the nucleus; the draw's window lies no lower */
+                    const double pd = (double) wide_prob(e[q], inv_hi, inv_lo);
+                    a_cut += k >= c_hi ? pd : 0.0;
+                    a_pick += k >= k_hi ? pd : 0.0;
+                    above += k >= c_hi ? 1 : 0;
+                    listed |= (k - c_lo < c_hi - c_lo || k - k_lo < k_hi - k_lo) ? 1u << q : 0u;
+                }
+            }
+            if (listed != 0u) {
+#pragma unroll
+                for (int q = 0; q < kPer; q++) {
+                    if ((listed >> q) & 1u) {
+                        const unsigned k  = __float_as_uint(e[q]);
+                        const float    pv = wide_prob(e[q], inv_hi, inv_lo);
+                        const int      id = s0 + column(step, q);
+                        if (k - c_lo < c_hi - c_lo) {
+                            note(&ctl->n_cut, list, pv, id);
+                        }
+                        if (k - k_lo < k_hi - k_lo) {
+                            note(&ctl->n_pick, list + half, pv, id);
+                        }
+                    }
+                }
+            }
+        }
+        a_cut  = warp_sum_d(a_cut);
+        a_pick = warp_sum_d(a_pick);
+        above  = __reduce_add_sync(0xffffffffu, above);
+        if (g.lane == 0) {
+            parts[piece].above_cut  = a_cut;
+            parts[piece].above_pick = a_pick;
+            parts[piece].n_above    = above;
+        }
+        piece = next;
+        __syncwarp();
+    }
+    /* The row is done, and its slot free for another one, when every thread block that works on it is through here: each
+     * was dealt a piece of pass 1 at least, and counts its own once more. */
+    __threadfence();
+    g.sync();
+    if (g.tid == 0) {
+        ws->next = atomicAdd(&ctl->done2, ws->mine) + ws->mine == pieces ? 1 : 0;
+        __threadfence();
+    }
+    g.sync();
+    if (ws->next != 0) {
+        wide_finish(p, gs, ws, r, slot, inv_hi, inv_lo, rc.rng, save_mem);
+    }
+}
+
+/* Opens the row in a slot that the thread block has claimed, for everybody; the block then works on it itself. */
+__device__ __forceinline__ void wide_open(const SampleParams &p, GroupShared *gs, WideShared *ws, int slot, int row, int st, float row_max, int row_arg, double S0, void *save_mem) {
+    WideCtl *ctl = p.wide_ctl + slot;
+    if (threadIdx.x == 0) {
+        const int pieces = (p.V + kWidePiece - 1) / kWidePiece;
+        ctl->done1       = 0;
+        ctl->done2       = 0;
+        ctl->n_cut       = 0;
+        ctl->n_pick      = 0;
+        ctl->row         = row;
+        ctl->st          = st;
+        ctl->row_max     = row_max;
+        ctl->row_arg     = row_arg;
+        ctl->S0          = S0;
+        ctl->rem2        = pieces;
+        __threadfence();
+        atomicExch(&ctl->rem1, pieces - 1); /* piece 0 is the block's own */
+    }
+    __syncthreads();
+    if (threadIdx.x == 32) {
+        __threadfence();
+        atomicAdd(&p.wide_head->rows, (1ull << 32) + 1ull);
+    }
+    wide_join(p, gs, ws, slot, 0, save_mem);
+    __syncthreads();
+}
+
+/* A thread block that has no rows of its own left helps with wide ones, as long as there can be any: rows that have not
+ * been decided on yet, but no longer than kWideHelpNs without a piece to take. */
+constexpr unsigned long long kWideHelpNs = 50000ull;
+__device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, WideShared *ws, void *save_mem) {
+    const Grp          g      = whole_block();
+    const int          pieces = (p.V + kWidePiece - 1) / kWidePiece, start = (int) (blockIdx.x % (unsigned) p.pool_slots);
+    unsigned           looked = 0u; /* rows that had been opened when the slots were last looked through in vain */
+    for (;;) {
+        if (g.tid == 0) {
+            const unsigned long long t0 = global_ns();
+            unsigned long long       rows;
+            for (;;) {
+                rows = *reinterpret_cast<volatile unsigned long long *>(&p.wide_head->rows);
+                if ((unsigned) (rows >> 32) > looked || (int) (unsigned) rows >= p.n_rows || global_ns() - t0 > kWideHelpNs) {
+                    break;
+                }
+                __nanosleep(40);
+            }
+            ws->next = (unsigned) (rows >> 32) > looked ? (int) (rows >> 32) : 0;
+            ws->slot = 0x7fffffff;
+            __threadfence();
+        }
+        g.sync();
+        const int opened = ws->next;
+        if (opened == 0) {
+            return;
+        }
+        for (int i = g.tid; i < p.pool_slots; i += g.n) {
+            const int rem = ld_volatile(&p.wide_ctl[i].rem1);
+            if (rem > kWarps / 2) {
+                /* a row with much left to do; among equals each block begins elsewhere */
+                const int at = i >= start ? i - start : i + p.pool_slots - start;
+                atomicMin(&ws->slot, ((kWidePiecesMax - rem) >> 3 << 16) | at);
+            }
+        }
+        g.sync();
+        const int at   = ws->slot;
+        const int slot = at == 0x7fffffff ? -1 : ((at & 0xffff) + start) % p.pool_slots;
+        if (g.tid == 0) {
+            const int left = slot < 0 ? 0 : atomicSub(&p.wide_ctl[slot].rem1, 1);
+            ws->next       = left > 0 ? pieces - left : -1;
+            __threadfence();
+        }
+        g.sync();
+        const int piece = ws->next;
+        g.sync();
+        if (piece >= 0) {
+            wide_join(p, gs, ws, slot, piece, save_mem);
+            g.sync();
+        } else if (slot < 0) {
+            looked = (unsigned) opened;
+        }
+    }
+}
+
+} /* namespace gb */

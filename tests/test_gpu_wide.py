@@ -1,0 +1,65 @@
+"""Top-p rows with wide nuclei (sampler_wide.cuh) against the CPU checker: rows around the pieces they are dealt out in,
+off the 16-byte grid, more rows than row copies, every way a row can be changed, ties, and long lists."""
+import numpy as np
+import pytest
+
+import oracle
+from geistlib_b200 import api
+from helpers import histories, independent_states, normal_logits, to_dev
+from test_gpu_parity import check_tokens, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def same(g, o):
+    check_tokens(g, o)
+    assert np.array_equal(g["kept_n"], o["detail_n"])
+
+
+@pytest.mark.parametrize("V,rows", [(33, 5), (511, 7), (512, 7), (513, 9), (1025, 3), (1537, 700), (4099, 40), (100003, 24), (128256, 3)])
+@pytest.mark.parametrize("kind", ["plain", "rep", "freq", "mask"])
+def test_pieces_and_changes(ctx, V, rows, kind):
+    x = normal_logits(rows, V, 1.0, V + rows)
+    st = independent_states(oracle.port, 3, rows)
+    P = np.linspace(0.5, 0.98, rows).astype(np.float32)
+    kw, okw, xo = {}, {}, x
+    if kind in ("rep", "freq"):
+        h = histories(rows, 70 if kind == "rep" else 1100, V, 4)
+        kw = {"history": h, "rep": 1.3, "freq": 0.1 if kind == "freq" else 0.0, "pres": 0.2}
+        okw = {"hist": h, "rep": 1.3, "freq": kw["freq"], "pres": 0.2}
+    if kind == "mask":
+        allowed = np.random.default_rng(5).random((rows, V)) < 0.7
+        allowed[:, :2] = True
+        words = np.zeros((rows, (V + 31) // 32 * 32), bool)
+        words[:, :V] = allowed
+        kw = {"logit_mask": to_dev(np.packbits(words, axis=1, bitorder="little").view(np.int32))}
+        xo = np.where(allowed, x, np.float32(-np.inf)).astype(np.float32)
+    g = run_gpu(ctx, x, 1.1, 0, P, st, kept_cap=4, **kw)
+    same(g, oracle.port.sample_batch(xo, 1.1, 0, P, st, detail_cap=4, **okw))
+    if V > 4000 and kind == "plain":
+        assert (g["status"] & api.ROW_SLOW_PATH).any()
+
+
+@pytest.mark.parametrize("V,step", [(6000, 0.25), (50000, 0.0625), (50000, 0.5), (9001, 100.0)])
+def test_rows_of_few_values(ctx, V, step):
+    """Ties by the hundred or the thousand, as logits that were 16 bits wide have them: long lists, and where they outrun
+    their room the multi-pass path."""
+    rows = 12
+    x = (np.round(normal_logits(rows, V, 1.5, 6) / step) * step).astype(np.float32)
+    st = independent_states(oracle.port, 7, rows)
+    P = np.linspace(0.3, 0.97, rows).astype(np.float32)
+    same(run_gpu(ctx, x, 0.9, 0, P, st, kept_cap=4), oracle.port.sample_batch(x, 0.9, 0, P, st, detail_cap=4))
+
+
+def test_rows_written_out_and_mixed_with_others(ctx):
+    """Wide rows between greedy, top-k and temperature ones, launched several times over, their logits written out."""
+    rows, V, H = 64, 30000, 40
+    x = normal_logits(rows, V, 1.2, 8)
+    h = histories(rows, H, V, 9)
+    T = np.where(np.arange(rows) % 4 == 0, 0.0, 0.9).astype(np.float32)
+    K = np.where(np.arange(rows) % 4 == 1, 30, 0).astype(np.int32)
+    P = np.where(np.arange(rows) % 4 == 2, 1.0, 0.9).astype(np.float32)
+    for seed in range(6):
+        st = independent_states(oracle.port, 100 * seed, rows)
+        g = run_gpu(ctx, x, T, K, P, st, history=h, rep=1.2, want_logits=seed % 2 == 1)
+        check_tokens(g, oracle.port.sample_batch(x, T, K, P, st, hist=h, rep=1.2))

@@ -318,7 +318,7 @@ __device__ __forceinline__ float penalise(float x, int cnt, float rep, float fre
  * did not prefetch: have_first = false). All threads of the group call this.
  * Returns status bits.
  */
-__device__ __forceinline__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const RowCfg &r, int V, int vocab_offset, unsigned *bitmap, PenEntry *dlist, int cap, int *n_dlist,
+__device__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const RowCfg &r, int V, int vocab_offset, unsigned *bitmap, PenEntry *dlist, int cap, int *n_dlist,
                                bool have_first, int first_id) {
     int       st    = 0;
     const int total = r.H + r.E;
@@ -1399,8 +1399,7 @@ __device__ __forceinline__ int top_bin(const int *hist, int lane, int kq) {
  * the bin that holds the kq-th entry; entries in higher bins are in, only that one bin is ranked exactly. cand is
  * overwritten. Called by the whole thread block.
  */
-__device__ __noinline__ void select_sorted(FinishShared *sh, Pair *cand, int total, int kq, Pair *sorted) {
-    const Grp g = whole_block();
+__device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int total, int kq, Pair *sorted) {
     Pair     e[kFinPer];
     unsigned lo = 0xffffffffu, hi = 0u;
 #pragma unroll
@@ -1896,7 +1895,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 }
                 g.sync();
             } else {
-                select_sorted(sh, cbuf, total, k, sh->fsort);
+                select_sorted(g, sh, cbuf, total, k, sh->fsort);
             }
             PROF(11);
             if (r.select_only) {
@@ -2028,7 +2027,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 }
                 g.sync();
             } else {
-                select_sorted(sh, cbuf, total, kq, sh->fsort);
+                select_sorted(g, sh, cbuf, total, kq, sh->fsort);
             }
             /* The walks over the kq entries, one per lane of a warp. Their running sums are exact wherever no entry is smaller
              * than 2^-29, so the order of additions is not seen; one thread that adds them one by one, three times over,
@@ -2052,6 +2051,9 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 const float    p_cut = __shfl_sync(0xffffffffu, e.v, max(cut - 1, 0));
                 const bool     ok    = cut > 0 && (reached == 0u || p_cut > p_floor || all_in);
                 if (ok) {
+                    if (g.lane == 0) {
+                        atomicAdd(&p.wide_head->rows, 1ull); /* the row is not wide: said as early as it is known */
+                    }
                     const double   N    = __shfl_sync(0xffffffffu, cum, cut - 1);
                     const double   u    = (double) unit_from(xorshift_next(r.rng)) * N;
                     const unsigned over = __ballot_sync(0xffffffffu, g.lane < cut && u < cum);
@@ -3401,7 +3403,7 @@ __device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *s
         wide_open(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), slot, row, st, bm, ba, S0, sh->save); /* done by whoever completes it */
         return;
     }
-    if (g.tid == 0) {
+    if (g.tid == 0 && r.mode == M_TOPP) {
         atomicAdd(&p.wide_head->rows, 1ull);
     }
     if (slot < 0) {
@@ -3453,8 +3455,12 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
         }
         PROF(8);
         if constexpr (!kFast) {
-            if (g.tid == 0 && r.mode == M_TOPP) {
-                *reinterpret_cast<volatile int *>(&p.wide_head->any) = 1;
+            if (g.tid == 0) {
+                if (r.mode == M_TOPP) {
+                    *reinterpret_cast<volatile int *>(&p.wide_head->any) = 1;
+                } else {
+                    atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
+                }
             }
         }
         int          st = finish_row<kFast>(g, p, sh, r, cmem, any);
@@ -3472,10 +3478,6 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
                 deferred_row(p, sh, cmem, row, st & ~ST_DEFERRED);
                 continue;
             }
-        } else if constexpr (!kFast) {
-            if (g.tid == 0) {
-                atomicAdd(&p.wide_head->rows, 1ull);
-            }
         }
         if (g.tid == 0) {
             row_epilogue(p, r, row, st, rc.rng);
@@ -3490,7 +3492,13 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
             } while (any == 0 && global_ns() - t0 < 3000ull);
         }
         if (__syncthreads_or(any) != 0) {
-            wide_help(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), sh->save);
+            int opened = 0;
+            if (g.tid == 0) {
+                opened = wide_wait(p, 0u);
+            }
+            if (__syncthreads_or(opened) != 0) {
+                wide_help(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), sh->save);
+            }
         }
     }
     PROF(kFast ? 6 : 7);

@@ -674,25 +674,30 @@ __device__ __forceinline__ void wide_open(const SampleParams &p, GroupShared *gs
     __syncthreads();
 }
 
-/* A thread block that has no rows of its own left helps with wide ones, as long as there can be any: rows that have not
- * been decided on yet, but no longer than kWideHelpNs without a piece to take. */
+/* A thread block that has no rows of its own left helps with wide ones, as long as there can be any: it waits for rows
+ * that have not been decided on, but no longer than kWideHelpNs. How many rows have been opened, 0 where those are no more
+ * than `looked` and there is nothing to wait for. One thread. */
 constexpr unsigned long long kWideHelpNs = 50000ull;
+__device__ __forceinline__ int wide_wait(const SampleParams &p, unsigned looked) {
+    const unsigned long long t0 = global_ns();
+    for (;;) {
+        const unsigned long long rows = *reinterpret_cast<volatile unsigned long long *>(&p.wide_head->rows);
+        if ((unsigned) (rows >> 32) > looked) {
+            return (int) (rows >> 32);
+        }
+        if ((int) (unsigned) rows >= p.n_rows || global_ns() - t0 > kWideHelpNs) {
+            return 0;
+        }
+        __nanosleep(40);
+    }
+}
 __device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, WideShared *ws, void *save_mem) {
     const Grp          g      = whole_block();
     const int          pieces = (p.V + kWidePiece - 1) / kWidePiece, start = (int) (blockIdx.x % (unsigned) p.pool_slots);
     unsigned           looked = 0u; /* rows that had been opened when the slots were last looked through in vain */
     for (;;) {
         if (g.tid == 0) {
-            const unsigned long long t0 = global_ns();
-            unsigned long long       rows;
-            for (;;) {
-                rows = *reinterpret_cast<volatile unsigned long long *>(&p.wide_head->rows);
-                if ((unsigned) (rows >> 32) > looked || (int) (unsigned) rows >= p.n_rows || global_ns() - t0 > kWideHelpNs) {
-                    break;
-                }
-                __nanosleep(40);
-            }
-            ws->next = (unsigned) (rows >> 32) > looked ? (int) (rows >> 32) : 0;
+            ws->next = wide_wait(p, looked);
             ws->slot = 0x7fffffff;
             __threadfence();
         }

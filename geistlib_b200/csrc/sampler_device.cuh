@@ -93,6 +93,15 @@ __device__ __forceinline__ void copy_word_async(void *dst_shared, const void *sr
 __device__ __forceinline__ void async_copies_wait() {
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
+/* The copies asked for since the last call become a group; all groups but the newest n (0 or 1) have arrived. */
+__device__ __forceinline__ void async_copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void async_copies_wait_but(int n) {
+    if (n == 0) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    }
+}
 
 __device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -2583,8 +2583,33 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             isrc += p.row_stride - (long long) p.n_slices * p.slice; /* on to the next row */
         }
     };
-    if (lane == 0 && aligned) {
-        for (int jj = 0; jj < min(kStages, my_count); jj++) {
+    /* Rows off the 16-byte grid: the same ring, filled by all lanes with 4-byte asynchronous copies, a group per item. With
+     * plain loads of the share in hand and nothing ahead every slice paid its own round trip to memory. */
+    auto issue_words = [&]() {
+        const bool last = ic == p.n_slices - 1;
+        const int  lo   = 4 * (last ? w4lo_l : w4lo_f), m = 4 * (last ? mine4_l : mine4_f), n_ = last ? n_last : n_full;
+        float     *dst  = reinterpret_cast<float *>(wring + (size_t) (ijj % kStages) * kWarpStageBytes);
+#pragma unroll 8
+        for (int i = lane; i < m; i += 32) {
+            if (lo + i < n_) {
+                copy_word_async(dst + i, isrc + lo + i);
+            } else {
+                dst[i] = -CUDART_INF_F;
+            }
+        }
+        async_copies_commit();
+        ijj++;
+        ic++;
+        isrc += p.slice;
+        if (last) {
+            ic = 0;
+            isrc += p.row_stride - (long long) p.n_slices * p.slice;
+        }
+    };
+    for (int jj = 0; jj < min(kStages, my_count); jj++) {
+        if (!aligned) {
+            issue_words();
+        } else if (lane == 0) {
             issue_next();
         }
     }
@@ -2835,11 +2860,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                     }
                 }
             } else {
-                /* rows off the 16-byte grid: plain loads into the warp's own stage */
-                for (int i = lane; i < 4 * mine4; i += 32) {
-                    const int gi = 4 * w4lo + i;
-                    sl[i]        = gi < n ? grow[gi] : -CUDART_INF_F;
-                }
+                async_copies_wait_but(j + 1 < my_count ? 1 : 0); /* the next item's group may be on its way */
             }
             __syncwarp();
             CYC(0);
@@ -2884,7 +2905,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             /* the share has been read: the stage is free again and the warp refills it itself */
             auto refill = [&]() {
                 __syncwarp();
-                if (lane == 0 && aligned && j + kStages < my_count && ring_dead < 0) {
+                if (!aligned) {
+                    if (j + kStages < my_count) {
+                        issue_words();
+                    }
+                } else if (lane == 0 && j + kStages < my_count && ring_dead < 0) {
                     if (wrote) { /* ordinary stores of this warp come before the copy engine's */
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     }

@@ -351,7 +351,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
                 }
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        async_copies_commit();
     };
     auto take_values = [&](int from, int step, float (&e)[kPer]) {
 #pragma unroll
@@ -361,11 +361,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         }
     };
     auto one_behind = [&](bool more) { /* the piece in work has arrived; the next may be on its way */
-        if (more) {
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        async_copies_wait_but(more ? 1 : 0);
         __syncwarp();
     };
     int       mine  = 0;

@@ -280,15 +280,34 @@ __device__ __forceinline__ float prologue_one(float x, int i, float cap, const u
  * slice; mine4 float4 groups, lane-strided; n: the slice's length, what lies behind it stays -inf). Kept out of
  * line: the stream kernel's loop stays short for the launches that have neither cap nor mask. */
 __device__ __noinline__ void prologue_share(float *sl, int lane, int mine4, int e0, int n, int s0, float cap, const unsigned *mrow) {
-    float4 *w4 = reinterpret_cast<float4 *>(sl) + lane;
-    for (int i = 0; lane + 32 * i < mine4; i++) {
-        const int e = e0 + 4 * (lane + 32 * i);
-        float4    v = w4[32 * i];
-        if (e + 0 < n) v.x = prologue_one(v.x, s0 + e + 0, cap, mrow);
-        if (e + 1 < n) v.y = prologue_one(v.y, s0 + e + 1, cap, mrow);
-        if (e + 2 < n) v.z = prologue_one(v.z, s0 + e + 2, cap, mrow);
-        if (e + 3 < n) v.w = prologue_one(v.w, s0 + e + 3, cap, mrow);
-        w4[32 * i] = v;
+    float4  *w4 = reinterpret_cast<float4 *>(sl) + lane;
+    unsigned allowed[kNV4]; /* four columns each: a float4 lies on a multiple of four, so inside one word of the mask */
+    if (mrow != nullptr) { /* all of the share's words at once: a word per column and use took a round trip for every float4 */
+#pragma unroll
+        for (int i = 0; i < kNV4; i++) {
+            const int at = s0 + e0 + 4 * (lane + 32 * i);
+            allowed[i]   = lane + 32 * i < mine4 ? __ldg(mrow + (at >> 5)) >> (at & 31) : 0u;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kNV4; i++) {
+        if (lane + 32 * i < mine4) {
+            const int e = e0 + 4 * (lane + 32 * i);
+            float4    v = w4[32 * i];
+            if (cap > 0.0f) {
+                if (e + 0 < n) v.x = soft_cap(v.x, cap);
+                if (e + 1 < n) v.y = soft_cap(v.y, cap);
+                if (e + 2 < n) v.z = soft_cap(v.z, cap);
+                if (e + 3 < n) v.w = soft_cap(v.w, cap);
+            }
+            if (mrow != nullptr) { /* what lies behind the row's end is -inf already */
+                v.x = (allowed[i] & 1u) != 0u ? v.x : -CUDART_INF_F;
+                v.y = (allowed[i] & 2u) != 0u ? v.y : -CUDART_INF_F;
+                v.z = (allowed[i] & 4u) != 0u ? v.z : -CUDART_INF_F;
+                v.w = (allowed[i] & 8u) != 0u ? v.w : -CUDART_INF_F;
+            }
+            w4[32 * i] = v;
+        }
     }
     __syncwarp();
 }

@@ -3550,8 +3550,6 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
 
 /* ------------------------------------------------ long histories, prepared -- */
 
-constexpr int kRowIdThreads = 256;
-
 /* Which (slice, warp) share a column lies in, and where in it. */
 __device__ __forceinline__ int share_of(const SampleParams &p, int id, int &off) {
     const int c = id / p.slice, local = id - c * p.slice;
@@ -3561,16 +3559,18 @@ __device__ __forceinline__ int share_of(const SampleParams &p, int id, int &off)
     return c * kWarps + w;
 }
 
-/* One CTA per row whose history (plus fed tokens) is longer than the stream kernel counts
+/* One thread block per row whose history (plus fed tokens) is longer than the stream kernel counts
  * by itself: the row's distinct ids with their counts, grouped by the (slice, warp) share they fall into.
  * pre_off[row][g] .. pre_off[row][g + 1] is share g's run in pre_list[row]; an entry is
- * (offset in the share) | (count << 10). Shorter rows are left to the stream kernel. */
-__global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_constant__ SampleParams p) {
+ * (offset in the share) | (count << 10). Shorter rows are left to the stream kernel. A thread keeps its kPer ids in
+ * registers: they are on their way while the table is cleared, and the thread whose id opened a slot of the table writes
+ * that id's entry, at the place in its share's run that counting the share gave it. */
+template <int kIdThreads, int kPer>
+__global__ void __launch_bounds__(kIdThreads) row_ids_kernel(const __grid_constant__ SampleParams p) {
     extern __shared__ __align__(16) int row_ids_smem[];
     int *tkey = row_ids_smem;          /* open-addressing table: the id ... */
     int *tcnt = tkey + p.id_slots;     /* ... and how often it occurs */
     int *bcnt = tcnt + p.id_slots;     /* entry g + 1: distinct ids in share g; after the scan, entry g: ids in the shares before */
-    int *bpos = bcnt + p.bucket_cap;   /* next free place of each share's run */
 
     /* the stream kernel behind this one may start now: it copies logits and sets itself up while the
      * lists are made, and waits for them where it first needs one */
@@ -3586,31 +3586,42 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
     }
     const int *hrow = p.hist ? p.hist + (size_t) seq * (size_t) p.hist_stride : nullptr;
     const int *erow = p.extra ? p.extra + (size_t) seq0 * (size_t) p.extra_stride : nullptr;
-    for (int i = tid; i < p.id_slots; i += kRowIdThreads) {
-        tkey[i] = -1;
-        tcnt[i] = 0;
+    int id[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        const int j = tid + q * kIdThreads;
+        id[q]       = j < H + E ? (j < H ? hrow[j] : erow[1 + j - H]) - p.vocab_offset : -1;
     }
-    for (int i = tid; i <= n_shares; i += kRowIdThreads) {
+    for (int i = tid; i < p.id_slots / 4; i += kIdThreads) {
+        reinterpret_cast<int4 *>(tkey)[i] = make_int4(-1, -1, -1, -1);
+        reinterpret_cast<int4 *>(tcnt)[i] = make_int4(0, 0, 0, 0);
+    }
+    for (int i = tid; i <= n_shares; i += kIdThreads) {
         bcnt[i] = 0;
     }
     __syncthreads();
     const unsigned smask = (unsigned) p.id_slots - 1u;
-    for (int j = tid; j < H + E; j += kRowIdThreads) {
-        const int id = (j < H ? hrow[j] : erow[1 + j - H]) - p.vocab_offset;
-        if (id >= 0 && id < p.V) {
-            unsigned hsh = ((unsigned) id * 2654435761u) & smask;
+    int            slot[kPer], share[kPer], place[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        slot[q] = -1;
+        if (id[q] >= 0 && id[q] < p.V) {
+            unsigned hsh = ((unsigned) id[q] * 2654435761u) & smask;
             for (int probe = 0; probe < p.id_slots; probe++) { /* at most half of the slots are ever taken */
-                const int old = atomicCAS(&tkey[hsh], -1, id);
-                if (old == -1 || old == id) {
+                const int old = atomicCAS(&tkey[hsh], -1, id[q]);
+                if (old == -1 || old == id[q]) {
                     atomicAdd(&tcnt[hsh], 1);
-                    if (old == -1) {
-                        int off;
-                        atomicAdd(&bcnt[share_of(p, id, off) + 1], 1);
-                    }
+                    slot[q] = old == -1 ? (int) hsh : -1;
                     break;
                 }
                 hsh = (hsh + 1u) & smask;
             }
+        }
+        if (slot[q] >= 0) {
+            int off;
+            share[q] = share_of(p, id[q], off);
+            place[q] = atomicAdd(&bcnt[share[q] + 1], 1);
+            id[q]    = off;
         }
     }
     __syncthreads();
@@ -3629,7 +3640,6 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
             }
             if (i <= n_shares) {
                 bcnt[i] = carry + incl;
-                bpos[i] = carry + incl;
                 off[i]  = carry + incl;
             }
             carry += __shfl_sync(0xffffffffu, incl, 31);
@@ -3637,15 +3647,15 @@ __global__ void __launch_bounds__(kRowIdThreads) row_ids_kernel(const __grid_con
     }
     __syncthreads();
     unsigned *list = p.pre_list + (size_t) row * (size_t) p.row_cap;
-    for (int i = tid; i < p.id_slots; i += kRowIdThreads) {
-        const int id = tkey[i];
-        if (id >= 0) {
-            int       off;
-            const int pos = atomicAdd(&bpos[share_of(p, id, off)], 1);
-            list[pos]     = (unsigned) off | ((unsigned) tcnt[i] << 10);
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        if (slot[q] >= 0) {
+            list[bcnt[share[q]] + place[q]] = (unsigned) id[q] | ((unsigned) tcnt[slot[q]] << 10);
         }
     }
 }
+
+constexpr int kIdsFew = 1024; /* ids a row can bring: up to here 256 threads with four each, else 1024 with eight (8192 ids at most: id_slots) */
 
 /* ----------------------------------------------------------------- launchers -- */
 
@@ -3709,22 +3719,22 @@ cudaError_t sample_stream_ctas_per_sm(size_t smem_bytes, int *out) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, sample_stream_kernel<K_SEL | K_SUMS | K_PEN>, kThreads, smem_bytes);
 }
 
-static cudaError_t ensure_row_ids_attributes(size_t smem_bytes) {
-    static int  configured_smem[64] = {0};
-    int         dev                 = 0;
-    cudaError_t e                   = cudaGetDevice(&dev);
+static cudaError_t ensure_row_ids_attributes(const void *kernel, int which, size_t smem_bytes) {
+    static int  configured_smem[64][2] = {{0}};
+    int         dev                    = 0;
+    cudaError_t e                      = cudaGetDevice(&dev);
     if (e != cudaSuccess) {
         return e;
     }
     if (dev < 0 || dev >= 64) {
         return cudaErrorInvalidDevice;
     }
-    if (smem_bytes > 48 * 1024 && (int) smem_bytes > configured_smem[dev]) {
-        e = cudaFuncSetAttribute(row_ids_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes);
+    if (smem_bytes > 48 * 1024 && (int) smem_bytes > configured_smem[dev][which]) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes);
         if (e != cudaSuccess) {
             return e;
         }
-        configured_smem[dev] = (int) smem_bytes;
+        configured_smem[dev][which] = (int) smem_bytes;
     }
     return cudaSuccess;
 }
@@ -3775,12 +3785,18 @@ cudaError_t launch_sample_stream(const SampleParams &p, int grid, size_t smem_by
         return e;
     }
     if (p.id_slots > 0) { /* rows may bring more ids than the stream kernel counts by itself: prepare their lists first */
-        const size_t ids_smem = ((size_t) p.id_slots * 2 + (size_t) p.bucket_cap * 2) * sizeof(int);
-        e                     = ensure_row_ids_attributes(ids_smem);
+        const size_t ids_smem = ((size_t) p.id_slots * 2 + (size_t) p.bucket_cap) * sizeof(int);
+        const bool   few      = p.row_cap <= kIdsFew;
+        const void  *kernel   = few ? reinterpret_cast<const void *>(row_ids_kernel<256, 4>) : reinterpret_cast<const void *>(row_ids_kernel<1024, 8>);
+        e                     = ensure_row_ids_attributes(kernel, few ? 0 : 1, ids_smem);
         if (e != cudaSuccess) {
             return e;
         }
-        row_ids_kernel<<<dim3((unsigned) p.n_rows), dim3(kRowIdThreads), ids_smem, stream>>>(p);
+        if (few) {
+            row_ids_kernel<256, 4><<<dim3((unsigned) p.n_rows), dim3(256), ids_smem, stream>>>(p);
+        } else {
+            row_ids_kernel<1024, 8><<<dim3((unsigned) p.n_rows), dim3(1024), ids_smem, stream>>>(p);
+        }
         e = cudaGetLastError();
         if (e != cudaSuccess) {
             return e;

@@ -377,6 +377,11 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     p.extra_stride = (long long) b->fed_stride;
     p.rng_in       = reinterpret_cast<const unsigned long long *>(b->rng_in);
     p.rng_out      = reinterpret_cast<unsigned long long *>(b->rng_out);
+    const void *const words[gb::kRawWords] = {nullptr, b->temperature, b->top_p, b->top_k, b->history ? b->history_len : nullptr, b->repetition_penalty, b->frequency_penalty,
+                                              b->presence_penalty, b->softcap, nullptr, b->rng_in, b->rng_in};
+    for (int i = 0; i < gb::kRawWords; i++) {
+        p.raw_word[i] = static_cast<const unsigned *>(words[i]);
+    }
     p.tokens       = b->tokens;
     p.status       = b->row_status;
     p.out_logits   = b->out_logits;

@@ -103,6 +103,8 @@ constexpr int kWideBins      = 1 << kWideBinsLog; /* bins of a row's histogram *
 constexpr int kWideCtlInts   = 16;
 constexpr int kWidePartBytes = 32;
 
+constexpr int kRawWords = 12; /* 32-bit words of a row's raw parameters: sequence, T, top_p, top_k, history length, rep, freq, pres, cap, (none), generator low and high */
+
 struct SampleParams {
     const float *logits;      /* [n_rows, V], row_stride floats apart */
     long long    row_stride;
@@ -128,6 +130,10 @@ struct SampleParams {
     const int *hist_len;      /* [n_seq] */
     const int *extra;         /* [n_seq, extra_stride] or null: tokens fed through a verify pass */
     long long  extra_stride;
+
+    /* The per-sequence words once more, as the stream kernel's warp asks for them, a lane each: where word i of a row's raw
+     * parameters comes from (null: its default) */
+    const unsigned *raw_word[kRawWords];
 
     const unsigned long long *rng_in;  /* [n_seq] */
     unsigned long long       *rng_out; /* [n_seq]; may alias rng_in only when rows_per_seq == 1 */

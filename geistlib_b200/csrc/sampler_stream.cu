@@ -1654,18 +1654,11 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             const double sm  = __ldcg(&segs[t].sum);
             return sm * ref_move(ref, row_max, r.inv_t);
         };
-        double part = 0.0;
-        for (int t = g.tid; t < nseg; t += g.n) {
-            part += seg_at(t);
-        }
-        const double S     = group_sum_d(g, gs, part);
-        const double u     = (double) unit_from(xorshift_next(r.rng)) * S;
-        double       carry = 0.0;
-        int          found = -1;
-        double       fbase = -CUDART_INF; /* nothing crosses: the walk ends on its last id */
-        for (int t0 = 0; t0 < nseg; t0 += g.n) {
-            const int    t    = t0 + g.tid;
-            const double val  = t < nseg ? seg_at(t) : 0.0;
+        int    found = -1;
+        double u, fbase = -CUDART_INF; /* nothing crosses: the walk ends on its last id */
+        if (nseg <= kThreads) {
+            /* a segment per thread: its sum is read and moved once, the scan's total is the row's sum */
+            const double val  = g.tid < nseg ? seg_at(g.tid) : 0.0;
             double       incl = val;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1674,7 +1667,6 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                     incl += up;
                 }
             }
-            g.sync();
             if (g.lane == 31) {
                 gs->wred_d[g.warp] = incl;
             }
@@ -1682,27 +1674,73 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 gs->pick = 0x7fffffff;
             }
             g.sync();
-            double woff = carry;
-            for (int w = 0; w < g.warp; w++) {
-                woff += gs->wred_d[w];
+            double S = 0.0, woff = 0.0;
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) {
+                woff = w == g.warp ? S : woff;
+                S += gs->wred_d[w];
             }
             incl += woff;
-            if (t < nseg && u < incl) {
-                atomicMin(&gs->pick, t);
+            u = (double) unit_from(xorshift_next(r.rng)) * S;
+            if (g.tid < nseg && u < incl) {
+                atomicMin(&gs->pick, g.tid);
             }
             g.sync();
-            const int pk = gs->pick;
-            if (pk != 0x7fffffff) {
-                if (t == pk) {
-                    gs->S = incl - val;
+            found = gs->pick == 0x7fffffff ? -1 : gs->pick;
+            if (g.tid == found) {
+                gs->S = incl - val;
+            }
+            g.sync();
+            fbase = found >= 0 ? gs->S : fbase;
+        } else {
+            double part = 0.0;
+            for (int t = g.tid; t < nseg; t += g.n) {
+                part += seg_at(t);
+            }
+            const double S = group_sum_d(g, gs, part);
+            u = (double) unit_from(xorshift_next(r.rng)) * S;
+            double carry = 0.0;
+            for (int t0 = 0; t0 < nseg; t0 += g.n) {
+                const int    t    = t0 + g.tid;
+                const double val  = t < nseg ? seg_at(t) : 0.0;
+                double       incl = val;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double up = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (g.lane >= o) {
+                        incl += up;
+                    }
                 }
                 g.sync();
-                found = pk;
-                fbase = gs->S;
-                break;
-            }
-            for (int w = 0; w < g.nw; w++) {
-                carry += gs->wred_d[w];
+                if (g.lane == 31) {
+                    gs->wred_d[g.warp] = incl;
+                }
+                if (g.tid == 0) {
+                    gs->pick = 0x7fffffff;
+                }
+                g.sync();
+                double woff = carry;
+                for (int w = 0; w < g.warp; w++) {
+                    woff += gs->wred_d[w];
+                }
+                incl += woff;
+                if (t < nseg && u < incl) {
+                    atomicMin(&gs->pick, t);
+                }
+                g.sync();
+                const int pk = gs->pick;
+                if (pk != 0x7fffffff) {
+                    if (t == pk) {
+                        gs->S = incl - val;
+                    }
+                    g.sync();
+                    found = pk;
+                    fbase = gs->S;
+                    break;
+                }
+                for (int w = 0; w < g.nw; w++) {
+                    carry += gs->wred_d[w];
+                }
             }
         }
         if (found < 0) {

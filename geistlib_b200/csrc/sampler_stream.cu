@@ -1294,6 +1294,7 @@ struct __align__(16) StreamShared {
                                                              * grouped by the (slice, warp) share they fall into, and where each group's run starts */
     alignas(16) unsigned id_bits[kIdBits / 32];             /* which values of the part an id has changed (slices s and s + 4 share their bits) */
     /* the part's select */
+    uint2              key_ends[kWarps];      /* smallest and largest key of a warp's thread maxima */
     int                n_grp, n_cand;         /* groups that reach the threshold; candidates in them */
     int                max_cnt;               /* how often the part's most frequent id occurs (asked where that raises a value) */
     unsigned short     grp[kGroupSlots * kThreads]; /* (slot << 8) | thread */
@@ -3139,8 +3140,26 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 sel1 = sel1 == -CUDART_INF_F ? sel1 : soft_cap(sel1, sh->cap);
             }
             const unsigned key0 = order_key(sel0), key1 = order_key(sel1);
-            unsigned       tkey = 0u;
-            for (int bit = 31; bit >= 0; bit--) {
+            /* The kq-th largest lies between the smallest and the largest of them: the search begins below their common bits
+             * (keys of a warp's extremes, one barrier; it saves half of the rounds, each of which is a barrier). */
+            const unsigned kmin = __reduce_min_sync(0xffffffffu, kq <= kThreads / 2 ? key0 : min(key0, key1)), kmax = __reduce_max_sync(0xffffffffu, max(key0, key1));
+            if (lane == 0) {
+                sh->key_ends[warp] = make_uint2(kmin, kmax);
+            }
+            __syncthreads();
+            unsigned all_min = 0xffffffffu, all_max = 0u;
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) {
+                const uint2 e = sh->key_ends[w];
+                all_min       = min(all_min, e.x);
+                all_max       = max(all_max, e.y);
+            }
+            const int same = __clz(all_min ^ all_max); /* leading bits that all have in common */
+            unsigned  tkey = same == 0 ? 0u : all_max & ~(0xffffffffu >> same);
+            if (same == 32) {
+                tkey = all_max;
+            }
+            for (int bit = 31 - same; bit >= 0; bit--) {
                 const unsigned t = tkey | (1u << bit);
                 int            n = __syncthreads_count(key0 >= t);
                 if (kq > kThreads / 2) {

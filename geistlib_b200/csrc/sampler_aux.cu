@@ -239,9 +239,12 @@ __global__ void __launch_bounds__(256) merge_sample_kernel(const __grid_constant
 
 /* ------------------------------------------------------ speculative accept -- */
 
-/* session.c:599-625, one thread per sequence. */
+/* session.c:599-625, one thread per sequence. A programmatic dependent of the sampling kernels: its thread blocks are there
+ * when those end. */
 __global__ void accept_kernel(const AcceptParams p) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
     if (s >= p.n_seq) {
         return;
     }
@@ -486,8 +489,16 @@ cudaError_t launch_merge_sample(const MergeParams &p, cudaStream_t stream) {
 }
 
 cudaError_t launch_accept(const AcceptParams &p, cudaStream_t stream) {
-    accept_kernel<<<(p.n_seq + 127) / 128, 128, 0, stream>>>(p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t  cfg{};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim                                        = dim3((unsigned) (p.n_seq + 127) / 128);
+    cfg.blockDim                                       = dim3(128);
+    cfg.stream                                         = stream;
+    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs                                          = attr;
+    cfg.numAttrs                                       = 1;
+    return cudaLaunchKernelEx(&cfg, accept_kernel, p);
 }
 
 cudaError_t launch_post_step(const int *slot, int n_seq, int per_seq, int first, const int *tokens, const int *counts, int *hist, int hist_cap, int *hist_len, long long *hist_total,

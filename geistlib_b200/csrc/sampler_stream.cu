@@ -2644,11 +2644,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
      * the gap between two grids. The kernel behind this one may be placed likewise. */
     if (lane == 0 && aligned) {
         /* While it waits, the thread block asks L2 for what its ring will copy first (the warp's shares of the run's
-         * first kStages items). Nothing is read: a line that the kernel before this one is still writing arrives in
+         * first kStages items, two more of a long run whose rows are not summed: the ring is full long before the first row's parameters are there; in
+         * runs of four or five items that delays what is wanted first, 64 x 151936 greedy 14.1 -> 14.8 us, in runs of sixteen
+         * it is worth 0.7 of 30.5). Nothing is read: a line that the kernel before this one is still writing arrives in
          * L2 with its stores either way. Back to back this is worth 0.5 us per launch: the last thread blocks of the
          * grid before leave DRAM idle. */
         const int n_full_ = min(p.slice, p.V), n_last_ = p.V - (p.n_slices - 1) * p.slice;
-        for (int jj = 0; jj < min(kStages, my_count); jj++) {
+        for (int jj = 0; jj < ((kKinds & K_SUMS) == 0 && my_count >= 12 ? kStages + 2 : min(kStages, my_count)); jj++) {
             const int item = my_first + jj, r_ = item / p.n_slices, c_ = item - r_ * p.n_slices;
             const int n_   = c_ == p.n_slices - 1 ? n_last_ : n_full_;
             const int nv4_ = (n_ + 3) >> 2, L_ = share_len(nv4_);

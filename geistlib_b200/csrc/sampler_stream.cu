@@ -28,9 +28,9 @@
  *   records; greedy rows end there; top-k rows (k <= 256) get their surviving candidates ordered, their
  *   probabilities evaluated exactly (double exp rounded once) and the draw made; temperature rows walk the
  *   per-warp segment sums and re-read the one segment that the draw falls into; top-p rows with a small nucleus
- *   are served from the candidates and the sums of the rest; rows whose kept set is too large for one pass
- *   (top-k beyond 256, wide nuclei) are worked on a private copy of the row in global scratch (the multi-pass
- *   path, ROW_SLOW_PATH). finish_rows_kernel<false> carries all of that; finish_rows_kernel<true> carries greedy
+ *   are served from the candidates and the sums of the rest; wide nuclei are worked on by all thread blocks that
+ *   have no row left (sampler_wide.cuh); top-k rows beyond 256 and what neither serves take a private copy of the row
+ *   in global scratch (the multi-pass path; ROW_SLOW_PATH in both cases). finish_rows_kernel<false> carries all of that; finish_rows_kernel<true> carries greedy
  *   and top-k alone and is launched instead when the caller vouched for such rows (F_FAST_ONLY); with
  *   F_GREEDY_ONLY, and with F_INLINE_TOPK (whole rows per thread block, greedy and top-k rows), the stream kernel
  *   writes the tokens itself and no finishing kernel runs.
@@ -3535,9 +3535,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
 /*
  * Run behind the stream kernel, one thread block per row at a time (rows blockIdx.x, blockIdx.x + gridDim.x, ...):
  * it merges the records that the row's parts left and finishes the row. finish_rows_kernel<false> carries the
- * code for every kind of row: greedy, top-k, temperature (segment walks), top-p (nucleus sums), and the
- * multi-pass path over a private copy of the row (the copies come from a small pool that the thread blocks claim
- * slots of). finish_rows_kernel<true> carries greedy and top-k (k <= 256) alone: a tenth of the code, 7 - 8 us
+ * code for every kind of row: greedy, top-k, temperature (segment walks), top-p (nucleus sums), wide nuclei, which
+ * thread blocks without a row of their own help with, and the multi-pass path over a private copy of the row (a copy per
+ * row, or a pool that the thread blocks claim slots of). finish_rows_kernel<true> carries greedy and top-k (k <= 256) alone: a tenth of the code, 7 - 8 us
  * less per launch; it is launched instead when the caller vouched for such rows, and reports any other row as
  * ROW_INTERNAL. Both write the row's status and, behind a sequence's last row, its generator.
  */

@@ -447,17 +447,22 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
             CUDA_TRY(cudaMalloc((void **) &ln->buf, need));
             ln->bytes = need;
         }
-        if (ln->counter_cap < slots && (p.flags & gb::F_FAST_ONLY) == 0u) {
-            cudaFree(ln->counters);
-            ln->counters    = nullptr;
-            ln->counter_cap = 0;
-            const size_t cap = round_up(slots, 32);
+        if (ln->counters == nullptr) {
             /* per row copy of the multi-pass path a flag, and a wide row's words and histogram, all zero between launches
-             * (whoever takes a copy gives it back as it was). Zeroed on the launch's own stream, so the first kernel that
-             * uses them comes behind it. */
+             * (whoever takes a copy gives it back as it was). As many as any launch of the device can use (4.9 MB on a B200),
+             * by the lane's first launch of whatever kind: they are never replaced, so a launch that was captured keeps
+             * them, and no later launch has to allocate for them or to wait for the device. Zeroed on the launch's own
+             * stream, so the first kernel that uses them comes behind it. */
+            const size_t cap   = (size_t) pl.fin_ctas;
             const size_t bytes = (kHeadInts + cap * (size_t) (1 + gb::kWideCtlInts + gb::kWideBins)) * sizeof(int);
-            CUDA_TRY(cudaMalloc((void **) &ln->counters, bytes));
-            CUDA_TRY(cudaMemsetAsync(ln->counters, 0, bytes, st));
+            int         *words = nullptr;
+            CUDA_TRY(cudaMalloc((void **) &words, bytes));
+            const cudaError_t ze = cudaMemsetAsync(words, 0, bytes, st);
+            if (ze != cudaSuccess) { /* words that are not zero are not kept */
+                cudaFree(words);
+                CUDA_TRY(ze);
+            }
+            ln->counters    = words;
             ln->counter_cap = cap;
         }
         if ((p.flags & gb::F_GREEDY_ONLY) != 0u && ln->arrive_cap < n_rows) {
@@ -471,12 +476,10 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
             ln->arrive_cap = cap;
         }
     }
-    if (ln->counters != nullptr) {
-        p.wide_head = reinterpret_cast<gb::WideHead *>(ln->counters);
-        p.wide_ctl  = reinterpret_cast<gb::WideCtl *>(ln->counters + kHeadInts);
-        p.wide_hist = reinterpret_cast<unsigned *>(ln->counters + kHeadInts + ln->counter_cap * (size_t) gb::kWideCtlInts);
-        p.pool      = ln->counters + kHeadInts + ln->counter_cap * (size_t) (gb::kWideCtlInts + gb::kWideBins);
-    }
+    p.wide_head        = reinterpret_cast<gb::WideHead *>(ln->counters);
+    p.wide_ctl         = reinterpret_cast<gb::WideCtl *>(ln->counters + kHeadInts);
+    p.wide_hist        = reinterpret_cast<unsigned *>(ln->counters + kHeadInts + ln->counter_cap * (size_t) gb::kWideCtlInts);
+    p.pool             = ln->counters + kHeadInts + ln->counter_cap * (size_t) (gb::kWideCtlInts + gb::kWideBins);
     p.wide_part        = reinterpret_cast<gb::WidePart *>(ln->buf + off_wp);
     p.arrive           = ln->arrive;
     p.pool_slots       = (int) slots;

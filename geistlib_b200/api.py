@@ -143,6 +143,7 @@ PROTOTYPES = {
                                                     c_void_p]),
     "geist_b200_argmax_rows_static": (C.c_int, [C.c_int, c_void_p, c_size_t, c_size_t, c_size_t, c_void_p, c_void_p]),
     "geist_b200_grid": (C.c_int, [c_size_t, c_size_t, c_size_t, C.POINTER(c_int32), C.POINTER(c_int32)]),
+    "geist_b200_wide_counts": (C.c_int, [c_void_p, C.POINTER(c_int32), C.POINTER(c_int32), C.POINTER(c_int32)]),
     "geist_b200_plan": (C.c_int, [c_size_t, c_size_t, C.POINTER(c_int32), C.POINTER(c_int32), C.POINTER(c_int32),
                                   C.POINTER(c_int32)]),
 }
@@ -252,6 +253,12 @@ class Context:
         """Launch a descriptor prepared by sample_batch(..., launch=False) again (asynchronous)."""
         fn = lib.geist_b200_shard_select if out.get("_select") else lib.geist_b200_sample_batch
         _check(fn(self.handle, C.byref(out["_desc"]), c_void_p(stream)))
+
+    def wide_counts(self):
+        """Of the last launch's wide top-p rows: (shared out, decided by their lists, longest list)."""
+        n = [c_int32() for _ in range(3)]
+        _check(lib.geist_b200_wide_counts(self.handle, *(C.byref(v) for v in n)))
+        return tuple(v.value for v in n)
 
     def argmax_f32(self, row) -> int:
         idx = c_int32(-1)

@@ -67,6 +67,7 @@ namespace {
 
 constexpr size_t kSmemMax = 227 * 1024; /* opt-in shared memory per CTA on sm_100 */
 constexpr size_t kHeadInts = 16;       /* words in front of a lane's per-slot words */
+static_assert(sizeof(gb::WideHead) <= kHeadInts * sizeof(int), "the launch's words lie in front");
 constexpr int    kLanes   = 4;          /* launches of one context that may overlap on the GPU */
 
 struct Plan {
@@ -577,6 +578,30 @@ extern "C" enum geist_status geist_b200_scatter_kept(struct geist_b200_ctx *ctx,
     }
     CUDA_TRY(cudaSetDevice(ctx->device));
     CUDA_TRY(gb::launch_scatter_kept(kept_n, kept_idx, kept_prob, kept_cap, (int) n_rows, (int) n_vocab, vocab_offset, dense, as_stream(stream)));
+    return GEIST_OK;
+}
+
+extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest) {
+    if (ctx == nullptr) {
+        return fail(GEIST_E_INVALID_ARG, "wide_counts: NULL context");
+    }
+    CUDA_TRY(cudaSetDevice(ctx->device));
+    gb::WideHead                h{};
+    std::lock_guard<std::mutex> lk(ctx->lane_mu);
+    const geist_b200_ctx::Lane &ln = ctx->lane[(ctx->next_lane + kLanes - 1) % kLanes];
+    if (ln.counters != nullptr) {
+        CUDA_TRY(cudaDeviceSynchronize());
+        CUDA_TRY(cudaMemcpy(&h, ln.counters, sizeof h, cudaMemcpyDeviceToHost));
+    }
+    if (opened) {
+        *opened = (int32_t) (h.rows >> 32);
+    }
+    if (by_lists) {
+        *by_lists = h.by_lists;
+    }
+    if (longest) {
+        *longest = h.longest;
+    }
     return GEIST_OK;
 }
 

@@ -94,7 +94,10 @@ struct WidePart;
 struct WideHead {
     unsigned long long rows; /* rows of the launch that are done or open for everybody; in the upper half those that were opened */
     int                any;  /* there are top-p rows */
-    int                pad;
+    /* for geist_b200_wide_counts */
+    int                by_lists; /* rows that their two lists decided; the other opened ones went the multi-pass way */
+    int                longest;  /* entries of the longest list that was walked */
+    int                pad[3];
 };
 constexpr int kWidePiece     = 512;  /* columns that are dealt out at a time, to a warp */
 constexpr int kWidePiecesMax = 4096; /* rows of more pieces go the multi-pass way */

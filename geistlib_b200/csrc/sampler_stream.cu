@@ -2663,7 +2663,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if ((kKinds & K_SUMS) != 0 && tid == 0 && blockIdx.x == 0 && p.wide_head != nullptr) { /* the finishing kernel's count of rows begins at nothing */
-        *reinterpret_cast<int4 *>(p.wide_head) = make_int4(0, 0, 0, 0);
+        static_assert(sizeof(WideHead) == 32, "two words of 16 bytes");
+        reinterpret_cast<int4 *>(p.wide_head)[0] = make_int4(0, 0, 0, 0);
+        reinterpret_cast<int4 *>(p.wide_head)[1] = make_int4(0, 0, 0, 0);
     }
     asm volatile("griddepcontrol.launch_dependents;");
 #ifdef GB_PROFILE

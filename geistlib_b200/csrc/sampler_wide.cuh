@@ -270,6 +270,8 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
             if (p.kept_cap > 0) {
                 p.kept_n[r.row] = (int) (above + cut.rank);
             }
+            atomicAdd(&p.wide_head->by_lists, 1);
+            atomicMax(&p.wide_head->longest, max(n_cut, n_pick));
         }
         st |= ST_SLOW_PATH | (p.kept_cap > 0 ? (int) ST_KEPT_PARTIAL : 0);
     } else {

@@ -408,6 +408,12 @@ enum geist_status geist_b200_plan(size_t n_vocab, size_t max_history, int32_t *s
 enum geist_status geist_b200_grid(size_t n_vocab, size_t max_history, size_t n_rows, int32_t *thread_blocks,
                                   int32_t *blocks_per_sm);
 
+/* What became of the wide top-p rows (nuclei beyond the finishing kernel's first 32 candidates) of the context's last
+ * launch: how many were shared out to all thread blocks, how many of those the two lists of entries near the crossing and
+ * the draw decided (the others took the multi-pass path), and the longest such list. Waits for the device; for tests and
+ * for looking into a workload. A launch whose hint leaves no top-p rows does not touch the counts. */
+enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest);
+
 /* Greedy argmax of n_rows rows [n_rows, n_vocab] (device memory, row_stride floats apart)
  * into out_index [n_rows] (device memory), ties -> lowest index, WITHOUT allocating: no
  * context, no cudaMalloc, no growth on larger batches. No counterpart in the reference; it

@@ -9,6 +9,7 @@ from helpers import histories, independent_states, normal_logits, to_dev
 from test_gpu_parity import check_tokens, run_gpu
 
 pytestmark = pytest.mark.gpu
+RANKED = 512  # lists up to here are walked by ranking (kWideRank)
 
 
 def same(g, o):
@@ -36,8 +37,10 @@ def test_pieces_and_changes(ctx, V, rows, kind):
         xo = np.where(allowed, x, np.float32(-np.inf)).astype(np.float32)
     g = run_gpu(ctx, x, 1.1, 0, P, st, kept_cap=4, **kw)
     same(g, oracle.port.sample_batch(xo, 1.1, 0, P, st, detail_cap=4, **okw))
-    if V > 4000 and kind == "plain":
-        assert (g["status"] & api.ROW_SLOW_PATH).any()
+    opened, by_lists, longest = ctx.wide_counts()
+    if V > 1000:  # normal rows: wide, and all of them decided where they are shared out
+        assert opened > rows // 2 and by_lists == opened and 0 < longest <= RANKED, (opened, by_lists, longest)
+        assert ((g["status"] & api.ROW_SLOW_PATH) != 0).sum() == opened
 
 
 @pytest.mark.parametrize("V,step", [(6000, 0.25), (50000, 0.0625), (50000, 0.5), (9001, 100.0)])
@@ -49,6 +52,26 @@ def test_rows_of_few_values(ctx, V, step):
     st = independent_states(oracle.port, 7, rows)
     P = np.linspace(0.3, 0.97, rows).astype(np.float32)
     same(run_gpu(ctx, x, 0.9, 0, P, st, kept_cap=4), oracle.port.sample_batch(x, 0.9, 0, P, st, detail_cap=4))
+    opened, by_lists, longest = ctx.wide_counts()
+    if step == 100.0:  # one value: the candidates outrun their room already, the row is not shared out
+        assert opened == 0
+    else:
+        assert by_lists > 0
+    if V == 50000:
+        assert longest > RANKED, (opened, by_lists, longest)
+
+
+def test_rows_that_their_lists_do_not_decide(ctx):
+    """A few hundred large values and then 40000 equal ones, in which the crossing falls: more than a list holds."""
+    rows, V = 8, 40400
+    rng = np.random.default_rng(12)
+    x = np.zeros((rows, V), np.float32)
+    for r in range(rows):
+        x[r, rng.choice(V, 400, replace=False)] = rng.uniform(3.0, 4.5, 400)
+    st = independent_states(oracle.port, 13, rows)
+    P = np.linspace(0.6, 0.97, rows).astype(np.float32)
+    same(run_gpu(ctx, x, 0.9, 0, P, st, kept_cap=4), oracle.port.sample_batch(x, 0.9, 0, P, st, detail_cap=4))
+    assert ctx.wide_counts()[:2] == (rows, 0)
 
 
 def test_rows_written_out_and_mixed_with_others(ctx):

@@ -68,6 +68,7 @@ namespace {
 constexpr size_t kSmemMax = 227 * 1024; /* opt-in shared memory per CTA on sm_100 */
 constexpr size_t kHeadInts = 16;       /* words in front of a lane's per-slot words */
 static_assert(sizeof(gb::WideHead) <= kHeadInts * sizeof(int), "the launch's words lie in front");
+constexpr unsigned long long kWideWaitNs = 1000000000ull; /* a second, as the kernels' other waits */
 constexpr int    kLanes   = 4;          /* launches of one context that may overlap on the GPU */
 
 struct Plan {
@@ -242,6 +243,7 @@ struct geist_b200_ctx {
         size_t         counter_cap = 0;
     } lane[kLanes];
     unsigned   next_lane = 0;
+    unsigned long long wide_wait_ns = kWideWaitNs;
     std::mutex lane_mu;
 };
 
@@ -482,6 +484,7 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     p.wide_hist        = reinterpret_cast<unsigned *>(ln->counters + kHeadInts + ln->counter_cap * (size_t) gb::kWideCtlInts);
     p.pool             = ln->counters + kHeadInts + ln->counter_cap * (size_t) (gb::kWideCtlInts + gb::kWideBins);
     p.wide_part        = reinterpret_cast<gb::WidePart *>(ln->buf + off_wp);
+    p.wide_wait_ns     = ctx->wide_wait_ns;
     p.arrive           = ln->arrive;
     p.pool_slots       = (int) slots;
     p.parts            = ln->buf;
@@ -581,7 +584,7 @@ extern "C" enum geist_status geist_b200_scatter_kept(struct geist_b200_ctx *ctx,
     return GEIST_OK;
 }
 
-extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest) {
+extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest, int32_t *gave_up) {
     if (ctx == nullptr) {
         return fail(GEIST_E_INVALID_ARG, "wide_counts: NULL context");
     }
@@ -602,6 +605,17 @@ extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, 
     if (longest) {
         *longest = h.longest;
     }
+    if (gave_up) {
+        *gave_up = h.gave_up;
+    }
+    return GEIST_OK;
+}
+
+extern "C" enum geist_status geist_b200_set_wide_wait(struct geist_b200_ctx *ctx, uint64_t ns) {
+    if (ctx == nullptr) {
+        return fail(GEIST_E_INVALID_ARG, "set_wide_wait: NULL context");
+    }
+    ctx->wide_wait_ns = std::min<unsigned long long>(ns, kWideWaitNs);
     return GEIST_OK;
 }
 

@@ -97,7 +97,8 @@ struct WideHead {
     /* for geist_b200_wide_counts */
     int                by_lists; /* rows that their two lists decided; the other opened ones went the multi-pass way */
     int                longest;  /* entries of the longest list that was walked */
-    int                pad[3];
+    int                gave_up;  /* thread blocks that went on without the others' pieces */
+    int                pad[2];
 };
 constexpr int kWidePiece     = 512;  /* columns that are dealt out at a time, to a warp */
 constexpr int kWidePiecesMax = 4096; /* rows of more pieces go the multi-pass way */
@@ -183,6 +184,7 @@ struct SampleParams {
     WideCtl   *wide_ctl;    /* [pool_slots] */
     unsigned  *wide_hist;   /* [pool_slots, kWideBins] */
     WidePart  *wide_part;   /* [pool_slots, pieces of a row] */
+    unsigned long long wide_wait_ns; /* how long a thread block waits for the others' pieces of a wide row */
     int        gen_hist_cap;
 };
 

@@ -219,8 +219,11 @@ __device__ __forceinline__ int wide_got(int left, int pieces) {
     return l > 0 ? pieces - l : -1;
 }
 
-/* The last of a row's thread blocks: the two walks, the token, and the slot made ready for its next row. */
-__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, RowCfg &r, int slot, float inv_hi, float inv_lo, unsigned long long rng0, void *save_mem) {
+/* The last of a row's thread blocks: the two walks, the token, and the slot made ready for its next row. `listed`: the block
+ * took part in pass 2, so that is through; one that had given up waiting for pass 1 does not know its windows, and nobody
+ * need have made the lists. */
+__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, RowCfg &r, int slot, bool listed, float inv_hi, float inv_lo, unsigned long long rng0,
+                                         void *save_mem) {
     const Grp       g      = whole_block();
     WideCtl        *ctl    = p.wide_ctl + slot;
     const int       V      = p.V, pieces = (V + kWidePiece - 1) / kWidePiece, idx_bits = 32 - __clz(max(V - 1, 1));
@@ -246,7 +249,7 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
         return pv > 0.0f && (hi >= kWideBins - 1 || pv < p_at(bins.edge(hi + 1))) && pv > p_at(bins.edge(lo) - 1u);
     };
     const int w0 = ws->win[0], w1 = ws->win[1], w2 = ws->win[2], w3 = ws->win[3];
-    bool      ok = n_cut <= half && n_pick <= half && n_cut > 0 && a_cut < (double) r.top_p;
+    bool      ok = listed && n_cut <= half && n_pick <= half && n_cut > 0 && a_cut < (double) r.top_p;
     WideHit   cut{}, pick{};
     if (ok) {
         cut = wide_walk(g, gs, ws, list, n_cut, a_cut, (double) r.top_p, true, idx_bits);
@@ -480,18 +483,31 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         bool                     in = true;
         while (ld_volatile(&ctl->done1) < pieces && in) {
             __nanosleep(50);
-            in = global_ns() - t0 < kWaitLimitNs;
+            in = global_ns() - t0 < p.wide_wait_ns;
         }
         __threadfence();
         ws->next = in ? 1 : 0;
     }
     g.sync();
-    if (ws->next == 0) {
+    /* A row's last thread block finishes it, whoever that is: each was dealt a piece of pass 1 at least, and counts its own
+     * once more when it is through here. The slot is then free for another row. */
+    auto leave = [&](bool listed, float inv_hi, float inv_lo) {
+        __threadfence();
+        g.sync();
         if (g.tid == 0) {
-            p.tokens[row] = -1;
-            p.status[row] = ST_INTERNAL;
+            ws->next = atomicAdd(&ctl->done2, ws->mine) + ws->mine == pieces ? 1 : 0;
+            __threadfence();
         }
         g.sync();
+        if (ws->next != 0) {
+            wide_finish(p, gs, ws, r, slot, listed, inv_hi, inv_lo, rc.rng, save_mem);
+        }
+    };
+    if (ws->next == 0) { /* gave up: its pieces of pass 1 are done all the same, so the row goes on without the block */
+        if (g.tid == 0) {
+            atomicAdd(&p.wide_head->gave_up, 1);
+        }
+        leave(false, 0.0f, 0.0f);
         return;
     }
     left = wide_ask(&ctl->rem2, g.lane);
@@ -639,18 +655,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         piece = next;
         __syncwarp();
     }
-    /* The row is done, and its slot free for another one, when every thread block that works on it is through here: each
-     * was dealt a piece of pass 1 at least, and counts its own once more. */
-    __threadfence();
-    g.sync();
-    if (g.tid == 0) {
-        ws->next = atomicAdd(&ctl->done2, ws->mine) + ws->mine == pieces ? 1 : 0;
-        __threadfence();
-    }
-    g.sync();
-    if (ws->next != 0) {
-        wide_finish(p, gs, ws, r, slot, inv_hi, inv_lo, rc.rng, save_mem);
-    }
+    leave(true, inv_hi, inv_lo);
 }
 
 /* Opens the row in a slot that the thread block has claimed, for everybody; the block then works on it itself. */

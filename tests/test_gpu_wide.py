@@ -37,7 +37,7 @@ def test_pieces_and_changes(ctx, V, rows, kind):
         xo = np.where(allowed, x, np.float32(-np.inf)).astype(np.float32)
     g = run_gpu(ctx, x, 1.1, 0, P, st, kept_cap=4, **kw)
     same(g, oracle.port.sample_batch(xo, 1.1, 0, P, st, detail_cap=4, **okw))
-    opened, by_lists, longest = ctx.wide_counts()
+    opened, by_lists, longest, _ = ctx.wide_counts()
     if V > 1000:  # normal rows: wide, and all of them decided where they are shared out
         assert opened > rows // 2 and by_lists == opened and 0 < longest <= RANKED, (opened, by_lists, longest)
         assert ((g["status"] & api.ROW_SLOW_PATH) != 0).sum() == opened
@@ -52,7 +52,7 @@ def test_rows_of_few_values(ctx, V, step):
     st = independent_states(oracle.port, 7, rows)
     P = np.linspace(0.3, 0.97, rows).astype(np.float32)
     same(run_gpu(ctx, x, 0.9, 0, P, st, kept_cap=4), oracle.port.sample_batch(x, 0.9, 0, P, st, detail_cap=4))
-    opened, by_lists, longest = ctx.wide_counts()
+    opened, by_lists, longest, _ = ctx.wide_counts()
     if step == 100.0:  # one value: the candidates outrun their room already, the row is not shared out
         assert opened == 0
     else:
@@ -86,3 +86,25 @@ def test_rows_written_out_and_mixed_with_others(ctx):
         st = independent_states(oracle.port, 100 * seed, rows)
         g = run_gpu(ctx, x, T, K, P, st, history=h, rep=1.2, want_logits=seed % 2 == 1)
         check_tokens(g, oracle.port.sample_batch(x, T, K, P, st, hist=h, rep=1.2))
+
+
+@pytest.mark.parametrize("rows,V", [(24, 60000), (330, 9000)])
+def test_a_wait_that_runs_out(rows, V):
+    """Thread blocks that wait no time for the others' pieces go on without them: the rows come out the same, and what the
+    launch leaves behind serves the next ones as before."""
+    ctx = api.Context(0)
+    x = normal_logits(rows, V, 1.0, 21)
+    st = independent_states(oracle.port, 22, rows)
+    o = oracle.port.sample_batch(x, 1.1, 0, 0.95, st, detail_cap=4)
+    gave_up = 0
+    for wait in (10 ** 12, 0, 10 ** 12):
+        api._check(api.lib.geist_b200_set_wide_wait(ctx.handle, wait))
+        for _ in range(4):  # every set of scratch
+            same(run_gpu(ctx, x, 1.1, 0, 0.95, st, kept_cap=4), o)
+            counts = ctx.wide_counts()
+            assert counts[0] == rows
+            if wait:
+                assert counts[1] == rows and counts[3] == 0
+            gave_up += counts[3]
+    assert gave_up > 0 or V < 60000
+    ctx.close()

@@ -1,0 +1,35 @@
+/* The wide rows' arithmetic against what the multi-pass path computes, on the device: built and called by
+ * test_gpu_wide_math.py. */
+#include "../geistlib_b200/csrc/sampler_wide_math.cuh"
+
+/* Arguments -|x| by their bits, first and up: how many come out otherwise than exp_exact's, and the bits of one. */
+__global__ void exp_kernel(unsigned first, unsigned n, unsigned long long *differ, unsigned *which) {
+    const double   t32  = exp2((double) (threadIdx.x & 31u) * 0x1p-5);
+    const unsigned step = gridDim.x * blockDim.x;
+    for (unsigned i0 = blockIdx.x * blockDim.x; i0 < n; i0 += step) { /* whole warps: the table is shared among the lanes */
+        const unsigned bits = first + min(i0 + threadIdx.x, n - 1u);
+        const float    a    = -__uint_as_float(bits);
+        if (__float_as_uint(gb::wide_exp(a, t32)) != __float_as_uint(gb::exp_exact(a)) && i0 + threadIdx.x < n) {
+            atomicAdd(differ, 1ull);
+            *which = bits;
+        }
+    }
+}
+
+extern "C" int exp_differs(unsigned first, unsigned n, unsigned long long *differ, unsigned *which) {
+    struct Out {
+        unsigned long long differ;
+        unsigned           which;
+    } h{}, *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, sizeof h);
+    if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof h);
+    if (e == cudaSuccess) {
+        exp_kernel<<<148 * 8, 256>>>(first, n, &d->differ, &d->which);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof h, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    *differ = h.differ;
+    *which  = h.which;
+    return (int) e;
+}

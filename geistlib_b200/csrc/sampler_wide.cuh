@@ -10,7 +10,7 @@
  *           as the stream kernel formed it).
  *   pass 2  starts when every piece is through pass 1: S is known, and from the histogram the bins in which the walk
  *           reaches top_p and in which the draw will fall, with a margin for the units' rounding. p_i = (float)(e_i / S);
- *           what lies above a window is summed in double, what lies in it is listed (a few entries, or a few hundred).
+ *           what lies above a window is summed in units of 2^-62, what lies in it is listed (a few entries, or a few hundred).
  *   end     the thread block that completes pass 2 walks the two lists exactly, in (p desc, id asc) order, and has the
  *           token. Whatever the lists do not decide (more entries than they hold, a crossing outside its window, equal
  *           probabilities at a window's edge) goes to multipass_row.
@@ -48,10 +48,10 @@ static_assert(sizeof(WideCtl) == 4 * kWideCtlInts, "a slot's words");
 
 /* What a piece adds up to. */
 struct __align__(16) WidePart {
-    double sum;                   /* of e */
-    double above_cut, above_pick; /* of p, above the two windows */
-    int    n_above;               /* entries above the window of the crossing */
-    int    pad;
+    double    sum;                   /* of e */
+    long long above_cut, above_pick; /* of p, above the two windows (wide_mass) */
+    int       n_above;               /* entries above the window of the crossing */
+    int       pad;
 };
 static_assert(sizeof(WidePart) == kWidePartBytes, "the host sizes the parts");
 
@@ -99,8 +99,8 @@ struct WideHit {
 };
 
 /* The first of the n listed entries, in (p desc, id asc) order, at which base + running mass reaches (inclusive) or
- * exceeds the target. Masses are added in units of 2^-62, so the order of the list does not matter. All threads call. */
-__device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, const Pair *list, int n, double base, double target, bool inclusive, int idx_bits) {
+ * exceeds the target. Masses are added in units of 2^-62 (wide_mass), so the order of the list does not matter. All threads call. */
+__device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, const Pair *list, int n, long long base, double target, bool inclusive, int idx_bits) {
     WideHit out;
     if (n <= kWideRank) {
         unsigned long long *word = reinterpret_cast<unsigned long long *>(&ws->x[0][0][0]), *mass = word + kWideRank;
@@ -110,7 +110,7 @@ __device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, cons
             const unsigned long long w  = __ldcg(reinterpret_cast<const unsigned long long *>(list + i)); /* p, then the id */
             const float              pv = __uint_as_float((unsigned) w);
             word[i]                     = composite(__float_as_uint(pv), (int) (w >> 32), idx_bits);
-            mass[i]                     = __double2ull_rz((double) pv * 0x1p62);
+            mass[i]                     = (unsigned long long) wide_mass(pv);
         }
         if (g.tid == 0) {
             ws->best = 0ull;
@@ -131,7 +131,7 @@ __device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, cons
                     my_sum[q] += up ? mass[j] : 0ull;
                     my_rank[q] += up ? 1 : 0;
                 }
-                const double at = base + (double) my_sum[q] * 0x1p-62;
+                const double at = mass_value(base + (long long) my_sum[q]);
                 if (inclusive ? at >= target : at > target) {
                     mine = max(mine, me);
                 }
@@ -152,7 +152,7 @@ __device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, cons
         }
         g.sync();
         out.found = out.word != 0ull;
-        out.mass  = base + (double) ws->best_mass * 0x1p-62;
+        out.mass  = mass_value(base + (long long) ws->best_mass);
         out.rank  = (long long) ws->best_rank;
         g.sync();
         return out;
@@ -164,18 +164,18 @@ __device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, cons
     double  *hm    = reinterpret_cast<double *>(&ws->x[0][0][0]);
     int     *hc    = reinterpret_cast<int *>(hm + kWarps * 256);
     static_assert(sizeof(ws->x) >= (size_t) kWarps * 256 * 12, "a byte histogram per warp fits");
-    const RadixOut ro = radix_mass(g, gs, hm, hc, kWarps, 0x1p62, sweep, target - base, inclusive, keyf, massf);
-    out.found         = ro.found;
-    out.word          = ro.found ? resolve_ties(g, gs, sweep, idx_bits, ro, target - base, inclusive, keyf, massf) : 0ull;
-    double    m = 0.0;
-    long long c = 0;
+    const double   rest = target - mass_value(base);
+    const RadixOut ro   = radix_mass(g, gs, hm, hc, kWarps, 0x1p62, sweep, rest, inclusive, keyf, massf);
+    out.found           = ro.found;
+    out.word            = ro.found ? resolve_ties(g, gs, sweep, idx_bits, ro, rest, inclusive, keyf, massf) : 0ull;
+    long long m = 0, c = 0;
     sweep([&](float pv, int i) {
         if (composite(__float_as_uint(pv), i, idx_bits) >= out.word) {
-            m += (double) pv;
+            m += wide_mass(pv);
             c++;
         }
     });
-    out.mass = base + group_sum_d(g, gs, m);
+    out.mass = mass_value(base + group_sum_ll(g, gs, m));
     out.rank = group_sum_ll(g, gs, c);
     return out;
 }
@@ -200,16 +200,15 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     const Pair     *list   = p.gen_list + (size_t) slot * (size_t) p.gen_list_cap;
     const int       half   = p.gen_list_cap / 2;
     const WideBins  bins(__ldcg(&ctl->S0), r.top_p, V);
-    double          a_cut = 0.0, a_pick = 0.0;
-    long long       above = 0;
+    long long       a_cut = 0, a_pick = 0, above = 0;
     for (int t = g.tid; t < pieces; t += g.n) {
         a_cut += __ldcg(&parts[t].above_cut);
         a_pick += __ldcg(&parts[t].above_pick);
         above += __ldcg(&parts[t].n_above);
     }
     const int n_cut = __ldcg(&ctl->n_cut), n_pick = __ldcg(&ctl->n_pick);
-    a_cut           = group_sum_d(g, gs, a_cut);
-    a_pick          = group_sum_d(g, gs, a_pick);
+    a_cut           = group_sum_ll(g, gs, a_cut);
+    a_pick          = group_sum_ll(g, gs, a_pick);
     above           = group_sum_ll(g, gs, above);
     /* p of the nearest entries outside a window: an entry of the window that shares it cannot be placed */
     auto p_at   = [&](unsigned k) { return wide_prob(__uint_as_float(k), inv_hi, inv_lo); };
@@ -218,7 +217,7 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
         return pv > 0.0f && (hi >= kWideBins - 1 || pv < p_at(bins.edge(hi + 1))) && pv > p_at(bins.edge(lo) - 1u);
     };
     const int w0 = ws->win[0], w1 = ws->win[1], w2 = ws->win[2], w3 = ws->win[3];
-    bool      ok = listed && n_cut <= half && n_pick <= half && n_cut > 0 && a_cut < (double) r.top_p;
+    bool      ok = listed && n_cut <= half && n_pick <= half && n_cut > 0 && mass_value(a_cut) < (double) r.top_p;
     WideHit   cut{}, pick{};
     if (ok) {
         cut = wide_walk(g, gs, ws, list, n_cut, a_cut, (double) r.top_p, true, idx_bits);
@@ -227,7 +226,7 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     if (ok) {
         unsigned long long rng = r.rng;
         const double       u   = (double) unit_from(xorshift_next(rng)) * cut.mass;
-        ok                     = a_pick <= u;
+        ok                     = mass_value(a_pick) <= u;
         if (ok) {
             pick = wide_walk(g, gs, ws, list + half, n_pick, a_pick, u, false, idx_bits);
             ok   = pick.found && inside(pick.word, w2, w3);
@@ -578,8 +577,8 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
             fetch(gr, true, (int) p.gen_stride, next, in ^ 1, 0.0f);
         }
         one_behind(next >= 0);
-        double a_cut = 0.0, a_pick = 0.0;
-        int    above = 0;
+        long long a_cut = 0, a_pick = 0;
+        int       above = 0;
 #pragma unroll 1
         for (int step = 0; step < kSteps; step++) {
             float    e[kPer];
@@ -589,9 +588,9 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
             for (int q = 0; q < kPer; q++) {
                 const unsigned k = __float_as_uint(e[q]);
                 if (__any_sync(0xffffffffu, k >= c_lo)) { /* most of a row lies below the nucleus; the draw's window lies no lower */
-                    const double pd = (double) wide_prob(e[q], inv_hi, inv_lo);
-                    a_cut += k >= c_hi ? pd : 0.0;
-                    a_pick += k >= k_hi ? pd : 0.0;
+                    const long long m = wide_mass(wide_prob(e[q], inv_hi, inv_lo));
+                    a_cut += k >= c_hi ? m : 0;
+                    a_pick += k >= k_hi ? m : 0;
                     above += k >= c_hi ? 1 : 0;
                     listed |= (k - c_lo < c_hi - c_lo || k - k_lo < k_hi - k_lo) ? 1u << q : 0u;
                 }
@@ -613,8 +612,8 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
                 }
             }
         }
-        a_cut  = warp_sum_d(a_cut);
-        a_pick = warp_sum_d(a_pick);
+        a_cut  = warp_sum_ll(a_cut);
+        a_pick = warp_sum_ll(a_pick);
         above  = __reduce_add_sync(0xffffffffu, above);
         if (g.lane == 0) {
             parts[piece].above_cut  = a_cut;

@@ -40,4 +40,9 @@ __device__ __forceinline__ float wide_prob(float e, float inv_hi, float inv_lo) 
     return __fadd_rn(q, __fmaf_rn(e, inv_lo, __fmaf_rn(e, inv_hi, -q)));
 }
 
+/* A probability in units of 2^-62, as the multi-pass path adds them up: a row's add up to less than 2^63, exactly down to
+ * p = 2^-38 and in any order. */
+__device__ __forceinline__ long long wide_mass(float p) { return __float2ll_rz(p * 0x1p62f); }
+__device__ __forceinline__ double mass_value(long long m) { return (double) m * 0x1p-62; }
+
 } /* namespace gb */

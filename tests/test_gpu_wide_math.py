@@ -26,3 +26,10 @@ def test_every_exponential(lib):
         differ, which = C.c_ulonglong(), C.c_uint()
         assert lib.exp_differs(C.c_uint(a), C.c_uint(b - a + 1), C.byref(differ), C.byref(which)) == 0
         assert differ.value == 0, (differ.value, -np.uint32(which.value).view(np.float32))
+
+
+def test_every_mass(lib):
+    """All floats from 0 to 1 as 64-bit masses in units of 2^-62."""
+    differ = C.c_ulonglong()
+    assert lib.mass_differs(C.c_uint(int(np.float32(1.0).view(np.uint32))), C.byref(differ)) == 0
+    assert differ.value == 0

@@ -33,3 +33,25 @@ extern "C" int exp_differs(unsigned first, unsigned n, unsigned long long *diffe
     *which  = h.which;
     return (int) e;
 }
+/* Probabilities by their bits, from 0 to 1: how many get another mass than the multi-pass path's histograms give them. */
+__global__ void mass_kernel(unsigned last, unsigned long long *differ) {
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k <= last; k += gridDim.x * blockDim.x) {
+        const float p = __uint_as_float(k);
+        if ((unsigned long long) gb::wide_mass(p) != __double2ull_rz((double) p * 0x1p62)) {
+            atomicAdd(differ, 1ull);
+        }
+    }
+}
+
+extern "C" int mass_differs(unsigned last, unsigned long long *differ) {
+    unsigned long long *d = nullptr;
+    cudaError_t         e = cudaMalloc(&d, sizeof *d);
+    if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof *d);
+    if (e == cudaSuccess) {
+        mass_kernel<<<148 * 8, 256>>>(last, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(differ, d, sizeof *d, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return (int) e;
+}

@@ -191,7 +191,7 @@ __device__ __forceinline__ int wide_got(int left, int pieces) {
 /* The last of a row's thread blocks: the two walks, the token, and the slot made ready for its next row. `listed`: the block
  * took part in pass 2, so that is through; one that had given up waiting for pass 1 does not know its windows, and nobody
  * need have made the lists. */
-__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, RowCfg &r, int slot, bool listed, float inv_hi, float inv_lo, unsigned long long rng0,
+__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, RowCfg &r, int slot, bool listed, double S, unsigned long long rng0,
                                          void *save_mem) {
     const Grp       g      = whole_block();
     WideCtl        *ctl    = p.wide_ctl + slot;
@@ -211,7 +211,8 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     a_pick          = group_sum_ll(g, gs, a_pick);
     above           = group_sum_ll(g, gs, above);
     /* p of the nearest entries outside a window: an entry of the window that shares it cannot be placed */
-    auto p_at   = [&](unsigned k) { return wide_prob(__uint_as_float(k), inv_hi, inv_lo); };
+    const WideQuotient quot(S);
+    auto p_at   = [&](unsigned k) { return quot(__uint_as_float(k)); };
     auto inside = [&](unsigned long long word, int lo, int hi) {
         const float pv = __uint_as_float((unsigned) (word >> idx_bits));
         return pv > 0.0f && (hi >= kWideBins - 1 || pv < p_at(bins.edge(hi + 1))) && pv > p_at(bins.edge(lo) - 1u);
@@ -459,7 +460,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
     g.sync();
     /* A row's last thread block finishes it, whoever that is: each was dealt a piece of pass 1 at least, and counts its own
      * once more when it is through here. The slot is then free for another row. */
-    auto leave = [&](bool listed, float inv_hi, float inv_lo) {
+    auto leave = [&](bool listed, double S) {
         __threadfence();
         g.sync();
         if (g.tid == 0) {
@@ -468,14 +469,14 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         }
         g.sync();
         if (ws->next != 0) {
-            wide_finish(p, gs, ws, r, slot, listed, inv_hi, inv_lo, rc.rng, save_mem);
+            wide_finish(p, gs, ws, r, slot, listed, S, rc.rng, save_mem);
         }
     };
     if (ws->next == 0) { /* gave up: its pieces of pass 1 are done all the same, so the row goes on without the block */
         if (g.tid == 0) {
             atomicAdd(&p.wide_head->gave_up, 1);
         }
-        leave(false, 0.0f, 0.0f);
+        leave(false, 1.0);
         return;
     }
     left = wide_ask(&ctl->rem2, g.lane);
@@ -493,8 +494,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         S += __ldcg(&parts[t].sum);
     }
     S = group_sum_d(g, gs, S);
-    const double inv    = 1.0 / S;
-    const float  inv_hi = __double2float_rn(inv), inv_lo = __double2float_rn(inv - (double) inv_hi);
+    const WideQuotient quot(S);
     {
 #pragma unroll
         for (int q = 0; q < kOwn; q++) {
@@ -583,16 +583,31 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         for (int step = 0; step < kSteps; step++) {
             float    e[kPer];
             unsigned listed = 0u; /* which of the lane's values lie in a window */
+            unsigned divide = 0u; /* ... and which want the division */
             take_values(in, step, e);
 #pragma unroll
             for (int q = 0; q < kPer; q++) {
                 const unsigned k = __float_as_uint(e[q]);
                 if (__any_sync(0xffffffffu, k >= c_lo)) { /* most of a row lies below the nucleus; the draw's window lies no lower */
-                    const long long m = wide_mass(wide_prob(e[q], inv_hi, inv_lo));
+                    bool            sure;
+                    const long long m = wide_mass(quot.quick(e[q], sure));
+                    divide |= sure ? 0u : 1u << q;
                     a_cut += k >= c_hi ? m : 0;
                     a_pick += k >= k_hi ? m : 0;
                     above += k >= c_hi ? 1 : 0;
                     listed |= (k - c_lo < c_hi - c_lo || k - k_lo < k_hi - k_lo) ? 1u << q : 0u;
+                }
+            }
+            if (divide != 0u) { /* masses are whole numbers: what went in comes out again */
+#pragma unroll
+                for (int q = 0; q < kPer; q++) {
+                    if ((divide >> q) & 1u) {
+                        const unsigned  k = __float_as_uint(e[q]);
+                        bool            sure;
+                        const long long m = wide_mass(quot(e[q])) - wide_mass(quot.quick(e[q], sure));
+                        a_cut += k >= c_hi ? m : 0;
+                        a_pick += k >= k_hi ? m : 0;
+                    }
                 }
             }
             if (listed != 0u) {
@@ -600,7 +615,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
                 for (int q = 0; q < kPer; q++) {
                     if ((listed >> q) & 1u) {
                         const unsigned k  = __float_as_uint(e[q]);
-                        const float    pv = wide_prob(e[q], inv_hi, inv_lo);
+                        const float    pv = quot(e[q]);
                         const int      id = s0 + column(step, q);
                         if (k - c_lo < c_hi - c_lo) {
                             note(&ctl->n_cut, list, pv, id);
@@ -623,7 +638,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         piece = next;
         __syncwarp();
     }
-    leave(true, inv_hi, inv_lo);
+    leave(true, S);
 }
 
 /* Opens the row in a slot that the thread block has claimed, for everybody; the block then works on it itself. */

@@ -33,12 +33,30 @@ __device__ __forceinline__ float wide_exp(float a, double t32) {
     return __double2float_rn(__fma_rn(T, q, T));
 }
 
-/* (float) (e / S): the quotient to 2^-47, then one rounding (inv_hi + inv_lo = 1 / S). None of 3e7 differed from the
- * rounded quotient of 64 bits. */
-__device__ __forceinline__ float wide_prob(float e, float inv_hi, float inv_lo) {
-    const float q = __fmul_rn(e, inv_hi);
-    return __fadd_rn(q, __fmaf_rn(e, inv_lo, __fmaf_rn(e, inv_hi, -q)));
-}
+/*
+ * (float) ((double) e / S), for quotients in the normal range. With 1 / S in two floats the remainder r = e / S - q of
+ * q = fl(e * hi) is known to 1.5 * 2^-47 of the quotient. That decides the rounding unless the quotient lies so close to a
+ * midpoint of two floats; r is then at least 2^-26 of it, and a 2^19-th of r covers the error: where q + r does not round
+ * the same with that much less and more, the division has to decide (one quotient in 10^6).
+ */
+struct WideQuotient {
+    double S;
+    float  hi, lo;
+    __device__ __forceinline__ explicit WideQuotient(double s) : S(s) {
+        const double inv = 1.0 / s;
+        hi               = __double2float_rn(inv);
+        lo               = __double2float_rn(inv - (double) hi);
+    }
+    /* in five FP32 operations; `sure`: it is the rounded quotient, else that or its neighbour */
+    __device__ __forceinline__ float quick(float e, bool &sure) const {
+        const float q    = __fmul_rn(e, hi);
+        const float r    = __fmaf_rn(e, lo, __fmaf_rn(e, hi, -q));
+        const float less = __fmaf_rn(r, 1.0f - 0x1p-19f, q);
+        sure             = less == __fmaf_rn(r, 1.0f + 0x1p-19f, q);
+        return less;
+    }
+    __device__ __forceinline__ float operator()(float e) const { return __double2float_rn((double) e / S); }
+};
 
 /* A probability in units of 2^-62, as the multi-pass path adds them up: a row's add up to less than 2^63, exactly down to
  * p = 2^-38 and in any order. */

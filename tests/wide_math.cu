@@ -15,6 +15,18 @@ __global__ void exp_kernel(unsigned first, unsigned n, unsigned long long *diffe
         }
     }
 }
+__global__ void quot_kernel(const float *e, const double *S, float *p, int *unsure, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        bool                   sure;
+        const gb::WideQuotient quot(S[i]);
+        p[i] = quot.quick(e[i], sure);
+        if (!sure) {
+            p[i] = quot(e[i]);
+            atomicAdd(unsure, 1);
+        }
+    }
+}
 
 extern "C" int exp_differs(unsigned first, unsigned n, unsigned long long *differ, unsigned *which) {
     struct Out {
@@ -54,4 +66,9 @@ extern "C" int mass_differs(unsigned last, unsigned long long *differ) {
     if (e == cudaSuccess) e = cudaMemcpy(differ, d, sizeof *d, cudaMemcpyDeviceToHost);
     cudaFree(d);
     return (int) e;
+}
+extern "C" int quotients(const float *e_dev, const double *S_dev, float *p_dev, int *unsure_dev, int n) {
+    quot_kernel<<<(n + 255) / 256, 256>>>(e_dev, S_dev, p_dev, unsure_dev, n);
+    const cudaError_t e = cudaGetLastError();
+    return (int) (e != cudaSuccess ? e : cudaDeviceSynchronize());
 }

@@ -1950,10 +1950,11 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         /* More entries than are ranked one against all: those that cannot be among the kq best, by the bins their values
          * fall into, stay out of the ranking (rows of many parts have kq of every part; a second list behind the first takes
          * the rest). With what is staged of every part: one row of 128256 in 16 parts, top-k 40, 39.7 -> 35.6 us;
-         * 8 x 151936 top-p in 19 parts 48.3 -> 43.8; 2 x 262144 top-p in 32 parts 37.2 -> 32.4. */
+         * 8 x 151936 top-p in 19 parts 48.3 -> 43.8; 2 x 262144 top-p in 32 parts 37.2 -> 32.4. Not where the kq best alone
+         * are more than are ranked: 64 x 32000 top-k 256, general kernel, 34.4 -> 32.1; 1000 x 8192 102.4 -> 97.3. */
         float few_scale = 0.0f;
         int   few_min   = -1; /* -1: all of them are ranked */
-        if (!need_multipass && total > kRankAll && row_max > tau_row && row_max - tau_row < CUDART_INF_F) {
+        if (!need_multipass && total > kRankAll && r.kq <= kRankAll && row_max > tau_row && row_max - tau_row < CUDART_INF_F) {
             few_scale = (float) kHistBins / (row_max - tau_row);
             sh->bhist[g.tid] = 0;
             static_assert(kHistBins == kThreads, "a bin per thread");

@@ -1905,10 +1905,13 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             for (int f0 = 0; f0 < others; f0 += g.n) {
                 const int  f  = f0 + g.tid;
                 const bool ok = f < others;
-                int        pi = 0;
-                for (int q = 1; q < n_parts; q++) {
-                    if (f >= sh->poff[q]) {
-                        pi = q; /* offsets ascend */
+                /* the last part that begins at f or before: offsets ascend. One after the other they were most of a row of many
+                 * parts: 2 x 262144 in 32 parts, top-k 256, 156 -> 107 us. */
+                int pi = 0;
+#pragma unroll
+                for (int step = kMaxParts / 2; step > 0; step >>= 1) {
+                    if (pi + step < n_parts && f >= sh->poff[pi + step]) {
+                        pi += step;
                     }
                 }
                 const int i = f - sh->poff[pi] + (pi < st_parts ? st_cand : 0);

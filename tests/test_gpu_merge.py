@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("K", [2, 219, 220, 221, 256])
-@pytest.mark.parametrize("rows,V", [(1, 128256), (9, 50257), (2, 262144)])
+@pytest.mark.parametrize("rows,V", [(1, 128256), (9, 50257), (2, 262144), (1, 524287)])
 @pytest.mark.parametrize("hint", [api.FINISH_AUTO, api.FINISH_GREEDY_TOPK])
 def test_k_around_what_is_ranked(ctx, rows, V, K, hint):
     x = normal_logits(rows, V, 2.0, V + K)

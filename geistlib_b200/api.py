@@ -143,7 +143,7 @@ PROTOTYPES = {
                                                     c_void_p]),
     "geist_b200_argmax_rows_static": (C.c_int, [C.c_int, c_void_p, c_size_t, c_size_t, c_size_t, c_void_p, c_void_p]),
     "geist_b200_grid": (C.c_int, [c_size_t, c_size_t, c_size_t, C.POINTER(c_int32), C.POINTER(c_int32)]),
-    "geist_b200_wide_counts": (C.c_int, [c_void_p] + [C.POINTER(c_int32)] * 4),
+    "geist_b200_wide_counts": (C.c_int, [c_void_p] + [C.POINTER(c_int32)] * 5),
     "geist_b200_set_wide_wait": (C.c_int, [c_void_p, C.c_uint64]),
     "geist_b200_plan": (C.c_int, [c_size_t, c_size_t, C.POINTER(c_int32), C.POINTER(c_int32), C.POINTER(c_int32),
                                   C.POINTER(c_int32)]),
@@ -256,8 +256,9 @@ class Context:
         _check(fn(self.handle, C.byref(out["_desc"]), c_void_p(stream)))
 
     def wide_counts(self):
-        """Of the last launch's wide top-p rows: (shared out, decided by their lists, longest list, waits that ran out)."""
-        n = [c_int32() for _ in range(4)]
+        """Of the last launch's wide top-p rows: (shared out, decided by their lists, longest list, waits that ran out, thread
+        blocks that waited for rows to help with)."""
+        n = [c_int32() for _ in range(5)]
         _check(lib.geist_b200_wide_counts(self.handle, *(C.byref(v) for v in n)))
         return tuple(v.value for v in n)
 

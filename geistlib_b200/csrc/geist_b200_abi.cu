@@ -241,6 +241,7 @@ struct geist_b200_ctx {
         int           *arrive      = nullptr; /* one counter per row: parts that have published (greedy launches); zero between launches */
         size_t         arrive_cap  = 0;
         size_t         counter_cap = 0;
+        unsigned       launches    = 0;
     } lane[kLanes];
     unsigned   next_lane = 0;
     unsigned long long wide_wait_ns = kWideWaitNs;
@@ -427,7 +428,7 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     const size_t slots    = std::min<size_t>((size_t) pl.fin_ctas, n_rows); /* row copies of the multi-pass path: one per finishing thread block that can run at a time */
     /* The general finishing kernel gets thread blocks that own no row as well: they help with wide top-p rows, two pieces
      * per warp. */
-    const bool   general  = (p.flags & (gb::F_FAST_ONLY | gb::F_SELECT_ONLY)) == 0u;
+    const bool   general  = (p.flags & (gb::F_FAST_ONLY | gb::F_SELECT_ONLY | gb::F_NO_TOP_P)) == 0u;
     const size_t pieces   = (b->n_vocab + gb::kWidePiece - 1) / gb::kWidePiece;
     const int    fin_grid = (int) std::min<size_t>((size_t) pl.fin_ctas, general ? n_rows * std::max<size_t>(1, pieces / (2 * gb::kWarps)) : n_rows);
     const size_t off_rows = round_up(off_seg + n_items * (size_t) gb::kWarps * sizeof(gb::SegRec), 256);
@@ -442,7 +443,8 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     geist_b200_ctx::Lane *ln;
     {
         std::lock_guard<std::mutex> lk(ctx->lane_mu);
-        ln = &ctx->lane[ctx->next_lane++ % kLanes];
+        ln       = &ctx->lane[ctx->next_lane++ % kLanes];
+        p.launch = ++ln->launches;
         if (ln->bytes < need) {
             cudaFree(ln->buf); /* waits for work that may still use it */
             ln->buf   = nullptr;
@@ -584,7 +586,7 @@ extern "C" enum geist_status geist_b200_scatter_kept(struct geist_b200_ctx *ctx,
     return GEIST_OK;
 }
 
-extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest, int32_t *gave_up) {
+extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest, int32_t *gave_up, int32_t *waited) {
     if (ctx == nullptr) {
         return fail(GEIST_E_INVALID_ARG, "wide_counts: NULL context");
     }
@@ -607,6 +609,9 @@ extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, 
     }
     if (gave_up) {
         *gave_up = h.gave_up;
+    }
+    if (waited) {
+        *waited = h.waited;
     }
     return GEIST_OK;
 }
@@ -1276,7 +1281,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
         }
     }
     /* which finishing kernels the launch needs: the sessions' sampler settings are known here */
-    bool any_fast = false, any_rest = false, all_greedy = true;
+    bool any_fast = false, any_rest = false, any_top_p = false, all_greedy = true;
     for (size_t i = 0; i < n; i++) {
         const size_t sl   = (size_t) sessions[i];
         const float  T    = b->h_T[sl];
@@ -1284,6 +1289,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
         const bool   fast = !(T > 0.0f) || (K > 1 && (size_t) K < b->V && K <= gb::kFastKMax);
         any_fast |= fast;
         any_rest |= !fast;
+        any_top_p |= !fast && b->h_P[sl] < 1.0f;
         all_greedy &= !(T > 0.0f);
     }
     int32_t hint = !any_rest ? GEIST_B200_FINISH_GREEDY_TOPK : (!any_fast ? GEIST_B200_FINISH_GENERAL : GEIST_B200_FINISH_AUTO);
@@ -1360,7 +1366,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
             d.fed_tokens = (pen && verify) ? b->d_fed : nullptr;
             d.tokens     = tok_dst;
             d.row_status = h_stat;
-            enum geist_status s = geist_b200_sample_batch(b->ctx, &d, st);
+            enum geist_status s = launch_batch(b->ctx, &d, st, any_top_p ? 0u : gb::F_NO_TOP_P);
             if (s != GEIST_OK) {
                 return s;
             }
@@ -1397,7 +1403,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
                 d.fed_tokens = (pen && verify) ? b->d_fed + s0 * k : nullptr;
                 d.tokens     = tok_dst + s0 * k;
                 d.row_status = h_stat + s0 * k;
-                enum geist_status s = geist_b200_sample_batch(b->ctx, &d, cs);
+                enum geist_status s = launch_batch(b->ctx, &d, cs, any_top_p ? 0u : gb::F_NO_TOP_P);
                 if (s != GEIST_OK) {
                     return s;
                 }

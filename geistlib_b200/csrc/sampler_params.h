@@ -47,6 +47,7 @@ enum : unsigned {
     F_SELECT_ONLY = 1u << 0, /* vocabulary shard: emit the row's best k (value, global id), no draw */
     F_FAST_ONLY   = 1u << 1, /* the caller vouches that every row is greedy or top-k <= kFastKMax: the small finishing kernel runs instead of the general one */
     F_INLINE_TOPK = 1u << 2, /* with F_FAST_ONLY, whole rows per thread block and no kept-set output: the stream kernel finishes top-k rows itself from its own candidate lists; no finishing kernel runs; what does not fit asks for ST_RETRY */
+    F_NO_TOP_P    = 1u << 4, /* the caller knows that no row is a top-p row: the general finishing kernel gets no thread blocks to help with wide ones */
     F_GREEDY_ONLY = 1u << 3, /* the caller vouches that every row is greedy: the stream kernel writes the tokens itself (the thread block that streamed the whole row, or the last of its parts to arrive) and no finishing kernel runs */
 };
 
@@ -93,12 +94,14 @@ struct WideCtl;
 struct WidePart;
 struct WideHead {
     unsigned long long rows; /* rows of the launch that are done or open for everybody; in the upper half those that were opened */
-    int                any;  /* there are top-p rows */
     /* for geist_b200_wide_counts */
     int                by_lists; /* rows that their two lists decided; the other opened ones went the multi-pass way */
     int                longest;  /* entries of the longest list that was walked */
     int                gave_up;  /* thread blocks that went on without the others' pieces */
-    int                pad[2];
+    unsigned           any;      /* the number of the lane's last launch that had top-p rows: never put back, so no order between
+                                  * the stream kernel's thread blocks matters */
+    int                waited;   /* thread blocks that waited for rows to help with; for geist_b200_wide_counts as well */
+    int                pad;
 };
 constexpr int kWidePiece     = 512;  /* columns that are dealt out at a time, to a warp */
 constexpr int kWidePiecesMax = 4096; /* rows of more pieces go the multi-pass way */
@@ -184,6 +187,7 @@ struct SampleParams {
     WideCtl   *wide_ctl;    /* [pool_slots] */
     unsigned  *wide_hist;   /* [pool_slots, kWideBins] */
     WidePart  *wide_part;   /* [pool_slots, pieces of a row] */
+    unsigned   launch;      /* the launch's number in its lane */
     unsigned long long wide_wait_ns; /* how long a thread block waits for the others' pieces of a wide row */
     int        gen_hist_cap;
 };

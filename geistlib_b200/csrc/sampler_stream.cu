@@ -1515,7 +1515,7 @@ __device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int to
  * room for the merged list. Returns the row's status bits (ST_DEFERRED: the multi-pass path has to serve it).
  */
 template <bool kFast>
-__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, unsigned char *cmem, int &any) {
+__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, unsigned char *cmem) {
     const int  row     = r.row;
     int       *kept_i  = p.kept_cap > 0 ? p.kept_idx + (size_t) row * (size_t) p.kept_cap : nullptr;
     float     *kept_v  = p.kept_cap > 0 ? p.kept_val + (size_t) row * (size_t) p.kept_cap : nullptr;
@@ -1613,9 +1613,6 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     }
     g.sync();
     PROF(9);
-    if constexpr (!kFast) {
-        any = ld_volatile(&p.wide_head->any); /* wanted when the row is done */
-    }
     for (int w = 0; w < g.nw; w++) {
         st |= gs->wred_a[w];
     }
@@ -2667,9 +2664,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if ((kKinds & K_SUMS) != 0 && tid == 0 && blockIdx.x == 0 && p.wide_head != nullptr) { /* the finishing kernel's count of rows begins at nothing */
-        static_assert(sizeof(WideHead) == 32, "two words of 16 bytes");
-        reinterpret_cast<int4 *>(p.wide_head)[0] = make_int4(0, 0, 0, 0);
-        reinterpret_cast<int4 *>(p.wide_head)[1] = make_int4(0, 0, 0, 0);
+        static_assert(offsetof(WideHead, gave_up) == 16, "the words in front of it are one of 16 bytes");
+        *reinterpret_cast<int4 *>(p.wide_head) = make_int4(0, 0, 0, 0);
+        p.wide_head->gave_up                   = 0;
+        p.wide_head->waited                    = 0;
     }
     asm volatile("griddepcontrol.launch_dependents;");
 #ifdef GB_PROFILE
@@ -3459,6 +3457,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                     bsum += sh->wb_sum[w];
                 }
                 bsum = bsum < 0.0 ? 0.0 : bsum; /* a NaN stays one: the walk ends on the row's last id, as the reference's does */
+                p.wide_head->any = p.launch; /* the finishing kernel's blocks without a row of their own wait for wide ones */
             }
             int4           h, h2;
             h.x  = __float_as_int((unsigned) (bw >> 32) == 0u ? -CUDART_INF_F : part_top(sh, cap_late));
@@ -3623,7 +3622,8 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     asm volatile("griddepcontrol.wait;" ::: "memory"); /* the records of the kernel before this one are complete and visible */
     asm volatile("griddepcontrol.launch_dependents;");
     PROF(kFast ? 5 : 7);
-    int any = 0; /* the launch has top-p rows */
+    /* the launch has top-p rows: the stream kernel has said so; wanted when the block's own rows are done */
+    const bool any = !kFast && *reinterpret_cast<volatile const unsigned *>(&p.wide_head->any) == p.launch;
     for (int row = (int) blockIdx.x; row < p.n_rows; row += (int) gridDim.x) {
         const RawCfg rc = row == (int) blockIdx.x ? rc0 : raw_config(p, row, true);
         RowCfg       r  = row_config(p, row, rc, true);
@@ -3634,15 +3634,11 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
         }
         PROF(8);
         if constexpr (!kFast) {
-            if (g.tid == 0) {
-                if (r.mode == M_TOPP) {
-                    *reinterpret_cast<volatile int *>(&p.wide_head->any) = 1;
-                } else {
-                    atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
-                }
+            if (g.tid == 0 && r.mode != M_TOPP) {
+                atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
             }
         }
-        int          st = finish_row<kFast>(g, p, sh, r, cmem, any);
+        int          st = finish_row<kFast>(g, p, sh, r, cmem);
         PROF(13);
         if (st & ST_DEFERRED) {
             if constexpr (kFast) {
@@ -3664,15 +3660,13 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
         __syncthreads();
     }
     if constexpr (!kFast) {
-        if ((int) blockIdx.x >= p.n_rows && g.tid == 0) { /* here to help alone: top-p rows say so when their blocks begin */
-            const unsigned long long t0 = global_ns();
-            do {
-                any = ld_volatile(&p.wide_head->any);
-            } while (any == 0 && global_ns() - t0 < 3000ull);
-        }
-        if (__syncthreads_or(any) != 0) {
+        /* Else there is nothing to help with, and the blocks that have no row end where they begin. (They watched three
+         * microseconds for a top-p row to be named: a matmul on another stream took 16.6 us next to launches of one temperature
+         * row without such blocks, 22.7 with them, and 19.7 since they end at once.) */
+        if (any) {
             int opened = 0;
             if (g.tid == 0) {
+                atomicAdd(&p.wide_head->waited, 1);
                 opened = wide_wait(p, 0u);
             }
             if (__syncthreads_or(opened) != 0) {

@@ -410,11 +410,11 @@ enum geist_status geist_b200_grid(size_t n_vocab, size_t max_history, size_t n_r
 
 /* What became of the wide top-p rows (nuclei beyond the finishing kernel's first 32 candidates) of the context's last
  * launch: how many were shared out to all thread blocks, how many of those the two lists of entries near the crossing and
- * the draw decided (the others took the multi-pass path), the longest such list, and how many thread blocks' waits for the
- * others' pieces ran out. Waits for the device; for tests and for looking into a workload. A launch whose hint leaves no
+ * the draw decided (the others took the multi-pass path), the longest such list, how many thread blocks' waits for the
+ * others' pieces ran out, and how many waited for wide rows to help with. Waits for the device; for tests and for looking into a workload. A launch whose hint leaves no
  * top-p rows does not touch the counts. */
 enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest,
-                                         int32_t *gave_up);
+                                         int32_t *gave_up, int32_t *waited);
 /* How long a thread block of the context's later launches waits for other thread blocks' pieces of a wide row before it goes
  * on without them (at most, and by default, a second). The row's result does not depend on it, only the time it takes: for
  * tests of what happens when the wait runs out. */

@@ -5,7 +5,7 @@ import pytest
 
 import oracle
 from geistlib_b200 import api
-from helpers import histories, independent_states, normal_logits, to_dev
+from helpers import histories, independent_states, normal_logits, per_seq, to_dev, u64_to_dev
 from test_gpu_parity import check_tokens, run_gpu
 
 pytestmark = pytest.mark.gpu
@@ -37,7 +37,7 @@ def test_pieces_and_changes(ctx, V, rows, kind):
         xo = np.where(allowed, x, np.float32(-np.inf)).astype(np.float32)
     g = run_gpu(ctx, x, 1.1, 0, P, st, kept_cap=4, **kw)
     same(g, oracle.port.sample_batch(xo, 1.1, 0, P, st, detail_cap=4, **okw))
-    opened, by_lists, longest, _ = ctx.wide_counts()
+    opened, by_lists, longest = ctx.wide_counts()[:3]
     if V > 1000:  # normal rows: wide, and all of them decided where they are shared out
         assert opened > rows // 2 and by_lists == opened and 0 < longest <= RANKED, (opened, by_lists, longest)
         assert ((g["status"] & api.ROW_SLOW_PATH) != 0).sum() == opened
@@ -52,7 +52,7 @@ def test_rows_of_few_values(ctx, V, step):
     st = independent_states(oracle.port, 7, rows)
     P = np.linspace(0.3, 0.97, rows).astype(np.float32)
     same(run_gpu(ctx, x, 0.9, 0, P, st, kept_cap=4), oracle.port.sample_batch(x, 0.9, 0, P, st, detail_cap=4))
-    opened, by_lists, longest, _ = ctx.wide_counts()
+    opened, by_lists, longest = ctx.wide_counts()[:3]
     if step == 100.0:  # one value: the candidates outrun their room already, the row is not shared out
         assert opened == 0
     else:
@@ -107,4 +107,44 @@ def test_a_wait_that_runs_out(rows, V):
                 assert counts[1] == rows and counts[3] == 0
             gave_up += counts[3]
     assert gave_up > 0 or V < 60000
+    ctx.close()
+
+
+def test_nobody_waits_in_launches_without_top_p_rows():
+    """Thread blocks without a row of their own wait for wide rows only where a launch has top-p rows; a captured launch whose
+    rows become top-p rows and temperature rows again between its replays finds out each time."""
+    import torch
+    ctx = api.Context(0)
+    rows, V = 5, 40000
+    x = normal_logits(rows, V, 1.0, 31)
+    st = independent_states(oracle.port, 32, rows)
+    narrow, wide = np.ones(rows, np.float32), np.array([1.0, 0.9, 0.95, 1.0, 0.8], np.float32)
+    dev = [to_dev(x), *per_seq(rows, 1.1, 0, narrow), u64_to_dev(st)]
+    d = ctx.sample_batch(*dev, launch=False)
+    s = torch.cuda.Stream()
+    for _ in range(4):
+        ctx.relaunch(d, s.cuda_stream)
+    s.synchronize()
+    assert ctx.wide_counts()[0] == 0 and ctx.wide_counts()[4] == 0
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        ctx.relaunch(d, s.cuda_stream)
+    for P in (narrow, wide, wide, narrow, wide):
+        dev[3].copy_(to_dev(P))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            g.replay()
+        s.synchronize()
+        o = oracle.port.sample_batch(x, 1.1, 0, P, st)
+        assert np.array_equal(d["tokens"].cpu().numpy(), o["tokens"])
+        counts = ctx.wide_counts()
+        assert counts[:2] == ((3, 3) if P is wide else (0, 0))
+        assert counts[4] > rows if P is wide else True
+    del g
+    for P, waits in ((narrow, False), (wide, True), (narrow, False)):  # launched anew, each is told apart
+        dev[3].copy_(to_dev(P))
+        for _ in range(4):
+            ctx.relaunch(d, s.cuda_stream)
+            s.synchronize()
+            assert (ctx.wide_counts()[4] > rows) == waits
     ctx.close()

@@ -265,8 +265,9 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     g.sync();
 }
 
-/* Works on the row of a slot. `first`: a piece that the thread block has been dealt already, its first warp's (all threads call). */
-__device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, WideShared *ws, int slot, int first, void *save_mem) {
+/* Works on the row of a slot. `first`: the first of the n_first pieces that the thread block has been dealt already, one for each
+ * of its first warps (all threads call). */
+__device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, WideShared *ws, int slot, int first, int n_first, void *save_mem) {
     const Grp       g       = whole_block();
     WideCtl        *ctl     = p.wide_ctl + slot;
     const int       V       = p.V, pieces = (V + kWidePiece - 1) / kWidePiece;
@@ -347,7 +348,7 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         __syncwarp();
     };
     int       mine  = 0;
-    int       piece = first >= 0 && g.warp == 0 ? first : -1;
+    int       piece = g.warp < n_first ? first + g.warp : -1;
     unsigned *cnt   = ws->cnt[g.warp];
     if (piece < 0) {
         piece = wide_got(left, pieces);
@@ -643,9 +644,9 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
 
 /* Opens the row in a slot that the thread block has claimed, for everybody; the block then works on it itself. */
 __device__ __forceinline__ void wide_open(const SampleParams &p, GroupShared *gs, WideShared *ws, int slot, int row, int st, float row_max, int row_arg, double S0, void *save_mem) {
-    WideCtl *ctl = p.wide_ctl + slot;
+    WideCtl  *ctl    = p.wide_ctl + slot;
+    const int pieces = (p.V + kWidePiece - 1) / kWidePiece, own = min(pieces, kWarps);
     if (threadIdx.x == 0) {
-        const int pieces = (p.V + kWidePiece - 1) / kWidePiece;
         ctl->done1       = 0;
         ctl->done2       = 0;
         ctl->n_cut       = 0;
@@ -657,14 +658,14 @@ __device__ __forceinline__ void wide_open(const SampleParams &p, GroupShared *gs
         ctl->S0          = S0;
         ctl->rem2        = pieces;
         __threadfence();
-        atomicExch(&ctl->rem1, pieces - 1); /* piece 0 is the block's own */
+        atomicExch(&ctl->rem1, pieces - own); /* the first are the block's own */
     }
     __syncthreads();
     if (threadIdx.x == 32) {
         __threadfence();
         atomicAdd(&p.wide_head->rows, (1ull << 32) + 1ull);
     }
-    wide_join(p, gs, ws, slot, 0, save_mem);
+    wide_join(p, gs, ws, slot, 0, own, save_mem);
     __syncthreads();
 }
 
@@ -712,7 +713,8 @@ __device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, W
         const int at   = ws->slot;
         const int slot = at == 0x7fffffff ? -1 : ((at & 0xffff) + start) % p.pool_slots;
         if (g.tid == 0) {
-            const int left = slot < 0 ? 0 : atomicSub(&p.wide_ctl[slot].rem1, 1);
+            /* a piece for every warp: with one for the block a row that is opened first was taken up by all of them */
+            const int left = slot < 0 ? 0 : atomicSub(&p.wide_ctl[slot].rem1, kWarps);
             ws->next       = left > 0 ? pieces - left : -1;
             __threadfence();
         }
@@ -720,7 +722,7 @@ __device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, W
         const int piece = ws->next;
         g.sync();
         if (piece >= 0) {
-            wide_join(p, gs, ws, slot, piece, save_mem);
+            wide_join(p, gs, ws, slot, piece, min(kWarps, pieces - piece), save_mem);
             g.sync();
         } else if (slot < 0) {
             looked = (unsigned) opened;

@@ -17,7 +17,7 @@ def same(g, o):
     assert np.array_equal(g["kept_n"], o["detail_n"])
 
 
-@pytest.mark.parametrize("V,rows", [(33, 5), (511, 7), (512, 7), (513, 9), (1025, 3), (1537, 700), (4099, 40), (100003, 24), (128256, 3)])
+@pytest.mark.parametrize("V,rows", [(33, 5), (511, 7), (512, 7), (513, 9), (1025, 3), (1537, 700), (4096, 24), (4099, 40), (8193, 300), (100003, 24), (128256, 3)])
 @pytest.mark.parametrize("kind", ["plain", "rep", "freq", "mask"])
 def test_pieces_and_changes(ctx, V, rows, kind):
     x = normal_logits(rows, V, 1.0, V + rows)

@@ -796,8 +796,11 @@ __device__ __forceinline__ bool again_aligned(const SampleParams &p) {
     return p.out_logits != nullptr ? (reinterpret_cast<unsigned long long>(p.out_logits) & 15ull) == 0ull && (p.V & 3) == 0 : p.aligned != 0;
 }
 
-/* All threads of the thread block serve a row whose kept set does not fit the one-pass path. */
-__device__ __noinline__ int multipass_row(const Grp &g, const SampleParams &p, GroupShared *sh, RowCfg &r, float row_max, int row_arg, void *hist_mem, int hist_bytes, int slot, void *save_mem) {
+/* All threads of the thread block serve a row whose kept set does not fit the one-pass path. The row's configuration comes
+ * in shared memory: handed on by reference it, and the group, would lie in the callers' frames. */
+__device__ __noinline__ int multipass_row(const SampleParams &p, GroupShared *sh, const RowCfg *cfg, float row_max, int row_arg, void *hist_mem, int hist_bytes, int slot, void *save_mem) {
+    const Grp g = whole_block();
+    RowCfg    r = *cfg;
     /* room for the byte histograms of the radix walks: per warp where it fits, else one for all */
     const int copies = hist_bytes >= g.nw * 256 * 12 ? g.nw : 1;
     double   *hm     = reinterpret_cast<double *>(hist_mem);
@@ -3552,8 +3555,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
  */
 /*
  * A row that the candidates could not serve, all threads of its thread block: a wide nucleus becomes everybody's, any
- * other row takes the multi-pass path over a private copy. Out of line, and it asks for the row's parameters again: with
- * them handed on by reference the kernel had a stack frame that every launch paid for.
+ * other row takes the multi-pass path over a private copy. Out of line, and it asks for the row's parameters again; what the
+ * functions behind it need of them lies in shared memory. Handed on by reference, the parameters and the group had lain in
+ * the kernel's stack frame, and the out-of-line functions had spilled around them: a frame of 464 bytes, 144 now (spills of
+ * the kernel's own code, mostly the select's); 1000 wide rows of 8192 212 -> 196 us, 24 of 100003 among 96 rows 80 -> 75.
+ * Narrow launches did not change: for those the frame alone costs nothing that was measured.
  */
 __device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *sh, unsigned char *cmem, int row, int st) {
     const Grp    g  = whole_block();
@@ -3591,7 +3597,12 @@ __device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *s
     if (slot < 0) {
         st |= ST_INTERNAL;
     } else {
-        st |= multipass_row(g, p, &sh->gs, r, bm, ba, cmem, kFinGeneralBytes, slot, sh->save);
+        WideShared *ws = reinterpret_cast<WideShared *>(cmem);
+        if (g.tid == 0) {
+            ws->cfg = r;
+        }
+        __syncthreads();
+        st |= multipass_row(p, &sh->gs, &ws->cfg, bm, ba, cmem, offsetof(WideShared, cfg), slot, sh->save);
         __syncthreads();
         if (g.tid == 0 && p.n_rows > p.pool_slots) {
             __threadfence();

@@ -66,6 +66,7 @@ struct __align__(16) WideShared {
     int                next, slot, mine;
     int                best_rank;
     unsigned long long best, best_mass;
+    RowCfg             cfg; /* the row's, for the functions that finish it */
 };
 
 __device__ __forceinline__ void copy_quad_async(void *dst_shared, const void *src_global) {
@@ -191,9 +192,9 @@ __device__ __forceinline__ int wide_got(int left, int pieces) {
 /* The last of a row's thread blocks: the two walks, the token, and the slot made ready for its next row. `listed`: the block
  * took part in pass 2, so that is through; one that had given up waiting for pass 1 does not know its windows, and nobody
  * need have made the lists. */
-__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, RowCfg &r, int slot, bool listed, double S, unsigned long long rng0,
-                                         void *save_mem) {
+__device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs, WideShared *ws, int slot, bool listed, double S, unsigned long long rng0, void *save_mem) {
     const Grp       g      = whole_block();
+    const RowCfg    r      = ws->cfg;
     WideCtl        *ctl    = p.wide_ctl + slot;
     const int       V      = p.V, pieces = (V + kWidePiece - 1) / kWidePiece, idx_bits = 32 - __clz(max(V - 1, 1));
     const WidePart *parts  = p.wide_part + (size_t) slot * (size_t) pieces;
@@ -247,7 +248,7 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
         }
         st |= ST_SLOW_PATH | (p.kept_cap > 0 ? (int) ST_KEPT_PARTIAL : 0);
     } else {
-        st |= multipass_row(g, p, gs, r, __ldcg(&ctl->row_max), __ldcg(&ctl->row_arg), ws, (int) sizeof(WideShared), slot, save_mem);
+        st |= multipass_row(p, gs, &ws->cfg, __ldcg(&ctl->row_max), __ldcg(&ctl->row_arg), ws, (int) offsetof(WideShared, cfg), slot, save_mem);
     }
     if (g.tid == 0) {
         row_epilogue(p, r, r.row, st, rng0);
@@ -466,11 +467,12 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         g.sync();
         if (g.tid == 0) {
             ws->next = atomicAdd(&ctl->done2, ws->mine) + ws->mine == pieces ? 1 : 0;
+            ws->cfg  = r;
             __threadfence();
         }
         g.sync();
         if (ws->next != 0) {
-            wide_finish(p, gs, ws, r, slot, listed, S, rc.rng, save_mem);
+            wide_finish(p, gs, ws, slot, listed, S, rc.rng, save_mem);
         }
     };
     if (ws->next == 0) { /* gave up: its pieces of pass 1 are done all the same, so the row goes on without the block */

@@ -560,11 +560,19 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
     const unsigned k_lo = bins.edge(ws->win[2]), k_hi = ws->win[3] >= kWideBins - 1 ? 0xffffffffu : bins.edge(ws->win[3] + 1);
     const int      half = p.gen_list_cap / 2;
     Pair          *list = p.gen_list + (size_t) slot * (size_t) p.gen_list_cap;
-    auto           note = [&](int *count, Pair *to, float pv, int id) {
-        const int pos = atomicAdd(count, 1);
-        if (pos < half) {
-            to[pos].v   = pv;
-            to[pos].idx = id;
+    /* A lane that finds a list full counts nothing more in it: its count is beyond its room already, which is all that is
+     * asked of it then. (Counted on, 10^5 equal values of a row queued for one word: 256 rows of 128256 that end in equal
+     * values took 12.6 ms, 8.1 on the multi-pass path alone.) */
+    bool           full_cut = false, full_pick = false;
+    auto           note = [&](bool &full, int *count, Pair *to, float pv, int id) {
+        if (!full) {
+            const int pos = atomicAdd(count, 1);
+            if (pos < half) {
+                to[pos].v   = pv;
+                to[pos].idx = id;
+            } else {
+                full = true;
+            }
         }
     };
     piece = wide_got(left, pieces);
@@ -621,10 +629,10 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
                         const float    pv = quot(e[q]);
                         const int      id = s0 + column(step, q);
                         if (k - c_lo < c_hi - c_lo) {
-                            note(&ctl->n_cut, list, pv, id);
+                            note(full_cut, &ctl->n_cut, list, pv, id);
                         }
                         if (k - k_lo < k_hi - k_lo) {
-                            note(&ctl->n_pick, list + half, pv, id);
+                            note(full_pick, &ctl->n_pick, list + half, pv, id);
                         }
                     }
                 }

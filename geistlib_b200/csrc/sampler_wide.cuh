@@ -292,6 +292,9 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         r.mrow   = nullptr;
         r.pen_on = false;
     }
+    if (g.tid == 0) {
+        ws->cfg = r; /* here, not where the row is finished: nothing of it need be kept in registers until then */
+    }
     const WideBins bins(S0, r.top_p, V);
     const float   *src    = row_again(p, row);
     const bool     src_al = again_aligned(p);
@@ -467,7 +470,6 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         g.sync();
         if (g.tid == 0) {
             ws->next = atomicAdd(&ctl->done2, ws->mine) + ws->mine == pieces ? 1 : 0;
-            ws->cfg  = r;
             __threadfence();
         }
         g.sync();
@@ -594,31 +596,30 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         for (int step = 0; step < kSteps; step++) {
             float    e[kPer];
             unsigned listed = 0u; /* which of the lane's values lie in a window */
-            unsigned divide = 0u; /* ... and which want the division */
+            bool     unsure = false; /* one of them wants the division */
             take_values(in, step, e);
 #pragma unroll
             for (int q = 0; q < kPer; q++) {
                 const unsigned k = __float_as_uint(e[q]);
                 if (__any_sync(0xffffffffu, k >= c_lo)) { /* most of a row lies below the nucleus; the draw's window lies no lower */
-                    bool            sure;
-                    const long long m = wide_mass(quot.quick(e[q], sure));
-                    divide |= sure ? 0u : 1u << q;
-                    a_cut += k >= c_hi ? m : 0;
-                    a_pick += k >= k_hi ? m : 0;
-                    above += k >= c_hi ? 1 : 0;
+                    const long long m = __float2ll_rz(quot.quick(e[q], unsure));
+                    if (k >= c_hi) {
+                        a_cut += m;
+                        above++;
+                    }
+                    if (k >= k_hi) {
+                        a_pick += m;
+                    }
                     listed |= (k - c_lo < c_hi - c_lo || k - k_lo < k_hi - k_lo) ? 1u << q : 0u;
                 }
             }
-            if (divide != 0u) { /* masses are whole numbers: what went in comes out again */
+            if (unsure) { /* masses are whole numbers: what went in comes out again */
 #pragma unroll
                 for (int q = 0; q < kPer; q++) {
-                    if ((divide >> q) & 1u) {
-                        const unsigned  k = __float_as_uint(e[q]);
-                        bool            sure;
-                        const long long m = wide_mass(quot(e[q])) - wide_mass(quot.quick(e[q], sure));
-                        a_cut += k >= c_hi ? m : 0;
-                        a_pick += k >= k_hi ? m : 0;
-                    }
+                    const unsigned  k = __float_as_uint(e[q]);
+                    const long long m = wide_mass(quot.divide(e[q])) - __float2ll_rz(quot.quick(e[q], unsure));
+                    a_cut += k >= c_hi ? m : 0;
+                    a_pick += k >= k_hi ? m : 0;
                 }
             }
             if (listed != 0u) {

@@ -41,21 +41,26 @@ __device__ __forceinline__ float wide_exp(float a, double t32) {
  */
 struct WideQuotient {
     double S;
-    float  hi, lo;
+    float  hi, lo; /* 2^62 / S: whole units of a mass, so that nothing has to be scaled behind them */
     __device__ __forceinline__ explicit WideQuotient(double s) : S(s) {
-        const double inv = 1.0 / s;
+        const double inv = 0x1p62 / s;
         hi               = __double2float_rn(inv);
         lo               = __double2float_rn(inv - (double) hi);
     }
-    /* in five FP32 operations; `sure`: it is the rounded quotient, else that or its neighbour */
-    __device__ __forceinline__ float quick(float e, bool &sure) const {
+    /* 2^62 p in five FP32 operations; sets `unsure` where it may be the rounded quotient's neighbour */
+    __device__ __forceinline__ float quick(float e, bool &unsure) const {
         const float q    = __fmul_rn(e, hi);
         const float r    = __fmaf_rn(e, lo, __fmaf_rn(e, hi, -q));
         const float less = __fmaf_rn(r, 1.0f - 0x1p-19f, q);
-        sure             = less == __fmaf_rn(r, 1.0f + 0x1p-19f, q);
+        unsure |= less != __fmaf_rn(r, 1.0f + 0x1p-19f, q);
         return less;
     }
-    __device__ __forceinline__ float operator()(float e) const { return __double2float_rn((double) e / S); }
+    __device__ __forceinline__ float divide(float e) const { return __double2float_rn((double) e / S); }
+    __device__ __forceinline__ float operator()(float e) const {
+        bool        unsure = false;
+        const float p      = quick(e, unsure) * 0x1p-62f;
+        return unsure ? divide(e) : p;
+    }
 };
 
 /* A probability in units of 2^-62, as the multi-pass path adds them up: a row's add up to less than 2^63, exactly down to

@@ -18,11 +18,11 @@ __global__ void exp_kernel(unsigned first, unsigned n, unsigned long long *diffe
 __global__ void quot_kernel(const float *e, const double *S, float *p, int *unsure, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        bool                   sure;
+        bool                   divide = false;
         const gb::WideQuotient quot(S[i]);
-        p[i] = quot.quick(e[i], sure);
-        if (!sure) {
-            p[i] = quot(e[i]);
+        (void) quot.quick(e[i], divide);
+        p[i] = quot(e[i]);
+        if (divide) {
             atomicAdd(unsure, 1);
         }
     }

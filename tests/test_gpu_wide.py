@@ -148,3 +148,61 @@ def test_nobody_waits_in_launches_without_top_p_rows():
             s.synchronize()
             assert (ctx.wide_counts()[4] > rows) == waits
     ctx.close()
+
+
+@pytest.mark.parametrize("V,seqs,k", [(5000, 3, 4), (40001, 8, 6), (9000, 80, 5)])
+def test_wide_verify_rows(ctx, V, seqs, k):
+    """Rows of one sequence share a generator word, and each counts the tokens fed before it; also more rows than row copies."""
+    rows = seqs * k
+    x = normal_logits(rows, V, 1.0, 41)
+    st = independent_states(oracle.port, 42, seqs)
+    h, fed = histories(seqs, 50, V, 43), histories(seqs, k, V, 44)
+    P = np.linspace(0.6, 0.97, seqs).astype(np.float32)
+    g = run_gpu(ctx, x, 1.1, 0, P, st, rows_per_seq=k, history=h, fed=fed, rep=1.3, freq=0.05, kept_cap=4)
+    same(g, oracle.port.sample_batch(x, 1.1, 0, P, st, rows_per_seq=k, hist=h, extra=fed, rep=1.3, freq=0.05, detail_cap=4))
+    assert ctx.wide_counts()[:2] == (rows, rows)
+
+
+@pytest.mark.parametrize("cap", [0.0, 3.0])
+def test_wide_rows_with_all_changes(ctx, cap):
+    """Cap, then mask, then the penalties of a long history, on rows on and off the 16-byte grid."""
+    for V, rows in ((20000, 9), (20003, 9)):
+        x = normal_logits(rows, V, 1.0, 51)
+        st = independent_states(oracle.port, 52, rows)
+        h = histories(rows, 700, V, 53)
+        allowed = np.random.default_rng(54).random((rows, V)) < 0.8
+        words = np.zeros((rows, (V + 31) // 32 * 32), bool)
+        words[:, :V] = allowed
+        kw = {"logit_mask": to_dev(np.packbits(words, axis=1, bitorder="little").view(np.int32))}
+        xo = np.where(allowed, x, np.float32(-np.inf)).astype(np.float32)
+        if cap > 0.0:
+            # the capped row as the device writes it out for a temperature draw: tanhf is not the subject here
+            kw["softcap"] = to_dev(np.full(rows, cap, np.float32))
+            xo = run_gpu(ctx, x, 1.1, 0, 1.0, st, want_logits=True, **kw)["logits"]
+        g = run_gpu(ctx, x, 1.1, 0, 0.95, st, history=h, rep=1.2, freq=0.1, pres=0.1, kept_cap=4, **kw)
+        same(g, oracle.port.sample_batch(xo, 1.1, 0, 0.95, st, hist=h, rep=1.2, freq=0.1, pres=0.1, detail_cap=4))
+        assert ctx.wide_counts()[:2] == (rows, rows)
+
+
+def test_wide_rows_on_two_streams_at_once():
+    """Launches with wide rows, each with scratch of its own, that overlap on the GPU."""
+    import torch
+    ctx = api.Context(0)
+    jobs = []
+    for i, (rows, V) in enumerate([(12, 60000), (40, 30001)]):
+        x, st = normal_logits(rows, V, 1.0, 61 + i), independent_states(oracle.port, 63 + i, rows)
+        dev = to_dev(x), *per_seq(rows, 1.1, 0, 0.93), u64_to_dev(st)
+        outs = [ctx.sample_batch(*dev, launch=False) for _ in range(2)]
+        jobs.append((torch.cuda.Stream(), outs, dev, oracle.port.sample_batch(x, 1.1, 0, 0.93, st)["tokens"]))
+    torch.cuda.synchronize()
+    for _ in range(10):
+        for n in range(2):  # four launches at most in flight: one set of scratch each
+            for stream, outs, _, _ in jobs:
+                ctx.relaunch(outs[n], stream.cuda_stream)
+        torch.cuda.synchronize()
+        for _, outs, _, want in jobs:
+            for out in outs:
+                assert np.array_equal(out["tokens"].cpu().numpy(), want)
+                out["tokens"].fill_(-7)
+        torch.cuda.synchronize()
+    ctx.close()

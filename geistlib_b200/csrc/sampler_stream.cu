@@ -21,7 +21,7 @@
  *
  *   Part boundaries. The thread block meets and writes the part's record (maximum, first id, threshold, sums;
  *   two 16-byte slots) followed by its candidates to the part's place in global scratch. Nothing else is
- *   shared between thread blocks: no counters, no thread block waits for another one.
+ *   shared between the stream kernel's thread blocks: no counters, no thread block waits for another one.
  *
  *   Finishing is left to a kernel of its own behind the stream kernel, launched as a programmatic dependent so
  *   that its thread blocks are placed while the stream kernel drains: one thread block per row merges the parts'
@@ -3948,8 +3948,10 @@ cudaError_t launch_sample_stream(const SampleParams &p, int grid, size_t smem_by
     }
     /* Programmatic dependent launch, both kernels: the thread blocks are placed while the kernel before them
      * in the stream drains, and wait (griddepcontrol.wait) until that kernel is complete and visible before they
-     * touch global memory. No thread block ever waits for another one of its grid, so neither grid needs
-     * co-residency. */
+     * touch global memory. No thread block of the stream kernel or of the small finishing kernel ever waits for another one of
+     * its grid. Those of the general finishing kernel do, where a launch has wide top-p rows: for pieces of such a row that
+     * have been dealt out, and every one of those lies with a thread block that is running (a block takes pieces for the
+     * warps it has); and, before they end, a bounded while for rows to help with. So neither grid needs co-residency. */
     cudaLaunchConfig_t  cfg{};
     cudaLaunchAttribute attr[1];
     cfg.gridDim          = dim3((unsigned) grid);

@@ -13,16 +13,20 @@
  *           what lies above a window is summed in units of 2^-62, what lies in it is listed (a few entries, or a few hundred).
  *   end     the thread block that completes pass 2 walks the two lists exactly, in (p desc, id asc) order, and has the
  *           token. Whatever the lists do not decide (more entries than they hold, a crossing outside its window, equal
- *           probabilities at a window's edge) goes to multipass_row.
+ *           probabilities at a window's edge) goes to multipass_row, one thread block for the row. Rows with thousands of
+ *           equal values are where that happens: the lists outrun their room, and equal masses round to units alike, so
+ *           that the window misses its target by more than the margin allows for. The two passes are lost then: 256 rows
+ *           of 128256 that end in 10^5 equal values 8.1 -> 8.6 ms. Logits that were 16 bits wide do not come near it.
  *
  * Nobody waits for a thread block that has not begun: the block that owns the row takes pieces like any other, and once
- * they are all dealt out, every piece lies with a block that runs. Sums and lists do not depend on who took which piece.
+ * they are all dealt out, every piece lies with a block that runs. A wait that runs out all the same leaves the row to the
+ * blocks that are still at it. Sums do not depend on who took which piece, nor does the order of the lists matter.
  *
  * Pass 1 is bound by the issue of its instructions at the finishing kernel's 16 warps per SM: 25 SM cycles per 32 values,
  * where its double arithmetic takes 6 and its conversions 8; a launch's first piece waits for the code as well, 4 us. 256
- * rows of 128256 columns, top-p 0.95 (105 of them wide): 428 us with a thread block and a dozen sweeps per row, 167 now;
- * 24 wide rows of 100003 among 96: 402 -> 93. Pieces of 512 for a warp: with 1024 the 24 rows take 99 us, and pieces of
- * 2048 for a thread block, a barrier each, took 204 us on the 105.
+ * rows of 128256 columns, top-p 0.95 (105 of them wide): 428 us with a thread block and a dozen sweeps per row, 168 now;
+ * 24 wide rows of 100003 among 96: 402 -> 74. Pieces of 512 for a warp: when they came in (the 24 rows took 93 us) pieces of
+ * 1024 took 99, and pieces of 2048 for a thread block, a barrier each, 204 us on the 105.
  */
 #pragma once
 

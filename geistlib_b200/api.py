@@ -256,8 +256,8 @@ class Context:
         _check(fn(self.handle, C.byref(out["_desc"]), c_void_p(stream)))
 
     def wide_counts(self):
-        """Of the last launch's wide top-p rows: (shared out, decided by their lists, longest list, waits that ran out, thread
-        blocks that waited for rows to help with)."""
+        """Of the last launch's wide top-p rows: (shared out, decided by their lists, longest list, waits that ran out, whether
+        thread blocks without a row of their own waited for rows to help with)."""
         n = [c_int32() for _ in range(5)]
         _check(lib.geist_b200_wide_counts(self.handle, *(C.byref(v) for v in n)))
         return tuple(v.value for v in n)

@@ -100,7 +100,7 @@ struct WideHead {
     int                gave_up;  /* thread blocks that went on without the others' pieces */
     unsigned           any;      /* the number of the lane's last launch that had top-p rows: never put back, so no order between
                                   * the stream kernel's thread blocks matters */
-    int                waited;   /* thread blocks that waited for rows to help with; for geist_b200_wide_counts as well */
+    int                waited;   /* 1: thread blocks without a row of their own waited for rows to help with; for geist_b200_wide_counts as well */
     int                pad;
 };
 constexpr int kWidePiece     = 512;  /* columns that are dealt out at a time, to a warp */

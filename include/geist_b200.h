@@ -411,7 +411,8 @@ enum geist_status geist_b200_grid(size_t n_vocab, size_t max_history, size_t n_r
 /* What became of the wide top-p rows (nuclei beyond the finishing kernel's first 32 candidates) of the context's last
  * launch: how many were shared out to all thread blocks, how many of those the two lists of entries near the crossing and
  * the draw decided (the others took the multi-pass path), the longest such list, how many thread blocks' waits for the
- * others' pieces ran out, and how many waited for wide rows to help with. Waits for the device; for tests and for looking into a workload. A launch whose hint leaves no
+ * others' pieces ran out, and (1 or 0) whether thread blocks without a row of their own waited for wide
+ * ones to help with. Waits for the device; for tests and for looking into a workload. A launch whose hint leaves no
  * top-p rows does not touch the counts. */
 enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, int32_t *opened, int32_t *by_lists, int32_t *longest,
                                          int32_t *gave_up, int32_t *waited);

@@ -3557,8 +3557,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
  * A row that the candidates could not serve, all threads of its thread block: a wide nucleus becomes everybody's, any
  * other row takes the multi-pass path over a private copy. Out of line, and it asks for the row's parameters again; what the
  * functions behind it need of them lies in shared memory. Handed on by reference, the parameters and the group had lain in
- * the kernel's stack frame, and the out-of-line functions had spilled around them: a frame of 464 bytes, 144 now (spills of
- * the kernel's own code, mostly the select's); 1000 wide rows of 8192 212 -> 196 us, 24 of 100003 among 96 rows 80 -> 75.
+ * the kernel's stack frame, and the out-of-line functions had spilled around them: a frame of 464 bytes, 112 now (spills of
+ * the kernel's own code, mostly the select's); 1000 wide rows of 8192 212 -> 194 us, 24 of 100003 among 96 rows 80 -> 75.
  * Narrow launches did not change: for those the frame alone costs nothing that was measured.
  */
 __device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *sh, unsigned char *cmem, int row, int st) {

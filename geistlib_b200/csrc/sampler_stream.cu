@@ -1269,6 +1269,8 @@ constexpr int kIdBits = 4 * kSliceMax;
 /* Where the bit of a value lies: slice of the part, warp, offset in the share. */
 __device__ __forceinline__ int id_bit(int s, int w, int off) { return ((s & 3) * kWarps + w) * (kSliceMax / kWarps) + off; }
 
+constexpr int kKeyBins = 512; /* among which the threshold is sought */
+
 /* A part whose candidates outran their list, for raise_threshold. */
 struct PartAgain {
     int             row, c0, part_len, gm_shift, kq;
@@ -1305,8 +1307,11 @@ struct __align__(16) StreamShared {
     PartAgain          again;                 /* what raise_threshold needs to know of the part */
     /* finishing inside the stream kernel (F_INLINE_TOPK): the k best in order, their weights */
     int                cur_rr;
-    Pair               fin_s[kFastKMax];
-    float              fin_q[kFastKMax];
+    union {
+        alignas(16) Pair fin_s[kFastKMax];
+        int              key_bins[kKeyBins]; /* before that, while the threshold is sought */
+    };
+    alignas(8) float   fin_q[kFastKMax];
     unsigned long long cur_rng;         /* the generator word the part's sequence came with, its sequence, and whether the row is the sequence's last */
     int                cur_seq, cur_last;
     float              cap;             /* the part's soft cap and mask row (0 / null: none) */
@@ -2235,6 +2240,190 @@ __device__ __forceinline__ int row_id_count(const SampleParams &p, int hist_len,
     return H + E;
 }
 
+/*
+ * A lower bound of the kq-th largest of the threads' keys (one each, two with `two`) that kq of them reach and few more: the keys
+ * are counted in kKeyBins bins between the smallest and the largest, and where the bin that the kq-th falls into holds too many,
+ * once more between that bin's ends. `bins` is zero when this is called. Bound by latency: two barriers, an atomic and a scan
+ * (0.84 us of one row of 4096) where building the key bit by bit took a barrier for each of about ten bits (1.25 - 1.5 us).
+ * Ordered lists per warp, and halving in all of them, took as long as this alone on an SM and 0.3 us longer with another thread
+ * block beside it: every instruction of it is issued by all eight warps. All threads call.
+ */
+__device__ __forceinline__ unsigned kth_key(unsigned key0, unsigned key1, bool two, int kq, int *bins, uint2 *ends, int lane, int warp) {
+    unsigned lo = __reduce_min_sync(0xffffffffu, two ? min(key0, key1) : key0), hi = __reduce_max_sync(0xffffffffu, two ? max(key0, key1) : key0);
+    if (lane == 0) {
+        ends[warp] = make_uint2(lo, hi);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        const uint2 e = ends[w];
+        lo            = min(lo, e.x);
+        hi            = max(hi, e.y);
+    }
+    int need = kq; /* of the keys from lo to hi */
+    for (;;) {
+        const int shift = max(0, 32 - __clz(hi - lo) - 9); /* (hi - lo) >> shift < kKeyBins */
+        static_assert(kKeyBins == 1 << 9 && kKeyBins == 16 * 32, "sixteen bins per lane");
+        if (key0 - lo <= hi - lo) {
+            atomicAdd(&bins[(key0 - lo) >> shift], 1);
+        }
+        if (two && key1 - lo <= hi - lo) {
+            atomicAdd(&bins[(key1 - lo) >> shift], 1);
+        }
+        __syncthreads();
+        int4 c[4]; /* the lane's bins */
+        int  sum = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            c[i] = reinterpret_cast<const int4 *>(bins)[4 * lane + i];
+            sum += (c[i].x + c[i].y) + (c[i].z + c[i].w);
+        }
+        int up = sum; /* keys in the lane's bins and above */
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int more = __shfl_down_sync(0xffffffffu, up, o);
+            up += lane + o < 32 ? more : 0;
+        }
+        const int from = 31 - __clz(__ballot_sync(0xffffffffu, up >= need)); /* the last lane from which up enough are */
+        /* in it: the last of its bins from which up enough are, and how many are from there up */
+        int b = 0, n = up, above = up - sum;
+#pragma unroll
+        for (int i = 3; i >= 0; i--) {
+            const int q[4] = {c[i].x, c[i].y, c[i].z, c[i].w};
+#pragma unroll
+            for (int j = 3; j >= 0; j--) {
+                const bool before = above < need;
+                above += q[j];
+                if (before && above >= need) {
+                    b = 4 * i + j;
+                    n = above;
+                }
+            }
+        }
+        b = __shfl_sync(0xffffffffu, 16 * lane + b, from);
+        n = __shfl_sync(0xffffffffu, n, from);
+        const unsigned key = lo + ((unsigned) b << shift);
+        if (n - need <= 4 + kq / 4 || shift == 0) {
+            return key;
+        }
+        const int in = bins[b];
+        __syncthreads(); /* every warp has read the bins */
+        for (int i = (int) threadIdx.x; i < kKeyBins; i += kThreads) {
+            bins[i] = 0;
+        }
+        __syncthreads();
+        need -= n - in;
+        lo = key;
+        hi = min(hi, key + ((1u << shift) - 1u));
+    }
+}
+
+/* At most kRankFew candidates in order, the k best to out_s, their weights e^((x - max) / T) to out_q. Four threads (two beyond
+ * 64 candidates) compare a candidate with a share of the others each, eight at a time without a branch between them.
+ * All threads call; the caller's barrier follows. */
+constexpr int kRankFew = 128;
+static_assert(2 * kRankFew == kThreads, "two threads per candidate");
+__device__ __forceinline__ void rank_few(const Pair *cand, int total, int k, float inv_t, Pair *out_s, float *out_q) {
+    const int  log = total <= kRankFew / 2 ? 2 : 1, i = (int) threadIdx.x >> log, step = 1 << log, sub = (int) threadIdx.x & (step - 1);
+    const Pair me   = cand[min(i, total - 1)];
+    int        rank = 0;
+    float      top  = -CUDART_INF_F;
+#pragma unroll 1
+    for (int j0 = sub; j0 < total; j0 += 8 * step) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const Pair o = cand[min(j0 + j * step, total - 1)];
+            rank += j0 + j * step < total && pair_before(o.v, o.idx, me.v, me.idx) ? 1 : 0;
+            top = fmaxf(top, o.v);
+        }
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    if (log == 2) {
+        rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    }
+    if (sub == 0 && i < total && rank < k) {
+        out_s[rank] = me;
+        out_q[rank] = exp_exact(scaled_arg(me.v, top, inv_t));
+    }
+}
+
+/*
+ * The reference's draw over k <= 256 weights in descending order (sampler.c:90-102): the sum and the walk in its order, in
+ * double. Where the smallest weight is at least 2^-22 every partial sum is a whole number of 2^-45 below 2^53 of them, so
+ * exact in any order, and the warp adds in parallel; else one lane adds one by one. The whole warp calls: the place that
+ * u01 times the sum falls on, and the sum. (Between the candidates and the token of one row, top-k 40: 1.9 us with a thread per
+ * candidate to rank them, the exponentials behind a barrier and one thread over the weights, twice; 1.25 us.)
+ */
+__device__ __forceinline__ int draw_sorted(int lane, const float *q, int k, float u01, double *S_out) {
+    const float2 two = 2 * lane < k ? *reinterpret_cast<const float2 *>(q + 2 * lane) : make_float2(0.0f, 0.0f); /* what lies behind the k-th weight is not used */
+    if (q[k - 1] >= 0x1p-22f) {
+        const int per  = k <= 64 ? 2 : (k + 31) >> 5, i0 = lane * per;
+        double    incl = (double) two.x + (2 * lane + 1 < k ? (double) two.y : 0.0);
+        if (k > 64) {
+            incl = 0.0;
+#pragma unroll 1
+            for (int i = i0; i < min(i0 + per, k); i++) {
+                incl += (double) q[i];
+            }
+        }
+        const double mine = incl;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) {
+                incl += up;
+            }
+        }
+        const double S = __shfl_sync(0xffffffffu, incl, 31), u = (double) u01 * S;
+        const int    from = __ffs(__ballot_sync(0xffffffffu, u < incl)) - 1; /* the lane whose run crosses u, -1: none */
+        double       a    = incl - mine;
+        int          pick = i0;
+        if (k <= 64) {
+            pick += u < a + (double) two.x ? 0 : 1;
+        } else {
+#pragma unroll 1
+            for (; pick < min(i0 + per, k) - 1; pick++) {
+                a += (double) q[pick];
+                if (u < a) {
+                    break;
+                }
+            }
+        }
+        *S_out = S;
+        return from < 0 ? k - 1 : __shfl_sync(0xffffffffu, pick, from);
+    }
+    double S    = 0.0;
+    int    pick = k - 1;
+    if (lane == 0) {
+#pragma unroll 1
+        for (int i0 = 0; i0 < k; i0 += 8) { /* eight weights per round: their loads overlap, the sum keeps its order */
+            float w8[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                w8[i] = i0 + i < k ? q[i0 + i] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                S += (double) w8[i]; /* adding +0 behind the last weight changes nothing */
+            }
+        }
+        const double u = (double) u01 * S;
+        double       a = 0.0;
+#pragma unroll 1
+        for (int i = 0; i < k; i++) {
+            a += (double) q[i];
+            if (u < a) {
+                pick = i;
+                break;
+            }
+        }
+    }
+    *S_out = __shfl_sync(0xffffffffu, S, 0);
+    return __shfl_sync(0xffffffffu, pick, 0);
+}
+
 /* The part's maximum, as its candidates are. */
 __device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late) {
     unsigned long long b = 0ull;
@@ -2250,7 +2439,6 @@ __device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late)
  * values, the highest in front, and ranked against their own bin: one against all costs a thread block total^2 / 32
  * rounds of six instructions. 1000 rows of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9;
  * 256 x 128256 top-k 200 48.9 -> 41.0. */
-constexpr int kRankFew = 128;
 __device__ __noinline__ void rank_in_bins(StreamShared *sh, unsigned char *gmem, int total, int k, float lo, bool cap_late) {
     const int tid = (int) threadIdx.x, lane = tid & 31;
     Pair       *srt   = reinterpret_cast<Pair *>(gmem); /* the group maxima are done with */
@@ -2457,89 +2645,40 @@ __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, Stream
     }
     if (ok) {
         if (total <= kRankFew) {
-#pragma unroll 1
-            for (int i = tid; i < total; i += kThreads) {
-                const Pair me   = sh->cand[i];
-                int        rank = 0;
-#pragma unroll 4
-                for (int j = 0; j < total; j++) {
-                    rank += pair_before(sh->cand[j].v, sh->cand[j].idx, me.v, me.idx) ? 1 : 0;
-                }
-                if (rank < k) {
-                    sh->fin_s[rank] = me;
-                }
-            }
+            rank_few(sh->cand, total, k, inv_t, sh->fin_s, sh->fin_q);
         } else {
             rank_in_bins(sh, gmem, total, k, lo, cap_late);
-        }
-        __syncthreads();
-        const float m = sh->fin_s[0].v;
-        for (int i = tid; i < k; i += kThreads) {
-            sh->fin_q[i] = exp_exact(scaled_arg(sh->fin_s[i].v, m, inv_t));
+            __syncthreads();
+            const float m = sh->fin_s[0].v;
+            for (int i = tid; i < k; i += kThreads) {
+                sh->fin_q[i] = exp_exact(scaled_arg(sh->fin_s[i].v, m, inv_t));
+            }
         }
         __syncthreads();
     }
-    if (tid == 0) {
+    /* The draw, by a warp that has nothing to do at the next row's set-up: the others go there (its first barrier comes before
+     * anything that is read here is written again). */
+    if (tid >> 5 == kWarps - 1) {
         unsigned long long rng = sh->cur_rng; /* the sequence's word; this row starts cur_rr draws behind it */
         for (int i = 0; i < sh->cur_rr; i++) {
             (void) xorshift_next(rng);
         }
-        int tok = -1;
+        const float u01 = unit_from(xorshift_next(rng));
+        int         tok = -1;
         if (ok) {
-            /* sampler.c:90-102: the sum and the walk in the reference's order, eight weights per step (their loads overlap) */
-            double S = 0.0;
-#pragma unroll 1
-            for (int i0 = 0; i0 < k; i0 += 8) {
-                float w8[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    w8[q] = i0 + q < k ? sh->fin_q[i0 + q] : 0.0f;
-                }
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    S += (double) w8[q];
-                }
-            }
-            const double u    = (double) unit_from(xorshift_next(rng)) * S;
-            double       a    = 0.0;
-            int          pick = k - 1;
-#pragma unroll 1
-            for (int i0 = 0; i0 < k; i0 += 8) {
-                float w8[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    w8[q] = i0 + q < k ? sh->fin_q[i0 + q] : 0.0f;
-                }
-                double pre[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    a += (double) w8[q];
-                    pre[q] = a;
-                }
-                int first = 8;
-#pragma unroll
-                for (int q = 7; q >= 0; q--) {
-                    if (u < pre[q] && i0 + q < k) {
-                        first = q;
-                    }
-                }
-                if (first < 8) {
-                    pick = i0 + first;
-                    break;
-                }
-            }
-            tok = sh->fin_s[pick].idx + p.vocab_offset;
+            double S;
+            tok = sh->fin_s[draw_sorted(tid & 31, sh->fin_q, k, u01, &S)].idx + p.vocab_offset;
         } else {
-            (void) xorshift_next(rng);
             st_bits |= ST_RETRY;
         }
-        p.tokens[row] = tok;
-        p.status[row] = st_bits;
-        if (p.rng_out != nullptr && sh->cur_last) {
-            p.rng_out[sh->cur_seq] = rng; /* the word after the sequence's last row */
+        if ((tid & 31) == 0) {
+            p.tokens[row] = tok;
+            p.status[row] = st_bits;
+            if (p.rng_out != nullptr && sh->cur_last) {
+                p.rng_out[sh->cur_seq] = rng; /* the word after the sequence's last row */
+            }
         }
     }
-    __syncthreads();
 }
 
 __device__ __noinline__ void finish_raised(const SampleParams &p, StreamShared *sh, unsigned char *gmem, float lo, bool cap_late, int st_bits) {
@@ -2824,6 +2963,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             sh->n_grp  = 0;
             sh->n_cand = 0;
             sh->max_cnt = 1;
+        }
+        if (sel) {
+            reinterpret_cast<int2 *>(sh->key_bins)[tid] = make_int2(0, 0);
+            static_assert(kKeyBins == 2 * kThreads, "two bins per thread");
         }
         if (pen_on && sel) {
             for (int i = tid; i < kIdBits / 128; i += kThreads) {
@@ -3206,51 +3349,21 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             /*
              * The threshold: the kq-th largest (or one a little below) of the 256 thread maxima, a lower bound of the
              * part's kq-th largest value that lies close to it (k of 256 threads hold about k + k^2 / 512 of the
-             * values above it; beyond k = 128 the 512 half maxima are asked). Found by building its key from the top
-             * bit down, each step counting the threads that reach it: a dozen short barriers, no memory.
+             * values above it; beyond k = 128 the 512 half maxima are asked).
              * Against capturing candidates above a rising threshold while the part streams (465 instead of about 100
              * instructions per warp and slice, two barriers and shared-memory atomics inside the part): 256 x 128256
              * top-k 40 with penalties 33.2 -> 32.2 us, 4096 x 128256 top-k 50 549 -> 541 us, 256 x 262144 top-p
              * 97.0 -> 85.2 us with the sums' new form, 48 x 262144 soft-capped top-k 64 116 -> 104 us a step.
              */
-            float sel0 = kq <= kThreads / 2 ? fmaxf(top0, top1) : top0, sel1 = kq <= kThreads / 2 ? -CUDART_INF_F : top1;
+            const bool two  = kq > kThreads / 2;
+            float      sel0 = two ? top0 : fmaxf(top0, top1), sel1 = top1;
             if (cap_late) { /* as the values they belong to will be once they are read again */
                 sel0 = sel0 == -CUDART_INF_F ? sel0 : soft_cap(sel0, sh->cap);
-                sel1 = sel1 == -CUDART_INF_F ? sel1 : soft_cap(sel1, sh->cap);
-            }
-            const unsigned key0 = order_key(sel0), key1 = order_key(sel1);
-            /* The kq-th largest lies between the smallest and the largest of them: the search begins below their common bits
-             * (keys of a warp's extremes, one barrier; it saves half of the rounds, each of which is a barrier). */
-            const unsigned kmin = __reduce_min_sync(0xffffffffu, kq <= kThreads / 2 ? key0 : min(key0, key1)), kmax = __reduce_max_sync(0xffffffffu, max(key0, key1));
-            if (lane == 0) {
-                sh->key_ends[warp] = make_uint2(kmin, kmax);
-            }
-            __syncthreads();
-            unsigned all_min = 0xffffffffu, all_max = 0u;
-#pragma unroll
-            for (int w = 0; w < kWarps; w++) {
-                const uint2 e = sh->key_ends[w];
-                all_min       = min(all_min, e.x);
-                all_max       = max(all_max, e.y);
-            }
-            const int same = __clz(all_min ^ all_max); /* leading bits that all have in common */
-            unsigned  tkey = same == 0 ? 0u : all_max & ~(0xffffffffu >> same);
-            if (same == 32) {
-                tkey = all_max;
-            }
-            for (int bit = 31 - same; bit >= 0; bit--) {
-                const unsigned t = tkey | (1u << bit);
-                int            n = __syncthreads_count(key0 >= t);
-                if (kq > kThreads / 2) {
-                    n += __syncthreads_count(key1 >= t);
-                }
-                if (n >= kq) {
-                    tkey = t;
-                    if (n <= kq + kq / 8) {
-                        break;
-                    }
+                if (two) {
+                    sel1 = sel1 == -CUDART_INF_F ? sel1 : soft_cap(sel1, sh->cap);
                 }
             }
+            const unsigned tkey = kth_key(order_key(sel0), order_key(sel1), two, kq, sh->key_bins, sh->key_ends, lane, warp);
             tau = tkey <= order_key(-CUDART_INF_F) ? -CUDART_INF_F : key_to_float(tkey); /* fewer than kq of them: everything passes */
             float tau_grp = tau;
             if (cap_late && tau > -CUDART_INF_F) {
@@ -3261,12 +3374,22 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 const float t = y > -1.0f ? c * atanhf(y) : -CUDART_INF_F;
                 tau_grp       = t - fabsf(t) * 0x1p-20f - c * 0x1p-140f - 0x1p-120f;
             }
-            /* the thread's groups that reach it */
+            /* the thread's groups that reach it: listed by the warp, a place in the list for all of the warp's at once */
             const int slots = ((part_len - 1) >> gm_shift) + 1;
+            unsigned  hits  = 0u; /* of the thread's slots */
+            if (fmaxf(top0, top1) >= tau_grp) {
 #pragma unroll 4
-            for (int i = 0; i < slots; i++) {
-                if (gmax[i * kThreads + tid] >= tau_grp) {
-                    sh->grp[atomicAdd(&sh->n_grp, 1)] = (unsigned short) ((i << 8) | tid);
+                for (int i = 0; i < slots; i++) {
+                    hits |= gmax[i * kThreads + tid] >= tau_grp ? 1u << i : 0u;
+                }
+            }
+            const int hits_w = __reduce_add_sync(0xffffffffu, __popc(hits));
+            int       at     = lane == 0 && hits_w > 0 ? atomicAdd(&sh->n_grp, hits_w) : 0;
+            at               = __shfl_sync(0xffffffffu, at, 0);
+            for (unsigned any; (any = __ballot_sync(0xffffffffu, hits != 0u)) != 0u; at += __popc(any)) {
+                if (hits != 0u) {
+                    sh->grp[at + __popc(any & ((1u << lane) - 1u))] = (unsigned short) (((__ffs(hits) - 1) << 8) | tid);
+                    hits &= hits - 1u;
                 }
             }
             __syncthreads();
@@ -3282,37 +3405,54 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 tau_raw       = fminf(tau, x - fabsf(x) * 0x1p-20f);
             }
             /* a candidate at least in each: more groups than candidates fit need no look (uncapped values may fall short) */
-            over            = sh->n_grp > kPartCand && !(cap_late && tau > -CUDART_INF_F);
-            const int  n_grp = over ? 0 : sh->n_grp, per_log = kNV4Log + gm_shift;
-            double    fix   = 0.0;
-            for (int t0 = 32 * warp; t0 < n_grp << per_log; t0 += kThreads) { /* whole warps: ids are looked up by all lanes together */
-                const int  t = t0 + lane, name = t < n_grp << per_log ? sh->grp[t >> per_log] : 0, f = t & ((1 << per_log) - 1), w = (name & 255) >> 5, l = name & 31;
-                const int  s = ((name >> 8) << gm_shift) + f / kNV4, c = c0 + s, i4 = l + 32 * (f % kNV4);
-                const bool last_c = c == p.n_slices - 1;
-                const int  n = last_c ? n_last : n_full, nv4 = (n + 3) >> 2, L = share_len(nv4), w4 = min(w * L, nv4);
-                const bool own = t < n_grp << per_log && s < part_len && i4 < min(L, nv4 - w4);
-                const int  e0  = 4 * (w4 + i4), id0 = c * p.slice + e0;
-                float      v[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                if ((kKinds & K_PEN) == 0 && !own) {
-                    continue;
-                }
-                if (own) {
-                    const float *src = (kPlain ? p.logits + (size_t) row * (size_t) p.row_stride : row_again(p, row)) + id0;
+            over = sh->n_grp > kPartCand && !(cap_late && tau > -CUDART_INF_F);
+            const int per_log = kNV4Log + gm_shift, n_again = over ? 0 : sh->n_grp << per_log;
+            double    fix     = 0.0;
+            /* the float4 that item t of the groups names: slice of the part, warp, index in the share, where in the slice; whether there is one */
+            auto named = [&](int t, int &s, int &w, int &i4, int &e0, int &n) {
+                const int name = t < n_again ? sh->grp[t >> per_log] : 0, f = t & ((1 << per_log) - 1);
+                s              = ((name >> 8) << gm_shift) + f / kNV4;
+                w              = (name & 255) >> 5;
+                i4             = (name & 31) + 32 * (f % kNV4);
+                n              = c0 + s == p.n_slices - 1 ? n_last : n_full;
+                const int nv4 = (n + 3) >> 2, L = share_len(nv4), w4 = min(w * L, nv4);
+                e0 = 4 * (w4 + i4);
+                return t < n_again && s < part_len && i4 < min(L, nv4 - w4);
+            };
+            const float *src_row = kPlain ? p.logits + (size_t) row * (size_t) p.row_stride : row_again(p, row);
+            auto         fetched = [&](int t) {
+                float4 v = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+                int    s, w, i4, e0, n;
+                if (named(t, s, w, i4, e0, n)) {
+                    const float *src = src_row + (c0 + s) * p.slice + e0;
                     if (src_al && e0 + 4 <= n) {
-                        const float4 q = *reinterpret_cast<const float4 *>(src);
-                        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+                        v = *reinterpret_cast<const float4 *>(src);
                     } else {
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            v[q] = e0 + q < n ? src[q] : -CUDART_INF_F;
-                        }
+                        v.x = e0 + 0 < n ? src[0] : -CUDART_INF_F;
+                        v.y = e0 + 1 < n ? src[1] : -CUDART_INF_F;
+                        v.z = e0 + 2 < n ? src[2] : -CUDART_INF_F;
+                        v.w = e0 + 3 < n ? src[3] : -CUDART_INF_F;
                     }
-                    if (pro_on && !rewritten) {
+                }
+                return v;
+            };
+            float4 ahead{};
+#pragma unroll 1
+            for (int t0 = 32 * warp; t0 < n_again; t0 += kThreads) { /* whole warps: ids are looked up by all lanes together */
+                const bool   first = ((t0 / kThreads) & 1) == 0; /* two of a lane's float4 on their way at a time */
+                const float4 got   = first ? fetched(t0 + lane) : ahead;
+                if (first) {
+                    ahead = fetched(t0 + kThreads + lane);
+                }
+                float      v[4] = {got.x, got.y, got.z, got.w};
+                int        s, w, i4, e0, n;
+                const bool own = named(t0 + lane, s, w, i4, e0, n);
+                const int  c = c0 + s, id0 = c * p.slice + e0;
+                if (pro_on && !rewritten && own) {
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            if (e0 + q < n) {
-                                v[q] = prologue_one(v[q], id0 + q, sh->cap, sh->mrow);
-                            }
+                    for (int q = 0; q < 4; q++) {
+                        if (e0 + q < n) {
+                            v[q] = prologue_one(v[q], id0 + q, sh->cap, sh->mrow);
                         }
                     }
                 }
@@ -3365,16 +3505,26 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                         }
                     }
                 }
-                bool any = false;
+                unsigned hit[4], found = 0u; /* which lanes' values are candidates */
+                bool     any = false;
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    if (own && v[q] >= tau && e0 + q < n) {
-                        const int pos = atomicAdd(&sh->n_cand, 1);
-                        if (pos < kPartCand) {
-                            sh->cand[pos].v   = v[q];
-                            sh->cand[pos].idx = id0 + q;
+                    const bool cand = own && v[q] >= tau && e0 + q < n;
+                    hit[q]          = __ballot_sync(0xffffffffu, cand);
+                    found += __popc(hit[q]);
+                    any |= cand;
+                }
+                if (found != 0u) {
+                    int pos = lane == 0 ? atomicAdd(&sh->n_cand, (int) found) : 0;
+                    pos     = __shfl_sync(0xffffffffu, pos, 0);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int at = pos + __popc(hit[q] & ((1u << lane) - 1u));
+                        if (((hit[q] >> lane) & 1u) != 0u && at < kPartCand) {
+                            sh->cand[at].v   = v[q];
+                            sh->cand[at].idx = id0 + q;
                         }
-                        any = true;
+                        pos += __popc(hit[q]);
                     }
                 }
                 if ((kKinds & K_SUMS) != 0 && sums && any) {

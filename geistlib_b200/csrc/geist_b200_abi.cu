@@ -76,6 +76,7 @@ struct Plan {
     int    slice        = 0;
     int    row_cap      = 0;
     int    bucket_cap   = 0;
+    int    many_ids     = 0;
     int    id_slots     = 0;
     int    hist_cap     = 0;
     size_t smem         = 0;
@@ -100,12 +101,13 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
     }
     pl.n_slices     = (int) n_slices;
     pl.slice        = (int) slice;
-    /* histories of more than kRowIds ids are counted by a kernel of their own, in a shared-memory table with at
+    /* histories of more than kRowIdsMax ids are counted by a kernel of their own, in a shared-memory table with at
      * least two slots per id */
     pl.id_slots     = 0;
     pl.row_cap      = 0;
     pl.bucket_cap   = 0;
-    if (hist_max > (size_t) gb::kRowIds) {
+    pl.many_ids     = hist_max > (size_t) gb::kRowIds ? 1 : 0;
+    if (hist_max > (size_t) gb::kRowIdsMax) {
         size_t slots = 1024;
         while (slots < 2 * hist_max) {
             slots *= 2;
@@ -118,7 +120,7 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
         pl.bucket_cap = (int) round_up(n_slices * (size_t) gb::kWarps + 1, 4);
     }
     pl.hist_cap = hist_max ? (int) round_up(std::min<size_t>(hist_max, 1024), 4) : 0; /* the finisher walks segments of at most 1024 ids */
-    pl.smem     = gb::sample_stream_smem(pl.n_slices, pl.id_slots > 0 ? 1 : 0);
+    pl.smem     = gb::sample_stream_smem(pl.n_slices, pl.many_ids);
     if (pl.smem > kSmemMax) {
         return false;
     }
@@ -376,6 +378,7 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     p.mask_stride  = (long long) b->logit_mask_stride;
     p.hist         = b->history;
     p.hist_stride  = (long long) b->history_stride;
+    p.hist_quads   = (reinterpret_cast<uintptr_t>(b->history) & 15u) == 0 && (b->history_stride & 3u) == 0 ? 1 : 0;
     p.hist_len     = b->history_len;
     p.extra        = b->fed_tokens;
     p.extra_stride = (long long) b->fed_stride;
@@ -395,8 +398,12 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     p.kept_val     = b->kept_prob;
     p.n_slices     = pl.n_slices;
     p.slice        = pl.slice;
+    p.slice_rcp    = 1.0f / (float) pl.slice;
+    p.share_rcp    = 1.0f / (float) gb::share_len(((int) std::min<size_t>((size_t) pl.slice, b->n_vocab) + 3) >> 2);
+    p.share_rcp_last = 1.0f / (float) gb::share_len((int) ((b->n_vocab - (size_t) (pl.n_slices - 1) * (size_t) pl.slice + 3) >> 2));
     p.row_cap      = pl.row_cap;
     p.bucket_cap   = pl.bucket_cap;
+    p.many_ids     = pl.many_ids;
     p.id_slots     = pl.id_slots;
     p.hist_cap     = pl.hist_cap;
     p.aligned      = ((reinterpret_cast<uintptr_t>(b->logits) & 15u) == 0 && (b->row_stride & 3u) == 0) ? 1 : 0;

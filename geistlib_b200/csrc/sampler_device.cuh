@@ -90,6 +90,9 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned
 __device__ __forceinline__ void copy_word_async(void *dst_shared, const void *src_global) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned) __cvta_generic_to_shared(dst_shared)), "l"(src_global) : "memory");
 }
+__device__ __forceinline__ void copy_quad_async(void *dst_shared, const void *src_global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned) __cvta_generic_to_shared(dst_shared)), "l"(src_global) : "memory");
+}
 __device__ __forceinline__ void async_copies_wait() {
     asm volatile("cp.async.wait_all;" ::: "memory");
 }

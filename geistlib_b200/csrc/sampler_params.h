@@ -30,7 +30,11 @@ constexpr int kGroupSlots   = 16;             /* group maxima a thread keeps of 
 constexpr int kPartCand     = 1024;           /* candidates that one row part can hand on */
 constexpr int kPartBytes    = 32 + kPartCand * 8; /* a part in global scratch: its record, then its candidates */
 constexpr int kSliceRefs    = 32;             /* slices of a part whose references are remembered in shared memory */
-constexpr int kRowIds       = 256;            /* ids of a row (history + fed tokens) counted inside the stream kernel, one per thread */
+constexpr int kRowIds       = 256;            /* ids of a row (history + fed tokens) that a thread block of the stream kernel counts, one per thread ... */
+constexpr int kRowIdsMax    = 1024;           /* ... and where a launch's rows can bring more, four per thread; beyond this a kernel ahead of it counts them */
+
+/* float4 of a slice that one warp owns: an equal share, rounded up to whole warp steps */
+__host__ __device__ __forceinline__ int share_len(int nv4) { return ((nv4 + kWarps - 1) / kWarps + 31) & ~31; }
 
 /* status word, one per row (bit set) */
 enum : int {
@@ -134,6 +138,7 @@ struct SampleParams {
 
     const int *hist;          /* [n_seq, hist_stride] or null */
     long long  hist_stride;
+    int        hist_quads;    /* the rows of hist lie on the 16-byte grid, and their length is whole quads */
     const int *hist_len;      /* [n_seq] */
     const int *extra;         /* [n_seq, extra_stride] or null: tokens fed through a verify pass */
     long long  extra_stride;
@@ -157,9 +162,11 @@ struct SampleParams {
     /* launch shape */
     int      n_slices;     /* work items per row */
     int      slice;        /* floats per slice, multiple of 4, <= kSliceMax */
+    float    slice_rcp, share_rcp, share_rcp_last; /* 1 / slice; 1 / float4 per warp of a full slice and of a row's last one */
     int      parts_max;    /* thread blocks one row can be spread over */
     RunMap   map;          /* how the items are dealt out to the stream kernel's thread blocks */
-    /* rows with more than kRowIds ids: their distinct ids are prepared by a kernel of their own */
+    int      many_ids;    /* rows can bring more than kRowIds ids */
+    /* rows with more than kRowIdsMax ids: their distinct ids are prepared by a kernel of their own */
     int       id_slots;    /* slots of that kernel's id table (a power of two, at least twice the ids a row can bring); 0: no such rows */
     int       row_cap;     /* entries of one row's prepared list */
     int       bucket_cap;  /* n_slices * kWarps + 1 rounded up to a multiple of 4 */

@@ -34,7 +34,7 @@
  *   and top-k alone and is launched instead when the caller vouched for such rows (F_FAST_ONLY); with
  *   F_GREEDY_ONLY, and with F_INLINE_TOPK (whole rows per thread block, greedy and top-k rows), the stream kernel
  *   writes the tokens itself and no finishing kernel runs.
- *   Histories of more than kRowIds ids are counted per row by row_ids_kernel ahead of all this.
+ *   Histories of more than kRowIdsMax ids are counted per row by row_ids_kernel ahead of all this.
  *
  *   The stream kernel is a template over what a launch can meet (kinds of rows vouched for, penalties at all,
  *   plain input, short histories), chosen by the host at the launch: an instantiation carries no code for the
@@ -155,9 +155,6 @@ struct __align__(16) GroupShared {
     int       flag;
     int       pick;
 };
-
-/* float4 of a slice that one warp owns: an equal share, rounded up to whole warp steps */
-__host__ __device__ __forceinline__ int share_len(int nv4) { return ((nv4 + kWarps - 1) / kWarps + 31) & ~31; }
 
 static_assert(kSliceMax / kWarps <= 1024, "an offset in a share takes ten bits of an id list entry");
 static_assert(kNV4 == 1 << kNV4Log, "the float4 of a group are named by bits");
@@ -1265,6 +1262,7 @@ namespace gb {
 
 /* ------------------------------------------------------------ shared state -- */
 
+constexpr int kTagAt  = 21; /* above an entry's ten bits of offset and eleven of count (kRowIdsMax at most) */
 constexpr int kIdBits = 4 * kSliceMax;
 /* Where the bit of a value lies: slice of the part, warp, offset in the share. */
 __device__ __forceinline__ int id_bit(int s, int w, int off) { return ((s & 3) * kWarps + w) * (kSliceMax / kWarps) + off; }
@@ -1280,8 +1278,8 @@ struct PartAgain {
     float           rep, freq, pres;
     double          rep_rcp;
     const int      *long_off;  /* long histories: where the part's shares' runs start ... */
-    const unsigned *long_list; /* ... in this list */
-    bool            long_smem; /* the runs are in shared memory, as a short history's are */
+    const unsigned *list;      /* the ids' entries */
+    bool            long_smem; /* where the runs start lies in shared memory, as for ids counted here */
 };
 
 /* What the warps of one thread block share. The ring (every warp's two stages) lies in front of it in dynamic
@@ -1295,14 +1293,15 @@ struct __align__(16) StreamShared {
     double             wb_acc[kWarps];             /* ... that sum ... */
     double             wb_sum[kWarps];             /* ... and the sum without the candidates, relative to the part's reference */
     float              ref_at[kSliceRefs][kWarps]; /* top-p: what a slice's terms were formed relative to */
-    int                rl_id[kRowIds], rl_cnt[kRowIds + 4]; /* the row's distinct history ids as (offset in the share | count << 10 | tag << 20),
-                                                             * grouped by the (slice, warp) share they fall into, and where each group's run starts */
+    unsigned           rl_id[kRowIds]; /* the row's distinct history ids as (offset in the share | count << 10 | tag << kTagAt),
+                                        * grouped by the (slice, warp) share they fall into (rows that can bring more: behind the group maxima) ... */
+    alignas(16) int    rl_cnt[kRowIds + 4]; /* ... and where each group's run starts */
     alignas(16) unsigned id_bits[kIdBits / 32];             /* which values of the part an id has changed (slices s and s + 4 share their bits) */
     /* the part's select */
     uint2              key_ends[kWarps];      /* smallest and largest key of a warp's thread maxima */
     int                n_grp, n_cand;         /* groups that reach the threshold; candidates in them */
     int                max_cnt;               /* how often the part's most frequent id occurs (asked where that raises a value) */
-    unsigned short     grp[kGroupSlots * kThreads]; /* (slot << 8) | thread */
+    alignas(16) unsigned short grp[kGroupSlots * kThreads]; /* (slot << 8) | thread; at a part's set-up, how many ids each group of them has */
     alignas(8) Pair    cand[kPartCand];
     PartAgain          again;                 /* what raise_threshold needs to know of the part */
     /* finishing inside the stream kernel (F_INLINE_TOPK): the k best in order, their weights */
@@ -1316,8 +1315,9 @@ struct __align__(16) StreamShared {
     int                cur_seq, cur_last;
     float              cap;             /* the part's soft cap and mask row (0 / null: none) */
     const unsigned    *mrow;
+    const unsigned    *raw_word[kRawWords]; /* SampleParams::raw_word: lanes that read different words of a constant take turns */
     RawCfg             raw_nxt;         /* parameters of the next row of this run, copied in while the part streams */
-    int                nxt_ids[kRowIds]; /* that row's history ids (raw): the first words of its history row ... */
+    alignas(16) int    nxt_ids[kRowIds]; /* that row's history ids (raw): the first words of its history row ... */
     int                nxt_ext[kRowIds]; /* ... and the tokens fed before it */
 };
 
@@ -1344,7 +1344,7 @@ struct __align__(16) FinishShared {
 };
 
 constexpr int kGroupBytes = kGroupSlots * kThreads * 4; /* one maximum per slot and thread */
-constexpr int kListSmem   = 1024;             /* prepared id-list entries of a part that are kept in shared memory */
+constexpr int kListSmem   = kRowIdsMax;       /* id-list entries of a part that are kept in shared memory */
 constexpr int kFinCap     = 2048;             /* candidates the finisher can order per row (8 per thread) */
 constexpr int kFinPer     = kFinCap / kThreads;
 constexpr int kRankAll    = 220;              /* up to this many candidates the finisher ranks one against all (220 against 384, us: 1000 x 16384 top-k 128 79.5 -> 71.7,
@@ -1352,7 +1352,7 @@ constexpr int kRankAll    = 220;              /* up to this many candidates the 
 constexpr int kFinBytes   = kWarps * 256 * 12;    /* finisher: the merged candidate list; the multi-pass path keeps one byte histogram per warp there */
 constexpr int kFinGeneralBytes = sizeof(WideShared) > (size_t) kFinBytes ? (int) sizeof(WideShared) : kFinBytes; /* the general kernel works on wide rows there as well */
 static_assert(kFinCap * (int) sizeof(Pair) <= kFinBytes, "the merged list fits");
-static_assert(kGroupBytes >= 4 * kRowIds * 4, "the id table of a part's set-up lies in the group maxima's memory");
+static_assert(kGroupBytes >= 2 * kRowIdsMax * 8, "the id table of a part's set-up lies in the group maxima's memory");
 static_assert(kGroupSlots <= 256 && kThreads == 256, "a group's name fits 16 bits");
 
 /* Part `k` of a row in global scratch: its record (two int4), then its candidates. */
@@ -1362,6 +1362,13 @@ __device__ __forceinline__ int4 *part_rec(const SampleParams &p, int row, int k)
 
 /* n things dealt out in runs of q + 1 (the first r runs) and q: which run holds thing i */
 __device__ __forceinline__ int run_of(int i, int q, int r) { return i < r * (q + 1) ? i / (q + 1) : r + (i - r * (q + 1)) / q; }
+
+/* a / d for a quotient of at most 1024, given 1 / d: the float product is off by one at most */
+__device__ __forceinline__ int quotient(int a, int d, float rcp) {
+    int       q = __float2int_rz((float) a * rcp);
+    const int r = a - q * d;
+    return q + (r >= d ? 1 : 0) - (r < 0 ? 1 : 0);
+}
 
 /* The thread block that streams item i, and the run [first, first + count) of thread block b (RunMap). */
 __device__ __forceinline__ int cta_of_item(const SampleParams &p, int i) {
@@ -2232,14 +2239,6 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
 
 /* ------------------------------------------------------------------ kernel -- */
 
-/* How many ids (history + tokens fed before this row) a row brings. */
-__device__ __forceinline__ int row_id_count(const SampleParams &p, int hist_len, int row) {
-    const int seq0 = p.rows_per_seq == 1 ? row : row / p.rows_per_seq;
-    const int H    = p.hist ? (int) min((long long) max(hist_len, 0), p.hist_stride) : 0;
-    const int E    = p.extra ? row - seq0 * p.rows_per_seq : 0;
-    return H + E;
-}
-
 /*
  * A lower bound of the kq-th largest of the threads' keys (one each, two with `two`) that kq of them reach and few more: the keys
  * are counted in kKeyBins bins between the smallest and the largest, and where the bin that the kq-th falls into holds too many,
@@ -2563,11 +2562,10 @@ __device__ __noinline__ float raise_threshold(const SampleParams &p, StreamShare
                 }
                 if (a.pen && ((sh->id_bits[bit >> 5] >> (bit & 31)) & 1u) != 0u) {
                     const int       g   = a.long_ids ? s * kWarps + w : (s & 31) * kWarps + w;
-                    const unsigned *ent = a.long_ids ? a.long_list : reinterpret_cast<const unsigned *>(sh->rl_id);
                     const int       lo  = a.long_smem ? sh->rl_cnt[g] : a.long_off[g], hi = a.long_smem ? sh->rl_cnt[g + 1] : a.long_off[g + 1];
                     for (int i = lo; i < hi; i++) {
-                        if ((int) (ent[i] & 0x3ffu) == off && (a.long_ids || (int) (ent[i] >> 20) == s >> 5)) {
-                            v[q] = penalise_rcp(v[q], (int) ((ent[i] >> 10) & (a.long_ids ? 0x3fffffu : 0x3ffu)), a.rep_rcp, a.rep, a.freq, a.pres);
+                        if ((int) (a.list[i] & 0x3ffu) == off && (a.long_ids || (int) (a.list[i] >> kTagAt) == s >> 5)) {
+                            v[q] = penalise_rcp(v[q], (int) ((a.list[i] >> 10) & (a.long_ids ? 0x3fffffu : 0x7ffu)), a.rep_rcp, a.rep, a.freq, a.pres);
                         }
                     }
                 }
@@ -2720,7 +2718,7 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
         static_assert(offsetof(RawCfg, T) == 4 && offsetof(RawCfg, top_p) == 8 && offsetof(RawCfg, top_k) == 12 && offsetof(RawCfg, hist_len) == 16 && offsetof(RawCfg, rep) == 20 &&
                               offsetof(RawCfg, freq) == 24 && offsetof(RawCfg, pres) == 28 && offsetof(RawCfg, cap) == 32 && offsetof(RawCfg, rng) == 40,
                       "raw_word is in the order of the words");
-        const unsigned *from = p.raw_word[lane];
+        const unsigned *from = sh->raw_word[lane];
         unsigned       *to   = reinterpret_cast<unsigned *>(&sh->raw_nxt) + lane;
         if (from != nullptr) {
             copy_word_async(to, from + (lane < 10 ? (size_t) seq : 2 * (size_t) seq + (size_t) (lane - 10)));
@@ -2730,8 +2728,19 @@ __device__ __forceinline__ void prefetch_step(const SampleParams &p, StreamShare
     }
     if (p.hist) {
         const int hs = (int) min((long long) kRowIds, p.hist_stride);
-        for (int t = lane; t < hs; t += 32) {
-            copy_word_async(&sh->nxt_ids[t], &p.hist[(size_t) seq * (size_t) p.hist_stride + t]);
+        const int *from = p.hist + (size_t) seq * (size_t) p.hist_stride;
+        if (p.hist_quads) { /* rows of ids on the 16-byte grid */
+            for (int t = 4 * lane; t < hs; t += 128) {
+                copy_quad_async(&sh->nxt_ids[t], from + t);
+            }
+        } else {
+            for (int t = lane; t < hs; t += 32) {
+                copy_word_async(&sh->nxt_ids[t], from + t);
+            }
+        }
+        /* what lies behind them is read where the row begins: L2 is asked for it */
+        for (int t = kRowIds + 32 * lane; t < (int) min((long long) kRowIdsMax, p.hist_stride); t += 32 * 32) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(from + t));
         }
     }
     if (p.extra) {
@@ -2783,6 +2792,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             }
         }
         mbar_init_fence();
+    }
+    if (tid >= 32 && tid < 32 + kRawWords) {
+        sh->raw_word[tid - 32] = p.raw_word[tid - 32];
     }
     __syncthreads();
     /* Launched as a programmatic dependent of the kernel before it in the stream: the thread block may have
@@ -2840,7 +2852,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     }
     const int    bulk4_f = max(0, min(mine4_f, (n_full >> 2) - w4lo_f)); /* float4 of the share that a bulk copy brings */
     const int    bulk4_l = max(0, min(mine4_l, (n_last >> 2) - w4lo_l));
-    int          irow = my_first / p.n_slices, ic = my_first - irow * p.n_slices, ijj = 0; /* the next item to request */
+    const int    row_first = my_first / p.n_slices, c_first = my_first - row_first * p.n_slices;
+    int          irow = row_first, ic = c_first, ijj = 0; /* the next item to request */
     const float *isrc = p.logits + (size_t) irow * (size_t) p.row_stride + (size_t) ic * (size_t) p.slice; /* ... and where its slice starts */
     auto issue_next = [&]() {
         const bool last  = ic == p.n_slices - 1;
@@ -2898,10 +2911,24 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
     int j         = 0;
     int ring_dead = -1; /* the item at which a copy of this warp failed to arrive in time (-1: none) */
     int pf        = 0; /* warp 0: how far the parameters of the row that begins next have been fetched */
-    while (j < my_count) {
-        const int  item0 = my_first + j, row = item0 / p.n_slices, c0 = item0 - row * p.n_slices;
+    for (int row = row_first, c0 = c_first; j < my_count; row++, c0 = 0) {
         const int  part_len   = min(p.n_slices - c0, my_count - j);
         const bool final_part = j + part_len == my_count;
+        /* the table in which a row's ids are counted, the counts of their groups and the marks of changed values: cleared while
+         * the row's parameters are on their way, or the row before is drawn from */
+        constexpr int kPerT = (kKinds & K_SHORT) != 0 ? 1 : kRowIdsMax / kThreads, kIdSlots = 2 * kRowIds * kPerT; /* ids of a thread */
+        int          *id_key = reinterpret_cast<int *>(gmem), *id_cnt = id_key + kIdSlots, *id_n = reinterpret_cast<int *>(sh->grp);
+        if ((kKinds & K_PEN) != 0) {
+#pragma unroll
+            for (int i = 0; i < kGroupBytes / 16; i += kThreads) {
+                reinterpret_cast<int4 *>(gmem)[i + tid] = make_int4(0, 0, 0, 0);
+            }
+            id_n[tid] = 0;
+            static_assert(kRowIds == kThreads, "a group's count per thread");
+            for (int i = tid; i < kIdBits / 128; i += kThreads) {
+                reinterpret_cast<uint4 *>(sh->id_bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
         CYC(6);
         if (warp == 0) { /* what has not been fetched while the previous part streamed (first part, short parts) */
             while (pf < kPrefetchDone) {
@@ -2912,7 +2939,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         }
         __syncthreads();
         PROF_ONCE(1);
-        int   mode, kq, n_ids, my_id = -1;
+        int   mode, kq, n_ids, id[kPerT];
         float inv_t, rep, freq, pres;
         bool  pen_on, pro_on, pro_part, cap_late;
         {
@@ -2941,21 +2968,28 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 sh->cur_last = r.rr == p.rows_per_seq - 1 ? 1 : 0;
                 sh->cur_rr   = r.rr;
             }
-            if (tid < n_ids && n_ids <= kRowIds) {
-                my_id = tid < r.H ? sh->nxt_ids[tid] : sh->nxt_ext[tid - r.H];
+            /* the thread's ids that fall into the part, or -1 */
+            const int at0 = c0 * p.slice, at_n = min(part_len * p.slice, p.V - at0);
+#pragma unroll
+            for (int q = 0; q < kPerT; q++) {
+                const int t = tid + q * kThreads;
+                id[q]       = -1;
+                if (pen_on && t < n_ids && n_ids <= kRowIds * kPerT) {
+                    const int at = (q == 0 ? (t < r.H ? sh->nxt_ids[t] : sh->nxt_ext[t - r.H]) : t < r.H ? r.hrow[t] : r.erow[1 + t - r.H]) - p.vocab_offset - at0;
+                    id[q]        = at >= 0 && at < at_n ? at : -1;
+                }
             }
         }
         /* the kind the row is streamed as */
         const int   smode   = ((kKinds & K_SUMS) == 0 && (mode == M_TEMP || mode == M_TOPP)) || ((kKinds & K_SEL) == 0 && mode == M_TOPK) ? (int) M_ARGMAX : mode;
         const bool  sel     = (kKinds & K_SEL) != 0 && (smode == M_TOPK || ((kKinds & K_SUMS) != 0 && smode == M_TOPP)) && kq > 0 && kq <= kFastKMax;
         const bool  sums    = (kKinds & K_SUMS) != 0 && (smode == M_TEMP || (smode == M_TOPP && sel));
-        const bool  long_ids = (kKinds & K_SHORT) == 0 && n_ids > kRowIds;
-        const int   b_first = cta_of_item(p, row * p.n_slices);
-        const int   part_idx = (int) blockIdx.x - b_first;
-        const int   n_parts = cta_of_item(p, row * p.n_slices + p.n_slices - 1) - b_first + 1;
+        const bool  long_ids = (kKinds & K_SHORT) == 0 && n_ids > kRowIdsMax;
 
         const int  *long_off  = (kKinds & K_SHORT) == 0 && long_ids ? p.pre_off + (size_t) row * (size_t) (p.n_slices * kWarps + 1) + c0 * kWarps : nullptr;
         bool        long_smem = true; /* a long list's part lies in shared memory like a short one's */
+
+        unsigned *id_list = (kKinds & K_SHORT) != 0 ? sh->rl_id : sl_list;
 
         /* ---- part set-up ---- */
         if (tid == 0) {
@@ -2968,77 +3002,60 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             reinterpret_cast<int2 *>(sh->key_bins)[tid] = make_int2(0, 0);
             static_assert(kKeyBins == 2 * kThreads, "two bins per thread");
         }
-        if (pen_on && sel) {
-            for (int i = tid; i < kIdBits / 128; i += kThreads) {
-                reinterpret_cast<uint4 *>(sh->id_bits)[i] = make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
         if (pen_on && !long_ids) {
-            /* The row's distinct ids with their counts: an open-addressing table in the group maxima's memory (free
-             * between two parts), one id per thread; the thread whose id opened a slot speaks for that id. The ids
+            /* The distinct ids that fall into the part, with their counts: an open-addressing table in the group maxima's memory (free
+             * between two parts), one id per thread at a time; the thread whose id opened a slot speaks for that id. The ids
              * are then grouped by the (slice, warp) share of the part that they fall into, so that a warp looks at
              * its own share's run alone (most shares hold none): kRowIds groups, slice c of the part and slice
-             * c + 32 share one and tell their ids apart by a tag. Entry: offset in the share | count << 10 | tag << 20. */
-            int *id_key = reinterpret_cast<int *>(gmem);
-            int *id_cnt = id_key + 2 * kRowIds;
-            for (int i = tid; i < 2 * kRowIds; i += kThreads) {
-                id_key[i] = -1;
-                id_cnt[i] = 0;
-            }
-            for (int i = tid; i <= kRowIds; i += kThreads) {
-                sh->rl_cnt[i] = 0; /* entry g + 1: ids in group g; after the scan, entry g: ids in the groups before g */
-            }
-            int id = my_id;
-            if (tid < n_ids) {
-                id -= p.vocab_offset;
-                if (id < 0 || id >= p.V) {
-                    id = -1;
-                }
-            } else {
-                id = -1;
-            }
-            /* which group holds the id (-1: a slice of another part of the row), and the rest of its entry */
-            auto group_of = [&](int gid, int &rest) {
-                const int c = gid / p.slice;
-                if (c < c0 || c >= c0 + part_len) {
-                    return -1;
-                }
-                const int local = gid - c * p.slice;
-                const int L     = share_len(((c == p.n_slices - 1 ? n_last : n_full) + 3) >> 2); /* float4 per warp */
-                const int w     = (local >> 2) / L;
-                rest            = (local - 4 * w * L) | (((c - c0) >> 5) << 20);
-                return ((c - c0) & 31) * kWarps + w;
-            };
-            __syncthreads();
-            int slot = -1, place = -1;
-            if (id >= 0) {
-                unsigned h = ((unsigned) id * 2654435761u) >> (32 - 9);
-                for (int probe = 0; probe < 2 * kRowIds; probe++) {
-                    const int old = atomicCAS(&id_key[h], -1, id);
-                    if (old == -1 || old == id) {
-                        atomicAdd(&id_cnt[h], 1);
-                        slot = old == -1 ? (int) h : -1;
-                        break;
+             * c + 32 share one and tell their ids apart by a tag. Bound by latency, of shared-memory atomics and four
+             * barriers: 64 ids of a row take 0.55 us, 2.2 with eight integer divisions (150 cycles each) per thread and
+             * a table cleared between barriers; 1024 ids 3, where a kernel ahead of the launch took 50 us for 4096 rows
+             * (4096 x 128256 with 1024 ids 453 -> 397 us, 8 x 50257 with 500 ids 25.2 -> 19.8). */
+            int      grp[kPerT], place[kPerT];
+            unsigned entry[kPerT];
+            int      slot[kPerT]; /* -1: the thread does not speak for the id */
+            /* Where the penalty does not ask how often an id occurs and a bit per column fits, whoever sets an id's bit speaks
+             * for it; else the ids are counted in an open-addressing table. */
+            const bool by_bit = freq == 0.0f && part_len * p.slice <= kGroupBytes * 8;
+#pragma unroll
+            for (int q = 0; q < kPerT; q++) {
+                slot[q] = -1;
+                if (id[q] >= 0) {
+                    if (by_bit) {
+                        const unsigned bit = 1u << (id[q] & 31);
+                        slot[q]            = (atomicOr(reinterpret_cast<unsigned *>(gmem) + (id[q] >> 5), bit) & bit) == 0u ? 0 : -1;
+                    } else {
+                        unsigned h = ((unsigned) id[q] * 2654435761u) >> (32 - ((kKinds & K_SHORT) != 0 ? 9 : 11));
+                        static_assert(kIdSlots == 1 << ((kKinds & K_SHORT) != 0 ? 9 : 11), "the bits that the hash keeps");
+                        for (int probe = 0; probe < kIdSlots; probe++) { /* at most half of the slots are ever taken */
+                            const int old = atomicCAS(&id_key[h], 0, id[q] + 1);
+                            if (old == 0 || old == id[q] + 1) {
+                                atomicAdd(&id_cnt[h], 1);
+                                slot[q] = old == 0 ? (int) h : -1;
+                                break;
+                            }
+                            h = (h + 1) & (kIdSlots - 1);
+                        }
                     }
-                    h = (h + 1) & (2 * kRowIds - 1);
                 }
-                if (slot >= 0) {
-                    int       rest;
-                    const int grp = group_of(id, rest);
-                    if (grp >= 0) {
-                        place = atomicAdd(&sh->rl_cnt[grp + 1], 1);
-                    }
+            }
+#pragma unroll
+            for (int q = 0; q < kPerT; q++) {
+                if (slot[q] >= 0) {
+                    const int  c = quotient(id[q], p.slice, p.slice_rcp), local = id[q] - c * p.slice;
+                    const bool last = c0 + c == p.n_slices - 1;
+                    const int  L = share_len(((last ? n_last : n_full) + 3) >> 2), w = quotient(local >> 2, L, last ? p.share_rcp_last : p.share_rcp); /* L float4 per warp */
+                    grp[q]   = (c & 31) * kWarps + w;
+                    entry[q] = (unsigned) (local - 4 * w * L) | ((unsigned) (c >> 5) << kTagAt);
+                    place[q] = atomicAdd(&id_n[grp[q]], 1);
                 }
             }
             __syncthreads();
             if (warp == 0) { /* running sums over the kRowIds counters, eight per lane */
-                int v[8], run = 0;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    run += sh->rl_cnt[1 + 8 * lane + i];
-                    v[i] = run;
-                }
-                int before = run;
+                static_assert(kRowIds == 8 * 32, "eight per lane");
+                const int4 a = reinterpret_cast<const int4 *>(id_n)[2 * lane], b = reinterpret_cast<const int4 *>(id_n)[2 * lane + 1];
+                const int  s0 = a.x, s1 = s0 + a.y, s2 = s1 + a.z, s3 = s2 + a.w, s4 = s3 + b.x, s5 = s4 + b.y, s6 = s5 + b.z, s7 = s6 + b.w;
+                int        before = s7;
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
                     const int o = __shfl_up_sync(0xffffffffu, before, d);
@@ -3046,17 +3063,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                         before += o;
                     }
                 }
-                before -= run;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    sh->rl_cnt[1 + 8 * lane + i] = before + v[i];
+                if (lane == 31) {
+                    sh->rl_cnt[kRowIds] = before;
                 }
+                before -= s7;
+                reinterpret_cast<int4 *>(sh->rl_cnt)[2 * lane]     = make_int4(before, before + s0, before + s1, before + s2);
+                reinterpret_cast<int4 *>(sh->rl_cnt)[2 * lane + 1] = make_int4(before + s3, before + s4, before + s5, before + s6);
             }
             __syncthreads();
-            if (place >= 0) {
-                int       rest;
-                const int grp = group_of(id, rest);
-                sh->rl_id[sh->rl_cnt[grp] + place] = rest | (id_cnt[slot] << 10);
+#pragma unroll
+            for (int q = 0; q < kPerT; q++) {
+                if (slot[q] >= 0) {
+                    id_list[sh->rl_cnt[grp[q]] + place[q]] = entry[q] | ((by_bit ? 1u : (unsigned) id_cnt[slot[q]]) << 10);
+                }
             }
         } else if (pen_on) {
             /* long histories: a kernel that ran before this one left the row's distinct ids with their counts in
@@ -3078,7 +3097,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             long_smem = part_len * kWarps <= kRowIds && e_n <= kListSmem;
         }
         __syncthreads();
-        static_assert(2 * kRowIds == 512, "the id table's hash keeps 9 bits");
 
         PROF_ONCE(3);
         CYC(5);
@@ -3088,7 +3106,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         auto ids_of = [&](int s_, int w, const unsigned *&ent, int &lo, int &hi, unsigned &tag) {
             if (!long_ids) {
                 const int grp = (s_ & 31) * kWarps + w;
-                ent           = reinterpret_cast<const unsigned *>(sh->rl_id);
+                ent           = id_list;
                 lo            = sh->rl_cnt[grp];
                 hi            = sh->rl_cnt[grp + 1];
                 tag           = (unsigned) s_ >> 5;
@@ -3100,7 +3118,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 tag           = 0u;
             }
         };
-        const unsigned cnt_mask = long_ids ? 0x3fffffu : 0x3ffu; /* above the offset's ten bits; a short list's entries carry a tag on top */
+        const unsigned cnt_mask = long_ids ? 0x3fffffu : 0x7ffu; /* above the offset's ten bits; entries of ids counted here carry a tag on top */
         unsigned       run_key = 0u; /* greedy: this warp's maximum of the part so far (key) and its first id */
         int            run_arg = 0x7fffffff;
         float          top0 = -CUDART_INF_F, top1 = -CUDART_INF_F; /* others: the thread's maxima over every other one of its float4 */
@@ -3164,7 +3182,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 ids_of(s, warp, ent, lo, hi, tag);
                 for (int e = lo + lane; e < hi; e += 32) {
                     const unsigned en = ent[e];
-                    if (long_ids || (en >> 20) == tag) {
+                    if (long_ids || (en >> kTagAt) == tag) {
                         most    = max(most, (int) ((en >> 10) & cnt_mask));
                         float *q = sl + (en & 0x3ffu);
                         *q       = penalise_rcp(*q, (int) ((en >> 10) & cnt_mask), rep_rcp, rep, freq, pres);
@@ -3482,7 +3500,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                             ids_of(__shfl_sync(0xffffffffu, s, from), __shfl_sync(0xffffffffu, w, from), ent, lo, hi, tag);
                             for (int base = lo; base < hi; base += 32) {
                                 const unsigned en = base + lane < hi ? ent[base + lane] : 0u;
-                                for (unsigned hit = __ballot_sync(0xffffffffu, base + lane < hi && (int) ((en & 0x3ffu) >> 2) == i4_ && (long_ids || (en >> 20) == tag)); hit != 0u; hit &= hit - 1u) {
+                                for (unsigned hit = __ballot_sync(0xffffffffu, base + lane < hi && (int) ((en & 0x3ffu) >> 2) == i4_ && (long_ids || (en >> kTagAt) == tag)); hit != 0u; hit &= hit - 1u) {
                                     const unsigned eh = __shfl_sync(0xffffffffu, en, __ffs(hit) - 1);
                                     if (lane == from) {
                                         found |= 1u << (eh & 3u);
@@ -3574,7 +3592,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             again.long_ids  = kLong && long_ids;
             again.long_off  = kLong ? long_off : nullptr;
             again.long_smem = !kLong || long_smem;
-            again.long_list = !kLong ? nullptr : long_smem ? sl_list : p.pre_list + (size_t) row * (size_t) p.row_cap;
+            again.list      = !kLong || !long_ids || long_smem ? id_list : p.pre_list + (size_t) row * (size_t) p.row_cap;
         };
         int       n_cand = over ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
         if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
@@ -3599,6 +3617,15 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             n_cand = min(sh->n_cand, kPartCand + 1);
         }
         const int held = sel ? min(n_cand, kPartCand) : 0;
+        int       part_idx = 0, n_parts = 1; /* which part of the row this is, of how many */
+        if (p.map.mode == RUN_PARTS) {
+            n_parts  = p.map.P;
+            part_idx = (int) blockIdx.x - row * n_parts;
+        } else if (p.map.mode == RUN_ITEMS) {
+            const int b_first = cta_of_item(p, row * p.n_slices);
+            part_idx          = (int) blockIdx.x - b_first;
+            n_parts           = cta_of_item(p, row * p.n_slices + p.n_slices - 1) - b_first + 1;
+        }
         if (tid == 0) {
             unsigned long long bw = 0ull;
 #pragma unroll
@@ -3861,7 +3888,7 @@ __device__ __forceinline__ int share_of(const SampleParams &p, int id, int &off)
  * (offset in the share) | (count << 10). Shorter rows are left to the stream kernel. A thread keeps its kPer ids in
  * registers: they are on their way while the table is cleared, and the thread whose id opened a slot of the table writes
  * that id's entry, at the place in its share's run that counting the share gave it. */
-template <int kIdThreads, int kPer>
+constexpr int kIdThreads = 1024, kPer = 8; /* 8192 ids at most: id_slots */
 __global__ void __launch_bounds__(kIdThreads) row_ids_kernel(const __grid_constant__ SampleParams p) {
     extern __shared__ __align__(16) int row_ids_smem[];
     int *tkey = row_ids_smem;          /* open-addressing table: the id ... */
@@ -3877,7 +3904,7 @@ __global__ void __launch_bounds__(kIdThreads) row_ids_kernel(const __grid_consta
     const int seq  = p.slot ? p.slot[seq0] : seq0;
     const int H    = p.hist ? (int) min((long long) max(p.hist_len[seq], 0), p.hist_stride) : 0;
     const int E    = p.extra ? row - seq0 * p.rows_per_seq : 0;
-    if (H + E <= kRowIds) {
+    if (H + E <= kRowIdsMax) {
         return;
     }
     const int *hrow = p.hist ? p.hist + (size_t) seq * (size_t) p.hist_stride : nullptr;
@@ -3951,7 +3978,6 @@ __global__ void __launch_bounds__(kIdThreads) row_ids_kernel(const __grid_consta
     }
 }
 
-constexpr int kIdsFew = 1024; /* ids a row can bring: up to here 256 threads with four each, else 1024 with eight (8192 ids at most: id_slots) */
 
 /* ----------------------------------------------------------------- launchers -- */
 
@@ -4015,22 +4041,22 @@ cudaError_t sample_stream_ctas_per_sm(size_t smem_bytes, int *out) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, sample_stream_kernel<K_SEL | K_SUMS | K_PEN>, kThreads, smem_bytes);
 }
 
-static cudaError_t ensure_row_ids_attributes(const void *kernel, int which, size_t smem_bytes) {
-    static int  configured_smem[64][2] = {{0}};
-    int         dev                    = 0;
-    cudaError_t e                      = cudaGetDevice(&dev);
+static cudaError_t ensure_row_ids_attributes(size_t smem_bytes) {
+    static int  configured_smem[64] = {0};
+    int         dev                 = 0;
+    cudaError_t e                   = cudaGetDevice(&dev);
     if (e != cudaSuccess) {
         return e;
     }
     if (dev < 0 || dev >= 64) {
         return cudaErrorInvalidDevice;
     }
-    if (smem_bytes > 48 * 1024 && (int) smem_bytes > configured_smem[dev][which]) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes);
+    if (smem_bytes > 48 * 1024 && (int) smem_bytes > configured_smem[dev]) {
+        e = cudaFuncSetAttribute(row_ids_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes);
         if (e != cudaSuccess) {
             return e;
         }
-        configured_smem[dev][which] = (int) smem_bytes;
+        configured_smem[dev] = (int) smem_bytes;
     }
     return cudaSuccess;
 }
@@ -4082,17 +4108,11 @@ cudaError_t launch_sample_stream(const SampleParams &p, int grid, size_t smem_by
     }
     if (p.id_slots > 0) { /* rows may bring more ids than the stream kernel counts by itself: prepare their lists first */
         const size_t ids_smem = ((size_t) p.id_slots * 2 + (size_t) p.bucket_cap) * sizeof(int);
-        const bool   few      = p.row_cap <= kIdsFew;
-        const void  *kernel   = few ? reinterpret_cast<const void *>(row_ids_kernel<256, 4>) : reinterpret_cast<const void *>(row_ids_kernel<1024, 8>);
-        e                     = ensure_row_ids_attributes(kernel, few ? 0 : 1, ids_smem);
+        e                     = ensure_row_ids_attributes(ids_smem);
         if (e != cudaSuccess) {
             return e;
         }
-        if (few) {
-            row_ids_kernel<256, 4><<<dim3((unsigned) p.n_rows), dim3(256), ids_smem, stream>>>(p);
-        } else {
-            row_ids_kernel<1024, 8><<<dim3((unsigned) p.n_rows), dim3(1024), ids_smem, stream>>>(p);
-        }
+        row_ids_kernel<<<dim3((unsigned) p.n_rows), dim3(kIdThreads), ids_smem, stream>>>(p);
         e = cudaGetLastError();
         if (e != cudaSuccess) {
             return e;
@@ -4119,7 +4139,7 @@ cudaError_t launch_sample_stream(const SampleParams &p, int grid, size_t smem_by
     const bool pen   = p.hist != nullptr || p.extra != nullptr;
     const int  kinds = (p.flags & F_SELECT_ONLY) != 0u ? (K_SEL | K_SUMS) : (p.flags & F_GREEDY_ONLY) != 0u ? 0 : (p.flags & F_FAST_ONLY) != 0u ? K_SEL : (K_SEL | K_SUMS);
     const bool plain     = p.aligned != 0 && p.softcap == nullptr && p.mask == nullptr && p.out_logits == nullptr;
-    const bool short_ids = !pen || p.id_slots == 0; /* no row brings more ids than a thread block counts by itself */
+    const bool short_ids = !pen || p.many_ids == 0; /* no row brings more ids than a thread block has threads */
 #define GB_STREAM_CASE(K)                                                  \
     case (K):                                                              \
         e = cudaLaunchKernelEx(&cfg, sample_stream_kernel<(K)>, p);        \

@@ -73,9 +73,6 @@ struct __align__(16) WideShared {
     RowCfg             cfg; /* the row's, for the functions that finish it */
 };
 
-__device__ __forceinline__ void copy_quad_async(void *dst_shared, const void *src_global) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned) __cvta_generic_to_shared(dst_shared)), "l"(src_global) : "memory");
-}
 __device__ __forceinline__ int ld_volatile(const int *q) { return *reinterpret_cast<const volatile int *>(q); }
 
 /* Bins of a row's histogram: the bits of e from the floor up to 1, in at most kWideBins equal steps of a power of two.

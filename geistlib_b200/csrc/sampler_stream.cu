@@ -1198,49 +1198,6 @@ __device__ __noinline__ int multipass_row(const SampleParams &p, GroupShared *sh
     return st;
 }
 
-/* Warp 0 of the group: S = sum of w[0..n) and the first i with u(S) < w[0] + .. + w[i] (n - 1 if
- * none), for n <= 256. u01 is the unit draw; the comparison is made against u01 * S like the
- * reference's inverse CDF (sampler.c:90-102). Sums are formed lane-wise and scanned across the
- * warp in double precision. Returns through *S_out and the return value (valid in every lane). */
-__device__ __forceinline__ int warp_inverse_cdf(int lane, const float *w, int n, float u01, double *S_out) {
-    const int per = (n + 31) / 32; /* <= 8 consecutive weights per lane */
-    const int b   = lane * per;
-    double    mine = 0.0;
-    for (int i = b; i < min(b + per, n); i++) {
-        mine += (double) w[i];
-    }
-    double incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) {
-            incl += up;
-        }
-    }
-    const double   S    = __shfl_sync(0xffffffffu, incl, 31);
-    const double   u    = (double) u01 * S;
-    const unsigned ball = __ballot_sync(0xffffffffu, b < n && u < incl);
-    int            pick = n - 1;
-    if (ball != 0u) {
-        const int src = __ffs(ball) - 1;
-        int       f   = n - 1;
-        if (lane == src) {
-            double a = incl - mine;
-            f        = min(b + per, n) - 1;
-            for (int i = b; i < min(b + per, n); i++) {
-                a += (double) w[i];
-                if (u < a) {
-                    f = i;
-                    break;
-                }
-            }
-        }
-        pick = __shfl_sync(0xffffffffu, f, src);
-    }
-    *S_out = S;
-    return pick;
-}
-
 /* Status of a finished row and, behind a sequence's last row, its generator. One thread. */
 __device__ __forceinline__ void row_epilogue(const SampleParams &p, const RowCfg &r, int row, int st, unsigned long long rng0) {
     p.status[row] = st;
@@ -1329,14 +1286,12 @@ constexpr int kStageLog   = 7;
 /* What the threads of one finishing thread block share; the merged candidate list lies behind it. */
 struct __align__(16) FinishShared {
     GroupShared gs; /* reductions of the whole thread block */
-    float       pmax[kMaxParts], ptau[kMaxParts], pbref[kMaxParts];
-    int         parg[kMaxParts], pn[kMaxParts], poff[kMaxParts];
-    double      pbsum[kMaxParts];
-    int         bhist[kHistBins]; /* select histogram */
+    int         poff[kMaxParts]; /* where a part's candidates begin among those that did not come in with the records */
+    alignas(16) int bhist[kHistBins]; /* select histogram */
     int         n_sel, n_border, n_ent, slot;
     unsigned    fin_bitmap[kFinBitmapWords];
     Pair        fsort[kFastKMax];
-    float       fq[kFastKMax];
+    alignas(8) float fq[kFastKMax];
     PenEntry    fdlist[512];
     alignas(16) unsigned long long stage[kStageWords]; /* the records and first candidates of the row's parts */
     unsigned long long save[256 + 128];                      /* the multi-pass path keeps a histogram here */
@@ -1526,6 +1481,117 @@ __device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int to
     g.sync();
 }
 
+/* ------------------------------------------------------ few candidates, weights -- */
+
+/* At most kRankFew candidates in order, the k best to out_s, with kWeigh their weights e^((x - max) / T) to out_q. Four threads (two beyond
+ * 64 candidates) compare a candidate with a share of the others each, eight at a time without a branch between them.
+ * All threads call; the caller's barrier follows. */
+constexpr int kRankFew = 128;
+static_assert(2 * kRankFew == kThreads, "two threads per candidate");
+template <bool kWeigh>
+__device__ __forceinline__ void rank_few(const Pair *cand, int total, int k, float inv_t, Pair *out_s, float *out_q) {
+    const int  log = total <= kRankFew / 2 ? 2 : 1, i = (int) threadIdx.x >> log, step = 1 << log, sub = (int) threadIdx.x & (step - 1);
+    const Pair me   = cand[min(i, total - 1)];
+    int        rank = 0;
+    float      top  = -CUDART_INF_F;
+#pragma unroll 1
+    for (int j0 = sub; j0 < total; j0 += 8 * step) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const Pair o = cand[min(j0 + j * step, total - 1)];
+            rank += j0 + j * step < total && pair_before(o.v, o.idx, me.v, me.idx) ? 1 : 0;
+            top = kWeigh ? fmaxf(top, o.v) : top;
+        }
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    top = kWeigh ? fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1)) : top;
+    if (log == 2) {
+        rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+        top = kWeigh ? fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2)) : top;
+    }
+    if (sub == 0 && i < total && rank < k) {
+        out_s[rank] = me;
+        if (kWeigh) {
+            out_q[rank] = exp_exact(scaled_arg(me.v, top, inv_t));
+        }
+    }
+}
+
+/*
+ * The reference's draw over k <= 256 weights in descending order (sampler.c:90-102): the sum and the walk in its order, in
+ * double. Where the smallest weight is at least 2^-22 every partial sum is a whole number of 2^-45 below 2^53 of them, so
+ * exact in any order, and the warp adds in parallel; else one lane adds one by one. The whole warp calls: the place that
+ * u01 times the sum falls on, and the sum. (Between the candidates and the token of one row, top-k 40: 1.9 us with a thread per
+ * candidate to rank them, the exponentials behind a barrier and one thread over the weights, twice; 1.25 us.)
+ */
+__device__ __forceinline__ int draw_sorted(int lane, const float *q, int k, float u01, double *S_out) {
+    const float2 two = 2 * lane < k ? *reinterpret_cast<const float2 *>(q + 2 * lane) : make_float2(0.0f, 0.0f); /* what lies behind the k-th weight is not used */
+    if (q[k - 1] >= 0x1p-22f) {
+        const int per  = k <= 64 ? 2 : (k + 31) >> 5, i0 = lane * per;
+        double    incl = (double) two.x + (2 * lane + 1 < k ? (double) two.y : 0.0);
+        if (k > 64) {
+            incl = 0.0;
+#pragma unroll 1
+            for (int i = i0; i < min(i0 + per, k); i++) {
+                incl += (double) q[i];
+            }
+        }
+        const double mine = incl;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) {
+                incl += up;
+            }
+        }
+        const double S = __shfl_sync(0xffffffffu, incl, 31), u = (double) u01 * S;
+        const int    from = __ffs(__ballot_sync(0xffffffffu, u < incl)) - 1; /* the lane whose run crosses u, -1: none */
+        double       a    = incl - mine;
+        int          pick = i0;
+        if (k <= 64) {
+            pick += u < a + (double) two.x ? 0 : 1;
+        } else {
+#pragma unroll 1
+            for (; pick < min(i0 + per, k) - 1; pick++) {
+                a += (double) q[pick];
+                if (u < a) {
+                    break;
+                }
+            }
+        }
+        *S_out = S;
+        return from < 0 ? k - 1 : __shfl_sync(0xffffffffu, pick, from);
+    }
+    double S    = 0.0;
+    int    pick = k - 1;
+    if (lane == 0) {
+#pragma unroll 1
+        for (int i0 = 0; i0 < k; i0 += 8) { /* eight weights per round: their loads overlap, the sum keeps its order */
+            float w8[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                w8[i] = i0 + i < k ? q[i0 + i] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                S += (double) w8[i]; /* adding +0 behind the last weight changes nothing */
+            }
+        }
+        const double u = (double) u01 * S;
+        double       a = 0.0;
+#pragma unroll 1
+        for (int i = 0; i < k; i++) {
+            a += (double) q[i];
+            if (u < a) {
+                pick = i;
+                break;
+            }
+        }
+    }
+    *S_out = __shfl_sync(0xffffffffu, S, 0);
+    return __shfl_sync(0xffffffffu, pick, 0);
+}
+
 /* ---------------------------------------------------------------- finisher -- */
 
 /*
@@ -1534,29 +1600,33 @@ __device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int to
  * room for the merged list. Returns the row's status bits (ST_DEFERRED: the multi-pass path has to serve it).
  */
 template <bool kFast>
-__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, unsigned char *cmem) {
+__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, int n_parts, unsigned char *cmem) {
     const int  row     = r.row;
     int       *kept_i  = p.kept_cap > 0 ? p.kept_idx + (size_t) row * (size_t) p.kept_cap : nullptr;
     float     *kept_v  = p.kept_cap > 0 ? p.kept_val + (size_t) row * (size_t) p.kept_cap : nullptr;
     Pair      *cbuf    = reinterpret_cast<Pair *>(cmem);
     GroupShared *gs    = &sh->gs;
-    const int  b_first = cta_of_item(p, row * p.n_slices);
-    const int  b_last  = cta_of_item(p, row * p.n_slices + p.n_slices - 1);
-    const int  n_parts = b_last - b_first + 1;
     int        st      = 0;
 
     g.sync(); /* the staging of the row before is no longer read */
-    if (!kFast && g.tid == 0) {
+    if (g.tid == 0) {
         sh->wide_S = 0.0;
+        sh->n_sel  = 0;
     }
+    sh->bhist[g.tid] = 0;
+    static_assert(kHistBins == kThreads, "a bin per thread");
     int st_log = kStageLog; /* words of a part that are staged */
     while ((n_parts << st_log) > kStageWords && st_log > 2) {
         st_log--;
     }
     const int st_parts = min(n_parts, kStageWords >> st_log), st_cand = (1 << st_log) - 4;
+    constexpr int      kOwnWords = kStageWords / kThreads;
+    unsigned long long tv[kOwnWords];
+    const bool         by_segs = !kFast && r.mode == M_TEMP && p.n_slices * kWarps <= kThreads; /* a segment per thread: asked for with the records */
+    float              seg_ref = 0.0f;
+    double             seg_sum = 0.0;
     {
         /* one round trip: the records and the first candidates of the parts, whatever their counts are */
-        unsigned long long tv[kStageWords / kThreads];
 #pragma unroll
         for (int q = 0; q < kStageWords / kThreads; q++) {
             const int t = g.tid + q * kThreads, k = t >> st_log, i = t & ((1 << st_log) - 1);
@@ -1567,6 +1637,11 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             if (q * kThreads < st_parts << st_log) {
                 sh->stage[g.tid + q * kThreads] = tv[q];
             }
+        }
+        if (by_segs && g.tid < p.n_slices * kWarps) {
+            const SegRec *seg = p.segs + (size_t) row * (size_t) (p.n_slices * kWarps) + g.tid;
+            seg_ref           = __ldcg(&seg->ref);
+            seg_sum           = __ldcg(&seg->sum);
         }
     }
     g.sync();
@@ -1608,51 +1683,56 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         g.sync();
         return st | ST_DEFERRED;
     }
-    if (g.tid < n_parts) {
-        int4 h, h2;
-        if (g.tid < st_parts) { /* the record came in with the part's first slots */
-            h  = *reinterpret_cast<const int4 *>(&sh->stage[g.tid << st_log]);
-            h2 = *reinterpret_cast<const int4 *>(&sh->stage[(g.tid << st_log) + 2]);
-        } else {
-            const int4 *rec = part_rec(p, row, g.tid);
-            h               = __ldcg(rec);
-            h2              = __ldcg(rec + 1);
+    /* The parts' records, two per lane, by every warp for itself: one after the other they took a microsecond of a row of
+     * sixteen parts. Rows of up to kMaxParts parts have all their records among the staged words. */
+    static_assert(kMaxParts == 64 && kStageWords >> 4 == kMaxParts, "two parts per lane, their records are staged");
+    unsigned max_key = 0u, tau_key = 0u;
+    int      row_arg = 0x7fffffff, others = 0;
+    bool     overflow = false;
+    {
+        int args[2], more[2];
+        unsigned keys[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int part = g.lane + 32 * h;
+            keys[h]        = 0u;
+            args[h]        = 0x7fffffff;
+            more[h]        = 0;
+            if (part < n_parts) {
+                const int4 a = *reinterpret_cast<const int4 *>(&sh->stage[part << st_log]), b = *reinterpret_cast<const int4 *>(&sh->stage[(part << st_log) + 2]);
+                keys[h] = order_key(__int_as_float(a.x));
+                args[h] = a.y;
+                overflow |= a.z > kPartCand;
+                more[h] = max(0, min(a.z, kPartCand + 1) - st_cand); /* what is not staged */
+                st |= a.w;
+                tau_key = max(tau_key, order_key(__int_as_float(b.x)));
+            }
         }
-        sh->pmax[g.tid]  = __int_as_float(h.x);
-        sh->parg[g.tid]  = h.y;
-        sh->pn[g.tid]    = h.z;
-        sh->ptau[g.tid]  = __int_as_float(h2.x);
-        sh->pbref[g.tid] = __int_as_float(h2.y);
-        sh->pbsum[g.tid] = __hiloint2double(h2.w, h2.z);
-        st |= h.w;
-    }
-    st = __reduce_or_sync(0xffffffffu, st);
-    if (g.lane == 0) {
-        gs->wred_a[g.warp] = st;
-    }
-    g.sync();
-    PROF(9);
-    for (int w = 0; w < g.nw; w++) {
-        st |= gs->wred_a[w];
-    }
-    float row_max  = -CUDART_INF_F, tau_row = -CUDART_INF_F;
-    int   row_arg  = 0x7fffffff;
-    int   others   = 0;
-    bool  overflow = false;
-    for (int i = 0; i < n_parts; i++) {
-        const float m = sh->pmax[i];
-        const int   a = sh->parg[i];
-        if (pair_before(m, a, row_max, row_arg)) { /* rows that are not greedy carry no id: the plain maximum */
-            row_max = m;
-            row_arg = a;
+        max_key  = __reduce_max_sync(0xffffffffu, max(keys[0], keys[1]));
+        row_arg  = __reduce_min_sync(0xffffffffu, min(keys[0] == max_key ? args[0] : 0x7fffffff, keys[1] == max_key ? args[1] : 0x7fffffff)); /* rows that are not greedy carry no id */
+        st       = __reduce_or_sync(0xffffffffu, st);
+        overflow = __any_sync(0xffffffffu, overflow);
+        if (r.mode == M_TOPK || r.mode == M_TOPP) {
+            tau_key = __reduce_max_sync(0xffffffffu, tau_key);
+            others  = __reduce_add_sync(0xffffffffu, more[0] + more[1]);
+            if (others > 0 && g.warp == 0) { /* for the passes over candidates that are not staged */
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    int upto = more[h];
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int up = __shfl_up_sync(0xffffffffu, upto, o);
+                        upto += g.lane >= o ? up : 0;
+                    }
+                    const int base = h == 0 ? 0 : __reduce_add_sync(0xffffffffu, more[0]);
+                    if (g.lane + 32 * h < n_parts) {
+                        sh->poff[g.lane + 32 * h] = base + upto - more[h];
+                    }
+                }
+            }
         }
-        tau_row = fmaxf(tau_row, sh->ptau[i]);
-        overflow |= sh->pn[i] > kPartCand;
-        if (g.tid == 0) {
-            sh->poff[i] = others;
-        }
-        others += max(0, min(sh->pn[i], kPartCand + 1) - (i < st_parts ? st_cand : 0)); /* what is not staged */
     }
+    const float row_max = key_to_float(max_key), tau_row = key_to_float(tau_key);
 
     if (r.mode == M_ARGMAX) {
         if (g.tid == 0) {
@@ -1681,7 +1761,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         double u, fbase = -CUDART_INF; /* nothing crosses: the walk ends on its last id */
         if (nseg <= kThreads) {
             /* a segment per thread: its sum is read and moved once, the scan's total is the row's sum */
-            const double val  = g.tid < nseg ? seg_at(g.tid) : 0.0;
+            const double val  = g.tid < nseg ? seg_sum * ref_move(seg_ref, row_max, r.inv_t) : 0.0;
             double       incl = val;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1694,7 +1774,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 gs->wred_d[g.warp] = incl;
             }
             if (g.tid == 0) {
-                gs->pick = 0x7fffffff;
+                gs->pick = -1;
             }
             g.sync();
             double S = 0.0, woff = 0.0;
@@ -1703,17 +1783,15 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 woff = w == g.warp ? S : woff;
                 S += gs->wred_d[w];
             }
-            incl += woff;
             u = (double) unit_from(xorshift_next(r.rng)) * S;
-            if (g.tid < nseg && u < incl) {
-                atomicMin(&gs->pick, g.tid);
+            /* the first segment whose end lies beyond u: every warp knows whether it lies in one before */
+            const unsigned over = __ballot_sync(0xffffffffu, g.tid < nseg && u < incl + woff);
+            if (over != 0u && (g.warp == 0 || !(u < woff)) && g.lane == __ffs(over) - 1) {
+                gs->pick = g.tid;
+                gs->S    = incl + woff - val;
             }
             g.sync();
-            found = gs->pick == 0x7fffffff ? -1 : gs->pick;
-            if (g.tid == found) {
-                gs->S = incl - val;
-            }
-            g.sync();
+            found = gs->pick;
             fbase = found >= 0 ? gs->S : fbase;
         } else {
             double part = 0.0;
@@ -1862,8 +1940,113 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     }
     /* ---- top-k and top-p: merge the parts' candidates ---- */
     bool need_multipass = !(r.kq > 0 && r.kq <= kFastKMax) || overflow; /* what counts is how many stay above the row's threshold: checked below */
-    if (!need_multipass) {
-        const bool keep_all = r.mode == M_TOPP; /* every marked entry was left out of the bulk sums */
+    const bool keep_all = r.mode == M_TOPP; /* every marked entry was left out of the bulk sums */
+    const float u01     = unit_from(xorshift_next(r.rng)); /* the row's draw */
+    bool        ordered = false; /* the kq best lie in fsort (top-k: their weights in fq) */
+    if (!need_multipass && others == 0) {
+        /* All candidates came in with the records, four words per thread. Those that cannot be among the kq best, by the bins
+         * their values fall into, are dropped where they are; the rest is ranked. Bound by latency: three barriers and a dozen
+         * shared-memory round trips. From the records to the token, one row of 128256 in 16 parts, top-k 40: 8.0 -> 5.1 us (the
+         * parts one after the other, lists written and read between the steps, one thread over the weights); 64 x 32000 top-k 40
+         * in 4 parts each 18.0 -> 14.0 us a pass, 4 x 128256 top-p 19.0 -> 14.9. */
+        const float range = row_max - tau_row, scale = row_max > tau_row && range < CUDART_INF_F ? (float) kHistBins / range : 0.0f;
+        int         bin[kOwnWords]; /* -1: nothing to keep */
+        float       v[kOwnWords];
+        double      part = 0.0;
+#pragma unroll
+        for (int q = 0; q < kOwnWords; q++) {
+            const int t = g.tid + q * kThreads, k = t >> st_log, i = (t & ((1 << st_log) - 1)) - 4;
+            const int held = k < n_parts ? (int) (unsigned) sh->stage[(k << st_log) + 1] : 0;
+            v[q]   = __uint_as_float((unsigned) tv[q]);
+            bin[q] = i >= 0 && i < held && (keep_all || v[q] >= tau_row) ? min(kHistBins - 1, max(0, __float2int_rz((v[q] - tau_row) * scale))) : -1;
+            if (bin[q] >= 0) {
+                atomicAdd(&sh->bhist[bin[q]], 1);
+            }
+        }
+        if constexpr (!kFast) {
+            if (r.mode == M_TOPP) { /* the candidates' weights, exact, and what the parts added up of the rest */
+#pragma unroll 1
+                for (int q = 0; q < kOwnWords; q++) {
+                    const bool one = bin[q] >= 0;
+                    if (__any_sync(0xffffffffu, one)) {
+                        const float e = exp_exact(scaled_arg(v[q], row_max, r.inv_t));
+                        v[q]          = e;
+                        part += one ? (double) e : 0.0;
+                    }
+                }
+                if (g.tid < n_parts) {
+                    const unsigned long long *rec = &sh->stage[(g.tid << st_log) + 2];
+                    part += ref_move(__uint_as_float((unsigned) (rec[0] >> 32)), row_max, r.inv_t) * __longlong_as_double((long long) rec[1]);
+                }
+                part = warp_sum_d(part);
+                if (g.lane == 0) {
+                    gs->wred_d[g.warp] = part;
+                }
+            }
+        }
+        g.sync();
+        const int few_min = top_bin(sh->bhist, g.lane, r.kq);
+        double    S       = 0.0;
+        if constexpr (!kFast) {
+            if (r.mode == M_TOPP) {
+#pragma unroll
+                for (int w = 0; w < kWarps; w++) {
+                    S += gs->wred_d[w];
+                }
+                if (g.tid == 0) {
+                    sh->wide_S = S;
+                }
+            }
+        }
+        unsigned in[kOwnWords];
+        int      mine = 0;
+#pragma unroll
+        for (int q = 0; q < kOwnWords; q++) {
+            in[q] = __ballot_sync(0xffffffffu, bin[q] >= 0 && bin[q] >= few_min);
+            mine += __popc(in[q]);
+        }
+        int at = g.lane == 0 && mine > 0 ? atomicAdd(&sh->n_sel, mine) : 0;
+        at     = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+        for (int q = 0; q < kOwnWords; q++) {
+            const int pos = at + __popc(in[q] & ((1u << g.lane) - 1u));
+            if (((in[q] >> g.lane) & 1u) != 0u && pos < kRankAll) {
+                cbuf[pos] = Pair{!kFast && r.mode == M_TOPP ? __double2float_rn((double) v[q] / S) : v[q], (int) (tv[q] >> 32)}; /* top-p: p_i as the reference normalises it */
+            }
+            at += __popc(in[q]);
+        }
+        g.sync();
+        const int n = sh->n_sel;
+        if (n >= r.kq && n <= kRankAll) {
+            if (n <= kRankFew) {
+                if (r.mode == M_TOPK && !r.select_only) {
+                    rank_few<true>(cbuf, n, r.kq, r.inv_t, sh->fsort, sh->fq);
+                } else {
+                    rank_few<false>(cbuf, n, r.kq, r.inv_t, sh->fsort, sh->fq);
+                }
+                g.sync();
+            } else {
+#pragma unroll 1
+                for (int i = g.tid; i < n; i += g.n) {
+                    const Pair me   = cbuf[i];
+                    int        rank = 0;
+#pragma unroll 4
+                    for (int j = 0; j < n; j++) {
+                        rank += pair_before(cbuf[j].v, cbuf[j].idx, me.v, me.idx) ? 1 : 0;
+                    }
+                    if (rank < r.kq) {
+                        sh->fsort[rank] = me;
+                        if (r.mode == M_TOPK) {
+                            sh->fq[rank] = exp_exact(scaled_arg(me.v, row_max, r.inv_t));
+                        }
+                    }
+                }
+                g.sync();
+            }
+            ordered = true;
+        }
+    }
+    if (!need_multipass && !ordered) {
         /* The candidates of all parts are merged in up to three passes of one rolled loop. The first keeps what
          * passes the row's threshold (the largest of the parts' thresholds). A row cut into many parts can have far
          * more of those than k (every part kept at least k of its own): if they do not fit, a second pass bins them
@@ -1913,7 +2096,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
 #pragma unroll 1
             for (int t0 = 0; t0 < st_parts << st_log; t0 += kThreads) {
                 const int                t = t0 + g.tid, k = t >> st_log, i = (t & ((1 << st_log) - 1)) - 4;
-                const bool               ok = k < st_parts && i >= 0 && i < sh->pn[k];
+                const bool               ok = k < st_parts && i >= 0 && i < (int) (unsigned) sh->stage[(min(k, st_parts - 1) << st_log) + 1];
                 const unsigned long long w  = ok ? sh->stage[t] : 0ull;
                 place(ok, Pair{__uint_as_float((unsigned) w), (int) (w >> 32)});
             }
@@ -1992,7 +2175,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         auto  is_few = [&](float v) { return min(kHistBins - 1, max(0, __float2int_rz((v - tau_row) * few_scale))) >= few_min; };
         static_assert((kFinCap + kRankAll) * (int) sizeof(Pair) <= kFinBytes, "the second list fits");
         if (!need_multipass && r.mode == M_TOPK) {
-            const int   k    = r.k;
+            const int   k         = r.k;
             const Pair *rank_from = cbuf;
             int         n_rank    = total;
             if (few_min >= 0) {
@@ -2032,99 +2215,18 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 g.sync(); /* n_sel is used again */
                 select_sorted(g, sh, cbuf, total, k, sh->fsort);
             }
-            PROF(11);
-            if (r.select_only) {
-                for (int i = g.tid; i < min(k, p.kept_cap); i += g.n) {
-                    kept_i[i] = sh->fsort[i].idx + p.vocab_offset;
-                    kept_v[i] = sh->fsort[i].v;
-                }
-                if (g.tid == 0) {
-                    p.kept_n[row] = k;
-                    p.tokens[row] = sh->fsort[0].idx + p.vocab_offset;
+            /* sampler.c:217-222: softmax over the k kept logits (max = the first) */
+            if (!r.select_only) {
+                const float m = sh->fsort[0].v;
+                for (int i = g.tid; i < k; i += g.n) {
+                    sh->fq[i] = exp_exact(scaled_arg(sh->fsort[i].v, m, r.inv_t));
                 }
                 g.sync();
-                return st;
             }
-            /* sampler.c:217-222: softmax over the k kept logits (max = the first), one draw */
-            const float m = sh->fsort[0].v;
-            for (int i = g.tid; i < k; i += g.n) {
-                sh->fq[i] = exp_exact(scaled_arg(sh->fsort[i].v, m, r.inv_t));
-            }
-            g.sync();
-            PROF(12);
-            if (k <= 64) {
-                if (g.tid == 0) { /* sampler.c:90-102 as it stands: the sum and the walk in the reference's order, by one thread */
-                    double S = 0.0;
-#pragma unroll 1
-                    for (int i0 = 0; i0 < k; i0 += 8) { /* eight weights per round: their loads overlap, the sum keeps its order */
-                        float w8[8];
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            w8[q] = i0 + q < k ? sh->fq[i0 + q] : 0.0f;
-                        }
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            S += (double) w8[q]; /* adding +0 behind the last weight changes nothing */
-                        }
-                    }
-                    const double u    = (double) unit_from(xorshift_next(r.rng)) * S;
-                    double       a    = 0.0;
-                    int          pick = k - 1;
-#pragma unroll 1
-                    for (int i0 = 0; i0 < k; i0 += 8) {
-                        float w8[8];
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            w8[q] = i0 + q < k ? sh->fq[i0 + q] : 0.0f;
-                        }
-                        double pre[8]; /* the running sums behind each of the eight, in walk order */
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            a += (double) w8[q];
-                            pre[q] = a;
-                        }
-                        int first = 8;
-#pragma unroll
-                        for (int q = 7; q >= 0; q--) {
-                            if (u < pre[q] && i0 + q < k) {
-                                first = q;
-                            }
-                        }
-                        if (first < 8) {
-                            pick = i0 + first;
-                            break;
-                        }
-                    }
-                    p.tokens[row] = sh->fsort[pick].idx + p.vocab_offset;
-                    gs->S         = S;
-                    if (p.kept_cap > 0) {
-                        p.kept_n[row] = k;
-                    }
-                }
-            } else if (g.warp == 0) {
-                double    S;
-                const int pick = warp_inverse_cdf(g.lane, sh->fq, k, unit_from(xorshift_next(r.rng)), &S);
-                if (g.lane == 0) {
-                    p.tokens[row] = sh->fsort[pick].idx + p.vocab_offset;
-                    gs->S         = S;
-                    if (p.kept_cap > 0) {
-                        p.kept_n[row] = k;
-                    }
-                }
-            }
-            if (p.kept_cap > 0) {
-                g.sync();
-                const double S = gs->S;
-                for (int i = g.tid; i < min(k, p.kept_cap); i += g.n) {
-                    kept_i[i] = sh->fsort[i].idx + p.vocab_offset;
-                    kept_v[i] = __double2float_rn((double) sh->fq[i] / S);
-                }
-            }
-            g.sync();
-            return st;
+            ordered = true;
         }
         if constexpr (!kFast) {
-        if (!need_multipass) {
+        if (!need_multipass && r.mode == M_TOPP) {
             /* top-p over a small nucleus (sampler.c:245-300). Candidates get their exact e_i relative to the row
              * maximum; the rest of the row was summed per part relative to the part's own maximum and is
              * rescaled here. */
@@ -2142,7 +2244,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 }
             }
             if (g.tid < n_parts) {
-                part += ref_move(sh->pbref[g.tid], row_max, r.inv_t) * sh->pbsum[g.tid];
+                const unsigned long long *rec = &sh->stage[(g.tid << st_log) + 2];
+                part += ref_move(__uint_as_float((unsigned) (rec[0] >> 32)), row_max, r.inv_t) * __longlong_as_double((long long) rec[1]);
             }
             const double S = group_sum_d(g, gs, part);
             if (g.tid == 0) {
@@ -2150,7 +2253,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             }
             /* the walk order is (p desc, id asc); the row's kq most probable ids are all candidates. Whatever is left out
              * here has a smaller value than the kq-th, so no larger p. */
-            const int   kq        = min(r.kq, total);
+            const int   kq        = r.kq;
             const bool  by_few    = few_min >= 0 && sh->n_sel <= kRankAll; /* read behind the sum's barriers */
             Pair       *rank_from = by_few ? few : cbuf;
             const int   n_rank    = by_few ? sh->n_sel : total;
@@ -2175,6 +2278,50 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             } else {
                 select_sorted(g, sh, cbuf, total, kq, sh->fsort);
             }
+            ordered = true;
+        }
+        }
+    }
+    if (ordered && r.mode == M_TOPK) {
+        PROF(11);
+        const int k = r.k;
+        if (r.select_only) {
+            for (int i = g.tid; i < min(k, p.kept_cap); i += g.n) {
+                kept_i[i] = sh->fsort[i].idx + p.vocab_offset;
+                kept_v[i] = sh->fsort[i].v;
+            }
+            if (g.tid == 0) {
+                p.kept_n[row] = k;
+                p.tokens[row] = sh->fsort[0].idx + p.vocab_offset;
+            }
+            g.sync();
+            return st;
+        }
+        if (g.warp == 0) { /* one draw */
+            double    S;
+            const int pick = draw_sorted(g.lane, sh->fq, k, u01, &S);
+            if (g.lane == 0) {
+                p.tokens[row] = sh->fsort[pick].idx + p.vocab_offset;
+                gs->S         = S;
+                if (p.kept_cap > 0) {
+                    p.kept_n[row] = k;
+                }
+            }
+        }
+        if (p.kept_cap > 0) {
+            g.sync();
+            const double S = gs->S;
+            for (int i = g.tid; i < min(k, p.kept_cap); i += g.n) {
+                kept_i[i] = sh->fsort[i].idx + p.vocab_offset;
+                kept_v[i] = __double2float_rn((double) sh->fq[i] / S);
+            }
+        }
+        g.sync();
+        return st;
+    }
+    if constexpr (!kFast) {
+        if (ordered) {
+            const int kq = r.kq;
             /* The walks over the kq entries, one per lane of a warp. Their running sums are exact wherever no entry is smaller
              * than 2^-29, so the order of additions is not seen; one thread that adds them one by one, three times over,
              * took 4 us of a row's 15. */
@@ -2201,7 +2348,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                         atomicAdd(&p.wide_head->rows, 1ull); /* the row is not wide: said as early as it is known */
                     }
                     const double   N    = __shfl_sync(0xffffffffu, cum, cut - 1);
-                    const double   u    = (double) unit_from(xorshift_next(r.rng)) * N;
+                    const double   u    = (double) u01 * N;
                     const unsigned over = __ballot_sync(0xffffffffu, g.lane < cut && u < cum);
                     const int      pick = over != 0u ? __ffs(over) - 1 : cut - 1;
                     if (g.lane == pick) {
@@ -2225,7 +2372,6 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             if (gs->flag) {
                 return st;
             }
-        }
         }
     }
     g.sync();
@@ -2315,112 +2461,6 @@ __device__ __forceinline__ unsigned kth_key(unsigned key0, unsigned key1, bool t
         lo = key;
         hi = min(hi, key + ((1u << shift) - 1u));
     }
-}
-
-/* At most kRankFew candidates in order, the k best to out_s, their weights e^((x - max) / T) to out_q. Four threads (two beyond
- * 64 candidates) compare a candidate with a share of the others each, eight at a time without a branch between them.
- * All threads call; the caller's barrier follows. */
-constexpr int kRankFew = 128;
-static_assert(2 * kRankFew == kThreads, "two threads per candidate");
-__device__ __forceinline__ void rank_few(const Pair *cand, int total, int k, float inv_t, Pair *out_s, float *out_q) {
-    const int  log = total <= kRankFew / 2 ? 2 : 1, i = (int) threadIdx.x >> log, step = 1 << log, sub = (int) threadIdx.x & (step - 1);
-    const Pair me   = cand[min(i, total - 1)];
-    int        rank = 0;
-    float      top  = -CUDART_INF_F;
-#pragma unroll 1
-    for (int j0 = sub; j0 < total; j0 += 8 * step) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const Pair o = cand[min(j0 + j * step, total - 1)];
-            rank += j0 + j * step < total && pair_before(o.v, o.idx, me.v, me.idx) ? 1 : 0;
-            top = fmaxf(top, o.v);
-        }
-    }
-    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
-    if (log == 2) {
-        rank += __shfl_xor_sync(0xffffffffu, rank, 2);
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-    }
-    if (sub == 0 && i < total && rank < k) {
-        out_s[rank] = me;
-        out_q[rank] = exp_exact(scaled_arg(me.v, top, inv_t));
-    }
-}
-
-/*
- * The reference's draw over k <= 256 weights in descending order (sampler.c:90-102): the sum and the walk in its order, in
- * double. Where the smallest weight is at least 2^-22 every partial sum is a whole number of 2^-45 below 2^53 of them, so
- * exact in any order, and the warp adds in parallel; else one lane adds one by one. The whole warp calls: the place that
- * u01 times the sum falls on, and the sum. (Between the candidates and the token of one row, top-k 40: 1.9 us with a thread per
- * candidate to rank them, the exponentials behind a barrier and one thread over the weights, twice; 1.25 us.)
- */
-__device__ __forceinline__ int draw_sorted(int lane, const float *q, int k, float u01, double *S_out) {
-    const float2 two = 2 * lane < k ? *reinterpret_cast<const float2 *>(q + 2 * lane) : make_float2(0.0f, 0.0f); /* what lies behind the k-th weight is not used */
-    if (q[k - 1] >= 0x1p-22f) {
-        const int per  = k <= 64 ? 2 : (k + 31) >> 5, i0 = lane * per;
-        double    incl = (double) two.x + (2 * lane + 1 < k ? (double) two.y : 0.0);
-        if (k > 64) {
-            incl = 0.0;
-#pragma unroll 1
-            for (int i = i0; i < min(i0 + per, k); i++) {
-                incl += (double) q[i];
-            }
-        }
-        const double mine = incl;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double up = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) {
-                incl += up;
-            }
-        }
-        const double S = __shfl_sync(0xffffffffu, incl, 31), u = (double) u01 * S;
-        const int    from = __ffs(__ballot_sync(0xffffffffu, u < incl)) - 1; /* the lane whose run crosses u, -1: none */
-        double       a    = incl - mine;
-        int          pick = i0;
-        if (k <= 64) {
-            pick += u < a + (double) two.x ? 0 : 1;
-        } else {
-#pragma unroll 1
-            for (; pick < min(i0 + per, k) - 1; pick++) {
-                a += (double) q[pick];
-                if (u < a) {
-                    break;
-                }
-            }
-        }
-        *S_out = S;
-        return from < 0 ? k - 1 : __shfl_sync(0xffffffffu, pick, from);
-    }
-    double S    = 0.0;
-    int    pick = k - 1;
-    if (lane == 0) {
-#pragma unroll 1
-        for (int i0 = 0; i0 < k; i0 += 8) { /* eight weights per round: their loads overlap, the sum keeps its order */
-            float w8[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                w8[i] = i0 + i < k ? q[i0 + i] : 0.0f;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                S += (double) w8[i]; /* adding +0 behind the last weight changes nothing */
-            }
-        }
-        const double u = (double) u01 * S;
-        double       a = 0.0;
-#pragma unroll 1
-        for (int i = 0; i < k; i++) {
-            a += (double) q[i];
-            if (u < a) {
-                pick = i;
-                break;
-            }
-        }
-    }
-    *S_out = __shfl_sync(0xffffffffu, S, 0);
-    return __shfl_sync(0xffffffffu, pick, 0);
 }
 
 /* The part's maximum, as its candidates are. */
@@ -2643,7 +2683,7 @@ __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, Stream
     }
     if (ok) {
         if (total <= kRankFew) {
-            rank_few(sh->cand, total, k, inv_t, sh->fin_s, sh->fin_q);
+            rank_few<true>(sh->cand, total, k, inv_t, sh->fin_s, sh->fin_q);
         } else {
             rank_in_bins(sh, gmem, total, k, lo, cap_late);
             __syncthreads();
@@ -3807,9 +3847,22 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     g.bar  = 0;
     /* The first row's parameters are inputs of the launch, written before the stream kernel began: they may be
      * read while that kernel's last thread blocks are still at work. Everything it wrote waits for the line below. */
-    RawCfg rc0{};
+    auto parts_of = [&](int row) { return cta_of_item(p, row * p.n_slices + p.n_slices - 1) - cta_of_item(p, row * p.n_slices) + 1; };
+    RawCfg rc{};
+    RowCfg r{};
+    int    n_parts = 0;
+    auto   configure = [&](int row) {
+        rc = raw_config(p, row, true);
+        r  = row_config(p, row, rc, true);
+        if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
+            r.cap    = 0.0f;
+            r.mrow   = nullptr;
+            r.pen_on = false;
+        }
+        n_parts = parts_of(row);
+    };
     if ((int) blockIdx.x < p.n_rows) {
-        rc0 = raw_config(p, (int) blockIdx.x, true);
+        configure((int) blockIdx.x);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory"); /* the records of the kernel before this one are complete and visible */
     asm volatile("griddepcontrol.launch_dependents;");
@@ -3817,12 +3870,8 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     /* the launch has top-p rows: the stream kernel has said so; wanted when the block's own rows are done */
     const bool any = !kFast && *reinterpret_cast<volatile const unsigned *>(&p.wide_head->any) == p.launch;
     for (int row = (int) blockIdx.x; row < p.n_rows; row += (int) gridDim.x) {
-        const RawCfg rc = row == (int) blockIdx.x ? rc0 : raw_config(p, row, true);
-        RowCfg       r  = row_config(p, row, rc, true);
-        if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
-            r.cap    = 0.0f;
-            r.mrow   = nullptr;
-            r.pen_on = false;
+        if (row != (int) blockIdx.x) {
+            configure(row);
         }
         PROF(8);
         if constexpr (!kFast) {
@@ -3830,7 +3879,7 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
                 atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
             }
         }
-        int          st = finish_row<kFast>(g, p, sh, r, cmem);
+        int st = finish_row<kFast>(g, p, sh, r, n_parts, cmem);
         PROF(13);
         if (st & ST_DEFERRED) {
             if constexpr (kFast) {

@@ -85,3 +85,39 @@ def test_fed_tokens_behind_a_history(ctx, H):
         st = independent_states(oracle.port, H, S)
         g = run_gpu(ctx, x, 0.9, 40, 1.0, st, rows_per_seq=R, rep=1.1, history=h, history_len=n, fed=fed)
         check_tokens(g, oracle.port.sample_batch(x, 0.9, 40, 1.0, st, rows_per_seq=R, rep=1.1, hist=h, hist_len=n, extra=fed))
+
+
+@pytest.mark.parametrize("k", [2, 50, 100, 129, 200, 256])
+@pytest.mark.parametrize("rows,V", [(1, 60001), (5, 60000), (70, 30000), (2, 262144)])
+def test_candidates_of_parts_merged(ctx, rows, V, k):
+    """Rows cut into parts: all candidates among the staged words and ranked (up to 128 of them, up to 220, more), more than were
+    staged, and values on a grid, whose ties at the last place outrun the few; kept sets and their probabilities."""
+    x = normal_logits(rows, V, 2.5, V + k)
+    x[1::3] = np.round(x[1::3] * 16) / 16
+    st = independent_states(oracle.port, V + k, rows)
+    o = oracle.port.sample_batch(x, 3.0, k, 1.0, st, detail_cap=k)
+    for hint in (0, 1):
+        g = run_gpu(ctx, x, 3.0, k, 1.0, st, kept_cap=k, finish_hint=hint)
+        assert (g["status"] & 32 == 0).all()
+        check_tokens(g, o)
+        full = (g["status"] & 8) == 0  # not by the multi-pass path
+        assert np.array_equal(g["kept_idx"][full], o["detail_idx"][full])
+        np.testing.assert_allclose(g["kept_prob"][full], o["detail_prob"][full], rtol=1e-5)
+
+
+@pytest.mark.parametrize("rows,V", [(3, 60001), (70, 30000), (300, 5000)])
+def test_narrow_nuclei_and_temperature_of_parts(ctx, rows, V):
+    """Top-p rows served from the candidates, equal values at the nucleus's edge among them; temperature rows whose draw falls
+    into every segment, segments of weight 0 and rows of more segments than a thread block has threads among them."""
+    from helpers import gumbel_logits
+    st = independent_states(oracle.port, V, rows)
+    x = gumbel_logits(rows, V, 4.0, V)
+    x[1::3] = np.round(x[1::3])
+    check_tokens(run_gpu(ctx, x, 0.8, 0, 0.9, st), oracle.port.sample_batch(x, 0.8, 0, 0.9, st))
+    y = normal_logits(rows, V, 2.0, V)
+    y[1::3, : V // 2] = -np.inf
+    y[2::3, V // 3:] -= 200.0
+    check_tokens(run_gpu(ctx, y, 1.0, 0, 1.0, st), oracle.port.sample_batch(y, 1.0, 0, 1.0, st))
+    if rows < 10:
+        z = normal_logits(rows, 300000, 2.0, V)
+        check_tokens(run_gpu(ctx, z, 1.0, 0, 1.0, st), oracle.port.sample_batch(z, 1.0, 0, 1.0, st))

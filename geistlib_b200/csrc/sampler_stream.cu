@@ -1279,9 +1279,9 @@ struct __align__(16) StreamShared {
 };
 
 /* What comes in of every part in one round trip, before its count of candidates is known: its record and the first
- * candidates behind it, 2^kStageLog words of 8 bytes of rows of up to eight parts, half of that up to sixteen and so on. */
+ * candidates behind it, kStageWords words of 8 bytes shared out over the parts, an even number each and no more than kStageMost. */
 constexpr int kStageWords = 1024;
-constexpr int kStageLog   = 7;
+constexpr int kStageMost  = 128;
 
 /* What the threads of one finishing thread block share; the merged candidate list lies behind it. */
 struct __align__(16) FinishShared {
@@ -1295,18 +1295,17 @@ struct __align__(16) FinishShared {
     PenEntry    fdlist[512];
     alignas(16) unsigned long long stage[kStageWords]; /* the records and first candidates of the row's parts */
     unsigned long long save[256 + 128];                      /* the multi-pass path keeps a histogram here */
+    RowCfg      cfg;    /* the row's: in registers it had left none for the code that finishes it */
     double      wide_S; /* a top-p row that the candidates could not serve: its sum, 0 where it is not known */
 };
 
 constexpr int kGroupBytes = kGroupSlots * kThreads * 4; /* one maximum per slot and thread */
 constexpr int kListSmem   = kRowIdsMax;       /* id-list entries of a part that are kept in shared memory */
 constexpr int kFinCap     = 2048;             /* candidates the finisher can order per row (8 per thread) */
-constexpr int kFinPer     = kFinCap / kThreads;
-constexpr int kRankAll    = 220;              /* up to this many candidates the finisher ranks one against all (220 against 384, us: 1000 x 16384 top-k 128 79.5 -> 71.7,
-                                               * top-k 200 97.9 -> 88.0; 64 x 128256 top-k 64 30.4 -> 23.4; against 128: 8 x 128256 top-k 128 46.1 -> 43.9) */
-constexpr int kFinBytes   = kWarps * 256 * 12;    /* finisher: the merged candidate list; the multi-pass path keeps one byte histogram per warp there */
+static_assert(kPartCand * (int) sizeof(Pair) + 2 * (kHistBins + 1) * 4 <= kGroupBytes, "a part's candidates are put in order there");
+constexpr int kFinBytes   = 2 * kFinCap * (int) sizeof(Pair) + 2 * (kHistBins + 1) * 4 + 8; /* finisher: the merged candidate list, what puts it in order; the multi-pass path keeps one byte histogram per warp there */
+static_assert(kFinBytes >= kWarps * 256 * 12, "a byte histogram per warp fits");
 constexpr int kFinGeneralBytes = sizeof(WideShared) > (size_t) kFinBytes ? (int) sizeof(WideShared) : kFinBytes; /* the general kernel works on wide rows there as well */
-static_assert(kFinCap * (int) sizeof(Pair) <= kFinBytes, "the merged list fits");
 static_assert(kGroupBytes >= 2 * kRowIdsMax * 8, "the id table of a part's set-up lies in the group maxima's memory");
 static_assert(kGroupSlots <= 256 && kThreads == 256, "a group's name fits 16 bits");
 
@@ -1385,102 +1384,6 @@ __device__ __forceinline__ int top_bin(const int *hist, int lane, int kq) {
     return __shfl_sync(0xffffffffu, b, ball != 0u ? 31 - __clz(ball) : 0);
 }
 
-/* ------------------------------------------- finisher: ordered select of kq -- */
-
-/*
- * cand[0..total) hold distinct ids, total >= kq >= 1, total <= kFinCap. Writes the kq best in (value desc, id asc)
- * order to sorted[0..kq). Every thread lifts its entries into registers; a histogram over their key range finds
- * the bin that holds the kq-th entry; entries in higher bins are in, only that one bin is ranked exactly. cand is
- * overwritten. Called by the whole thread block.
- * (The loops that rank say how far they are unrolled: left to the compiler, the general kernel's copy had become slower
- * when the code around it grew, top-k 256 of one row of 1000 28.5 -> 31.9 us; 30.7 so.)
- */
-__device__ void select_sorted(const Grp &g, FinishShared *sh, Pair *cand, int total, int kq, Pair *sorted) {
-    Pair     e[kFinPer];
-    unsigned lo = 0xffffffffu, hi = 0u;
-#pragma unroll
-    for (int i = 0; i < kFinPer; i++) {
-        const int f = g.tid + kThreads * i;
-        if (f < total) {
-            e[i]             = cand[f];
-            const unsigned k = order_key(e[i].v);
-            lo               = min(lo, k);
-            hi               = max(hi, k);
-        }
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    g.sync(); /* earlier readers of the scratch are done; every entry is in a register */
-    if (g.lane == 0) {
-        sh->gs.wred_a[g.warp]                               = (int) lo;
-        reinterpret_cast<unsigned *>(sh->gs.wred_f)[g.warp] = hi;
-    }
-    if (g.tid < kHistBins) {
-        sh->bhist[g.tid] = 0;
-    }
-    if (g.tid == 0) {
-        sh->n_sel    = 0;
-        sh->n_border = 0;
-    }
-    g.sync();
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        lo = min(lo, (unsigned) sh->gs.wred_a[w]);
-        hi = max(hi, reinterpret_cast<unsigned *>(sh->gs.wred_f)[w]);
-    }
-    const unsigned range = hi >= lo ? hi - lo : 0u;
-    const int      shift = max(0, (32 - __clz(range)) - 8); /* (range >> shift) < 256 */
-#pragma unroll
-    for (int i = 0; i < kFinPer; i++) {
-        if (g.tid + kThreads * i < total) {
-            atomicAdd(&sh->bhist[(order_key(e[i].v) - lo) >> shift], 1);
-        }
-    }
-    g.sync();
-    /* b* = largest bin with count(bins >= b*) >= kq; every warp finds it for itself */
-    const int b_star = top_bin(sh->bhist, g.lane, kq);
-    int       n_hi   = 0;
-    for (int b = b_star + 1 + g.lane; b < kHistBins; b += 32) {
-        n_hi += sh->bhist[b];
-    }
-    n_hi = __reduce_add_sync(0xffffffffu, n_hi);
-    /* entries above the bin fill cand from the front, the bin's entries follow */
-#pragma unroll
-    for (int i = 0; i < kFinPer; i++) {
-        if (g.tid + kThreads * i < total) {
-            const int bin = (int) ((order_key(e[i].v) - lo) >> shift);
-            if (bin > b_star) {
-                cand[atomicAdd(&sh->n_sel, 1)] = e[i];
-            } else if (bin == b_star) {
-                cand[n_hi + atomicAdd(&sh->n_border, 1)] = e[i];
-            }
-        }
-    }
-    g.sync();
-    const int nb   = sh->n_border;
-    const int need = kq - n_hi;
-    for (int i = g.tid; i < n_hi + nb; i += g.n) {
-        const Pair me   = cand[i];
-        int        rank = 0;
-        if (i < n_hi) {
-#pragma unroll 8
-            for (int j = 0; j < n_hi; j++) {
-                rank += pair_before(cand[j].v, cand[j].idx, me.v, me.idx) ? 1 : 0;
-            }
-            sorted[rank] = me;
-        } else {
-#pragma unroll 4
-            for (int j = n_hi; j < n_hi + nb; j++) {
-                rank += pair_before(cand[j].v, cand[j].idx, me.v, me.idx) ? 1 : 0;
-            }
-            if (rank < need) {
-                sorted[n_hi + rank] = me;
-            }
-        }
-    }
-    g.sync();
-}
-
 /* ------------------------------------------------------ few candidates, weights -- */
 
 /* At most kRankFew candidates in order, the k best to out_s, with kWeigh their weights e^((x - max) / T) to out_q. Four threads (two beyond
@@ -1513,6 +1416,74 @@ __device__ __forceinline__ void rank_few(const Pair *cand, int total, int k, flo
         out_s[rank] = me;
         if (kWeigh) {
             out_q[rank] = exp_exact(scaled_arg(me.v, top, inv_t));
+        }
+    }
+}
+
+/* More than kRankFew candidates in order, the k best to out_s; they lie between lo and hi. They are dealt out to 256 bins of
+ * values, the highest in front (srt takes them), and ranked against their own bin: one against all costs a thread block
+ * total^2 / 32 rounds of six instructions. 1000 rows of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9;
+ * 256 x 128256 top-k 200 48.9 -> 41.0. by_octave: bins of the values' bits, for probabilities (lo is not used); in even bins all but
+ * a few share the last, and eight top-p rows of 19 parts took 67 us instead of 41. start: room for 2 * (kHistBins + 1) words. All threads call; the caller's barrier follows. */
+__device__ __noinline__ void rank_in_bins(const Pair *in, int total, int k, float lo, float hi, bool by_octave, Pair *srt, int *start, Pair *out_s) {
+    const int   tid = (int) threadIdx.x, lane = tid & 31;
+    int        *next  = start + kHistBins + 1;
+    if (by_octave) {
+        hi = (float) __float_as_int(hi);
+        lo = hi - (float) (20 << 23); /* what is a millionth of the largest or less shares the last bin */
+    }
+    const float scale = hi > lo && hi - lo < CUDART_INF_F ? (float) kHistBins / (hi - lo) : 0.0f; /* 0: one bin for all */
+    auto        bin_of = [&](float v) { return kHistBins - 1 - min(kHistBins - 1, max(0, __float2int_rz(((by_octave ? (float) __float_as_int(v) : v) - lo) * scale))); };
+    for (int i = tid; i <= kHistBins; i += kThreads) {
+        start[i] = 0; /* entry b + 1: candidates in bin b; after the scan, entry b: candidates in the bins before b */
+    }
+    __syncthreads();
+    for (int i = tid; i < total; i += kThreads) {
+        atomicAdd(&start[bin_of(in[i].v) + 1], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int v[kHistBins / 32], run = 0;
+#pragma unroll
+        for (int i = 0; i < kHistBins / 32; i++) {
+            run += start[1 + kHistBins / 32 * lane + i];
+            v[i] = run;
+        }
+        int before = run;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, before, d);
+            if (lane >= d) {
+                before += o;
+            }
+        }
+        before -= run;
+#pragma unroll
+        for (int i = 0; i < kHistBins / 32; i++) {
+            start[1 + kHistBins / 32 * lane + i] = before + v[i];
+            next[1 + kHistBins / 32 * lane + i]  = before + v[i];
+        }
+        if (lane == 0) {
+            next[0] = 0;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < total; i += kThreads) {
+        const Pair me                           = in[i];
+        srt[atomicAdd(&next[bin_of(me.v)], 1)] = me;
+    }
+    __syncthreads();
+    for (int i = tid; i < total; i += kThreads) {
+        const Pair me   = srt[i];
+        const int  b    = bin_of(me.v), end = start[b + 1];
+        int        rank = start[b];
+        if (rank < k) {
+            for (int j = rank; j < end; j++) {
+                rank += pair_before(srt[j].v, srt[j].idx, me.v, me.idx) ? 1 : 0;
+            }
+            if (rank < k) {
+                out_s[rank] = me;
+            }
         }
     }
 }
@@ -1600,8 +1571,10 @@ __device__ __forceinline__ int draw_sorted(int lane, const float *q, int k, floa
  * room for the merged list. Returns the row's status bits (ST_DEFERRED: the multi-pass path has to serve it).
  */
 template <bool kFast>
-__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, RowCfg &r, int n_parts, unsigned char *cmem) {
+__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, int n_parts, unsigned char *cmem) {
+    const RowCfg &r    = sh->cfg;
     const int  row     = r.row;
+    unsigned long long rng = r.rng;
     int       *kept_i  = p.kept_cap > 0 ? p.kept_idx + (size_t) row * (size_t) p.kept_cap : nullptr;
     float     *kept_v  = p.kept_cap > 0 ? p.kept_val + (size_t) row * (size_t) p.kept_cap : nullptr;
     Pair      *cbuf    = reinterpret_cast<Pair *>(cmem);
@@ -1615,11 +1588,13 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     }
     sh->bhist[g.tid] = 0;
     static_assert(kHistBins == kThreads, "a bin per thread");
-    int st_log = kStageLog; /* words of a part that are staged */
-    while ((n_parts << st_log) > kStageWords && st_log > 2) {
-        st_log--;
-    }
-    const int st_parts = min(n_parts, kStageWords >> st_log), st_cand = (1 << st_log) - 4;
+    const int st_parts = min(n_parts, kStageWords / 4), st_w = min(kStageMost, (kStageWords / st_parts) & ~1), st_cand = st_w - 4; /* words of a part that are staged */
+    const float st_rcp = 1.0f / (float) st_w;
+    auto part_of = [&](int t, int &i) { /* which part staged word t is of, and its place behind that part's record */
+        const int k = quotient(t, st_w, st_rcp);
+        i           = t - k * st_w - 4;
+        return k;
+    };
     constexpr int      kOwnWords = kStageWords / kThreads;
     unsigned long long tv[kOwnWords];
     const bool         by_segs = !kFast && r.mode == M_TEMP && p.n_slices * kWarps <= kThreads; /* a segment per thread: asked for with the records */
@@ -1629,12 +1604,13 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         /* one round trip: the records and the first candidates of the parts, whatever their counts are */
 #pragma unroll
         for (int q = 0; q < kStageWords / kThreads; q++) {
-            const int t = g.tid + q * kThreads, k = t >> st_log, i = t & ((1 << st_log) - 1);
-            tv[q]       = q * kThreads < st_parts << st_log && k < st_parts ? __ldcg(reinterpret_cast<const unsigned long long *>(part_rec(p, row, k)) + i) : 0ull;
+            int       i;
+            const int t = g.tid + q * kThreads, k = part_of(t, i);
+            tv[q]       = q * kThreads < st_parts * st_w && k < st_parts ? __ldcg(reinterpret_cast<const unsigned long long *>(part_rec(p, row, k)) + 4 + i) : 0ull;
         }
 #pragma unroll
         for (int q = 0; q < kStageWords / kThreads; q++) {
-            if (q * kThreads < st_parts << st_log) {
+            if (q * kThreads < st_parts * st_w) {
                 sh->stage[g.tid + q * kThreads] = tv[q];
             }
         }
@@ -1685,7 +1661,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     }
     /* The parts' records, two per lane, by every warp for itself: one after the other they took a microsecond of a row of
      * sixteen parts. Rows of up to kMaxParts parts have all their records among the staged words. */
-    static_assert(kMaxParts == 64 && kStageWords >> 4 == kMaxParts, "two parts per lane, their records are staged");
+    static_assert(kMaxParts == 64 && kStageWords / kMaxParts >= 4, "two parts per lane, their records are staged");
     unsigned max_key = 0u, tau_key = 0u;
     int      row_arg = 0x7fffffff, others = 0;
     bool     overflow = false;
@@ -1699,7 +1675,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             args[h]        = 0x7fffffff;
             more[h]        = 0;
             if (part < n_parts) {
-                const int4 a = *reinterpret_cast<const int4 *>(&sh->stage[part << st_log]), b = *reinterpret_cast<const int4 *>(&sh->stage[(part << st_log) + 2]);
+                const int4 a = *reinterpret_cast<const int4 *>(&sh->stage[part * st_w]), b = *reinterpret_cast<const int4 *>(&sh->stage[part * st_w + 2]);
                 keys[h] = order_key(__int_as_float(a.x));
                 args[h] = a.y;
                 overflow |= a.z > kPartCand;
@@ -1783,7 +1759,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 woff = w == g.warp ? S : woff;
                 S += gs->wred_d[w];
             }
-            u = (double) unit_from(xorshift_next(r.rng)) * S;
+            u = (double) unit_from(xorshift_next(rng)) * S;
             /* the first segment whose end lies beyond u: every warp knows whether it lies in one before */
             const unsigned over = __ballot_sync(0xffffffffu, g.tid < nseg && u < incl + woff);
             if (over != 0u && (g.warp == 0 || !(u < woff)) && g.lane == __ffs(over) - 1) {
@@ -1799,7 +1775,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 part += seg_at(t);
             }
             const double S = group_sum_d(g, gs, part);
-            u = (double) unit_from(xorshift_next(r.rng)) * S;
+            u = (double) unit_from(xorshift_next(rng)) * S;
             double carry = 0.0;
             for (int t0 = 0; t0 < nseg; t0 += g.n) {
                 const int    t    = t0 + g.tid;
@@ -1941,8 +1917,10 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     /* ---- top-k and top-p: merge the parts' candidates ---- */
     bool need_multipass = !(r.kq > 0 && r.kq <= kFastKMax) || overflow; /* what counts is how many stay above the row's threshold: checked below */
     const bool keep_all = r.mode == M_TOPP; /* every marked entry was left out of the bulk sums */
-    const float u01     = unit_from(xorshift_next(r.rng)); /* the row's draw */
-    bool        ordered = false; /* the kq best lie in fsort (top-k: their weights in fq) */
+    const float u01     = unit_from(xorshift_next(rng)); /* the row's draw */
+    int         n_rank  = 0;   /* entries of cbuf, the kq best among them; top-p: their probabilities */
+    float       rank_hi = row_max;
+    static_assert(kStageWords <= kFinCap, "what is staged fits the list");
     if (!need_multipass && others == 0) {
         /* All candidates came in with the records, four words per thread. Those that cannot be among the kq best, by the bins
          * their values fall into, are dropped where they are; the rest is ranked. Bound by latency: three barriers and a dozen
@@ -1955,8 +1933,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         double      part = 0.0;
 #pragma unroll
         for (int q = 0; q < kOwnWords; q++) {
-            const int t = g.tid + q * kThreads, k = t >> st_log, i = (t & ((1 << st_log) - 1)) - 4;
-            const int held = k < n_parts ? (int) (unsigned) sh->stage[(k << st_log) + 1] : 0;
+            int       i;
+            const int t = g.tid + q * kThreads, k = part_of(t, i), held = k < n_parts ? (int) (unsigned) sh->stage[k * st_w + 1] : 0;
             v[q]   = __uint_as_float((unsigned) tv[q]);
             bin[q] = i >= 0 && i < held && (keep_all || v[q] >= tau_row) ? min(kHistBins - 1, max(0, __float2int_rz((v[q] - tau_row) * scale))) : -1;
             if (bin[q] >= 0) {
@@ -1975,7 +1953,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                     }
                 }
                 if (g.tid < n_parts) {
-                    const unsigned long long *rec = &sh->stage[(g.tid << st_log) + 2];
+                    const unsigned long long *rec = &sh->stage[g.tid * st_w + 2];
                     part += ref_move(__uint_as_float((unsigned) (rec[0] >> 32)), row_max, r.inv_t) * __longlong_as_double((long long) rec[1]);
                 }
                 part = warp_sum_d(part);
@@ -1993,6 +1971,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 for (int w = 0; w < kWarps; w++) {
                     S += gs->wred_d[w];
                 }
+                rank_hi = __double2float_rn(1.0 / S); /* the row's maximum is a candidate */
                 if (g.tid == 0) {
                     sh->wide_S = S;
                 }
@@ -2010,43 +1989,16 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
 #pragma unroll
         for (int q = 0; q < kOwnWords; q++) {
             const int pos = at + __popc(in[q] & ((1u << g.lane) - 1u));
-            if (((in[q] >> g.lane) & 1u) != 0u && pos < kRankAll) {
+            if (((in[q] >> g.lane) & 1u) != 0u) {
                 cbuf[pos] = Pair{!kFast && r.mode == M_TOPP ? __double2float_rn((double) v[q] / S) : v[q], (int) (tv[q] >> 32)}; /* top-p: p_i as the reference normalises it */
             }
             at += __popc(in[q]);
         }
         g.sync();
-        const int n = sh->n_sel;
-        if (n >= r.kq && n <= kRankAll) {
-            if (n <= kRankFew) {
-                if (r.mode == M_TOPK && !r.select_only) {
-                    rank_few<true>(cbuf, n, r.kq, r.inv_t, sh->fsort, sh->fq);
-                } else {
-                    rank_few<false>(cbuf, n, r.kq, r.inv_t, sh->fsort, sh->fq);
-                }
-                g.sync();
-            } else {
-#pragma unroll 1
-                for (int i = g.tid; i < n; i += g.n) {
-                    const Pair me   = cbuf[i];
-                    int        rank = 0;
-#pragma unroll 4
-                    for (int j = 0; j < n; j++) {
-                        rank += pair_before(cbuf[j].v, cbuf[j].idx, me.v, me.idx) ? 1 : 0;
-                    }
-                    if (rank < r.kq) {
-                        sh->fsort[rank] = me;
-                        if (r.mode == M_TOPK) {
-                            sh->fq[rank] = exp_exact(scaled_arg(me.v, row_max, r.inv_t));
-                        }
-                    }
-                }
-                g.sync();
-            }
-            ordered = true;
-        }
+        need_multipass = sh->n_sel < r.kq;
+        n_rank         = sh->n_sel;
     }
-    if (!need_multipass && !ordered) {
+    if (!need_multipass && others > 0) {
         /* The candidates of all parts are merged in up to three passes of one rolled loop. The first keeps what
          * passes the row's threshold (the largest of the parts' thresholds). A row cut into many parts can have far
          * more of those than k (every part kept at least k of its own): if they do not fit, a second pass bins them
@@ -2094,9 +2046,10 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             g.sync();
             /* what is staged, then one loop over the rest of all parts (rolled: code that runs once per row costs what it weighs) */
 #pragma unroll 1
-            for (int t0 = 0; t0 < st_parts << st_log; t0 += kThreads) {
-                const int                t = t0 + g.tid, k = t >> st_log, i = (t & ((1 << st_log) - 1)) - 4;
-                const bool               ok = k < st_parts && i >= 0 && i < (int) (unsigned) sh->stage[(min(k, st_parts - 1) << st_log) + 1];
+            for (int t0 = 0; t0 < st_parts * st_w; t0 += kThreads) {
+                int                      i;
+                const int                t = t0 + g.tid, k = part_of(t, i);
+                const bool               ok = k < st_parts && i >= 0 && i < (int) (unsigned) sh->stage[min(k, st_parts - 1) * st_w + 1];
                 const unsigned long long w  = ok ? sh->stage[t] : 0ull;
                 place(ok, Pair{__uint_as_float((unsigned) w), (int) (w >> 32)});
             }
@@ -2149,140 +2102,54 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         if (total > kFinCap || total < r.kq) {
             need_multipass = true;
         }
-        /* More entries than are ranked one against all: those that cannot be among the kq best, by the bins their values
-         * fall into, stay out of the ranking (rows of many parts have kq of every part; a second list behind the first takes
-         * the rest). With what is staged of every part: one row of 128256 in 16 parts, top-k 40, 39.7 -> 35.6 us;
-         * 8 x 151936 top-p in 19 parts 48.3 -> 43.8; 2 x 262144 top-p in 32 parts 37.2 -> 32.4. Not where the kq best alone
-         * are more than are ranked: 64 x 32000 top-k 256, general kernel, 34.4 -> 32.1; 1000 x 8192 102.4 -> 97.3. */
-        float few_scale = 0.0f;
-        int   few_min   = -1; /* -1: all of them are ranked */
-        if (!need_multipass && total > kRankAll && r.kq <= kRankAll && row_max > tau_row && row_max - tau_row < CUDART_INF_F) {
-            few_scale = (float) kHistBins / (row_max - tau_row);
-            sh->bhist[g.tid] = 0;
-            static_assert(kHistBins == kThreads, "a bin per thread");
-            if (g.tid == 0) {
-                sh->n_sel = 0;
-            }
-            g.sync();
-#pragma unroll 1
-            for (int i = g.tid; i < total; i += g.n) {
-                atomicAdd(&sh->bhist[min(kHistBins - 1, max(0, __float2int_rz((cbuf[i].v - tau_row) * few_scale)))], 1);
-            }
-            g.sync();
-            few_min = top_bin(sh->bhist, g.lane, r.kq);
-        }
-        Pair *few    = cbuf + kFinCap;
-        auto  is_few = [&](float v) { return min(kHistBins - 1, max(0, __float2int_rz((v - tau_row) * few_scale))) >= few_min; };
-        static_assert((kFinCap + kRankAll) * (int) sizeof(Pair) <= kFinBytes, "the second list fits");
-        if (!need_multipass && r.mode == M_TOPK) {
-            const int   k         = r.k;
-            const Pair *rank_from = cbuf;
-            int         n_rank    = total;
-            if (few_min >= 0) {
-#pragma unroll 1
-                for (int i = g.tid; i < total; i += g.n) {
-                    const Pair e = cbuf[i];
-                    if (is_few(e.v)) {
-                        const int pos = atomicAdd(&sh->n_sel, 1);
-                        if (pos < kRankAll) {
-                            few[pos] = e;
-                        }
-                    }
-                }
-                g.sync();
-                if (sh->n_sel <= kRankAll) {
-                    rank_from = few;
-                    n_rank    = sh->n_sel;
-                }
-            }
-            if (n_rank <= kRankAll) {
-                /* few candidates: every entry is ranked against all others (a short loop that stays in the
-                 * instruction cache, instead of the histogram select's long straight-line code) */
-#pragma unroll 1
-                for (int i = g.tid; i < n_rank; i += g.n) {
-                    const Pair me   = rank_from[i];
-                    int        rank = 0;
-#pragma unroll 4
-                    for (int j = 0; j < n_rank; j++) {
-                        rank += pair_before(rank_from[j].v, rank_from[j].idx, me.v, me.idx) ? 1 : 0;
-                    }
-                    if (rank < k) {
-                        sh->fsort[rank] = me;
-                    }
-                }
-                g.sync();
-            } else {
-                g.sync(); /* n_sel is used again */
-                select_sorted(g, sh, cbuf, total, k, sh->fsort);
-            }
-            /* sampler.c:217-222: softmax over the k kept logits (max = the first) */
-            if (!r.select_only) {
-                const float m = sh->fsort[0].v;
-                for (int i = g.tid; i < k; i += g.n) {
-                    sh->fq[i] = exp_exact(scaled_arg(sh->fsort[i].v, m, r.inv_t));
-                }
-                g.sync();
-            }
-            ordered = true;
-        }
+        n_rank = total;
         if constexpr (!kFast) {
-        if (!need_multipass && r.mode == M_TOPP) {
-            /* top-p over a small nucleus (sampler.c:245-300). Candidates get their exact e_i relative to the row
-             * maximum; the rest of the row was summed per part relative to the part's own maximum and is
-             * rescaled here. */
-            double part = 0.0;
-            for (int i = g.tid; i < total; i += g.n) {
-                const float x = cbuf[i].v;
-                const float e = exp_exact(scaled_arg(x, row_max, r.inv_t));
-                cbuf[i].v     = e;
-                part += (double) e;
-                if (few_min >= 0 && is_few(x)) {
-                    const int pos = atomicAdd(&sh->n_sel, 1);
-                    if (pos < kRankAll) {
-                        few[pos] = Pair{e, cbuf[i].idx};
-                    }
+            if (!need_multipass && r.mode == M_TOPP) {
+                /* Candidates get their exact e_i relative to the row maximum; the rest of the row was summed per part relative
+                 * to the part's own maximum and is rescaled here. */
+                double part = 0.0;
+                for (int i = g.tid; i < total; i += g.n) {
+                    const float e = exp_exact(scaled_arg(cbuf[i].v, row_max, r.inv_t));
+                    cbuf[i].v     = e;
+                    part += (double) e;
                 }
-            }
-            if (g.tid < n_parts) {
-                const unsigned long long *rec = &sh->stage[(g.tid << st_log) + 2];
-                part += ref_move(__uint_as_float((unsigned) (rec[0] >> 32)), row_max, r.inv_t) * __longlong_as_double((long long) rec[1]);
-            }
-            const double S = group_sum_d(g, gs, part);
-            if (g.tid == 0) {
-                sh->wide_S = S;
-            }
-            /* the walk order is (p desc, id asc); the row's kq most probable ids are all candidates. Whatever is left out
-             * here has a smaller value than the kq-th, so no larger p. */
-            const int   kq        = r.kq;
-            const bool  by_few    = few_min >= 0 && sh->n_sel <= kRankAll; /* read behind the sum's barriers */
-            Pair       *rank_from = by_few ? few : cbuf;
-            const int   n_rank    = by_few ? sh->n_sel : total;
-            for (int i = g.tid; i < n_rank; i += g.n) {
-                rank_from[i].v = __double2float_rn((double) rank_from[i].v / S); /* p_i as the reference normalises it */
-            }
-            g.sync();
-            if (n_rank <= kRankAll) {
-#pragma unroll 1
-                for (int i = g.tid; i < n_rank; i += g.n) {
-                    const Pair me   = rank_from[i];
-                    int        rank = 0;
-#pragma unroll 4
-                    for (int j = 0; j < n_rank; j++) {
-                        rank += pair_before(rank_from[j].v, rank_from[j].idx, me.v, me.idx) ? 1 : 0;
-                    }
-                    if (rank < kq) {
-                        sh->fsort[rank] = me;
-                    }
+                if (g.tid < n_parts) {
+                    const unsigned long long *rec = &sh->stage[g.tid * st_w + 2];
+                    part += ref_move(__uint_as_float((unsigned) (rec[0] >> 32)), row_max, r.inv_t) * __longlong_as_double((long long) rec[1]);
+                }
+                const double S = group_sum_d(g, gs, part);
+                if (g.tid == 0) {
+                    sh->wide_S = S;
+                }
+                rank_hi = __double2float_rn(1.0 / S);
+                for (int i = g.tid; i < total; i += g.n) {
+                    cbuf[i].v = __double2float_rn((double) cbuf[i].v / S); /* p_i as the reference normalises it */
                 }
                 g.sync();
-            } else {
-                select_sorted(g, sh, cbuf, total, kq, sh->fsort);
             }
-            ordered = true;
-        }
         }
     }
-    if (ordered && r.mode == M_TOPK) {
+    if (!need_multipass) { /* in order, (value or p desc, id asc); top-k: and the weights of the softmax over the k kept logits (sampler.c:217-222) */
+        const bool weigh = r.mode == M_TOPK && !r.select_only;
+        if (n_rank <= kRankFew) {
+            if (weigh) {
+                rank_few<true>(cbuf, n_rank, r.kq, r.inv_t, sh->fsort, sh->fq);
+            } else {
+                rank_few<false>(cbuf, n_rank, r.kq, r.inv_t, sh->fsort, sh->fq);
+            }
+        } else {
+            rank_in_bins(cbuf, n_rank, r.kq, tau_row, rank_hi, r.mode == M_TOPP, cbuf + kFinCap, reinterpret_cast<int *>(cbuf + 2 * kFinCap), sh->fsort);
+            g.sync();
+            if (weigh) {
+                const float m = sh->fsort[0].v;
+                for (int i = g.tid; i < r.kq; i += g.n) {
+                    sh->fq[i] = exp_exact(scaled_arg(sh->fsort[i].v, m, r.inv_t));
+                }
+            }
+        }
+        g.sync();
+    }
+    if (!need_multipass && r.mode == M_TOPK) {
         PROF(11);
         const int k = r.k;
         if (r.select_only) {
@@ -2320,7 +2187,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         return st;
     }
     if constexpr (!kFast) {
-        if (ordered) {
+        if (!need_multipass) { /* top-p over a small nucleus (sampler.c:245-300) */
             const int kq = r.kq;
             /* The walks over the kq entries, one per lane of a warp. Their running sums are exact wherever no entry is smaller
              * than 2^-29, so the order of additions is not seen; one thread that adds them one by one, three times over,
@@ -2474,71 +2341,6 @@ __device__ __forceinline__ float part_top(const StreamShared *sh, bool cap_late)
     return cap_late && top > -CUDART_INF_F ? soft_cap(top, sh->cap) : top;
 }
 
-/* More than kRankFew candidates in order, the k best to sh->fin_s; none lies below lo. They are dealt out to 256 bins of
- * values, the highest in front, and ranked against their own bin: one against all costs a thread block total^2 / 32
- * rounds of six instructions. 1000 rows of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9;
- * 256 x 128256 top-k 200 48.9 -> 41.0. */
-__device__ __noinline__ void rank_in_bins(StreamShared *sh, unsigned char *gmem, int total, int k, float lo, bool cap_late) {
-    const int tid = (int) threadIdx.x, lane = tid & 31;
-    Pair       *srt   = reinterpret_cast<Pair *>(gmem); /* the group maxima are done with */
-    int        *start = reinterpret_cast<int *>(srt + kPartCand), *next = start + kHistBins + 1;
-    const float hi    = part_top(sh, cap_late);
-    const float scale = hi > lo && hi - lo < CUDART_INF_F ? (float) kHistBins / (hi - lo) : 0.0f; /* 0: one bin for all */
-    auto        bin_of = [&](float v) { return kHistBins - 1 - min(kHistBins - 1, max(0, __float2int_rz((v - lo) * scale))); };
-    for (int i = tid; i <= kHistBins; i += kThreads) {
-        start[i] = 0; /* entry b + 1: candidates in bin b; after the scan, entry b: candidates in the bins before b */
-    }
-    __syncthreads();
-    for (int i = tid; i < total; i += kThreads) {
-        atomicAdd(&start[bin_of(sh->cand[i].v) + 1], 1);
-    }
-    __syncthreads();
-    if (tid < 32) {
-        int v[kHistBins / 32], run = 0;
-#pragma unroll
-        for (int i = 0; i < kHistBins / 32; i++) {
-            run += start[1 + kHistBins / 32 * lane + i];
-            v[i] = run;
-        }
-        int before = run;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, before, d);
-            if (lane >= d) {
-                before += o;
-            }
-        }
-        before -= run;
-#pragma unroll
-        for (int i = 0; i < kHistBins / 32; i++) {
-            start[1 + kHistBins / 32 * lane + i] = before + v[i];
-            next[1 + kHistBins / 32 * lane + i]  = before + v[i];
-        }
-        if (lane == 0) {
-            next[0] = 0;
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < total; i += kThreads) {
-        const Pair me                           = sh->cand[i];
-        srt[atomicAdd(&next[bin_of(me.v)], 1)] = me;
-    }
-    __syncthreads();
-    for (int i = tid; i < total; i += kThreads) {
-        const Pair me   = srt[i];
-        const int  b    = bin_of(me.v), end = start[b + 1];
-        int        rank = start[b];
-        if (rank < k) {
-            for (int j = rank; j < end; j++) {
-                rank += pair_before(srt[j].v, srt[j].idx, me.v, me.idx) ? 1 : 0;
-            }
-            if (rank < k) {
-                sh->fin_s[rank] = me;
-            }
-        }
-    }
-}
-
 /* The largest of the warps' references of a part. */
 __device__ __forceinline__ float part_ref(const StreamShared *sh) {
     float m = -CUDART_INF_F;
@@ -2685,7 +2487,8 @@ __device__ __forceinline__ void inline_finish_topk(const SampleParams &p, Stream
         if (total <= kRankFew) {
             rank_few<true>(sh->cand, total, k, inv_t, sh->fin_s, sh->fin_q);
         } else {
-            rank_in_bins(sh, gmem, total, k, lo, cap_late);
+            Pair *srt = reinterpret_cast<Pair *>(gmem); /* the group maxima are done with */
+            rank_in_bins(sh->cand, total, k, lo, part_top(sh, cap_late), false, srt, reinterpret_cast<int *>(srt + kPartCand), sh->fin_s);
             __syncthreads();
             const float m = sh->fin_s[0].v;
             for (int i = tid; i < k; i += kThreads) {
@@ -3848,18 +3651,22 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     /* The first row's parameters are inputs of the launch, written before the stream kernel began: they may be
      * read while that kernel's last thread blocks are still at work. Everything it wrote waits for the line below. */
     auto parts_of = [&](int row) { return cta_of_item(p, row * p.n_slices + p.n_slices - 1) - cta_of_item(p, row * p.n_slices) + 1; };
-    RawCfg rc{};
-    RowCfg r{};
-    int    n_parts = 0;
-    auto   configure = [&](int row) {
-        rc = raw_config(p, row, true);
-        r  = row_config(p, row, rc, true);
+    unsigned long long rng0    = 0ull; /* the generator word that the row's sequence came with */
+    int                n_parts = 0;
+    auto               configure = [&](int row) { /* the barrier in front of a row lies behind the last use of its predecessor's */
+        const RawCfg rc = raw_config(p, row, true);
+        RowCfg       r  = row_config(p, row, rc, true);
         if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
             r.cap    = 0.0f;
             r.mrow   = nullptr;
             r.pen_on = false;
         }
+        rng0    = rc.rng;
         n_parts = parts_of(row);
+        if (g.tid == 0) {
+            sh->cfg = r;
+        }
+        __syncthreads();
     };
     if ((int) blockIdx.x < p.n_rows) {
         configure((int) blockIdx.x);
@@ -3875,18 +3682,18 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
         }
         PROF(8);
         if constexpr (!kFast) {
-            if (g.tid == 0 && r.mode != M_TOPP) {
+            if (g.tid == 0 && sh->cfg.mode != M_TOPP) {
                 atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
             }
         }
-        int st = finish_row<kFast>(g, p, sh, r, n_parts, cmem);
+        int st = finish_row<kFast>(g, p, sh, n_parts, cmem);
         PROF(13);
         if (st & ST_DEFERRED) {
             if constexpr (kFast) {
                 /* This kernel does not carry the code for the row. A top-k row whose candidates did not fit (many
                  * equal values at the top) is the caller's to launch again without the hint; any other kind of
                  * row the caller said would not come. */
-                st = (st & ~ST_DEFERRED) | (r.mode == M_TOPK ? ST_RETRY : ST_INTERNAL);
+                st = (st & ~ST_DEFERRED) | (sh->cfg.mode == M_TOPK ? ST_RETRY : ST_INTERNAL);
                 if (g.tid == 0) {
                     p.tokens[row] = -1;
                 }
@@ -3896,7 +3703,7 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
             }
         }
         if (g.tid == 0) {
-            row_epilogue(p, r, row, st, rc.rng);
+            row_epilogue(p, sh->cfg, row, st, rng0);
         }
         __syncthreads();
     }

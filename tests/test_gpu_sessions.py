@@ -217,3 +217,57 @@ def test_batcher_propose_drafts_over_the_history_ring(ctx):
     with pytest.raises(api.GeistError, match="GEIST_E_INVALID_ARG"):
         bt.propose_drafts(sess[:3], 8, out_capacity=8)
     bt.close()
+
+
+def test_calls_in_a_row_commit_before_the_next_reads(ctx):
+    """Calls return when their tokens are there; what they commit (histories, generator words) is ordered before the next call
+    and before whoever asks for it. Steps and verify calls in turn over short rings that wrap, sessions opened and closed in
+    between, against the checker with the histories kept here."""
+    V, N, k, ring = 9001, 6, 3, 20
+    rg = np.random.default_rng(8)
+    bt = api.Batcher(ctx, V, N + 1, max_history=ring)
+    sess = [bt.open(temperature=0.9, top_k=20 if i % 2 else 0, top_p=0.7 if i % 3 == 0 else 1.0, seed=3 + i, rep=1.3, freq=0.1) for i in range(N)]
+    T, K, P = np.full(N, 0.9, np.float32), np.array([20 if i % 2 else 0 for i in range(N)]), np.array([0.7 if i % 3 == 0 else 1.0 for i in range(N)])
+    state = np.array([port.rng_seed(3 + i) for i in range(N)], np.uint64)
+    hist = [[] for _ in range(N)]
+
+    def padded():
+        h, n = np.zeros((N, ring), np.int32), np.zeros(N, np.int32)
+        for i, ids in enumerate(hist):
+            n[i] = len(ids[-ring:])
+            h[i, : n[i]] = ids[-ring:]
+        return h, n
+
+    for it in range(30):
+        h, n = padded()
+        if it % 3 < 2:
+            x = normal_logits(N, V, 2.0, 100 + it)
+            x[:, :30] += 5.0
+            got = bt.step(sess, to_dev(x))
+            o = port.sample_batch(x, T, K, P, state, rep=1.3, freq=0.1, pres=0.0, hist=h, hist_len=n)
+            assert np.array_equal(got, o["tokens"]), it
+            for i in range(N):
+                hist[i].append(int(got[i]))
+        else:
+            x = normal_logits(N * k, V, 2.0, 100 + it)
+            x[:, :4] += 9.0
+            fed = rg.integers(0, 4, (N, k)).astype(np.int32)
+            acc, nout, toks = bt.verify(sess, fed, to_dev(x))
+            o = port.sample_batch(x, T, K, P, state, rows_per_seq=k, rep=1.3, freq=0.1, pres=0.0, hist=h, hist_len=n, extra=fed)
+            out = o["tokens"].reshape(N, k)
+            for i in range(N):
+                a = 0
+                while a + 1 < k and out[i, a] == fed[i, a + 1]:
+                    a += 1
+                assert (acc[i], nout[i]) == (a, a + 2) and toks[i, : a + 2].tolist() == fed[i, : a + 1].tolist() + [int(out[i, a])], it
+                hist[i] += toks[i, 1 : a + 2].tolist()
+        state = o["rng_state"]
+        if it % 4 == 0:
+            assert [bt.get_rng(s) for s in sess] == [int(v) for v in state]
+        if it % 5 == 0:
+            bt.close_session(bt.open(temperature=0.0))
+        if it % 7 == 0:
+            state = state.copy()
+            state[1] = np.uint64(12345 + it)
+            bt.set_rng(sess[1], 12345 + it)
+    bt.close()

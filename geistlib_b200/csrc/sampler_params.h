@@ -105,14 +105,14 @@ struct WideHead {
     unsigned           any;      /* the number of the lane's last launch that had top-p rows: never put back, so no order between
                                   * the stream kernel's thread blocks matters */
     int                waited;   /* 1: thread blocks without a row of their own waited for rows to help with; for geist_b200_wide_counts as well */
-    int                pad;
+    int                turn;   /* thread blocks that have looked for a row to help with */
 };
 constexpr int kWidePiece     = 512;  /* columns that are dealt out at a time, to a warp */
 constexpr int kWidePiecesMax = 4096; /* rows of more pieces go the multi-pass way */
 constexpr int kWideBinsLog   = 12;
 constexpr int kWideBins      = 1 << kWideBinsLog; /* bins of a row's histogram */
-constexpr int kWideCtlInts   = 16;
-constexpr int kWidePartBytes = 32;
+constexpr int kWideCtlInts   = 20;
+constexpr int kWidePartBytes = 8;
 
 constexpr int kRawWords = 12; /* 32-bit words of a row's raw parameters: sequence, T, top_p, top_k, history length, rep, freq, pres, cap, (none), generator low and high */
 

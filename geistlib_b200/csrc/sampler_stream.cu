@@ -2697,6 +2697,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
         *reinterpret_cast<int4 *>(p.wide_head) = make_int4(0, 0, 0, 0);
         p.wide_head->gave_up                   = 0;
         p.wide_head->waited                    = 0;
+        p.wide_head->turn                      = 0;
     }
     asm volatile("griddepcontrol.launch_dependents;");
 #ifdef GB_PROFILE
@@ -3758,7 +3759,7 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
                 opened = wide_wait(p, 0u);
             }
             if (__syncthreads_or(opened) != 0) {
-                wide_help(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), sh->save);
+                wide_help(p, &sh->gs, reinterpret_cast<WideShared *>(cmem), opened, sh->save);
             }
         }
     }

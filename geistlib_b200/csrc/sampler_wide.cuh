@@ -24,8 +24,10 @@
  *
  * Pass 1 is bound by the issue of its instructions at the finishing kernel's 16 warps per SM: 25 SM cycles per 32 values,
  * where its double arithmetic takes 6 and its conversions 8; a launch's first piece waits for the code as well, 4 us. 256
- * rows of 128256 columns, top-p 0.95 (105 of them wide): 428 us with a thread block and a dozen sweeps per row, 168 now;
- * 24 wide rows of 100003 among 96: 402 -> 74. Pieces of 512 for a warp: when they came in (the 24 rows took 93 us) pieces of
+ * rows of 128256 columns, top-p 0.95 (98 of them wide): 428 us with a thread block and a dozen sweeps per row, 147 now;
+ * 24 wide rows of 100003 among 96: 402 -> 69. Of the 98 rows' 77 us from the first row opened to the last token pass 1 takes 38,
+ * what is added up and waited for between the passes 4, the windows 3, pass 2 12; 16 are the last row's end and uneven work.
+ * Pieces of 512 for a warp: when they came in (the 24 rows took 93 us) pieces of
  * 1024 took 99, and pieces of 2048 for a thread block, a barrier each, 204 us on the 105.
  */
 #pragma once
@@ -46,16 +48,15 @@ struct __align__(16) WideCtl {
     float  row_max;
     int    row_arg;
     double S0;
-    double pad[2];
+    unsigned long long above_cut, above_pick; /* of p, above the two windows (wide_mass): whole numbers, so in any order */
+    int                n_above;               /* entries above the window of the crossing */
+    int                pad[3];
 };
 static_assert(sizeof(WideCtl) == 4 * kWideCtlInts, "a slot's words");
 
 /* What a piece adds up to. */
-struct __align__(16) WidePart {
-    double    sum;                   /* of e */
-    long long above_cut, above_pick; /* of p, above the two windows (wide_mass) */
-    int       n_above;               /* entries above the window of the crossing */
-    int       pad;
+struct WidePart {
+    double sum; /* of e */
 };
 static_assert(sizeof(WidePart) == kWidePartBytes, "the host sizes the parts");
 
@@ -65,7 +66,7 @@ struct __align__(16) WideShared {
     float              x[kWarps][2][kWidePiece];    /* every warp's pieces: the one in work and the next on its way */
     unsigned           cnt[kWarps][kWidePiece / 2]; /* how often an id of the warp's piece occurs, 16 bits each; zero between pieces */
     int                ids[kWideIds];
-    unsigned           wsum[kWarps];
+    unsigned           wsum[kWarps], open[2 * kWarps];
     int                win[4]; /* the crossing's window, lowest and highest bin; the draw's */
     int                next, slot, mine;
     int                best_rank;
@@ -182,6 +183,37 @@ __device__ WideHit wide_walk(const Grp &g, GroupShared *gs, WideShared *ws, cons
     return out;
 }
 
+/* The same for at most 32 entries, by one warp: an entry per lane, each met with all others. The windows are a bin or two of
+ * thousands, most lists hold less than ten: a row's end, 10 us by all threads with their barriers, takes a warp 4. (Bins instead
+ * of one against all in wide_walk: 13 us.) */
+__device__ __forceinline__ WideHit wide_walk_few(int lane, const Pair *list, int n, long long base, double target, bool inclusive, int idx_bits) {
+    const unsigned long long e  = lane < n ? __ldcg(reinterpret_cast<const unsigned long long *>(list + lane)) : 0ull; /* p, then the id */
+    const unsigned long long me = lane < n ? composite((unsigned) e, (int) (e >> 32), idx_bits) : 0ull;
+    const long long          m  = lane < n ? wide_mass(__uint_as_float((unsigned) e)) : 0;
+    long long                to = 0; /* of the entries up to the lane's */
+    int                      rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; j++) {
+        const bool      up = __shfl_sync(0xffffffffu, me, j) >= me;
+        const long long mj = __shfl_sync(0xffffffffu, m, j);
+        to += up ? mj : 0;
+        rank += up ? 1 : 0;
+    }
+    const double             at = mass_value(base + to);
+    unsigned long long best = lane < n && (inclusive ? at >= target : at > target) ? me : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    }
+    const int from = __ffs(__ballot_sync(0xffffffffu, lane < n && me == best)) - 1;
+    WideHit   out;
+    out.found = best != 0ull;
+    out.word  = best;
+    out.mass  = mass_value(base + __shfl_sync(0xffffffffu, to, max(from, 0)));
+    out.rank  = (long long) __shfl_sync(0xffffffffu, rank, max(from, 0));
+    return out;
+}
+
 /* Takes a piece of a row of which *rem were left: its number, -1 when there was none. Called by a whole warp; the answer
  * takes a round trip, so a warp asks a piece ahead (lane 0 holds what came back). */
 __device__ __forceinline__ int wide_ask(int *rem, int lane) { return lane == 0 ? atomicSub(rem, 1) : 0; }
@@ -198,20 +230,21 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     const RowCfg    r      = ws->cfg;
     WideCtl        *ctl    = p.wide_ctl + slot;
     const int       V      = p.V, pieces = (V + kWidePiece - 1) / kWidePiece, idx_bits = 32 - __clz(max(V - 1, 1));
-    const WidePart *parts  = p.wide_part + (size_t) slot * (size_t) pieces;
     const Pair     *list   = p.gen_list + (size_t) slot * (size_t) p.gen_list_cap;
     const int       half   = p.gen_list_cap / 2;
     const WideBins  bins(__ldcg(&ctl->S0), r.top_p, V);
-    long long       a_cut = 0, a_pick = 0, above = 0;
-    for (int t = g.tid; t < pieces; t += g.n) {
-        a_cut += __ldcg(&parts[t].above_cut);
-        a_pick += __ldcg(&parts[t].above_pick);
-        above += __ldcg(&parts[t].n_above);
-    }
-    const int n_cut = __ldcg(&ctl->n_cut), n_pick = __ldcg(&ctl->n_pick);
-    a_cut           = group_sum_ll(g, gs, a_cut);
-    a_pick          = group_sum_ll(g, gs, a_pick);
-    above           = group_sum_ll(g, gs, above);
+    const int       n_cut = __ldcg(&ctl->n_cut), n_pick = __ldcg(&ctl->n_pick);
+    const bool      few   = listed && n_cut <= 32 && n_pick <= 32; /* nearly always: one warp finishes the row */
+    const int       w0 = ws->win[0], w1 = ws->win[1], w2 = ws->win[2], w3 = ws->win[3];
+    uint4          *gh    = reinterpret_cast<uint4 *>(p.wide_hist + (size_t) slot * kWideBins);
+    auto            clear = [&](int from, int step) { /* for the slot's next row */
+        for (int i = from; i < kWideBins / 4; i += step) {
+            gh[i] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    const long long a_cut = (long long) __ldcg(&ctl->above_cut), a_pick = (long long) __ldcg(&ctl->above_pick), above = __ldcg(&ctl->n_above);
+    WideHit   cut{}, pick{};
+    bool      ok = listed && n_cut <= half && n_pick <= half && n_cut > 0 && mass_value(a_cut) < (double) r.top_p;
     /* p of the nearest entries outside a window: an entry of the window that shares it cannot be placed */
     const WideQuotient quot(S);
     auto p_at   = [&](unsigned k) { return quot(__uint_as_float(k)); };
@@ -219,20 +252,37 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
         const float pv = __uint_as_float((unsigned) (word >> idx_bits));
         return pv > 0.0f && (hi >= kWideBins - 1 || pv < p_at(bins.edge(hi + 1))) && pv > p_at(bins.edge(lo) - 1u);
     };
-    const int w0 = ws->win[0], w1 = ws->win[1], w2 = ws->win[2], w3 = ws->win[3];
-    bool      ok = listed && n_cut <= half && n_pick <= half && n_cut > 0 && mass_value(a_cut) < (double) r.top_p;
-    WideHit   cut{}, pick{};
-    if (ok) {
-        cut = wide_walk(g, gs, ws, list, n_cut, a_cut, (double) r.top_p, true, idx_bits);
-        ok  = cut.found && inside(cut.word, w0, w1);
-    }
-    if (ok) {
-        unsigned long long rng = r.rng;
-        const double       u   = (double) unit_from(xorshift_next(rng)) * cut.mass;
-        ok                     = mass_value(a_pick) <= u;
+    auto drawn = [&](unsigned long long rng) { return (double) unit_from(xorshift_next(rng)) * cut.mass; };
+    if (few) {
+        if (g.warp != 0) {
+            clear(g.tid - 32, kThreads - 32);
+        } else {
+            if (ok) {
+                cut = wide_walk_few(g.lane, list, n_cut, a_cut, (double) r.top_p, true, idx_bits);
+                ok  = cut.found && inside(cut.word, w0, w1);
+            }
+            if (ok) {
+                const double u = drawn(r.rng);
+                ok             = mass_value(a_pick) <= u;
+                if (ok) {
+                    pick = wide_walk_few(g.lane, list + half, n_pick, a_pick, u, false, idx_bits);
+                    ok   = pick.found && inside(pick.word, w2, w3);
+                }
+            }
+        }
+        ok = __syncthreads_or(g.warp == 0 && ok) != 0; /* the first thread holds what there is to write */
+    } else {
         if (ok) {
-            pick = wide_walk(g, gs, ws, list + half, n_pick, a_pick, u, false, idx_bits);
-            ok   = pick.found && inside(pick.word, w2, w3);
+            cut = wide_walk(g, gs, ws, list, n_cut, a_cut, (double) r.top_p, true, idx_bits);
+            ok  = cut.found && inside(cut.word, w0, w1);
+        }
+        if (ok) {
+            const double u = drawn(r.rng);
+            ok             = mass_value(a_pick) <= u;
+            if (ok) {
+                pick = wide_walk(g, gs, ws, list + half, n_pick, a_pick, u, false, idx_bits);
+                ok   = pick.found && inside(pick.word, w2, w3);
+            }
         }
     }
     int st = __ldcg(&ctl->st);
@@ -254,9 +304,8 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     if (g.tid == 0) {
         row_epilogue(p, r, r.row, st, rng0);
     }
-    uint4 *gh = reinterpret_cast<uint4 *>(p.wide_hist + (size_t) slot * kWideBins);
-    for (int i = g.tid; i < kWideBins / 4; i += g.n) {
-        gh[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (!few) {
+        clear(g.tid, g.n);
     }
     __threadfence();
     g.sync();
@@ -532,15 +581,15 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
         const double       margin = 1024.0 + (double) (V >> 8);
         const double       t_cut  = (double) r.top_p * S * (double) bins.unit;
         auto place = [&](int which, double target) { /* the highest bin b so that the units in bins >= b reach the target */
-            target = fmax(target, 1e-3);
-            if ((double) before < target && (double) (before + run) >= target) {
+            const unsigned t = __double2uint_ru(fmax(target, 1e-3)); /* units are whole */
+            if (before < t && before + run >= t) {
                 unsigned acc = before;
                 int      b   = b0;
 #pragma unroll
                 for (int q = kOwn - 1; q >= 0; q--) {
-                    const bool below = (double) acc < target;
+                    const bool below = acc < t;
                     acc += h[q];
-                    b = below && (double) acc >= target ? b0 + q : b;
+                    b = below && acc >= t ? b0 + q : b;
                 }
                 ws->win[which] = b;
             }
@@ -583,6 +632,8 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
     if (piece >= 0) {
         fetch(gr, true, (int) p.gen_stride, piece, 0, 0.0f);
     }
+    long long a_cut = 0, a_pick = 0;
+    int       above = 0;
     for (int in = 0; piece >= 0; in ^= 1) {
         const int s0   = piece * kWidePiece;
         const int next = wide_got(left, pieces);
@@ -591,8 +642,6 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
             fetch(gr, true, (int) p.gen_stride, next, in ^ 1, 0.0f);
         }
         one_behind(next >= 0);
-        long long a_cut = 0, a_pick = 0;
-        int       above = 0;
 #pragma unroll 1
         for (int step = 0; step < kSteps; step++) {
             float    e[kPer];
@@ -640,16 +689,16 @@ __device__ __noinline__ void wide_join(const SampleParams &p, GroupShared *gs, W
                 }
             }
         }
-        a_cut  = warp_sum_ll(a_cut);
-        a_pick = warp_sum_ll(a_pick);
-        above  = __reduce_add_sync(0xffffffffu, above);
-        if (g.lane == 0) {
-            parts[piece].above_cut  = a_cut;
-            parts[piece].above_pick = a_pick;
-            parts[piece].n_above    = above;
-        }
         piece = next;
         __syncwarp();
+    }
+    a_cut  = warp_sum_ll(a_cut);
+    a_pick = warp_sum_ll(a_pick);
+    above  = __reduce_add_sync(0xffffffffu, above);
+    if (g.lane == 0 && (a_cut | a_pick) != 0) { /* what lies above has a mass */
+        atomicAdd(&ctl->above_cut, (unsigned long long) a_cut);
+        atomicAdd(&ctl->above_pick, (unsigned long long) a_pick);
+        atomicAdd(&ctl->n_above, above);
     }
     leave(true, S);
 }
@@ -668,6 +717,9 @@ __device__ __forceinline__ void wide_open(const SampleParams &p, GroupShared *gs
         ctl->row_max     = row_max;
         ctl->row_arg     = row_arg;
         ctl->S0          = S0;
+        ctl->above_cut   = 0ull;
+        ctl->above_pick  = 0ull;
+        ctl->n_above     = 0;
         ctl->rem2        = pieces;
         __threadfence();
         atomicExch(&ctl->rem1, pieces - own); /* the first are the block's own */
@@ -684,46 +736,89 @@ __device__ __forceinline__ void wide_open(const SampleParams &p, GroupShared *gs
 /* A thread block that has no rows of its own left helps with wide ones, as long as there can be any: it waits for rows
  * that have not been decided on, but no longer than kWideHelpNs. How many rows have been opened, 0 where those are no more
  * than `looked` and there is nothing to wait for. One thread. */
-constexpr unsigned long long kWideHelpNs = 50000ull;
+constexpr unsigned long long kWideHelpNs = 50000ull, kWideDecideNs = 4000ull; /* rows that go the same way are decided on within 3 us */
 __device__ __forceinline__ int wide_wait(const SampleParams &p, unsigned looked) {
     const unsigned long long t0 = global_ns();
+    unsigned long long       seen = 0ull; /* when a row was first there to help with */
     for (;;) {
-        const unsigned long long rows = *reinterpret_cast<volatile unsigned long long *>(&p.wide_head->rows);
+        const unsigned long long rows = *reinterpret_cast<volatile unsigned long long *>(&p.wide_head->rows), now = global_ns();
+        const bool               decided = (int) (unsigned) rows >= p.n_rows;
         if ((unsigned) (rows >> 32) > looked) {
-            return (int) (rows >> 32);
-        }
-        if ((int) (unsigned) rows >= p.n_rows || global_ns() - t0 > kWideHelpNs) {
+            /* who looks for the first time waits a little for the others, so that all of them can be shared out */
+            seen = seen == 0ull ? now : seen;
+            if (decided || looked > 0u || now - seen > kWideDecideNs) {
+                return (int) (rows >> 32);
+            }
+        } else if (decided || now - t0 > kWideHelpNs) {
             return 0;
         }
         __nanosleep(40);
     }
 }
-__device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, WideShared *ws, void *save_mem) {
+/* `opened`: what the first thread's wait has said. */
+__device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, WideShared *ws, int opened, void *save_mem) {
     const Grp          g      = whole_block();
-    const int          pieces = (p.V + kWidePiece - 1) / kWidePiece, start = (int) (blockIdx.x % (unsigned) p.pool_slots);
+    const int          pieces = (p.V + kWidePiece - 1) / kWidePiece;
     unsigned           looked = 0u; /* rows that had been opened when the slots were last looked through in vain */
     for (;;) {
         if (g.tid == 0) {
-            ws->next = wide_wait(p, looked);
-            ws->slot = 0x7fffffff;
+            ws->next = opened > 0 ? opened : wide_wait(p, looked);
             __threadfence();
         }
         g.sync();
-        const int opened = ws->next;
-        if (opened == 0) {
+        const int rows_seen = ws->next;
+        opened              = 0;
+        if (rows_seen == 0) {
             return;
         }
-        for (int i = g.tid; i < p.pool_slots; i += g.n) {
-            const int rem = ld_volatile(&p.wide_ctl[i].rem1);
-            if (rem > kWarps / 2) {
-                /* a row with much left to do; among equals each block begins elsewhere */
-                const int at = i >= start ? i - start : i + p.pool_slots - start;
-                atomicMin(&ws->slot, ((kWidePiecesMax - rem) >> 3 << 16) | at);
+        /* Of the rows that have more than half as much left to do as the one with the most, the blocks take up one each in turn, in
+         * the order in which they come: a block stays for both passes. Each going to the nearest row left some with two blocks next
+         * to others with nine (256 flat rows, 98 of them wide, 163 us; 152 so). */
+        constexpr int kLook = 2 * kThreads; /* slots that are looked at: more than a device holds thread blocks */
+        int           rem[2], most = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int i = g.tid + h * kThreads;
+            rem[h]      = i < p.pool_slots ? ld_volatile(&p.wide_ctl[i].rem1) : 0;
+            most        = max(most, rem[h]);
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (g.lane == 0) {
+            ws->wsum[g.warp] = (unsigned) most;
+        }
+        g.sync();
+        for (int w = 0; w < kWarps; w++) {
+            most = max(most, (int) ws->wsum[w]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const unsigned open = __ballot_sync(0xffffffffu, rem[h] > max(kWarps / 2, most / 2));
+            if (g.lane == 0) {
+                ws->open[h * kWarps + g.warp] = open;
             }
         }
         g.sync();
-        const int at   = ws->slot;
-        const int slot = at == 0x7fffffff ? -1 : ((at & 0xffff) + start) % p.pool_slots;
+        if (g.tid == 0) {
+            int rows = 0, found = -1;
+            for (int w = 0; w < kLook / 32; w++) {
+                rows += __popc(ws->open[w]);
+            }
+            int k = rows > 0 ? (int) ((unsigned) atomicAdd(&p.wide_head->turn, 1) % (unsigned) rows) : -1;
+            for (int w = 0; w < kLook / 32 && k >= 0; w++) {
+                const int c = __popc(ws->open[w]);
+                if (k < c) {
+                    unsigned bits = ws->open[w];
+                    for (int i = 0; i < k; i++) {
+                        bits &= bits - 1u;
+                    }
+                    found = 32 * w + __ffs(bits) - 1;
+                }
+                k -= c;
+            }
+            ws->slot = found;
+        }
+        g.sync();
+        const int slot = ws->slot;
         if (g.tid == 0) {
             /* a piece for every warp: with one for the block a row that is opened first was taken up by all of them */
             const int left = slot < 0 ? 0 : atomicSub(&p.wide_ctl[slot].rem1, kWarps);
@@ -737,7 +832,7 @@ __device__ __noinline__ void wide_help(const SampleParams &p, GroupShared *gs, W
             wide_join(p, gs, ws, slot, piece, min(kWarps, pieces - piece), save_mem);
             g.sync();
         } else if (slot < 0) {
-            looked = (unsigned) opened;
+            looked = (unsigned) rows_seen;
         }
     }
 }

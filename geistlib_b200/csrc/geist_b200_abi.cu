@@ -139,13 +139,15 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
 
 /* How a launch's (row, slice) items are dealt out to the stream kernel's thread blocks (gb::RunMap), the grid that
  * goes with it, and over how many thread blocks a row can be spread. A thread block's cost is taken as its items
- * plus kPartCost items' worth for every part of a row it touches (set-up, threshold, groups read again, record): five
- * where rows may be top-k rows (with three, us: 200 x 128256 top-k 40 26.0 -> 31.7, 1000 x 65536 64.0 -> 76.2; with eight
- * 150 x 128256 29.3 -> 22.3, 350 x 65536 34.9 -> 31.0, single rows of 8192 5 % slower), one where the caller said they
- * are temperature / top-p rows (a temperature part has no threshold: 150 x 65536 23.9 us against 26.3 with three; a
- * top-p part has one: 256 x 128256 on Gumbel rows 55.5 against 49.9, the hint does not tell them apart), eight where
- * the caller said they are greedy (whole rows need no finishing kernel; with three 200 x 128256 19.6 -> 21.5, with five
- * 350 x 65536 21.4 -> 19.7). */
+ * plus kPartCost items' worth for every part of a row it touches (set-up, threshold, groups read again, record), by what the
+ * caller said its rows are (over 49 shapes from 1 x 8192 to 1000 x 65536, us):
+ *   greedy and top-k rows 10: whole rows need no finishing kernel. Against five 150 x 128256 top-k 40 26.7 -> 21.3, with 64
+ *     ids 30.7 -> 23.1, 350 x 65536 34.9 -> 28.4, 160 x 200000 33.5 -> 30.4; 3 % over all, none slower by more than the noise;
+ *   greedy rows 8: with five 150 x 128256 17.2 -> 18.7, 350 x 65536 21.2 -> 19.7, no difference over all;
+ *   temperature / top-p rows 4: against one 256 x 128256 top-p 43.8 -> 39.0, 256 x 262144 65.6 -> 61.9, 224 x 128256 42.7 ->
+ *     37.7, 100 x 100000 30.0 -> 25.2; temperature rows, whose parts have no threshold, want two (150 x 65536 20.8 -> 21.6 with
+ *     four, 1000 x 65536 79.0 -> 83.5), which a caller that says there is no top-p row gets;
+ *   unknown rows 5. */
 struct Deal {
     gb::RunMap map;
     int        grid;
@@ -461,7 +463,8 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     /* scratch of this launch */
     const size_t n_rows   = (size_t) p.n_rows;
     const size_t n_items  = n_rows * (size_t) pl.n_slices;
-    const size_t part_cost = (flags & gb::F_SELECT_ONLY) ? 5 : (b->finish_hint == GEIST_B200_FINISH_GENERAL ? 1 : (b->finish_hint == GEIST_B200_FINISH_GREEDY ? 8 : 5));
+    const bool   any_kind  = (flags & gb::F_SELECT_ONLY) != 0u || b->finish_hint == GEIST_B200_FINISH_AUTO;
+    const size_t part_cost = any_kind ? 5 : b->finish_hint == GEIST_B200_FINISH_GREEDY ? 8 : b->finish_hint == GEIST_B200_FINISH_GREEDY_TOPK ? 10 : (flags & gb::F_NO_TOP_P) != 0u ? 2 : 4;
     const Deal   deal     = deal_items(n_rows, pl.n_slices, pl.ctas, part_cost);
     const int    grid     = deal.grid;
     const size_t parts    = (size_t) deal.parts_max;

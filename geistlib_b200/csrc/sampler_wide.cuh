@@ -229,7 +229,7 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     const Grp       g      = whole_block();
     const RowCfg    r      = ws->cfg;
     WideCtl        *ctl    = p.wide_ctl + slot;
-    const int       V      = p.V, pieces = (V + kWidePiece - 1) / kWidePiece, idx_bits = 32 - __clz(max(V - 1, 1));
+    const int       V      = p.V, idx_bits = 32 - __clz(max(V - 1, 1));
     const Pair     *list   = p.gen_list + (size_t) slot * (size_t) p.gen_list_cap;
     const int       half   = p.gen_list_cap / 2;
     const WideBins  bins(__ldcg(&ctl->S0), r.top_p, V);

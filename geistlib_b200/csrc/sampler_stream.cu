@@ -275,17 +275,31 @@ __device__ __forceinline__ float prologue_one(float x, int i, float cap, const u
     return x;
 }
 
+/* The mask words of a warp's share of a slice, at most 1024 columns: a word per lane, and the one behind them where the share
+ * begins inside a word. Asked for a slice ahead: read where they were used, every slice waited for them. */
+struct ShareMask {
+    unsigned w, x;
+};
+__device__ __forceinline__ ShareMask share_mask(const unsigned *mrow, int V, int lane, int column) {
+    ShareMask m;
+    const int at = column >> 5, words = (V + 31) >> 5;
+    m.w          = at + lane < words ? __ldg(mrow + at + lane) : 0u;
+    m.x          = (column & 31) != 0 && at + 32 < words ? __ldg(mrow + at + 32) : 0u;
+    return m;
+}
+
 /* The same over a warp's share of a slice in its stage (sl: the share's first float; e0: its index inside the
  * slice; mine4 float4 groups, lane-strided; n: the slice's length, what lies behind it stays -inf). Kept out of
  * line: the stream kernel's loop stays short for the launches that have neither cap nor mask. */
-__device__ __noinline__ void prologue_share(float *sl, int lane, int mine4, int e0, int n, int s0, float cap, const unsigned *mrow) {
+__device__ __noinline__ void prologue_share(float *sl, int lane, int mine4, int e0, int n, int s0, float cap, bool masked, const ShareMask &words) {
     float4  *w4 = reinterpret_cast<float4 *>(sl) + lane;
     unsigned allowed[kNV4]; /* four columns each: a float4 lies on a multiple of four, so inside one word of the mask */
-    if (mrow != nullptr) { /* all of the share's words at once: a word per column and use took a round trip for every float4 */
+    if (masked) {
 #pragma unroll
         for (int i = 0; i < kNV4; i++) {
-            const int at = s0 + e0 + 4 * (lane + 32 * i);
-            allowed[i]   = lane + 32 * i < mine4 ? __ldg(mrow + (at >> 5)) >> (at & 31) : 0u;
+            const int      at = ((s0 + e0) & 31) + 4 * (lane + 32 * i);
+            const unsigned in = __shfl_sync(0xffffffffu, words.w, (at >> 5) & 31);
+            allowed[i]        = ((at >> 5) < 32 ? in : words.x) >> (at & 31);
         }
     }
 #pragma unroll
@@ -299,7 +313,7 @@ __device__ __noinline__ void prologue_share(float *sl, int lane, int mine4, int 
                 if (e + 2 < n) v.z = soft_cap(v.z, cap);
                 if (e + 3 < n) v.w = soft_cap(v.w, cap);
             }
-            if (mrow != nullptr) { /* what lies behind the row's end is -inf already */
+            if (masked) { /* what lies behind the row's end is -inf already */
                 v.x = (allowed[i] & 1u) != 0u ? v.x : -CUDART_INF_F;
                 v.y = (allowed[i] & 2u) != 0u ? v.y : -CUDART_INF_F;
                 v.z = (allowed[i] & 4u) != 0u ? v.z : -CUDART_INF_F;
@@ -3003,6 +3017,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             gm_shift++;
         }
 
+        const bool masked = !kPlain && pro_part && sh->mrow != nullptr;
+        ShareMask  words{};
+        if (masked) {
+            words = share_mask(sh->mrow, p.V, lane, c0 * p.slice + 4 * (c0 == p.n_slices - 1 ? w4lo_l : w4lo_f));
+        }
+
         /* ---- the part's slices, every warp on its own ---- */
         for (int s = 0; s < part_len; s++, j++) {
             const int      stage  = j % kStages;
@@ -3042,7 +3062,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             /* ---- 1b. soft cap and mask, in place ---- */
             if (pro_part) {
                 wrote = true;
-                prologue_share(sl, lane, mine4, 4 * w4lo, n, s0, cap_late ? 0.0f : sh->cap, sh->mrow);
+                prologue_share(sl, lane, mine4, 4 * w4lo, n, s0, cap_late ? 0.0f : sh->cap, masked, words);
+                if (masked && s + 1 < part_len) {
+                    words = share_mask(sh->mrow, p.V, lane, s0 + p.slice + 4 * (c + 1 == p.n_slices - 1 ? w4lo_l : w4lo_f));
+                }
             }
 
             /* ---- 2. penalties on the share ---- */
@@ -3352,7 +3375,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         if (e0 + q < n) {
-                            v[q] = prologue_one(v[q], id0 + q, sh->cap, sh->mrow);
+                            v[q] = prologue_one(v[q], id0 + q, cap_late ? 0.0f : sh->cap, sh->mrow);
                         }
                     }
                 }
@@ -3409,7 +3432,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
                 bool     any = false;
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const bool cand = own && v[q] >= tau && e0 + q < n;
+                    const bool cand = own && v[q] >= tau_grp && e0 + q < n; /* tau itself, but for values that are capped below */
                     hit[q]          = __ballot_sync(0xffffffffu, cand);
                     found += __popc(hit[q]);
                     any |= cand;
@@ -3477,6 +3500,14 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             again.list      = !kLong || !long_ids || long_smem ? id_list : p.pre_list + (size_t) row * (size_t) p.row_cap;
         };
         int       n_cand = over ? kPartCand + 1 : min(sh->n_cand, kPartCand + 1); /* more than kPartCand: the list ran over */
+        if (!kPlain && cap_late && n_cand <= kPartCand) {
+            /* One candidate per thread, where every value that was read again took a tanhf and a division. What falls short of
+             * tau now is no more than a candidate too many. */
+            for (int i = tid; i < n_cand; i += kThreads) {
+                sh->cand[i].v = prologue_one(sh->cand[i].v, sh->cand[i].idx, sh->cap, sh->mrow); /* the mask again: the cap of -inf is not -inf */
+            }
+            __syncthreads();
+        }
         if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
             /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
              * part); a row of another kind is reported as the small finishing kernel would */

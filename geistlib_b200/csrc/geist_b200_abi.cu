@@ -971,6 +971,7 @@ struct geist_b200_batcher {
     int   *h_pin        = nullptr; /* pinned, written and read by the kernels where it lies: slots | fed | twice (tokens | status | accepted | nemit | emitted), taken in turn: the kernel that
                                     * commits a call's tokens may still read them when the next call begins */
     int    turn         = 0;
+    bool   committing   = false; /* a call's bookkeeping has been launched and nobody has waited for it yet */
     std::vector<int32_t> slots_sent; /* the session list that d_slot holds */
     size_t h_pin_ints   = 0;
 
@@ -1009,7 +1010,13 @@ struct geist_b200_batcher {
 
 /* What the last call committed may still be on its way when it returns: calls that read or write a session's state from
  * the host wait for it. */
-static cudaError_t settled(const geist_b200_batcher *b) { return cudaStreamSynchronize(b->ctx->stream); }
+static cudaError_t settled(geist_b200_batcher *b) {
+    if (!b->committing) {
+        return cudaSuccess;
+    }
+    b->committing = false;
+    return cudaStreamSynchronize(b->ctx->stream);
+}
 
 extern "C" void geist_b200_batcher_destroy(struct geist_b200_batcher *b) {
     if (b == nullptr) {
@@ -1540,6 +1547,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
     CUDA_TRY(gb::launch_post_step(b->d_slot, (int) n, per_seq, first, (append_history && b->max_history) ? append_tok : nullptr, append_cnt, b->d_hist, (int) b->max_history,
                                   b->d_hist_len, b->d_hist_tot, b->d_rng_tmp, b->d_rng, st));
     b->turn ^= 1;
+    b->committing = true;
     const float *dev_rows = logits_on_host ? b->d_logits : logits;
     const size_t dev_stride = logits_on_host ? b->V : row_stride;
     if (verify) {

@@ -154,7 +154,7 @@ struct geist_b200_batch {
     const float   *presence_penalty;   /* per sequence or NULL   (EXTENSION) */
     const int32_t *history;            /* [*, history_stride] or NULL */
     size_t         history_stride;     /* also the longest history a row can have: at most 8192 ids per row (history plus
-                                        * fed tokens), else GEIST_E_UNSUPPORTED. A batch whose rows can bring more than 256 ids
+                                        * fed tokens), else GEIST_E_UNSUPPORTED. A batch whose rows can bring more than 1024 ids
                                         * costs one more kernel launch (the rows' distinct ids are counted ahead of the stream
                                         * kernel). */
     const int32_t *history_len;        /* per sequence */

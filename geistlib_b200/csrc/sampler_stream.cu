@@ -1846,35 +1846,43 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         const int    e0    = min(4 * w * Lc, nc);
         const int    e1    = min(4 * min((w + 1) * Lc, nv4c), nc);
         const int    seg_n = max(e1 - e0, 0);
-        float       *wbuf  = reinterpret_cast<float *>(cmem); /* >= 1024 floats */
         const float *src   = row_again(p, row) + s0c + e0;
+        /* every thread takes a run of consecutive entries; the runs' sums are scanned over the group and the thread whose run
+         * crosses u walks it */
+        const int per = (seg_n + g.n - 1) / g.n; /* <= 4 */
+        const int i0  = g.tid * per;
+        float     ev[4];
         g.sync();
-        for (int i = g.tid; i < seg_n; i += g.n) {
-            wbuf[i] = prologue_one(src[i], s0c + e0 + i, r.cap, r.mrow);
-        }
         if (r.pen_on) {
+            float *wbuf = reinterpret_cast<float *>(cmem); /* >= 1024 floats */
+            for (int i = g.tid; i < seg_n; i += g.n) {
+                wbuf[i] = prologue_one(src[i], s0c + e0 + i, r.cap, r.mrow);
+            }
             for (int i = g.tid; i < kFinBitmapWords; i += g.n) {
                 sh->fin_bitmap[i] = 0u;
             }
             if (g.tid == 0) {
                 gs->n_dlist = 0;
             }
-        }
-        g.sync();
-        if (r.pen_on && seg_n > 0) {
-            st |= apply_penalties(g, wbuf, s0c + e0, seg_n, r, p.V, p.vocab_offset, sh->fin_bitmap, sh->fdlist, min(p.hist_cap, 512), &gs->n_dlist, false, 0);
-        }
-        {
-            /* every thread takes a run of consecutive entries; the runs' sums are scanned over the
-             * group and the thread whose run crosses u walks it */
-            const int per = (seg_n + g.n - 1) / g.n; /* <= 4 */
-            const int i0  = g.tid * per;
-            float     ev[4];
-            double    mine = 0.0;
+            g.sync();
+            if (seg_n > 0) {
+                st |= apply_penalties(g, wbuf, s0c + e0, seg_n, r, p.V, p.vocab_offset, sh->fin_bitmap, sh->fdlist, min(p.hist_cap, 512), &gs->n_dlist, false, 0);
+            }
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int i = i0 + q;
-                ev[q]       = (q < per && i < seg_n) ? expf(scaled_arg(wbuf[i], row_max, r.inv_t)) : 0.0f;
+                ev[q] = q < per && i0 + q < seg_n ? wbuf[i0 + q] : -CUDART_INF_F;
+            }
+        } else { /* nothing to change: each thread reads its own */
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                ev[q] = q < per && i0 + q < seg_n ? prologue_one(src[i0 + q], s0c + e0 + i0 + q, r.cap, r.mrow) : -CUDART_INF_F;
+            }
+        }
+        {
+            double mine = 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                ev[q] = q < per && i0 + q < seg_n ? expf(scaled_arg(ev[q], row_max, r.inv_t)) : 0.0f;
                 mine += (double) ev[q];
             }
             double incl = mine;
@@ -1885,28 +1893,22 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                     incl += up;
                 }
             }
-            g.sync();
             if (g.lane == 31) {
                 gs->wred_d[g.warp] = incl;
             }
-            if (g.tid == 0) {
-                gs->pick = 0x7fffffff;
-            }
             g.sync();
-            double base = fbase;
-            for (int ww = 0; ww < g.warp; ww++) {
-                base += gs->wred_d[ww];
+            double base = fbase, upto = fbase; /* up to the thread's warp, and in all */
+#pragma unroll
+            for (int ww = 0; ww < kWarps; ww++) {
+                base = ww == g.warp ? upto : base;
+                upto += gs->wred_d[ww];
             }
-            if (u < base + incl && i0 < seg_n) {
-                atomicMin(&gs->pick, g.tid);
-            }
-            g.sync();
-            const int pk = gs->pick;
-            if (pk == 0x7fffffff) {
+            const unsigned over = __ballot_sync(0xffffffffu, u < base + incl && i0 < seg_n);
+            if (!(u < upto) || seg_n == 0) {
                 if (g.tid == 0) { /* regrouped sums can end a hair below the segment's share; the row's last segment may be empty */
                     p.tokens[row] = max(s0c + e0 + seg_n - 1, 0) + p.vocab_offset;
                 }
-            } else if (g.tid == pk) {
+            } else if (over != 0u && (g.warp == 0 || !(u < base)) && g.lane == __ffs(over) - 1) { /* no warp before crosses it */
                 double a   = base + (incl - mine);
                 int    hit = min(i0 + per - 1, seg_n - 1);
 #pragma unroll

@@ -71,7 +71,8 @@ constexpr size_t kSmemMax = 227 * 1024; /* opt-in shared memory per CTA on sm_10
 constexpr size_t kHeadInts = 16;       /* words in front of a lane's per-slot words */
 static_assert(sizeof(gb::WideHead) <= kHeadInts * sizeof(int), "the launch's words lie in front");
 constexpr unsigned long long kWideWaitNs = 1000000000ull; /* a second, as the kernels' other waits */
-constexpr int    kLanes   = 4;          /* launches of one context that may overlap on the GPU */
+constexpr int    kLanes   = 4;          /* launches of one context that may overlap on the GPU ... */
+constexpr int    kOwnLane = kLanes;     /* ... and the set of the synchronous calls, whose launches follow one another on the context's stream */
 
 struct Plan {
     int    n_slices     = 0;
@@ -279,7 +280,9 @@ struct geist_b200_ctx {
     std::mutex small_mu;      /* one synchronous host-pointer call at a time stages through the two words above */
 
     /* kernel scratch: part records with their candidates, segment sums, row counters, multi-pass row copies. kLanes
-     * independent sets, used round-robin, so that up to kLanes launches may overlap on the GPU. */
+     * independent sets, used round-robin, so that up to kLanes launches may overlap on the GPU. A synchronous call returns
+     * when its words are there: its last thread blocks may still look into their set, so those calls have one of their own,
+     * which the stream's order keeps, and none of theirs counts among the caller's kLanes. */
     struct Lane {
         unsigned char *buf         = nullptr;
         size_t         bytes       = 0;
@@ -288,10 +291,12 @@ struct geist_b200_ctx {
         size_t         arrive_cap  = 0;
         size_t         counter_cap = 0;
         unsigned       launches    = 0;
-    } lane[kLanes];
+    } lane[kLanes + 1];
     unsigned   next_lane = 0;
+    int        last_lane = 0; /* that the last launch took */
     unsigned long long wide_wait_ns = kWideWaitNs;
     std::mutex lane_mu;
+    std::mutex own_mu; /* the synchronous calls' set: from where a launch takes it to the launch itself */
 };
 
 extern "C" enum geist_status geist_b200_ctx_create(int device, struct geist_b200_ctx **out) {
@@ -360,7 +365,8 @@ extern "C" void geist_b200_ctx_destroy(struct geist_b200_ctx *c) {
 
 /* ------------------------------------------------------- batched entries -- */
 
-static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct geist_b200_batch *b, void *stream, unsigned flags) {
+/* `own`: the launch of a synchronous call on the context's stream. */
+static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct geist_b200_batch *b, void *stream, unsigned flags, bool own = false) {
     if (ctx == nullptr || b == nullptr) {
         return fail(GEIST_E_INVALID_ARG, "sample_batch: NULL context or batch");
     }
@@ -492,10 +498,15 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     const size_t off_pl   = round_up(off_wp + slots * pieces * (size_t) gb::kWidePartBytes, 256);
     const size_t off_po   = round_up(off_pl + (pl.id_slots ? n_rows * (size_t) pl.row_cap * 4 : 0), 256);
     const size_t need     = round_up(off_po + (pl.id_slots ? n_rows * ((size_t) pl.n_slices * (size_t) gb::kWarps + 1) * 4 : 0), 256) + 256;
-    geist_b200_ctx::Lane *ln;
+    geist_b200_ctx::Lane        *ln;
+    std::unique_lock<std::mutex> in_turn(ctx->own_mu, std::defer_lock);
+    if (own) {
+        in_turn.lock();
+    }
     {
         std::lock_guard<std::mutex> lk(ctx->lane_mu);
-        ln       = &ctx->lane[ctx->next_lane++ % kLanes];
+        ctx->last_lane = own ? kOwnLane : (int) (ctx->next_lane++ % kLanes);
+        ln             = &ctx->lane[ctx->last_lane];
         p.launch = ++ln->launches;
         if (ln->bytes < need) {
             cudaFree(ln->buf); /* waits for work that may still use it */
@@ -645,7 +656,7 @@ extern "C" enum geist_status geist_b200_wide_counts(struct geist_b200_ctx *ctx, 
     CUDA_TRY(cudaSetDevice(ctx->device));
     gb::WideHead                h{};
     std::lock_guard<std::mutex> lk(ctx->lane_mu);
-    const geist_b200_ctx::Lane &ln = ctx->lane[(ctx->next_lane + kLanes - 1) % kLanes];
+    const geist_b200_ctx::Lane &ln = ctx->lane[ctx->last_lane];
     if (ln.counters != nullptr) {
         CUDA_TRY(cudaDeviceSynchronize());
         CUDA_TRY(cudaMemcpy(&h, ln.counters, sizeof h, cudaMemcpyDeviceToHost));
@@ -818,7 +829,7 @@ geist_token_t sample_host_row(size_t n, const float *logits, float *staging, flo
         h->token   = kUnwritten;
         h->status  = kUnwritten;
         h->rng_out = 0ull; /* no generator word comes to that */
-        if (geist_b200_sample_batch(c, &b, c->stream) != GEIST_OK) {
+        if (launch_batch(c, &b, c->stream, 0u, true) != GEIST_OK) {
             return -1;
         }
         e = await_words(&h->token, 1, kUnwritten, c->stream);
@@ -933,7 +944,7 @@ extern "C" enum geist_status geist_b200_argmax_f32(struct geist_b200_ctx *ctx, c
     b.tokens       = &h->token; /* written over the host link by the one kernel that the hint leaves */
     b.row_status   = &h->status;
     b.finish_hint  = GEIST_B200_FINISH_GREEDY;
-    enum geist_status s = geist_b200_sample_batch(ctx, &b, ctx->stream);
+    enum geist_status s = launch_batch(ctx, &b, ctx->stream, 0u, true);
     if (s != GEIST_OK) {
         return s;
     }
@@ -1440,7 +1451,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
             d.fed_tokens = (pen && verify) ? b->d_fed : nullptr;
             d.tokens     = tok_dst;
             d.row_status = h_stat;
-            enum geist_status s = launch_batch(b->ctx, &d, st, any_top_p ? 0u : gb::F_NO_TOP_P);
+            enum geist_status s = launch_batch(b->ctx, &d, st, any_top_p ? 0u : gb::F_NO_TOP_P, true);
             if (s != GEIST_OK) {
                 return s;
             }
@@ -1517,7 +1528,9 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
             gb::AcceptParams ap{h_fed, b->d_tokens, (int) n, (int) k, h_acc, h_nem, h_emit};
             CUDA_TRY(gb::launch_accept(ap, st));
         }
-        if (verify) { /* the accept kernel's words first: they come last, and until then nobody looks at a line that is written */
+        if (logits_on_host) { /* launches on other streams, with the sets that rotate: all of them are through when the call returns */
+            CUDA_TRY(cudaStreamSynchronize(st));
+        } else if (verify) { /* the accept kernel's words first: they come last, and until then nobody looks at a line that is written */
             CUDA_TRY(await_words(h_nem, n, kUnwritten, st));
             CUDA_TRY(await_words(h_acc, n, kUnwritten, st));
             CUDA_TRY(await_words(h_emit, n * (k + 1), kUnwritten, st));

@@ -301,17 +301,17 @@ __device__ __noinline__ void wide_finish(const SampleParams &p, GroupShared *gs,
     } else {
         st |= multipass_row(p, gs, &ws->cfg, __ldcg(&ctl->row_max), __ldcg(&ctl->row_arg), ws, (int) offsetof(WideShared, cfg), slot, save_mem);
     }
-    if (g.tid == 0) {
-        row_epilogue(p, r, r.row, st, rng0);
-    }
     if (!few) {
         clear(g.tid, g.n);
     }
     __threadfence();
     g.sync();
-    if (g.tid == 0 && p.n_rows > p.pool_slots) {
-        __threadfence();
-        atomicExch(&p.pool[slot], 0);
+    if (g.tid == 0) { /* the row's status comes behind all that is done to its slot */
+        if (p.n_rows > p.pool_slots) {
+            atomicExch(&p.pool[slot], 0);
+            __threadfence();
+        }
+        row_epilogue(p, r, r.row, st, rng0);
     }
     g.sync();
 }

@@ -107,7 +107,11 @@ geist_token_t geist_sampler_top_p_ws(struct geist_sampler_workspace *ws, const f
  * candidate lists, row counters), which grows on demand: the first call with a
  * larger batch allocates. At most four launches of one context may be in
  * flight on the GPU at a time (they rotate over four scratch sets); callers
- * that need more overlap create more contexts. */
+ * that need more overlap create more contexts. The launches of calls that
+ * hand out tokens on the host (the argmax slot, the sampler.h surface, the
+ * batcher over device logits) are not among the four: they have a set of
+ * their own and follow one another on the context's stream, also where a call
+ * has returned before its last thread blocks have. */
 struct geist_b200_ctx;
 
 enum geist_status geist_b200_ctx_create(int device, struct geist_b200_ctx **out);

@@ -206,3 +206,41 @@ def test_wide_rows_on_two_streams_at_once():
                 out["tokens"].fill_(-7)
         torch.cuda.synchronize()
     ctx.close()
+
+
+def test_steps_followed_by_launches_on_other_streams():
+    """A step returns when its tokens are there. What comes right behind it must not meet what is left of it: its logits are
+    overwritten from another stream, and four launches with wide rows go to four more."""
+    import torch
+    ctx = api.Context(0)
+    n, V, steps = 12, 30001, 12
+    bt = api.Batcher(ctx, V, n)
+    sess = [bt.open(temperature=1.1, top_p=0.93, seed=70 + i) for i in range(n)]
+    state = independent_states(oracle.port, 70, n)
+    jobs, keep = [], []  # a descriptor holds pointers only
+    for i, rows in enumerate([3, 40, 12, 7]):
+        x, st = normal_logits(rows, V, 1.0, 71 + i), independent_states(oracle.port, 90 + i, rows)
+        keep.append((to_dev(x), *per_seq(rows, 1.1, 0, 0.93), u64_to_dev(st)))
+        jobs.append((torch.cuda.Stream(), ctx.sample_batch(*keep[i], launch=False), oracle.port.sample_batch(x, 1.1, 0, 0.93, st)["tokens"]))
+    xs = [normal_logits(n, V, 1.0, 200 + i) for i in range(3)]
+    ready = [to_dev(x) for x in xs]
+    cur, side = torch.empty_like(ready[0]), torch.cuda.Stream()
+    for it in range(steps):
+        with torch.cuda.stream(side):
+            cur.copy_(ready[it % 3])
+        side.synchronize()
+        got = bt.step(sess, cur)
+        with torch.cuda.stream(side):
+            cur.fill_(float("nan"))
+        for stream, out, _ in jobs:
+            ctx.relaunch(out, stream.cuda_stream)
+        o = oracle.port.sample_batch(xs[it % 3], 1.1, 0, 0.93, state)
+        assert np.array_equal(got, o["tokens"]), it
+        state = o["rng_state"]
+        torch.cuda.synchronize()
+        for _, out, want in jobs:
+            assert np.array_equal(out["tokens"].cpu().numpy(), want), it
+            out["tokens"].fill_(-7)
+        torch.cuda.synchronize()
+    bt.close()
+    ctx.close()

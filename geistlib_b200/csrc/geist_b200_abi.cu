@@ -844,7 +844,7 @@ geist_token_t sample_host_row(size_t n, const float *logits, float *staging, flo
         }
         b.finish_hint = GEIST_B200_FINISH_AUTO; /* thousands of equal values at the top: the general kernel takes the row */
     }
-    if (h->status < 0 || (h->status & (GEIST_B200_ROW_LOAD_TIMEOUT | GEIST_B200_ROW_HIST_OVERFLOW | GEIST_B200_ROW_INTERNAL))) {
+    if (h->token == kUnwritten || h->status < 0 || (h->status & (GEIST_B200_ROW_LOAD_TIMEOUT | GEIST_B200_ROW_HIST_OVERFLOW | GEIST_B200_ROW_INTERNAL))) {
         fail(GEIST_E_BACKEND, "sampler: kernel reported row status 0x%x", h->status);
         return -1;
     }
@@ -1544,6 +1544,11 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
                 return fail(GEIST_E_BACKEND, "batcher: row %zu reported status 0x%x", i, h_stat[i]);
             }
             retry |= (h_stat[i] & GEIST_B200_ROW_RETRY) != 0;
+        }
+        /* the tokens are handed out as they are, so none may be what the host put there (the status says so too, unless only a token is missing) */
+        const int *const told = verify ? h_emit : h_tok;
+        if (std::find(told, told + (verify ? n * (k + 1) : n), kUnwritten) != told + (verify ? n * (k + 1) : n)) {
+            return fail(GEIST_E_BACKEND, "batcher: a row was left without a token");
         }
         if (!retry) {
             break;

@@ -1774,11 +1774,16 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 S += gs->wred_d[w];
             }
             u = (double) unit_from(xorshift_next(rng)) * S;
-            /* the first segment whose end lies beyond u: every warp knows whether it lies in one before */
-            const unsigned over = __ballot_sync(0xffffffffu, g.tid < nseg && u < incl + woff);
-            if (over != 0u && (g.warp == 0 || !(u < woff)) && g.lane == __ffs(over) - 1) {
-                gs->pick = g.tid;
-                gs->S    = incl + woff - val;
+            /* The first segment whose end lies beyond u. Every thread has the same sums up to each warp and, as lane 31's, with it:
+             * one warp takes it. Which of its lanes is asked of those that add something; their sums may end a last bit away from
+             * lane 31's, and the last of them takes it where none of theirs lies beyond u. */
+            const unsigned over = __ballot_sync(0xffffffffu, u < incl + woff);
+            if ((over >> 31) != 0u && !(u < woff)) {
+                const unsigned adds = __ballot_sync(0xffffffffu, val > 0.0);
+                if (g.lane == ((over & adds) != 0u ? __ffs(over & adds) - 1 : 31 - __clz(adds))) {
+                    gs->pick = g.tid;
+                    gs->S    = incl + woff - val;
+                }
             }
             g.sync();
             found = gs->pick;
@@ -1815,7 +1820,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                     woff += gs->wred_d[w];
                 }
                 incl += woff;
-                if (t < nseg && u < incl) {
+                if (val > 0.0 && u < incl) {
                     atomicMin(&gs->pick, t);
                 }
                 g.sync();
@@ -1897,29 +1902,51 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 gs->wred_d[g.warp] = incl;
             }
             g.sync();
-            double base = fbase, upto = fbase; /* up to the thread's warp, and in all */
+            u           = u < fbase ? fbase : u; /* the difference that fbase is may be a last bit too large */
+            double base = fbase, upto = fbase;   /* up to the thread's warp, and in all */
 #pragma unroll
             for (int ww = 0; ww < kWarps; ww++) {
                 base = ww == g.warp ? upto : base;
                 upto += gs->wred_d[ww];
             }
-            const unsigned over = __ballot_sync(0xffffffffu, u < base + incl && i0 < seg_n);
-            if (!(u < upto) || seg_n == 0) {
-                if (g.tid == 0) { /* regrouped sums can end a hair below the segment's share; the row's last segment may be empty */
-                    p.tokens[row] = max(s0c + e0 + seg_n - 1, 0) + p.vocab_offset;
-                }
-            } else if (over != 0u && (g.warp == 0 || !(u < base)) && g.lane == __ffs(over) - 1) { /* no warp before crosses it */
-                double a   = base + (incl - mine);
-                int    hit = min(i0 + per - 1, seg_n - 1);
+            const unsigned over = __ballot_sync(0xffffffffu, u < base + incl);
+            if (u < upto) {
+                if ((over >> 31) != 0u && !(u < base)) { /* one warp takes it, and which of its lanes is asked as above */
+                    const unsigned adds = __ballot_sync(0xffffffffu, mine > 0.0);
+                    if (g.lane == ((over & adds) != 0u ? __ffs(over & adds) - 1 : 31 - __clz(adds))) {
+                        double a   = base + (incl - mine);
+                        int    hit = i0;
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    a += (double) ev[q];
-                    if (q < per && u < a) {
-                        hit = i0 + q;
-                        break;
+                        for (int q = 0; q < 4; q++) {
+                            a += (double) ev[q];
+                            hit = ev[q] > 0.0f ? i0 + q : hit;
+                            if (ev[q] > 0.0f && u < a) {
+                                break;
+                            }
+                        }
+                        p.tokens[row] = s0c + e0 + hit + p.vocab_offset;
                     }
                 }
-                p.tokens[row] = s0c + e0 + min(hit, seg_n - 1) + p.vocab_offset;
+            } else {
+                /* The segment's share came out a hair larger than its entries add up to: the last entry that adds something. Nothing
+                 * does, or the row's sum is no number: its last id, as the reference's walk ends. */
+                if (g.tid == 0) {
+                    gs->pick = -1;
+                }
+                g.sync();
+                int last = -1;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    last = ev[q] > 0.0f ? i0 + q : last;
+                }
+                last = __reduce_max_sync(0xffffffffu, u == u ? last : -1);
+                if (g.lane == 0 && last >= 0) {
+                    atomicMax(&gs->pick, last);
+                }
+                g.sync();
+                if (g.tid == 0) {
+                    p.tokens[row] = max(s0c + e0 + (gs->pick >= 0 ? gs->pick : seg_n - 1), 0) + p.vocab_offset;
+                }
             }
             if (g.tid == 0 && p.kept_cap > 0) {
                 p.kept_n[row] = 0;

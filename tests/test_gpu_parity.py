@@ -317,6 +317,57 @@ def test_temperature_penalised_ids_late_in_the_crossing_segment(ctx):
     check_tokens(g, o)
 
 
+def state_drawing(n):
+    """A generator state whose next draw is n / 2^24: the multiplication and the three shifts undone."""
+    m = (1 << 64) - 1
+    s = (n << 40 | 0x1234567) * pow(0x2545F4914F6CDD1D, -1, 1 << 64) & m
+    for shift, left in ((27, False), (25, True), (12, False)):
+        t = s
+        for _ in range(64 // shift):
+            t = s ^ ((t << shift & m) if left else t >> shift)
+        s = t
+    assert oracle.port.rng_stream(s, 1)[0] >> 40 == n
+    return s
+
+
+def test_temperature_draw_on_the_end_of_a_ragged_segment(ctx):
+    """The draw is 1 of a row whose sum is 2: the crossing segment holds 12 ids (ids 4480 .. 4491 of 8984: the last warp's share of
+    the first slice), of weights e, e and 1, e < 2^-53. Added up lane by lane they come to 1, in another order to more: the token
+    lies here all the same, and is written."""
+    import torch
+    V = 8984
+    x = np.full((3, V), -np.inf, np.float32)
+    x[:, [4480, 4484]] = -37.0
+    x[:, [4488, 4497]] = 0.0
+    st = np.array([state_drawing(1 << 23), state_drawing((1 << 23) - 1), state_drawing((1 << 23) + 1)], np.uint64)
+    keep = to_dev(x), *per_seq(3, 1.0, 0, 1.0), u64_to_dev(st)
+    out = ctx.sample_batch(*keep, launch=False)
+    out["tokens"].fill_(-7)
+    ctx.relaunch(out, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert (oracle.port.sample_batch(x, 1.0, 0, 1.0, st)["tokens"] == [4488, 4488, 4497]).all()
+    assert out["tokens"].tolist() == [4488, 4488, 4497]
+
+
+def test_temperature_draw_never_ends_on_a_masked_column(ctx):
+    """The segments' sums are formed by the special-function unit, the crossing segment is walked with expf: a draw that lies
+    between the two sums ends on the segment's last id that can be drawn, not on one that the mask takes out. Rows whose draw
+    lies as near the first segment's end as 24 bits allow."""
+    rows, V = 2048, 8192  # a segment of 1024 ids per warp
+    rg = np.random.default_rng(3)
+    level = rg.uniform(-7.0, -2.0, rows).astype(np.float32)
+    x = np.repeat(level[:, None], V, axis=1)
+    x[:, 1024] = 0.0  # the row's maximum, and most of what follows
+    allowed = np.zeros(V, bool)
+    allowed[:1000] = allowed[1024:1030] = True
+    first = 1000 * np.exp(level.astype(np.float64))
+    S = first + 1.0 + 5 * np.exp(level.astype(np.float64))
+    st = np.array([state_drawing(int(n)) for n in np.round(first / S * 2 ** 24) + rg.integers(-2, 2, rows)], np.uint64)
+    words = np.packbits(allowed, bitorder="little").view(np.int32)
+    g = run_gpu(ctx, x, 1.0, 0, 1.0, st, logit_mask=to_dev(np.tile(words, (rows, 1))))
+    assert set(np.unique(g["tokens"])) == {999, 1024}
+
+
 def _long_history_case(rows, V, stride, seed):
     """Histories of mixed lengths around the 128-id limit of the loader's register path, ids drawn
     from small pools so that most repeat, some rows with every id in one slice."""

@@ -81,7 +81,6 @@ struct Plan {
     int    bucket_cap   = 0;
     int    many_ids     = 0;
     int    id_slots     = 0;
-    int    hist_cap     = 0;
     size_t smem         = 0;
     int    ctas         = 0; /* thread blocks of the stream kernel the device holds at once (its grid never exceeds this) */
     int    fin_ctas     = 0; /* ... and of the finishing kernel */
@@ -122,7 +121,6 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
         pl.row_cap    = (int) round_up(hist_max, 4);
         pl.bucket_cap = (int) round_up(n_slices * (size_t) gb::kWarps + 1, 4);
     }
-    pl.hist_cap = hist_max ? (int) round_up(std::min<size_t>(hist_max, 1024), 4) : 0; /* the finisher walks segments of at most 1024 ids */
     pl.smem     = gb::sample_stream_smem(pl.n_slices, pl.many_ids);
     if (pl.smem > kSmemMax) {
         return false;
@@ -455,7 +453,6 @@ static enum geist_status launch_batch(struct geist_b200_ctx *ctx, const struct g
     p.bucket_cap   = pl.bucket_cap;
     p.many_ids     = pl.many_ids;
     p.id_slots     = pl.id_slots;
-    p.hist_cap     = pl.hist_cap;
     p.aligned      = ((reinterpret_cast<uintptr_t>(b->logits) & 15u) == 0 && (b->row_stride & 3u) == 0) ? 1 : 0;
     p.flags        = flags;
     if ((flags & gb::F_SELECT_ONLY) == 0u) { /* a shard's select is a top-k row whatever its parameters say: the small kernel takes k <= kFastKMax, the general one the rest */

@@ -172,7 +172,6 @@ struct SampleParams {
     int       bucket_cap;  /* n_slices * kWarps + 1 rounded up to a multiple of 4 */
     unsigned *pre_list;    /* [n_rows][row_cap] (offset in the share) | (count << 10), grouped by (slice, warp) share */
     int      *pre_off;     /* [n_rows][n_slices * kWarps + 1] where each share's run starts */
-    int      hist_cap;     /* distinct-id entries the finisher reserves for one walked segment */
     int      aligned;      /* rows start on 16-byte boundaries: bulk copies allowed */
     unsigned flags;
 

@@ -387,7 +387,7 @@ __device__ int apply_penalties(const Grp &g, float *buf, int s0, int n, const Ro
     }
     g.sync();
     int nd = *n_dlist;
-    if (nd > cap) { /* cannot happen when the launcher sized the room; keep the run consistent anyway */
+    if (nd > cap) { /* cannot happen: the callers have room for an entry per value of the run, or per id; keep the run consistent anyway */
         st |= ST_HIST_OVERFLOW;
         nd = 0;
     }
@@ -1306,7 +1306,6 @@ struct __align__(16) FinishShared {
     unsigned    fin_bitmap[kFinBitmapWords];
     Pair        fsort[kFastKMax];
     alignas(8) float fq[kFastKMax];
-    PenEntry    fdlist[512];
     alignas(16) unsigned long long stage[kStageWords]; /* the records and first candidates of the row's parts */
     unsigned long long save[256 + 128];                      /* the multi-pass path keeps a histogram here */
     RowCfg      cfg;    /* the row's: in registers it had left none for the code that finishes it */
@@ -1859,7 +1858,10 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         float     ev[4];
         g.sync();
         if (r.pen_on) {
-            float *wbuf = reinterpret_cast<float *>(cmem); /* >= 1024 floats */
+            constexpr int kSegMost = kSliceMax / kWarps; /* entries of a segment, and so distinct ids in it */
+            static_assert(kSegMost * (sizeof(float) + sizeof(PenEntry)) <= (size_t) kFinBytes, "a segment and its ids fit");
+            float    *wbuf = reinterpret_cast<float *>(cmem);
+            PenEntry *ids  = reinterpret_cast<PenEntry *>(wbuf + kSegMost);
             for (int i = g.tid; i < seg_n; i += g.n) {
                 wbuf[i] = prologue_one(src[i], s0c + e0 + i, r.cap, r.mrow);
             }
@@ -1871,7 +1873,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             }
             g.sync();
             if (seg_n > 0) {
-                st |= apply_penalties(g, wbuf, s0c + e0, seg_n, r, p.V, p.vocab_offset, sh->fin_bitmap, sh->fdlist, min(p.hist_cap, 512), &gs->n_dlist, false, 0);
+                st |= apply_penalties(g, wbuf, s0c + e0, seg_n, r, p.V, p.vocab_offset, sh->fin_bitmap, ids, kSegMost, &gs->n_dlist, false, 0);
             }
 #pragma unroll
             for (int q = 0; q < 4; q++) {

@@ -368,6 +368,19 @@ def test_temperature_draw_never_ends_on_a_masked_column(ctx):
     assert set(np.unique(g["tokens"])) == {999, 1024}
 
 
+@pytest.mark.parametrize("V", [8192, 8191, 16384])
+def test_temperature_segments_with_hundreds_of_counted_ids(ctx, V):
+    """8000 ids over segments of 1024 columns, with a penalty that counts: the crossing segment holds up to 660 distinct ones,
+    and in the last rows, whose ids are a run, every column of it."""
+    rows = 24
+    x = normal_logits(rows, V, 2.0, V)
+    h = histories(rows, 8000, V, V + 1)
+    h[-4:, :6000] = np.arange(6000) % V
+    st = independent_states(oracle.port, V, rows)
+    g = run_gpu(ctx, x, 1.0, 0, 1.0, st, rep=1.1, freq=0.1, pres=0.2, history=h)
+    check_tokens(g, oracle.port.sample_batch(x, 1.0, 0, 1.0, st, rep=1.1, freq=0.1, pres=0.2, hist=h))
+
+
 def _long_history_case(rows, V, stride, seed):
     """Histories of mixed lengths around the 128-id limit of the loader's register path, ids drawn
     from small pools so that most repeat, some rows with every id in one slice."""

@@ -1314,9 +1314,10 @@ struct __align__(16) FinishShared {
 
 constexpr int kGroupBytes = kGroupSlots * kThreads * 4; /* one maximum per slot and thread */
 constexpr int kListSmem   = kRowIdsMax;       /* id-list entries of a part that are kept in shared memory */
+constexpr int kRankWords  = 2 * (kHistBins + 1) + 3; /* what puts candidates in order, beside them */
 constexpr int kFinCap     = 2048;             /* candidates the finisher can order per row (8 per thread) */
-static_assert(kPartCand * (int) sizeof(Pair) + 2 * (kHistBins + 1) * 4 <= kGroupBytes, "a part's candidates are put in order there");
-constexpr int kFinBytes   = 2 * kFinCap * (int) sizeof(Pair) + 2 * (kHistBins + 1) * 4 + 8; /* finisher: the merged candidate list, what puts it in order; the multi-pass path keeps one byte histogram per warp there */
+static_assert(kPartCand * (int) sizeof(Pair) + kRankWords * 4 <= kGroupBytes, "a part's candidates are put in order there");
+constexpr int kFinBytes   = 2 * kFinCap * (int) sizeof(Pair) + (kRankWords + 1) * 4; /* finisher: the merged candidate list, what puts it in order; the multi-pass path keeps one byte histogram per warp there */
 static_assert(kFinBytes >= kWarps * 256 * 12, "a byte histogram per warp fits");
 constexpr int kFinGeneralBytes = sizeof(WideShared) > (size_t) kFinBytes ? (int) sizeof(WideShared) : kFinBytes; /* the general kernel works on wide rows there as well */
 static_assert(kGroupBytes >= 2 * kRowIdsMax * 8, "the id table of a part's set-up lies in the group maxima's memory");
@@ -1433,22 +1434,15 @@ __device__ __forceinline__ void rank_few(const Pair *cand, int total, int k, flo
     }
 }
 
-/* More than kRankFew candidates in order, the k best to out_s; they lie between lo and hi. They are dealt out to 256 bins of
- * values, the highest in front (srt takes them), and ranked against their own bin: one against all costs a thread block
- * total^2 / 32 rounds of six instructions. 1000 rows of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9;
- * 256 x 128256 top-k 200 48.9 -> 41.0. by_octave: bins of the values' bits, for probabilities (lo is not used); in even bins all but
- * a few share the last, and eight top-p rows of 19 parts took 67 us instead of 41. start: room for 2 * (kHistBins + 1) words. All threads call; the caller's barrier follows. */
-__device__ __noinline__ void rank_in_bins(const Pair *in, int total, int k, float lo, float hi, bool by_octave, Pair *srt, int *start, Pair *out_s) {
-    const int   tid = (int) threadIdx.x, lane = tid & 31;
-    int        *next  = start + kHistBins + 1;
-    if (by_octave) {
-        hi = (float) __float_as_int(hi);
-        lo = hi - (float) (20 << 23); /* what is a millionth of the largest or less shares the last bin */
-    }
-    const float scale = hi > lo && hi - lo < CUDART_INF_F ? (float) kHistBins / (hi - lo) : 0.0f; /* 0: one bin for all */
-    auto        bin_of = [&](float v) { return kHistBins - 1 - min(kHistBins - 1, max(0, __float2int_rz(((by_octave ? (float) __float_as_int(v) : v) - lo) * scale))); };
+/* `total` candidates dealt out to kHistBins bins, the highest in front, in srt; entry b of start: candidates in the bins before b.
+ * Whether the bin that the k-th falls into holds more than kRankMost. All threads call. */
+constexpr int kRankMost = 256; /* entries of that bin that are ranked against each other: dealing them out again costs as much */
+template <class Bin>
+__device__ __forceinline__ bool deal_out(const Pair *in, int total, int k, Pair *srt, int *start, Bin &&bin_of) {
+    const int tid = (int) threadIdx.x, lane = tid & 31;
+    int      *next = start + kHistBins + 1;
     for (int i = tid; i <= kHistBins; i += kThreads) {
-        start[i] = 0; /* entry b + 1: candidates in bin b; after the scan, entry b: candidates in the bins before b */
+        start[i] = 0; /* entry b + 1: candidates in bin b, until the scan */
     }
     __syncthreads();
     for (int i = tid; i < total; i += kThreads) {
@@ -1485,8 +1479,13 @@ __device__ __noinline__ void rank_in_bins(const Pair *in, int total, int k, floa
         const Pair me                           = in[i];
         srt[atomicAdd(&next[bin_of(me.v)], 1)] = me;
     }
-    __syncthreads();
-    for (int i = tid; i < total; i += kThreads) {
+    static_assert(kHistBins == kThreads, "a bin per thread");
+    return __syncthreads_or(start[tid] < k && start[tid + 1] - start[tid] > kRankMost) != 0; /* bins further up hold less than k */
+}
+/* What deal_out left, each candidate ranked against its own bin. */
+template <class Bin>
+__device__ __forceinline__ void rank_dealt(const Pair *srt, int total, int k, const int *start, Pair *out_s, Bin &&bin_of) {
+    for (int i = (int) threadIdx.x; i < total; i += kThreads) {
         const Pair me   = srt[i];
         const int  b    = bin_of(me.v), end = start[b + 1];
         int        rank = start[b];
@@ -1498,6 +1497,80 @@ __device__ __noinline__ void rank_in_bins(const Pair *in, int total, int k, floa
                 out_s[rank] = me;
             }
         }
+    }
+}
+/* Bins of keys: those from lo to hi, 2^shift each, are dealt out to bins 1 to 254, what lies above to bin 0. */
+struct KeyBins {
+    unsigned lo, hi;
+    int      shift;
+    __device__ __forceinline__ int operator()(float v) const {
+        const unsigned key = order_key(v);
+        return key > hi ? 0 : key < lo ? kHistBins - 1 : kHistBins - 2 - (int) ((key - lo) >> shift);
+    }
+};
+/* Bins of values from lo on, scale of them to a unit, the highest in front; by_octave: of the values' bits. */
+struct ValueBins {
+    float lo, scale;
+    bool  by_octave;
+    __device__ __forceinline__ int operator()(float v) const {
+        return kHistBins - 1 - min(kHistBins - 1, max(0, __float2int_rz(((by_octave ? (float) __float_as_int(v) : v) - lo) * scale)));
+    }
+};
+/* The bin of `first` that the k-th of the candidates dealt out falls into holds too many: it is cut again between its smallest and its
+ * largest key, until the bin that the k-th is in holds few, or equal ones. Fewer than k lie above it, what lies below is not ranked. Out of
+ * line: rare. */
+__device__ __noinline__ void rank_crowded(const Pair *in, int total, int k, const ValueBins first, Pair *srt, int *start, Pair *out_s) {
+    const int tid  = (int) threadIdx.x;
+    unsigned *ends = reinterpret_cast<unsigned *>(start + 2 * (kHistBins + 1)); /* smallest and largest key of the bin, and which it is */
+    KeyBins   bins{0u, 0u, -1};
+    do {
+        if (start[tid] < k && start[tid + 1] >= k) {
+            ends[0] = 0xffffffffu;
+            ends[1] = 0u;
+            ends[2] = (unsigned) tid;
+        }
+        __syncthreads();
+        const int b  = (int) ends[2];
+        unsigned  lo = 0xffffffffu, hi = 0u;
+        for (int i = tid; i < total; i += kThreads) {
+            const float v = in[i].v;
+            if ((bins.shift < 0 ? first(v) : bins(v)) == b) {
+                lo = min(lo, order_key(v));
+                hi = max(hi, order_key(v));
+            }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if ((tid & 31) == 0) {
+            atomicMin(&ends[0], lo);
+            atomicMax(&ends[1], hi);
+        }
+        __syncthreads();
+        bins.lo              = ends[0];
+        bins.hi              = ends[1];
+        const unsigned range = bins.hi - bins.lo;
+        bins.shift           = max(0, 32 - __clz(range) - 8);
+        bins.shift += (range >> bins.shift) > (unsigned) (kHistBins - 3) ? 1 : 0;
+    } while (deal_out(in, total, k, srt, start, bins) && bins.shift > 0);
+    rank_dealt(srt, total, k, start, out_s, bins);
+}
+/* More than kRankFew candidates in order, the k best to out_s; they lie between lo and hi. They are dealt out to 256 bins of
+ * values, the highest in front (srt takes them), and ranked against their own bin: one against all costs a thread block
+ * total^2 / 32 rounds of six instructions. 1000 rows of 8192, us: top-k 128 54.3 -> 45.8, 200 81.5 -> 53.7, 250 105 -> 59.9;
+ * 256 x 128256 top-k 200 48.9 -> 41.0. by_octave: bins of the values' bits, for probabilities (lo is not used); in even bins all but
+ * a few share the last, and eight top-p rows of 19 parts took 67 us instead of 41. A value far above the rest does the same to the bins
+ * of values: rank_crowded (64 x 32000 with a value of 4000 in each row, top-k 256: 197 us without it, 30; 8 x 128256, top-k 129: 248 and 27).
+ * start: room for kRankWords words. All threads call; the caller's barrier follows. */
+__device__ __noinline__ void rank_in_bins(const Pair *in, int total, int k, float lo, float hi, bool by_octave, Pair *srt, int *start, Pair *out_s) {
+    if (by_octave) {
+        hi = (float) __float_as_int(hi);
+        lo = hi - (float) (20 << 23); /* what is a millionth of the largest or less shares the last bin */
+    }
+    const ValueBins bins{lo, hi > lo && hi - lo < CUDART_INF_F ? (float) kHistBins / (hi - lo) : 0.0f, by_octave}; /* 0: one bin for all */
+    if (deal_out(in, total, k, srt, start, bins)) {
+        rank_crowded(in, total, k, bins, srt, start, out_s);
+    } else {
+        rank_dealt(srt, total, k, start, out_s, bins);
     }
 }
 

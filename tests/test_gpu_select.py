@@ -121,3 +121,31 @@ def test_narrow_nuclei_and_temperature_of_parts(ctx, rows, V):
     if rows < 10:
         z = normal_logits(rows, 300000, 2.0, V)
         check_tokens(run_gpu(ctx, z, 1.0, 0, 1.0, st), oracle.port.sample_batch(z, 1.0, 0, 1.0, st))
+
+
+@pytest.mark.parametrize("k", [40, 129, 200, 256])
+@pytest.mark.parametrize("V", [4096, 20011, 128256])
+def test_candidates_crowded_into_few_bins(ctx, V, k):
+    """Many candidates that all but a few values push into one bin of values, and into few of keys: values far above the rest, of every
+    size; two clusters a few bits wide; values around zero under one far above; hundreds that are equal. Whole rows, and rows whose
+    parts are merged. Drawn nearly evenly, so that every place counts."""
+    for rows, hint in [(300 if V < 10000 else 24, 1), (24, 0)]:
+        rg = np.random.default_rng(V + k)
+        x = normal_logits(rows, V, 2.5, V + k)
+        T = np.full(rows, 4.0, np.float32)
+        far = rg.integers(0, V, rows)
+        x[np.arange(0, rows, 6), far[0::6]] = 4000.0
+        x[np.arange(1, rows, 6), far[1::6]] = 1e30
+        x[2::6] = np.float32(7.0) + rg.integers(0, 2 * V, x[2::6].shape).astype(np.float32) * np.float32(2.0 ** -21)
+        x[np.arange(2, rows, 6), far[2::6]] = 3e38
+        x[3::6] = np.where(rg.random(x[3::6].shape) < 0.5, np.float32(-2.0), np.float32(5.0)) + rg.integers(0, 64, x[3::6].shape).astype(np.float32) * np.float32(2.0 ** -20)
+        x[np.arange(3, rows, 6), far[3::6]] = 100.0
+        x[4::6] = np.where(rg.random(x[4::6].shape) < 400.0 / V, normal_logits(1, V, 0.01, V), np.float32(-3.0))
+        x[np.arange(4, rows, 6), far[4::6]] = 50.0
+        x[5::6] = np.where(rg.random(x[5::6].shape) < 600.0 / V, np.float32(1.0), x[5::6] - np.float32(20.0))
+        st = independent_states(oracle.port, V + k, rows)
+        g = run_gpu(ctx, x, T, k, 1.0, st, finish_hint=hint)
+        done = (g["status"] & 32) == 0
+        assert done.all() or (hint == 1 and done.sum() >= rows // 6)  # parts' candidates that outrun the small kernel's list ask for the other one
+        o = oracle.port.sample_batch(x, T, k, 1.0, st)
+        assert np.array_equal(g["tokens"][done], o["tokens"][done])

@@ -1309,6 +1309,7 @@ struct __align__(16) FinishShared {
     alignas(16) unsigned long long stage[kStageWords]; /* the records and first candidates of the row's parts */
     unsigned long long save[256 + 128];                      /* the multi-pass path keeps a histogram here */
     RowCfg      cfg;    /* the row's: in registers it had left none for the code that finishes it */
+    unsigned long long rng0; /* the generator word that the row's sequence came with */
     double      wide_S; /* a top-p row that the candidates could not serve: its sum, 0 where it is not known */
 };
 
@@ -1651,16 +1652,33 @@ __device__ __forceinline__ int draw_sorted(int lane, const float *q, int k, floa
 
 /* ---------------------------------------------------------------- finisher -- */
 
+/* A row's parameters, for all threads of the finishing thread block that takes it, behind a barrier. One thread. */
+__device__ __forceinline__ void configure_row(const SampleParams &p, FinishShared *sh, int row, const RawCfg &rc) {
+    RowCfg r = row_config(p, row, rc, true);
+    if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
+        r.cap    = 0.0f;
+        r.mrow   = nullptr;
+        r.pen_on = false;
+    }
+    sh->cfg  = r;
+    sh->rng0 = rc.rng;
+}
+/* Nobody has to wait for a row of another kind. The same thread. */
+template <bool kFast>
+__device__ __forceinline__ void not_wide(const SampleParams &p, const FinishShared *sh) {
+    if (!kFast && sh->cfg.mode != M_TOPP) {
+        atomicAdd(&p.wide_head->rows, 1ull);
+    }
+}
+
 /*
  * One row, all threads of a finishing thread block. Merges the parts' records, then by mode: argmax; temperature
  * (segment sums, then the crossing segment re-read and walked); top-k / top-p over the merged candidates. cmem:
- * room for the merged list. Returns the row's status bits (ST_DEFERRED: the multi-pass path has to serve it).
+ * room for the merged list. first: the thread block's. Returns the row's status bits (ST_DEFERRED: the multi-pass path has to serve it).
  */
 template <bool kFast>
-__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, int n_parts, unsigned char *cmem) {
-    const RowCfg &r    = sh->cfg;
-    const int  row     = r.row;
-    unsigned long long rng = r.rng;
+__device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, FinishShared *sh, int row, int n_parts, bool first, bool temp, unsigned char *cmem) {
+    const RowCfg &r    = sh->cfg; /* the thread block's first row's is there, any other's behind the second barrier */
     int       *kept_i  = p.kept_cap > 0 ? p.kept_idx + (size_t) row * (size_t) p.kept_cap : nullptr;
     float     *kept_v  = p.kept_cap > 0 ? p.kept_val + (size_t) row * (size_t) p.kept_cap : nullptr;
     Pair      *cbuf    = reinterpret_cast<Pair *>(cmem);
@@ -1683,16 +1701,28 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     };
     constexpr int      kOwnWords = kStageWords / kThreads;
     unsigned long long tv[kOwnWords];
-    const bool         by_segs = !kFast && r.mode == M_TEMP && p.n_slices * kWarps <= kThreads; /* a segment per thread: asked for with the records */
-    float              seg_ref = 0.0f;
-    double             seg_sum = 0.0;
+    /* a segment per thread: asked for with the records, where the first row, or the one before any other, is a temperature row (temp); a
+     * temperature row behind one of another kind reads its segments further down, as rows of more segments do */
+    const bool by_segs = !kFast && temp && p.n_slices * kWarps <= kThreads;
+    float      seg_ref = 0.0f;
+    double     seg_sum = 0.0;
     {
-        /* one round trip: the records and the first candidates of the parts, whatever their counts are */
+        /* one round trip: the records and the first candidates of the parts, whatever their counts are, and the parameters of a row
+         * behind the first (with a round trip of their own, 2000 x 16384 top-k 40, unhinted: 87.8 us, 82.3 so) */
 #pragma unroll
         for (int q = 0; q < kStageWords / kThreads; q++) {
             int       i;
             const int t = g.tid + q * kThreads, k = part_of(t, i);
             tv[q]       = q * kThreads < st_parts * st_w && k < st_parts ? __ldcg(reinterpret_cast<const unsigned long long *>(part_rec(p, row, k)) + 4 + i) : 0ull;
+        }
+        if (by_segs && g.tid < p.n_slices * kWarps) {
+            const SegRec *seg = p.segs + (size_t) row * (size_t) (p.n_slices * kWarps) + g.tid;
+            seg_ref           = __ldcg(&seg->ref);
+            seg_sum           = __ldcg(&seg->sum);
+        }
+        RawCfg rc{};
+        if (!first && g.tid == 0) {
+            rc = raw_config(p, row, true);
         }
 #pragma unroll
         for (int q = 0; q < kStageWords / kThreads; q++) {
@@ -1700,13 +1730,13 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 sh->stage[g.tid + q * kThreads] = tv[q];
             }
         }
-        if (by_segs && g.tid < p.n_slices * kWarps) {
-            const SegRec *seg = p.segs + (size_t) row * (size_t) (p.n_slices * kWarps) + g.tid;
-            seg_ref           = __ldcg(&seg->ref);
-            seg_sum           = __ldcg(&seg->sum);
+        if (!first && g.tid == 0) {
+            configure_row(p, sh, row, rc);
+            not_wide<kFast>(p, sh);
         }
     }
     g.sync();
+    unsigned long long rng = r.rng;
     if (n_parts > kMaxParts) {
         /* a row spread over that many thread blocks (a handful of rows on the whole chip): its maximum is
          * taken from the records one by one, everything else is left to the multi-pass path */
@@ -1821,7 +1851,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
         };
         int    found = -1;
         double u, fbase = -CUDART_INF; /* nothing crosses: the walk ends on its last id */
-        if (nseg <= kThreads) {
+        if (by_segs) {
             /* a segment per thread: its sum is read and moved once, the scan's total is the row's sum */
             const double val  = g.tid < nseg ? seg_sum * ref_move(seg_ref, row_max, r.inv_t) : 0.0;
             double       incl = val;
@@ -3839,43 +3869,35 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     g.bar  = 0;
     /* The first row's parameters are inputs of the launch, written before the stream kernel began: they may be
      * read while that kernel's last thread blocks are still at work. Everything it wrote waits for the line below. */
-    auto parts_of = [&](int row) { return cta_of_item(p, row * p.n_slices + p.n_slices - 1) - cta_of_item(p, row * p.n_slices) + 1; };
-    unsigned long long rng0    = 0ull; /* the generator word that the row's sequence came with */
-    int                n_parts = 0;
-    auto               configure = [&](int row) { /* the barrier in front of a row lies behind the last use of its predecessor's */
-        const RawCfg rc = raw_config(p, row, true);
-        RowCfg       r  = row_config(p, row, rc, true);
-        if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
-            r.cap    = 0.0f;
-            r.mrow   = nullptr;
-            r.pen_on = false;
-        }
-        rng0    = rc.rng;
-        n_parts = parts_of(row);
+    const RunMap &m        = p.map;
+    auto          parts_of = [&](int row) { /* over how many thread blocks the row was spread */
+        const int i = row * p.n_slices;
+        return m.mode == RUN_ROWS ? 1 : m.mode == RUN_PARTS ? m.P : run_of(i + p.n_slices - 1, m.q, m.r) - run_of(i, m.q, m.r) + 1;
+    };
+    const bool owns    = (int) blockIdx.x < p.n_rows;
+    int        n_parts = owns ? parts_of((int) blockIdx.x) : 0;
+    if (owns) {
+        const RawCfg rc = raw_config(p, (int) blockIdx.x, true);
         if (g.tid == 0) {
-            sh->cfg = r;
+            configure_row(p, sh, (int) blockIdx.x, rc);
         }
         __syncthreads();
-    };
-    if ((int) blockIdx.x < p.n_rows) {
-        configure((int) blockIdx.x);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory"); /* the records of the kernel before this one are complete and visible */
     asm volatile("griddepcontrol.launch_dependents;");
     PROF(kFast ? 5 : 7);
     /* the launch has top-p rows: the stream kernel has said so; wanted when the block's own rows are done */
     const bool any = !kFast && *reinterpret_cast<volatile const unsigned *>(&p.wide_head->any) == p.launch;
+    if (!kFast && g.tid == 0 && owns && sh->cfg.mode != M_TOPP) {
+        atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
+    }
     for (int row = (int) blockIdx.x; row < p.n_rows; row += (int) gridDim.x) {
-        if (row != (int) blockIdx.x) {
-            configure(row);
+        const bool first = row == (int) blockIdx.x, temp = sh->cfg.mode == M_TEMP; /* the row's, or the one's before it */
+        if (!first) {
+            n_parts = parts_of(row);
         }
         PROF(8);
-        if constexpr (!kFast) {
-            if (g.tid == 0 && sh->cfg.mode != M_TOPP) {
-                atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
-            }
-        }
-        int st = finish_row<kFast>(g, p, sh, n_parts, cmem);
+        int st = finish_row<kFast>(g, p, sh, row, n_parts, first, temp, cmem);
         PROF(13);
         if (st & ST_DEFERRED) {
             if constexpr (kFast) {
@@ -3892,9 +3914,8 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
             }
         }
         if (g.tid == 0) {
-            row_epilogue(p, sh->cfg, row, st, rng0);
+            row_epilogue(p, sh->cfg, row, st, sh->rng0);
         }
-        __syncthreads();
     }
     if constexpr (!kFast) {
         /* Else there is nothing to help with, and the blocks that have no row end where they begin. (They watched three

@@ -255,6 +255,27 @@ def test_mixed_modes_in_one_launch(ctx):
     check_tokens(g, o)
 
 
+@pytest.mark.parametrize("rows,V", [(700, 3000), (1300, 9001), (330, 40000)])
+@pytest.mark.parametrize("kinds", [0, 1])
+def test_rows_of_all_kinds_behind_one_another(ctx, rows, V, kinds):
+    """More rows than finishing thread blocks: each takes several, of kinds that follow one another in every order (or greedy and
+    top-k rows alone, by the small kernel), their settings through a slot table."""
+    rg = np.random.default_rng(rows + V)
+    x = normal_logits(rows, V, 2.5, V)
+    n = rows + 50
+    T = np.where(rg.random(n) < 0.2, 0.0, rg.choice([0.5, 0.9], n)).astype(np.float32)
+    K = rg.choice([0, 0, 2, 40, 200] if not kinds else [2, 40, 64, 200], n).astype(np.int32)
+    P = rg.choice([1.0, 0.6, 0.95], n).astype(np.float32)
+    slot = rg.permutation(n)[:rows].astype(np.int32)
+    st = independent_states(oracle.port, V, n)
+    dev = to_dev(x), to_dev(T), to_dev(K), to_dev(P), u64_to_dev(st)
+    out = ctx.sample_batch(*dev, slot=to_dev(slot), finish_hint=kinds)
+    o = oracle.port.sample_batch(x, T[slot], K[slot], P[slot], st[slot])
+    assert (out["status"].cpu().numpy() & (INVALID | 32) == 0).all()
+    assert np.array_equal(out["tokens"].cpu().numpy(), o["tokens"])
+    assert np.array_equal(u64_from_dev(out["rng_state"])[slot], o["rng_state"])
+
+
 def test_mixed_modes_large_batch_with_penalties(ctx):
     """Several hundred rows, all four modes interleaved row by row, two rows per generator, histories
     of different lengths: every CTA meets rows of every kind back to back."""

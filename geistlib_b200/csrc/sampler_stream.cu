@@ -1708,7 +1708,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
     double     seg_sum = 0.0;
     {
         /* one round trip: the records and the first candidates of the parts, whatever their counts are, and the parameters of a row
-         * behind the first (with a round trip of their own, 2000 x 16384 top-k 40, unhinted: 87.8 us, 82.3 so) */
+         * behind the first (with a round trip of their own: 2000 x 16384 top-k 40, unhinted, 87.8 us, so 82.3) */
 #pragma unroll
         for (int q = 0; q < kStageWords / kThreads; q++) {
             int       i;
@@ -3642,20 +3642,24 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             }
             __syncthreads();
         }
-        if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
-            /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
-             * part); a row of another kind is reported as the small finishing kernel would */
-            if (mode == M_TOPK) {
-                inline_finish_topk<true>(p, sh, gmem, row, n_cand, kq, tau, cap_late, inv_t, sh->st, part_again);
-            } else {
-                if (tid == 0) {
-                    p.tokens[row] = -1;
-                    p.status[row] = sh->st | ST_INTERNAL;
+        /* Rows are finished here in launches of greedy and top-k rows alone: the instantiations with sums carry none of it (with it, and
+         * the code behind it, a launch of one temperature row of 128256 takes 9.1 us and not 8.3) */
+        if constexpr ((kKinds & (K_SEL | K_SUMS)) == K_SEL) {
+            if ((p.flags & F_INLINE_TOPK) != 0u && mode != M_ARGMAX) {
+                /* whole rows, top-k: finished here, nothing goes to global scratch (every row of such a launch is one
+                 * part); a row of another kind is reported as the small finishing kernel would */
+                if (mode == M_TOPK) {
+                    inline_finish_topk<true>(p, sh, gmem, row, n_cand, kq, tau, cap_late, inv_t, sh->st, part_again);
+                } else {
+                    if (tid == 0) {
+                        p.tokens[row] = -1;
+                        p.status[row] = sh->st | ST_INTERNAL;
+                    }
+                    __syncthreads();
                 }
-                __syncthreads();
+                CYC(6);
+                continue;
             }
-            CYC(6);
-            continue;
         }
         if (sel && n_cand > kPartCand && tau > -CUDART_INF_F) {
             part_again();
@@ -3706,7 +3710,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             own_arg = h.y;
             own_st  = h.w;
         }
-        if ((p.flags & (F_GREEDY_ONLY | F_INLINE_TOPK)) != 0u && warp == 0) { /* in a launch that finishes its top-k rows here, the greedy ones are finished here as well */
+        if ((kKinds & K_SUMS) == 0 && (p.flags & (F_GREEDY_ONLY | F_INLINE_TOPK)) != 0u && warp == 0) { /* in a launch that finishes its top-k rows here, the greedy ones are finished here as well */
             /* The caller said that every row is greedy: no finishing kernel follows. A row that went through
              * this thread block as a whole is known here. A row cut into parts is finished by whichever of its
              * parts arrives last: every part publishes its record, then counts itself in; the one that finds

@@ -218,17 +218,19 @@ cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
  * the host puts kUnwritten there before it launches and looks until every one has changed. A word is written once a launch,
  * after everything its row reads of the caller's memory, so nothing of the caller's is in use behind the last of them; what
  * follows on the stream (the grid's end, the sessions' bookkeeping) is ordered before the next call's work as before. Every
- * 50 us the stream is asked as well: it ends the wait when it is through or has failed, whatever the words say.
+ * 50 us the stream is asked as well: it ends the wait when it is through or has failed, whatever the words say. Behind kLookFor
+ * the stream's own wait takes over, and it is all there is where the process chose waits that leave the core to others (`look`).
  * Against cudaStreamSynchronize, us a call: argmax slot 19.2 -> 15.5, a step of 8 top-p rows 40.0 -> 35.1, of 2 greedy rows 27.0 ->
  * 22.2, 32 verify calls of 7 rows 67.3 -> 63.5. Where the kernels of a call write one after the other, the last one's words are
  * looked at first: looking at lines that 224 rows were still writing to cost as much as the stream's wait.
  */
 constexpr int kUnwritten = INT_MIN;
+constexpr auto kLookFor  = std::chrono::microseconds(500); /* a call that takes longer gains nothing by a few us */
 template <class T>
-cudaError_t await_words(const T *words, size_t n, T unwritten, cudaStream_t st) {
-    size_t at   = 0;
-    auto   next = std::chrono::steady_clock::time_point{};
-    for (unsigned round = 1;; round++) {
+cudaError_t await_words(const T *words, size_t n, T unwritten, cudaStream_t st, bool look) {
+    size_t at = 0;
+    auto   next = std::chrono::steady_clock::time_point{}, last = next;
+    for (unsigned round = 1; look; round++) {
         while (at < n && __atomic_load_n(words + at, __ATOMIC_ACQUIRE) != unwritten) {
             at++;
         }
@@ -242,6 +244,9 @@ cudaError_t await_words(const T *words, size_t n, T unwritten, cudaStream_t st) 
             const auto now = std::chrono::steady_clock::now();
             if (round == 64) {
                 next = now + std::chrono::microseconds(50);
+                last = now + kLookFor;
+            } else if (now >= last) {
+                break;
             } else if (now >= next) {
                 const cudaError_t e = cudaStreamQuery(st);
                 if (e != cudaErrorNotReady) {
@@ -251,6 +256,7 @@ cudaError_t await_words(const T *words, size_t n, T unwritten, cudaStream_t st) 
             }
         }
     }
+    return cudaStreamSynchronize(st);
 }
 
 } /* namespace */
@@ -293,6 +299,7 @@ struct geist_b200_ctx {
     unsigned   next_lane = 0;
     int        last_lane = 0; /* that the last launch took */
     unsigned long long wide_wait_ns = kWideWaitNs;
+    bool       look = true; /* the process lets threads spin while they wait for the device */
     std::mutex lane_mu;
     std::mutex own_mu; /* the synchronous calls' set: from where a launch takes it to the launch itself */
 };
@@ -318,7 +325,12 @@ extern "C" enum geist_status geist_b200_ctx_create(int device, struct geist_b200
         return fail(GEIST_E_OOM, "ctx_create: host allocation");
     }
     c->device = device;
-    cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    unsigned    waits = 0;
+    cudaError_t e     = cudaGetDeviceFlags(&waits);
+    c->look           = (waits & (cudaDeviceScheduleYield | cudaDeviceScheduleBlockingSync)) == 0u;
+    if (e == cudaSuccess) {
+        e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    }
     if (e == cudaSuccess) {
         e = cudaMalloc(&c->d_small, sizeof(geist_b200_ctx::Small));
     }
@@ -829,9 +841,9 @@ geist_token_t sample_host_row(size_t n, const float *logits, float *staging, flo
         if (launch_batch(c, &b, c->stream, 0u, true) != GEIST_OK) {
             return -1;
         }
-        e = await_words(&h->token, 1, kUnwritten, c->stream);
-        e = e == cudaSuccess ? await_words(&h->status, 1, kUnwritten, c->stream) : e;
-        e = e == cudaSuccess ? await_words(&h->rng_out, 1, 0ull, c->stream) : e;
+        e = await_words(&h->token, 1, kUnwritten, c->stream, c->look);
+        e = e == cudaSuccess ? await_words(&h->status, 1, kUnwritten, c->stream, c->look) : e;
+        e = e == cudaSuccess ? await_words(&h->rng_out, 1, 0ull, c->stream, c->look) : e;
         if (e != cudaSuccess) {
             fail(GEIST_E_BACKEND, "sampler: %s", cudaGetErrorString(e));
             return -1;
@@ -945,8 +957,8 @@ extern "C" enum geist_status geist_b200_argmax_f32(struct geist_b200_ctx *ctx, c
     if (s != GEIST_OK) {
         return s;
     }
-    CUDA_TRY(await_words(&h->token, 1, kUnwritten, ctx->stream));
-    CUDA_TRY(await_words(&h->status, 1, kUnwritten, ctx->stream));
+    CUDA_TRY(await_words(&h->token, 1, kUnwritten, ctx->stream, ctx->look));
+    CUDA_TRY(await_words(&h->status, 1, kUnwritten, ctx->stream, ctx->look));
     if ((h->status & ~(GEIST_B200_ROW_SLOW_PATH | GEIST_B200_ROW_KEPT_PARTIAL)) != 0 || h->token < 0 || (size_t) h->token >= n) {
         return fail(GEIST_E_BACKEND, "argmax_f32: row status 0x%x, index %d", h->status, h->token);
     }
@@ -1528,13 +1540,13 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
         if (logits_on_host) { /* launches on other streams, with the sets that rotate: all of them are through when the call returns */
             CUDA_TRY(cudaStreamSynchronize(st));
         } else if (verify) { /* the accept kernel's words first: they come last, and until then nobody looks at a line that is written */
-            CUDA_TRY(await_words(h_nem, n, kUnwritten, st));
-            CUDA_TRY(await_words(h_acc, n, kUnwritten, st));
-            CUDA_TRY(await_words(h_emit, n * (k + 1), kUnwritten, st));
+            CUDA_TRY(await_words(h_nem, n, kUnwritten, st, b->ctx->look));
+            CUDA_TRY(await_words(h_acc, n, kUnwritten, st, b->ctx->look));
+            CUDA_TRY(await_words(h_emit, n * (k + 1), kUnwritten, st, b->ctx->look));
         } else {
-            CUDA_TRY(await_words(h_tok, n, kUnwritten, st));
+            CUDA_TRY(await_words(h_tok, n, kUnwritten, st, b->ctx->look));
         }
-        CUDA_TRY(await_words(h_stat, rows, kUnwritten, st));
+        CUDA_TRY(await_words(h_stat, rows, kUnwritten, st, b->ctx->look));
         bool retry = false;
         for (size_t i = 0; i < rows; i++) {
             if (h_stat[i] < 0 || h_stat[i] & (GEIST_B200_ROW_LOAD_TIMEOUT | GEIST_B200_ROW_HIST_OVERFLOW | GEIST_B200_ROW_INTERNAL)) {

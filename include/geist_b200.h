@@ -111,7 +111,10 @@ geist_token_t geist_sampler_top_p_ws(struct geist_sampler_workspace *ws, const f
  * hand out tokens on the host (the argmax slot, the sampler.h surface, the
  * batcher over device logits) are not among the four: they have a set of
  * their own and follow one another on the context's stream, also where a call
- * has returned before its last thread blocks have. */
+ * has returned before its last thread blocks have. Such a call looks at the
+ * words it waits for, for half a millisecond at most, and then leaves the wait
+ * to the CUDA runtime; it leaves it there from the start if the process had
+ * chosen cudaDeviceScheduleBlockingSync or Yield when the context was made. */
 struct geist_b200_ctx;
 
 enum geist_status geist_b200_ctx_create(int device, struct geist_b200_ctx **out);

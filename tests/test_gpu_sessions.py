@@ -271,3 +271,51 @@ def test_calls_in_a_row_commit_before_the_next_reads(ctx):
             state[1] = np.uint64(12345 + it)
             bt.set_rng(sess[1], 12345 + it)
     bt.close()
+
+
+def test_a_generator_that_never_leaves_zero():
+    """The word that a host row's generator comes to is 0, which is what the host waits to see changed: the call ends with the
+    stream."""
+    row = normal_logits(1, 9001, 2.0, 17)[0]
+    for _ in range(3):
+        rng = api.Rng(0)
+        tok, state = port.sampler_call("temperature", row, T=0.8, state=0)
+        assert api.sampler_temperature(row, 0.8, rng) == tok and rng.state == state == 0
+
+
+BLOCKING = """
+import ctypes, sys, time
+rt = ctypes.CDLL("libcudart.so.12")
+assert rt.cudaSetDeviceFlags(int(sys.argv[1])) == 0
+import numpy as np, torch
+from geistlib_b200 import api
+ctx = api.Context(0)
+n, V = 64, 128256
+bt = api.Batcher(ctx, V, n)
+sess = [bt.open(temperature=1.0, top_p=0.9, seed=1 + i) for i in range(n)]
+x = torch.zeros(n, V, device="cuda")  # one value: the multi-pass path, milliseconds
+torch.cuda.synchronize()
+first = bt.step(sess, x)
+wall, cpu = time.perf_counter(), time.thread_time()
+for _ in range(8):
+    bt.step(sess, x)
+print(time.perf_counter() - wall, time.thread_time() - cpu, *first)
+"""
+
+
+def test_waits_leave_the_core_where_the_process_says_so():
+    """cudaDeviceScheduleBlockingSync, chosen before the context is made: a step that takes milliseconds does not spin through
+    them. The tokens are those of a process that does."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    out = {}
+    for flags in (4, 0):
+        r = subprocess.run([sys.executable, "-c", BLOCKING, str(flags)], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr[-2000:]
+        v = r.stdout.split()
+        out[flags] = float(v[0]), float(v[1]), v[2:]
+    assert out[4][2] == out[0][2]
+    wall, cpu, _ = out[4]
+    assert wall > 8 * 0.5e-3  # longer than the host looks by itself
+    assert cpu < 0.5 * wall, (wall, cpu)

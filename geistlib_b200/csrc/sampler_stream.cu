@@ -2353,7 +2353,7 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
                 }
                 const float    p_floor = __shfl_sync(0xffffffffu, e.v, kq - 1); /* nothing outside fsort has a larger p */
                 const unsigned reached = __ballot_sync(0xffffffffu, g.lane < kq && cum >= (double) r.top_p);
-                const bool     all_in  = kq >= p.V;
+                const bool     all_in  = kq >= p.V && __shfl_sync(0xffffffffu, cum, kq - 1) >= 0.0; /* no numbers: nothing of this is in order */
                 /* never reached top_p: the nucleus is the whole row, if all of it is here */
                 const int      cut = reached != 0u ? __ffs(reached) : (all_in ? kq : -1);
                 const float    p_cut = __shfl_sync(0xffffffffu, e.v, max(cut - 1, 0));

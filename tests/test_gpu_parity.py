@@ -672,6 +672,25 @@ def test_nan_in_a_summed_row(ctx, V, P):
         check_tokens(run_gpu(ctx, x, 0.9, 0, P, st, finish_hint=hint), o)
 
 
+@pytest.mark.parametrize("V", [2, 5, 20, 31, 32, 33, 1000, 9001])
+@pytest.mark.parametrize("K,P", [(0, 1.0), (0, 0.9), (2, 1.0), (30, 1.0)])
+def test_infinite_logits(ctx, V, K, P):
+    """One or two values of +inf: their weights are no numbers, nor is any sum. A summed row's walk ends on the last id, a top-k row's
+    on the last that is kept; the rows between them are drawn as ever. (Rows of at most 32 ids hold all of them in the top-p
+    probe's list.)"""
+    rows = 40
+    x = normal_logits(rows, V, 2.0, V)
+    x[0::4, V // 2] = np.inf
+    x[2::8, 0] = np.inf
+    x[2::8, V - 1] = np.inf
+    st = independent_states(oracle.port, V, rows)
+    o = oracle.port.sample_batch(x, 0.9, K, P, st)
+    if K == 0 or K >= V:
+        assert (o["tokens"][[0, 2, 4, 8]] == V - 1).all()
+    for hint in (0, 2) if K == 0 else (0,):
+        check_tokens(run_gpu(ctx, x, 0.9, K, P, st, finish_hint=hint), o)
+
+
 @pytest.mark.parametrize("H", [200, 1000, 1500])
 @pytest.mark.parametrize("V", [4096, 32768, 40000, 70001])
 def test_candidates_among_many_ids(ctx, V, H):

@@ -1529,13 +1529,17 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
         } else {
             std::fill(h_tok, h_tok + n, kUnwritten);
         }
-        const enum geist_status ls = launch_sampling(attempt == 0);
-        if (ls != GEIST_OK) {
-            return ls;
+        enum geist_status ls = launch_sampling(attempt == 0);
+        if (ls == GEIST_OK && verify) {
+            gb::AcceptParams  ap{h_fed, b->d_tokens, (int) n, (int) k, h_acc, h_nem, h_emit};
+            const cudaError_t e = gb::launch_accept(ap, st);
+            ls                  = e == cudaSuccess ? ls : fail(GEIST_E_BACKEND, "batcher: accept: %s", cudaGetErrorString(e));
         }
-        if (verify) {
-            gb::AcceptParams ap{h_fed, b->d_tokens, (int) n, (int) k, h_acc, h_nem, h_emit};
-            CUDA_TRY(gb::launch_accept(ap, st));
+        if (ls != GEIST_OK) { /* what has been launched of the call still writes its words: not into the next call's, which are the same */
+            cudaStreamSynchronize(b->copy_stream[0]);
+            cudaStreamSynchronize(b->copy_stream[1]);
+            cudaStreamSynchronize(st);
+            return ls;
         }
         if (logits_on_host) { /* launches on other streams, with the sets that rotate: all of them are through when the call returns */
             CUDA_TRY(cudaStreamSynchronize(st));

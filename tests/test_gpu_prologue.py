@@ -379,8 +379,8 @@ def test_softcapped_rows_stay_on_the_short_path(ctx, V):
 @pytest.mark.parametrize("V,rows", [(8200, 12), (40004, 6), (100004, 300), (262144, 3)])
 @pytest.mark.parametrize("c", [0.5, 30.0])
 def test_masked_rows_capped_behind_the_select(ctx, V, rows, c):
-    """Top-k rows under a cap and a mask: shares of a slice that begin inside a word of the mask, rows with few allowed columns
-    (the cap of a masked column is not -inf), and caps that most of a row reaches."""
+    """Top-k rows under a cap and a mask: shares of a slice that begin inside a word of the mask, and rows with few allowed columns
+    (the cap of a masked column is not -inf). What is kept at caps that rows come close to: the two tests below."""
     rg = np.random.default_rng(V + rows)
     x = normal_logits(rows, V, 2.5, V)
     allowed = rg.random((rows, V)) < 0.5
@@ -408,3 +408,40 @@ def test_masked_rows_capped_behind_the_select(ctx, V, rows, c):
             done = (status & 32) == 0  # row 0: more columns of value -inf at its parts' thresholds than a list holds
             assert done[1:].all() and (hint or done[0])
             assert np.mean((got[hint] == o["tokens"])[done]) >= (1.0 if rows < 100 else 0.99)
+
+
+@pytest.mark.parametrize("V,rows", [(8200, 300), (40004, 24), (100004, 300), (262144, 12)])
+@pytest.mark.parametrize("c", [1.5, 3.0])
+def test_kept_values_close_below_the_cap(ctx, V, rows, c):
+    """Caps near the rows' largest values, which crowd below them: every row is served by the select, and keeps all ids whose
+    capped value is above the k-th by more than the device's and the host's tanhf can differ, and none that is below it by that."""
+    k, x = 40, normal_logits(rows, V, 2.5, V) * np.float32(min(1.0, 5.0 * c / (2.5 * 5.3)))  # the largest at about 5 c, where tanh is 1 - 1e-4
+    allowed = np.random.default_rng(V).random((rows, V)) < 0.5
+    y = np.where(allowed, np.tanh(x.astype(np.float64) / c) * c, -np.inf)
+    kth = -np.partition(-y, k - 1, axis=1)[:, k - 1]
+    tol = c * 2.0 ** -20  # tanhf, the quotient and the product: 2^-21 of c, on either side of the comparison
+    st = np.array([oracle.port.rng_seed(5 + i) for i in range(rows)], np.uint64)
+    dT, dK, dP = per_seq(rows, 0.5, k, 1.0)
+    for hint in (0, 1):
+        out = ctx.sample_batch(to_dev(x), dT, dK, dP, u64_to_dev(st), softcap=cap_dev(rows, c), logit_mask=to_dev(mask_words(allowed)), kept_cap=k, finish_hint=hint)
+        assert (out["status"].cpu().numpy() == 0).all()
+        for r, kept in enumerate(out["kept_idx"].cpu().numpy()):
+            assert len(set(kept)) == k and (y[r, kept] >= kth[r] - tol).all()
+            assert set(np.nonzero(y[r] > kth[r] + tol)[0]) <= set(kept)
+
+
+@pytest.mark.parametrize("V,rows", [(8200, 12), (40004, 6), (100004, 300), (262144, 3)])
+def test_rows_whose_kept_ids_all_reach_the_cap(ctx, V, rows):
+    """A few per cent of every row come to the cap itself: the k first of them by id are kept, with equal weights. No value lies where
+    a tanhf that is good to 2 ulp may or may not come to 1: 2 e^(-2z) is 2.5 * 2^-24 at z = 8.2 and 2^-25 at 9.01. So tokens are those of
+    the checker."""
+    c, k = 0.5, 40
+    x = normal_logits(rows, V, 2.5, V)
+    x[(x > 8.1 * c) & (x < 9.5 * c)] = np.float32(10.0 * c)
+    allowed = np.random.default_rng(V).random((rows, V)) < 0.5
+    y = np.where(allowed, np.tanh(x.astype(np.float64) / c).astype(np.float32) * np.float32(c), np.float32(-np.inf)).astype(np.float32)
+    assert ((y == c).sum(axis=1) > k).all()
+    st = np.array([oracle.port.rng_seed(5 + i) for i in range(rows)], np.uint64)
+    o = oracle.port.sample_batch(y, 0.5, k, 1.0, st)
+    g = run_gpu(ctx, x, 0.5, k, 1.0, st, softcap=cap_dev(rows, c), logit_mask=to_dev(mask_words(allowed)))
+    assert np.array_equal(g["tokens"], o["tokens"])

@@ -1450,6 +1450,10 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
     d.logit_mask_stride  = b->mask_words;
     d.finish_hint        = hint;
 
+    /* host logits are copied and sampled in chunks on two streams; a call of one chunk stays on the context's */
+    const size_t seq_chunk = std::max<size_t>(1, (32 + k - 1) / k);
+    const bool   chunked   = logits_on_host && n > seq_chunk;
+
     /* the sampling launch(es); run a second time without the hint when a row asked for that */
     auto launch_sampling = [&](bool copy_in) -> enum geist_status {
         if (!logits_on_host) {
@@ -1474,13 +1478,14 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
                 CUDA_TRY(cudaMalloc((void **) &b->d_logits, rows * b->V * sizeof(float)));
                 b->d_logits_cap = rows * b->V;
             }
-            CUDA_TRY(cudaEventRecord(b->ev[0], st)); /* slots / fed are on the way */
-            const size_t seq_chunk = std::max<size_t>(1, (32 + k - 1) / k);
-            int          which     = 0;
+            if (chunked) {
+                CUDA_TRY(cudaEventRecord(b->ev[0], st)); /* slots / fed are on the way */
+            }
+            int which = 0;
             for (size_t s0 = 0; s0 < n; s0 += seq_chunk, which ^= 1) {
                 const size_t ns = std::min(seq_chunk, n - s0);
-                cudaStream_t cs = b->copy_stream[which];
-                if (s0 < 2 * seq_chunk) {
+                cudaStream_t cs = chunked ? b->copy_stream[which] : st;
+                if (chunked && s0 < 2 * seq_chunk) {
                     CUDA_TRY(cudaStreamWaitEvent(cs, b->ev[0], 0));
                 }
                 if (!copy_in) {
@@ -1497,12 +1502,12 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
                 d.fed_tokens = (pen && verify) ? b->d_fed + s0 * k : nullptr;
                 d.tokens     = tok_dst + s0 * k;
                 d.row_status = h_stat + s0 * k;
-                enum geist_status s = launch_batch(b->ctx, &d, cs, any_top_p ? 0u : gb::F_NO_TOP_P);
+                enum geist_status s = launch_batch(b->ctx, &d, cs, any_top_p ? 0u : gb::F_NO_TOP_P, !chunked);
                 if (s != GEIST_OK) {
                     return s;
                 }
             }
-            for (int i = 0; i < 2; i++) {
+            for (int i = 0; chunked && i < 2; i++) {
                 CUDA_TRY(cudaEventRecord(b->ev[1], b->copy_stream[i]));
                 CUDA_TRY(cudaStreamWaitEvent(st, b->ev[1], 0));
             }
@@ -1541,7 +1546,7 @@ enum geist_status batcher_run(geist_b200_batcher *b, size_t n, const int32_t *se
             cudaStreamSynchronize(st);
             return ls;
         }
-        if (logits_on_host) { /* launches on other streams, with the sets that rotate: all of them are through when the call returns */
+        if (chunked) { /* launches on other streams, with the sets that rotate: all of them are through when the call returns */
             CUDA_TRY(cudaStreamSynchronize(st));
         } else if (verify) { /* the accept kernel's words first: they come last, and until then nobody looks at a line that is written */
             CUDA_TRY(await_words(h_nem, n, kUnwritten, st, b->ctx->look));

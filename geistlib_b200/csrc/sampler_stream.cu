@@ -1652,18 +1652,17 @@ __device__ __forceinline__ int draw_sorted(int lane, const float *q, int k, floa
 
 /* ---------------------------------------------------------------- finisher -- */
 
-/* A row's parameters, for all threads of the finishing thread block that takes it, behind a barrier. One thread. */
-__device__ __forceinline__ void configure_row(const SampleParams &p, FinishShared *sh, int row, const RawCfg &rc) {
+/* A row's parameters, as the finishing kernels need them. */
+__device__ __forceinline__ RowCfg finish_config(const SampleParams &p, int row, const RawCfg &rc) {
     RowCfg r = row_config(p, row, rc, true);
     if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
         r.cap    = 0.0f;
         r.mrow   = nullptr;
         r.pen_on = false;
     }
-    sh->cfg  = r;
-    sh->rng0 = rc.rng;
+    return r;
 }
-/* Nobody has to wait for a row of another kind. The same thread. */
+/* Nobody has to wait for a row of another kind. The thread that has written its parameters. */
 template <bool kFast>
 __device__ __forceinline__ void not_wide(const SampleParams &p, const FinishShared *sh) {
     if (!kFast && sh->cfg.mode != M_TOPP) {
@@ -1731,7 +1730,8 @@ __device__ __forceinline__ int finish_row(const Grp &g, const SampleParams &p, F
             }
         }
         if (!first && g.tid == 0) {
-            configure_row(p, sh, row, rc);
+            sh->cfg  = finish_config(p, row, rc);
+            sh->rng0 = rc.rng;
             not_wide<kFast>(p, sh);
         }
     }
@@ -3807,12 +3807,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
 __device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *sh, unsigned char *cmem, int row, int st) {
     const Grp    g  = whole_block();
     const RawCfg rc = raw_config(p, row, true);
-    RowCfg       r  = row_config(p, row, rc, true);
-    if (p.out_logits != nullptr) { /* read back as it is sampled from (row_again) */
-        r.cap    = 0.0f;
-        r.mrow   = nullptr;
-        r.pen_on = false;
-    }
+    const RowCfg r  = finish_config(p, row, rc);
     const float bm = sh->gs.blk_max;
     const int   ba = sh->gs.blk_arg;
     if (g.tid == 0) {
@@ -3882,8 +3877,10 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     int        n_parts = owns ? parts_of((int) blockIdx.x) : 0;
     if (owns) {
         const RawCfg rc = raw_config(p, (int) blockIdx.x, true);
+        const RowCfg r  = finish_config(p, (int) blockIdx.x, rc);
         if (g.tid == 0) {
-            configure_row(p, sh, (int) blockIdx.x, rc);
+            sh->cfg  = r;
+            sh->rng0 = rc.rng;
         }
         __syncthreads();
     }
@@ -3892,8 +3889,8 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
     PROF(kFast ? 5 : 7);
     /* the launch has top-p rows: the stream kernel has said so; wanted when the block's own rows are done */
     const bool any = !kFast && *reinterpret_cast<volatile const unsigned *>(&p.wide_head->any) == p.launch;
-    if (!kFast && g.tid == 0 && owns && sh->cfg.mode != M_TOPP) {
-        atomicAdd(&p.wide_head->rows, 1ull); /* nobody has to wait for it */
+    if (g.tid == 0 && owns) {
+        not_wide<kFast>(p, sh);
     }
     for (int row = (int) blockIdx.x; row < p.n_rows; row += (int) gridDim.x) {
         const bool first = row == (int) blockIdx.x, temp = sh->cfg.mode == M_TEMP; /* the row's, or the one's before it */
@@ -3920,6 +3917,7 @@ __global__ void __launch_bounds__(kThreads, 2) finish_rows_kernel(const __grid_c
         if (g.tid == 0) {
             row_epilogue(p, sh->cfg, row, st, sh->rng0);
         }
+        __syncthreads();
     }
     if constexpr (!kFast) {
         /* Else there is nothing to help with, and the blocks that have no row end where they begin. (They watched three

@@ -109,7 +109,7 @@ geist_token_t geist_sampler_top_p_ws(struct geist_sampler_workspace *ws, const f
  * flight on the GPU at a time (they rotate over four scratch sets); callers
  * that need more overlap create more contexts. The launches of calls that
  * hand out tokens on the host (the argmax slot, the sampler.h surface, the
- * batcher over device logits) are not among the four: they have a set of
+ * batcher but for host logits of more than 32 rows) are not among the four: they have a set of
  * their own and follow one another on the context's stream, also where a call
  * has returned before its last thread blocks have. Such a call looks at the
  * words it waits for, for half a millisecond at most, and then leaves the wait

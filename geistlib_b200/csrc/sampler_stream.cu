@@ -1518,9 +1518,9 @@ struct ValueBins {
     }
 };
 /* The bin of `first` that the k-th of the candidates dealt out falls into holds too many: it is cut again between its smallest and its
- * largest key, until the bin that the k-th is in holds few, or equal ones. Fewer than k lie above it, what lies below is not ranked. Out of
- * line: rare. */
-__device__ __noinline__ void rank_crowded(const Pair *in, int total, int k, const ValueBins first, Pair *srt, int *start, Pair *out_s) {
+ * largest key, until the bin that the k-th is in holds few, or equal ones. Fewer than k lie above it, what lies below is not ranked. False:
+ * its entries are equal, what has been dealt out stays as it is. Out of line: rare. */
+__device__ __noinline__ bool rank_crowded(const Pair *in, int total, int k, const ValueBins first, Pair *srt, int *start, Pair *out_s) {
     const int tid  = (int) threadIdx.x;
     unsigned *ends = reinterpret_cast<unsigned *>(start + 2 * (kHistBins + 1)); /* smallest and largest key of the bin, and which it is */
     KeyBins   bins{0u, 0u, -1};
@@ -1547,6 +1547,9 @@ __device__ __noinline__ void rank_crowded(const Pair *in, int total, int k, cons
             atomicMax(&ends[1], hi);
         }
         __syncthreads();
+        if (bins.shift < 0 && ends[0] == ends[1]) {
+            return false;
+        }
         bins.lo              = ends[0];
         bins.hi              = ends[1];
         const unsigned range = bins.hi - bins.lo;
@@ -1554,6 +1557,7 @@ __device__ __noinline__ void rank_crowded(const Pair *in, int total, int k, cons
         bins.shift += (range >> bins.shift) > (unsigned) (kHistBins - 3) ? 1 : 0;
     } while (deal_out(in, total, k, srt, start, bins) && bins.shift > 0);
     rank_dealt(srt, total, k, start, out_s, bins);
+    return true;
 }
 /* More than kRankFew candidates in order, the k best to out_s; they lie between lo and hi. They are dealt out to 256 bins of
  * values, the highest in front (srt takes them), and ranked against their own bin: one against all costs a thread block
@@ -1568,9 +1572,7 @@ __device__ __noinline__ void rank_in_bins(const Pair *in, int total, int k, floa
         lo = hi - (float) (20 << 23); /* what is a millionth of the largest or less shares the last bin */
     }
     const ValueBins bins{lo, hi > lo && hi - lo < CUDART_INF_F ? (float) kHistBins / (hi - lo) : 0.0f, by_octave}; /* 0: one bin for all */
-    if (deal_out(in, total, k, srt, start, bins)) {
-        rank_crowded(in, total, k, bins, srt, start, out_s);
-    } else {
+    if (!deal_out(in, total, k, srt, start, bins) || !rank_crowded(in, total, k, bins, srt, start, out_s)) {
         rank_dealt(srt, total, k, start, out_s, bins);
     }
 }

@@ -145,8 +145,9 @@ bool make_plan(size_t V, size_t hist_max, Plan &pl) {
  *   greedy rows 8: with five 150 x 128256 17.2 -> 18.7, 350 x 65536 21.2 -> 19.7, no difference over all;
  *   temperature / top-p rows 4: against one 256 x 128256 top-p 43.8 -> 39.0, 256 x 262144 65.6 -> 61.9, 224 x 128256 42.7 ->
  *     37.7, 100 x 100000 30.0 -> 25.2; temperature rows, whose parts have no threshold, want two (150 x 65536 20.8 -> 21.6 with
- *     four, 1000 x 65536 79.0 -> 83.5), which a caller that says there is no top-p row gets;
- *   unknown rows 5. */
+ *     four, 1000 x 65536 79.0 -> 83.5). The hint covers both kinds: only the batcher, which knows its sessions, says that there is no
+ *     top-p row and gets two. At four 256 rows of 32 slices cost the same both ways, and the tie goes to whole rows;
+ *   unknown rows 5, which is also what geist_b200_grid answers for. */
 struct Deal {
     gb::RunMap map;
     int        grid;

@@ -79,8 +79,8 @@ struct __align__(16) SegRec {
 };
 
 /* Which (row, slice) items a thread block of the stream kernel takes: always one contiguous run of the row-major
- * item list. The host picks the cheaper of two ways to cut the list (a part of a row costs a thread block
- * about as much as five slices):
+ * item list. The host picks the cheaper of two ways to cut the list (what a part of a row costs a thread block, in
+ * slices: deal_items, where the list is dealt out):
  *   RUN_ITEMS  runs of equal length (q or q + 1 items, the first r blocks the longer ones); runs may begin and
  *              end inside a row;
  *   RUN_ROWS   whole rows (q or q + 1 rows per block), when there are at least as many rows as blocks or one

@@ -1302,7 +1302,7 @@ struct __align__(16) FinishShared {
     GroupShared gs; /* reductions of the whole thread block */
     int         poff[kMaxParts]; /* where a part's candidates begin among those that did not come in with the records */
     alignas(16) int bhist[kHistBins]; /* select histogram */
-    int         n_sel, n_border, n_ent, slot;
+    int         n_sel, n_ent, slot;
     unsigned    fin_bitmap[kFinBitmapWords];
     Pair        fsort[kFastKMax];
     alignas(8) float fq[kFastKMax];
@@ -2979,7 +2979,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
             /* ... and it has to while the part streams. The soft cap is monotone: a top-k row that brings no ids is
              * selected from its uncapped logits, and only what is read again is capped: a tanhf, a division and a
              * call per logit less. 48 rows of 262144 columns, half of them masked, top-k 64: 104.6 us a step with every
-             * logit capped and 93.8 with these (then; 78 by now). */
+             * logit capped and 93.8 with these, when they came in (48 since). */
             cap_late = !kPlain && (kKinds & K_SEL) != 0 && r.cap > 0.0f && r.cap < 1e38f && mode == M_TOPK && kq <= kFastKMax && !pen_on && p.out_logits == nullptr;
             pro_part = !kPlain && ((r.cap > 0.0f && !cap_late) || r.mrow != nullptr);
             if (tid == 0) { /* read again by the warps only if pro_on; the barriers of the part set-up lie between */
@@ -3802,8 +3802,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) sample_stream_kernel(con
  * A row that the candidates could not serve, all threads of its thread block: a wide nucleus becomes everybody's, any
  * other row takes the multi-pass path over a private copy. Out of line, and it asks for the row's parameters again; what the
  * functions behind it need of them lies in shared memory. Handed on by reference, the parameters and the group had lain in
- * the kernel's stack frame, and the out-of-line functions had spilled around them: a frame of 464 bytes, 112 now (spills of
- * the kernel's own code, mostly the select's); 1000 wide rows of 8192 212 -> 194 us, 24 of 100003 among 96 rows 80 -> 75.
+ * the kernel's stack frame, and the out-of-line functions had spilled around them: a frame of 464 bytes, 96 now and
+ * no spills; 1000 wide rows of 8192 212 -> 194 us, 24 of 100003 among 96 rows 80 -> 75.
  * Narrow launches did not change: for those the frame alone costs nothing that was measured.
  */
 __device__ __noinline__ void deferred_row(const SampleParams &p, FinishShared *sh, unsigned char *cmem, int row, int st) {

@@ -24,8 +24,8 @@
  *
  * Pass 1 is bound by the issue of its instructions at the finishing kernel's 16 warps per SM: 25 SM cycles per 32 values,
  * where its double arithmetic takes 6 and its conversions 8; a launch's first piece waits for the code as well, 4 us. 256
- * rows of 128256 columns, top-p 0.95 (98 of them wide): 428 us with a thread block and a dozen sweeps per row, 147 now;
- * 24 wide rows of 100003 among 96: 402 -> 69. Of the 98 rows' 77 us from the first row opened to the last token pass 1 takes 38,
+ * rows of 128256 columns, top-p 0.95 (98 of them wide): 428 us with a thread block and a dozen sweeps per row, 135 - 139
+ * now; 24 wide rows of 100003 among 96: 402 -> 69. Of the 98 rows' 77 us from the first row opened to the last token pass 1 takes 38,
  * what is added up and waited for between the passes 4, the windows 3, pass 2 12; 16 are the last row's end and uneven work.
  * Pieces of 512 for a warp: when they came in (the 24 rows took 93 us) pieces of
  * 1024 took 99, and pieces of 2048 for a thread block, a barrier each, 204 us on the 105.

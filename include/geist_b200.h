@@ -109,9 +109,9 @@ geist_token_t geist_sampler_top_p_ws(struct geist_sampler_workspace *ws, const f
  * flight on the GPU at a time (they rotate over four scratch sets); callers
  * that need more overlap create more contexts. The launches of calls that
  * hand out tokens on the host (the argmax slot, the sampler.h surface, the
- * batcher but for host logits of more than 32 rows) are not among the four: they have a set of
- * their own and follow one another on the context's stream, also where a call
- * has returned before its last thread blocks have. Such a call looks at the
+ * batcher but for host logits of more than 32 rows) are not among the four:
+ * they have a set of their own and follow one another on the context's
+ * stream, also where a call has returned before its last thread blocks have. Such a call looks at the
  * words it waits for, for half a millisecond at most, and then leaves the wait
  * to the CUDA runtime; it leaves it there from the start if the process had
  * chosen cudaDeviceScheduleBlockingSync or Yield when the context was made. */
@@ -410,8 +410,8 @@ enum geist_status geist_b200_batcher_propose_drafts(struct geist_b200_batcher *b
 enum geist_status geist_b200_plan(size_t n_vocab, size_t max_history, int32_t *slices_per_row, int32_t *slice,
                                   int32_t *smem_bytes, int32_t *ring_stages);
 
-/* How one launch over n_rows rows of this vocabulary is spread over the current device: the number of thread
- * blocks (each takes a contiguous run of (row, slice) items) and how many of them one SM holds at a time. */
+/* How one launch over n_rows rows of this vocabulary is spread over the current device, if it has no finish_hint (a hint can
+ * have the rows cut otherwise): the number of thread blocks (each takes a contiguous run of (row, slice) items) and how many of them one SM holds at a time. */
 enum geist_status geist_b200_grid(size_t n_vocab, size_t max_history, size_t n_rows, int32_t *thread_blocks,
                                   int32_t *blocks_per_sm);
 

@@ -109,13 +109,13 @@ geist_token_t geist_sampler_top_p_ws(struct geist_sampler_workspace *ws, const f
  * flight on the GPU at a time (they rotate over four scratch sets); callers
  * that need more overlap create more contexts. The launches of calls that
  * hand out tokens on the host (the argmax slot, the sampler.h surface, the
- * batcher but for host logits of more rows than the 32 or so, whole
- * sequences, that it copies at a time) are not among the four:
- * they have a set of their own and follow one another on the context's
- * stream, also where a call has returned before its last thread blocks have. Such a call looks at the
- * words it waits for, for half a millisecond at most, and then leaves the wait
- * to the CUDA runtime; it leaves it there from the start if the process had
- * chosen cudaDeviceScheduleBlockingSync or Yield when the context was made. */
+ * batcher unless it copies host logits in more than one chunk, of about 32
+ * rows) are not among the four: they have a set of their own and follow one
+ * another on the context's stream, also where a call has returned before its
+ * last thread blocks have. Such a call looks at the words it waits for, for
+ * half a millisecond at most, and then leaves the wait to the CUDA runtime; it
+ * leaves it there from the start if the process had chosen
+ * cudaDeviceScheduleBlockingSync or Yield when the context was made. */
 struct geist_b200_ctx;
 
 enum geist_status geist_b200_ctx_create(int device, struct geist_b200_ctx **out);

@@ -273,6 +273,56 @@ def test_calls_in_a_row_commit_before_the_next_reads(ctx):
     bt.close()
 
 
+@pytest.mark.parametrize("n,k", [(6, 1), (32, 1), (33, 1), (70, 1), (5, 7), (6, 7)])
+def test_host_logits_of_one_chunk_and_of_several(ctx, n, k):
+    """Steps and verify calls over host logits right behind each other and between calls over device logits, around the sizes at
+    which the copies go in chunks; the host buffer is overwritten as soon as a call returns."""
+    import torch
+    V, ring = 5003, 16
+    bt = api.Batcher(ctx, V, n, max_history=ring)
+    sess = [bt.open(temperature=0.9, top_k=20 if i % 2 else 0, top_p=0.8 if i % 3 == 0 else 1.0, seed=3 + i, rep=1.3) for i in range(n)]
+    K, P = np.array([20 if i % 2 else 0 for i in range(n)]), np.array([0.8 if i % 3 == 0 else 1.0 for i in range(n)], np.float32)
+    state = np.array([port.rng_seed(3 + i) for i in range(n)], np.uint64)
+    hist = [[] for _ in range(n)]
+    host = torch.empty(n * k, V).pin_memory()
+    for it in range(9):
+        h, hl = np.zeros((n, ring), np.int32), np.zeros(n, np.int32)
+        for i, ids in enumerate(hist):
+            hl[i] = len(ids[-ring:])
+            h[i, : hl[i]] = ids[-ring:]
+        x = normal_logits(n * k, V, 2.0, 300 + it)
+        x[:, :4] += 7.0
+        if it % 3 < 2:
+            host.copy_(torch.from_numpy(x))
+            arg = host
+        else:
+            arg = to_dev(x)
+        kw = dict(rep=1.3, freq=0.0, pres=0.0, hist=h, hist_len=hl)
+        if k == 1:
+            got = bt.step(sess, arg)
+            host.fill_(float("nan"))
+            o = port.sample_batch(x, 0.9, K, P, state, **kw)
+            assert np.array_equal(got, o["tokens"]), it
+            new = [[int(t)] for t in got]
+        else:
+            fed = np.random.default_rng(it).integers(0, 4, (n, k)).astype(np.int32)
+            acc, nout, toks = bt.verify(sess, fed, arg)
+            host.fill_(float("nan"))
+            o = port.sample_batch(x, 0.9, K, P, state, rows_per_seq=k, extra=fed, **kw)
+            out, new = o["tokens"].reshape(n, k), []
+            for i in range(n):
+                a = 0
+                while a + 1 < k and out[i, a] == fed[i, a + 1]:
+                    a += 1
+                assert (acc[i], nout[i]) == (a, a + 2) and toks[i, : a + 2].tolist() == fed[i, : a + 1].tolist() + [int(out[i, a])], it
+                new.append(toks[i, 1 : a + 2].tolist())
+        for i in range(n):
+            hist[i] += new[i]
+        state = o["rng_state"]
+    assert [bt.get_rng(s) for s in sess] == [int(v) for v in state]
+    bt.close()
+
+
 def test_a_generator_that_never_leaves_zero():
     """The word that a host row's generator comes to is 0, which is what the host waits to see changed: the call ends with the
     stream."""
